@@ -9,7 +9,7 @@
 // band that its neighbours just wrote from their shared memory (distributed
 // shared memory, two cluster barriers per phase).  Chains never wait on other
 // clusters, so the launch needs no co-residency beyond the cluster itself.
-// The per-site arithmetic is that of the single-walk kernels (word_phase for
+// The per-site arithmetic is that of the single-walk kernels (WordOp for
 // the int8 models, Model::site for the int32 ones), and the draws are the
 // fast mode's, so every chain equals its single-chain fast-mode walk.
 #include <cooperative_groups.h>
@@ -81,12 +81,9 @@ __global__ void __launch_bounds__(1024, 1) batch_word_kernel(const __grid_consta
     const int BLOCK = blockDim.x, tid = threadIdx.x;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     unsigned char* lat = smem_raw + 16;
-    uint32_t shift_tab[3] = {0u, 0u, 0u};
-    if (!M::DOM) {
-        shift_tab[0] = lozenge_shift_table(0);
-        shift_tab[1] = lozenge_shift_table(1);
-        shift_tab[2] = lozenge_shift_table(2);
-    }
+    __shared__ WordPhase s_phase[kWordPhases];
+    __shared__ uint4 s_sel[kLozengeSel];
+    if (tid < kLozengeSel) s_sel[tid] = lozenge_sel_entry(tid);
 
     for (int q = cid; q < b.nchains; q += ncl) {
         const BatchChain& ch = b.chains[b.order[q]];
@@ -111,6 +108,7 @@ __global__ void __launch_bounds__(1024, 1) batch_word_kernel(const __grid_consta
                 s[e] = (unsigned char)v;
             }
         }
+        if (tid < kWordPhases) s_phase[tid] = word_phase_entry<FAM>(tid, plane);
         for (int rr = tid; rr < nrows; rr += BLOCK) {
             const int i = a0 + rr;
             row_cls[rr] = (unsigned char)(M::DOM ? (i & 1) : i % 3);
@@ -125,10 +123,11 @@ __global__ void __launch_bounds__(1024, 1) batch_word_kernel(const __grid_consta
                 if (j >= M::COFF && j < M::COFF + cols) vb |= 1u << bb;
             }
             col_um[w] = lane_bytes(ub) * 0xffu;
-            col_vm[w] = lane_bytes(vb);
+            col_vm[w] = lane_bytes(vb) << 7;
         }
         __syncthreads();
 
+        const uint32_t nt0 = 0u - (M::DOM ? b.thr[0] : ch.thr[0]), nt1 = 0u - ch.thr[1], nt2 = 0u - ch.thr[2];
         const uint32_t key0 = (uint32_t)ch.key, key1 = (uint32_t)(ch.key >> 32);
         int64_t dstep = *b.step0 + b.step_add;
         const int nwords = nrows * Gw;
@@ -136,7 +135,7 @@ __global__ void __launch_bounds__(1024, 1) batch_word_kernel(const __grid_consta
         for (int64_t ph = 0; ph < b.nphases; ++ph) {
             const uint32_t d = __ldg(b.phases + ph);
             const bool draws = (d & PH_DRAWS) != 0u;
-            const WordPhase P = word_phase_of<FAM>(d, lat, plane, shift_tab);
+            const WordPhase P = s_phase[word_phase_index(d)];
             int rr = tid / Gw, w = tid - (tid / Gw) * Gw;
             for (int u = tid; u < nwords; u += BLOCK) {
                 WordInfo wi;
@@ -148,15 +147,17 @@ __global__ void __launch_bounds__(1024, 1) batch_word_kernel(const __grid_consta
                 if (draws) {
                     const uint4 w4 = philox4((uint32_t)((a0 + rr) * Gw + w), (uint32_t)dstep,
                                              (uint32_t)((uint64_t)dstep >> 32), ch.chain, key0, key1);
-                    const uint32_t k[4] = {w4.x >> 9, w4.y >> 9, w4.z >> 9, w4.w >> 9};
-                    if (M::DOM) {
-                        m0 = below4(k, b.thr[0]);
-                    } else {
-                        m0 = below4(k, ch.thr[0]);
-                        m1 = below4(k, ch.thr[1]) & ~below4(k, ch.thr[2]);
-                    }
+                    const uint32_t k[4] = {w4.x, w4.y, w4.z, w4.w};
+                    m0 = below4(k, nt0);
+                    if (!M::DOM) m1 = below4(k, nt1) & ~below4(k, nt2);
                 }
-                word_phase<FAM>(P, 0, W, wi, m0, m1);
+                WordOp<FAM> op;
+                WordNbr nb;
+                op.begin(lat, P, wi, s_sel);
+                op.load_up(nb, lat, P, wi, W);
+                op.load_dn(nb, lat, P, wi, W);
+                op.finish(P, wi, nb, m0, m1);
+                op.store(lat, P, wi);
                 rr += drr;
                 w += dw;
                 if (w >= Gw) {

@@ -20,17 +20,22 @@ namespace rtb {
 //   bits 0..7   op
 //   bits 8..15  a   (colour rotated in this phase, or the last one for FINAL)
 //   bits 16..23 b   (colour rotated in the previous phase; 0xff = none)
-//   bit  24     the phase draws one number from every position's stream
+//   bit  24     the phase draws numbers from every position's stream
+//   bits 25..31 steps of the phase - 1: a run of steps that flip the same
+//               colour is one phase that draws once per step (word kernel)
 // ---------------------------------------------------------------------------
 enum : uint32_t {
     OP_STEP = 1,   // deferred update from colour b (if b != a), then flip colour a
     OP_FINAL = 2,  // update every other colour from colour a (end of walk)
     PH_DRAWS = 1u << 24,
+    PH_STEP = 1u << 25,  // one more step in the phase
+    PH_MAX_STEPS = 128,
     NO_COLOUR = 0xffu
 };
 __host__ __device__ inline uint32_t ph_op(uint32_t d) { return d & 0xffu; }
 __host__ __device__ inline uint32_t ph_a(uint32_t d) { return (d >> 8) & 0xffu; }
 __host__ __device__ inline uint32_t ph_b(uint32_t d) { return (d >> 16) & 0xffu; }
+__host__ __device__ inline uint32_t ph_steps(uint32_t d) { return 1u + (d >> 25); }
 __host__ __device__ inline uint32_t make_phase(uint32_t op, uint32_t a, uint32_t b, bool draws) {
     return op | (a << 8) | (b << 16) | (draws ? PH_DRAWS : 0u);
 }
@@ -68,9 +73,12 @@ __device__ __forceinline__ uint32_t tiny_output(const TinyState& s, const TinyPa
 // (tinymt32.clh:81-93, :125-129).  All acceptance tests compare k against an
 // integer threshold computed on the host, which reproduces the reference's
 // float / double comparisons exactly.
-__device__ __forceinline__ uint32_t tiny_draw23(TinyState& s, const TinyParams& p) {
+__device__ __forceinline__ uint32_t tiny_draw32(TinyState& s, const TinyParams& p) {
     tiny_advance(s, p);
-    return tiny_output(s, p) >> 9;
+    return tiny_output(s, p);
+}
+__device__ __forceinline__ uint32_t tiny_draw23(TinyState& s, const TinyParams& p) {
+    return tiny_draw32(s, p) >> 9;
 }
 
 __device__ __forceinline__ void tiny_seed(TinyState& s, const TinyParams& p, uint32_t seed) {

@@ -42,11 +42,15 @@ struct WalkPlan {
     int xslots = 1;  // arrays exchanged per phase
     int depth = 1;   // bit-plane kernel: phases per halo exchange
     int pwords = 0;  // bit-plane kernel: words per row
+    bool cluster = false;     // the CTAs are one thread-block cluster (else a cooperative launch)
+    bool merge_runs = false;  // the kernel takes a run of same-colour steps as one phase
     const void* fn = nullptr;
 };
 
 rt_status plan_walk(int family, int device, int nlat, int rows, int cols, int width, bool uniform, bool philox,
                     WalkPlan* plan, std::string* err);
+// Launch configuration of a one-cluster plan; `attr` outlives *cfg.
+void walk_launch_config(const WalkPlan& plan, cudaLaunchConfig_t* cfg, cudaLaunchAttribute (&attr)[1]);
 rt_status launch_walk(const WalkPlan& plan, WalkArgs& args, cudaStream_t stream, std::string* err);
 // Word-parallel kernel of the int8 models (rt_word.cu): uniform TinyMT32J
 // parameters or fast mode.  ctas_hint <= 0: one CTA per SM.
@@ -75,6 +79,10 @@ rt_status launch_split(bool merge, int elem_bytes, int kind, int ncol, int n, in
 // step s of an epoch; fast_phases appends a whole walk of `steps` steps
 // (with the final Update of the colour models).
 int64_t fast_step_phases(int kind, int64_t s, uint32_t* ph, int64_t at, uint32_t* prev);
+// Appends a bit-exact colour step of a two- or three-colour model: a phase of
+// its own, or (merge) one more step of the run that `ph` ends with, if that
+// run began at or after index `first`, the epoch's first phase.
+int64_t colour_step_phase(uint32_t colour, bool merge, int64_t first, uint32_t* ph, int64_t at, uint32_t* prev);
 void fast_phases(int kind, int64_t steps, std::vector<uint32_t>& ph);
 // Integer threshold K with (k * 2^-23 < x) <=> (k < K) for k in [0, 2^23).
 uint32_t below_threshold(double x);

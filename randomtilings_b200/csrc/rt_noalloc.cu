@@ -183,8 +183,7 @@ extern "C" rt_status rt_walk_device_noalloc(const rt_config* cfg, int32_t* d_til
             // uniform_int_distribution<int>(0,2) otherwise, LozengeTiler.cpp:50-55),
             // staged through a small stack buffer.
             uint32_t chunk[2048];
-            int64_t done = 0;
-            int fill = 0;
+            int64_t done = 0, fill = 0;
             uint32_t prev = NO_COLOUR;
             uint64_t tseed;
             std::mt19937 mt(seed);
@@ -206,10 +205,11 @@ extern "C" rt_status rt_walk_device_noalloc(const rt_config* cfg, int32_t* d_til
             };
             for (int64_t st = 0; st < steps; ++st) {
                 const uint32_t r = kind == 0 ? (uint32_t)(mt() % 2) : (uint32_t)dist(lcg);
-                chunk[fill++] = make_phase(OP_STEP, r, prev, true);
-                prev = r;
+                // a run cut by a full buffer goes on as a phase with no Update pending
                 if (fill == 2048 && (e = flush()) != cudaSuccess) break;
+                fill = colour_step_phase(r, plan.merge_runs, 0, chunk, fill, &prev);
             }
+            if (e == cudaSuccess && fill == 2048) e = flush();
             if (e == cudaSuccess) {
                 chunk[fill++] = make_phase(OP_FINAL, prev, NO_COLOUR, false);
                 e = flush();
@@ -250,7 +250,7 @@ extern "C" rt_status rt_walk_device_noalloc(const rt_config* cfg, int32_t* d_til
             a.mat2 = 0xfc78ff1fu;
             a.tmat = 0x3793fdffu;
             a.phases = reinterpret_cast<const uint32_t*>(base + off_ph);
-            a.nphases = nph;
+            a.nphases = done;  // runs of steps share a phase: at most nph
             a.epoch_start = reinterpret_cast<const int64_t*>(base + off_ep);
             a.epoch_seed = reinterpret_cast<const uint64_t*>(base + off_ep + 8);
             a.nepochs = 1;

@@ -337,6 +337,18 @@ rt_status plan_walk(int family, int device, int nlat, int rows, int cols, int wi
     return RT_E_INVAL;
 }
 
+void walk_launch_config(const WalkPlan& plan, cudaLaunchConfig_t* cfg, cudaLaunchAttribute (&attr)[1]) {
+    cfg->gridDim = dim3((unsigned)plan.ctas);
+    cfg->blockDim = dim3((unsigned)plan.block);
+    cfg->dynamicSmemBytes = plan.smem;
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)plan.ctas;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg->attrs = attr;
+    cfg->numAttrs = 1;
+}
+
 rt_status launch_walk(const WalkPlan& plan, WalkArgs& args, cudaStream_t stream, std::string* err) {
     args.rows_per_cta = plan.rows_per_cta;
     args.wpad = plan.wpad;
@@ -345,9 +357,18 @@ rt_status launch_walk(const WalkPlan& plan, WalkArgs& args, cudaStream_t stream,
     args.depth = plan.depth;
     args.pwords = plan.pwords;
     void* kargs[] = {&args};
-    cudaError_t e = cudaLaunchCooperativeKernel(plan.fn, dim3(plan.ctas), dim3(plan.block), kargs, plan.smem, stream);
+    cudaError_t e;
+    if (plan.cluster) {
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute attr[1];
+        walk_launch_config(plan, &cfg, attr);
+        cfg.stream = stream;
+        e = cudaLaunchKernelExC(&cfg, plan.fn, kargs);
+    } else {
+        e = cudaLaunchCooperativeKernel(plan.fn, dim3(plan.ctas), dim3(plan.block), kargs, plan.smem, stream);
+    }
     if (e != cudaSuccess) {
-        *err = std::string("cooperative launch failed: ") + cudaGetErrorString(e);
+        *err = std::string("walk launch failed: ") + cudaGetErrorString(e);
         return RT_E_CUDA;
     }
     return RT_OK;

@@ -1,20 +1,28 @@
 // rt_word.cu -- the word-parallel walk kernel of the int8 models.
 //
-// Dominoes (dominokernel.cl, dominokernelCFTP.cl) and uniform lozenges
-// (lozengekernel.cl) store one byte per site.  This kernel treats a 32-bit
-// word of four consecutive sites of a colour-array row as its unit of work:
-// the Update of a colour is a handful of masks and byte shifts on words of
-// the flipped colour (neighbours at j +- 1 are funnel shifts of two adjacent
-// words), the flip test is a per-byte compare, and each thread keeps the
-// TinyMT states of the four positions of each of its words in registers for
-// the whole walk (bit-exact mode) or draws them from one Philox call per word
-// (fast mode).  Schedule, bands, tagged halo slots and bounded waits are
-// those of the generic walk kernel (rt_walk.cu) and it produces the same
-// bytes.  With one word per thread, the owners of the band's edge words poll
-// their halo words themselves and only their warps meet at the halo barrier,
-// so the interior words of the other warps overlap the exchange; a colour
-// step then costs the longer of one interior word and (halo wait + one edge
-// word) rather than their sum.
+// Dominoes (dominokernel.cl, dominokernelCFTP.cl) and lozenges
+// (lozengekernel.cl, qlozengekernel.cl) store one byte per site.  This kernel
+// treats a 32-bit word of four consecutive sites of a colour-array row as its
+// unit of work: the Update of a colour is a handful of masks and byte shifts
+// on words of the flipped colour (neighbours at j +- 1 are byte permutes of
+// two adjacent words), the flip test is a per-byte compare, and each thread
+// keeps the TinyMT states of the four positions of each of its words in
+// registers for the whole walk (bit-exact mode) or draws them from one Philox
+// call per word (fast mode).
+//
+// A phase is a run of steps that flip the same colour (the reference's random
+// colour order repeats a colour with probability 1/2 or 1/3).  Within a run
+// the sites' neighbours do not change, so its draws combine into two byte
+// masks per word before the lattice is touched, and the lattice is refreshed,
+// flipped and exchanged once per run instead of once per step.  The masks of
+// the next phase are made while its rows are on their way.
+//
+// What bounds it: the integer work of the draws (about 100 instructions a
+// word and step), the latency of one word's update, and the exchange.  On the
+// a = b = c = 500 hexagon (148 CTAs) a step takes 0.98 us, 1.83 with a phase
+// per step, a halo row copied through shared memory and a block-wide vote; on
+// the Aztec diamond of order 100 (one cluster of 16) 0.43 us, 1.35 before; of
+// order 24 (one CTA) 0.34 us, 1.33 before.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -27,48 +35,130 @@
 
 namespace rtb {
 
-constexpr int kWordBlockMax = 512;
+constexpr int kWordBlockMax = 512;  // threads that keep 2 or 4 words' generator states each
+constexpr int kWordBlockMid = 640;  // 65,536 registers / 96, in whole warps
 
-// bar.red.or on named barrier `id`, which `n` threads (whole warps) execute;
-// returns the OR of their `v`.
-__device__ __forceinline__ bool bar_red_or_n(int id, int n, bool v) {
+// ---------------------------------------------------------------------------
+// Exchange of the rows next to a band.  A row of the colour flipped in phase
+// p is published as tagged 64-bit words (32 bits of lattice, p + 1), double
+// buffered by the parity of p; its reader is the thread that owns the word
+// next to it, which polls the words it needs in phase p + 1 (never a copy of
+// the row in shared memory), so a wait costs its own warp and no barrier.  A
+// CTA publishes phase p + 2 only after it read its neighbour's phase p + 1,
+// which the neighbour published after reading phase p: a slot is rewritten
+// only after it was read.
+//   CLUSTER = false: slots in global memory (any number of co-resident CTAs).
+//   CLUSTER = true: the CTAs are one thread-block cluster and a row is written
+//   straight into its reader's shared memory.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ uint32_t cluster_addr(uint32_t saddr, int rank) {
     uint32_t r;
-    asm volatile(
-        "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.or.pred q, %2, %3, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
-        : "=r"(r)
-        : "r"((uint32_t)v), "r"(id), "r"(n)
-        : "memory");
-    return r != 0u;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
+    return r;
 }
 
-// Shared memory: 16 bytes of slack, then for each lattice NC colour planes of
-// (band rows + 2 halo rows) x wpad bytes, then 16 bytes of slack (the funnel
-// shifts read one word beyond a row; those bytes only reach sites outside
-// the update / flip masks).
+template <bool CLUSTER>
+struct WordExchange {
+    const WalkArgs& a;
+    unsigned long long* inbox;  // CLUSTER: [side][parity][lattice][word] in this CTA's shared memory
+    int cta;
+
+    __device__ __forceinline__ int at(int side, int par, int l, int w) const {
+        return ((side * 2 + par) * a.nlat + l) * a.xwords + w;
+    }
+    __device__ __forceinline__ unsigned long long poll(const unsigned long long* p) const {
+        if (!CLUSTER) return ld_relaxed64(p);
+        unsigned long long x;
+        asm volatile("ld.relaxed.cluster.shared::cta.u64 %0, [%1];"
+                     : "=l"(x)
+                     : "r"((uint32_t)__cvta_generic_to_shared(p))
+                     : "memory");
+        return x;
+    }
+    // Words w and w2 (both polled in one round trip; w2 = w: one word) of the
+    // row above (side 0) or below (side 1) the band, tagged `tag`.
+    __device__ __forceinline__ bool read(int side, int par, int l, int w, int w2, uint32_t tag,
+                                         uint32_t (&out)[2]) const {
+        const unsigned long long* row =
+            CLUSTER ? inbox + at(side, par, l, 0) : slot(a, side == 0 ? cta - 1 : cta + 1, 1 - side, par, l, 0);
+        unsigned spins = 0;
+        uint64_t t0 = 0;
+        for (;;) {
+            const unsigned long long x = poll(row + w), y = w2 == w ? x : poll(row + w2);
+            if ((uint32_t)(x >> 32) == tag && (uint32_t)(y >> 32) == tag) {
+                out[0] = (uint32_t)x;
+                out[1] = (uint32_t)y;
+                return true;
+            }
+            if ((++spins & (CLUSTER ? 1023u : 63u)) == 0u) {
+                if (*(volatile int*)a.err) return false;
+                const uint64_t now = global_ns();
+                if (t0 == 0) {
+                    t0 = now;
+                } else if (now - t0 > a.timeout_ns) {
+                    atomicOr(a.err, ERR_TIMEOUT);
+                    return false;
+                }
+            }
+        }
+    }
+    // Word w of the band's first (side 0) or last (side 1) row for the CTA above / below.
+    __device__ __forceinline__ void write(int side, int par, int l, int w, uint32_t tag, uint32_t v) const {
+        const unsigned long long x = (unsigned long long)tag << 32 | v;
+        if (CLUSTER) {
+            // the upper CTA receives it as its row below, the lower one as its row above
+            const uint32_t mine = (uint32_t)__cvta_generic_to_shared(inbox + at(1 - side, par, l, w));
+            const uint32_t theirs = cluster_addr(mine, side == 0 ? cta - 1 : cta + 1);
+            asm volatile("st.relaxed.cluster.shared::cluster.u64 [%0], %1;" ::"r"(theirs), "l"(x) : "memory");
+        } else {
+            st_relaxed64(slot(a, cta, side, par, l, 0) + w, x);
+        }
+    }
+};
+
+__device__ __forceinline__ void cluster_sync_all() {
+    asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+}
+
+// Shared memory: the inbox (CLUSTER), 16 bytes of slack, then for each lattice
+// NC colour planes of (band rows + 2) x wpad bytes, then 16 bytes of slack
+// (the funnel shifts read one word beyond a row; those bytes only reach sites
+// outside the update / flip masks).
+// MAXW: words per thread kept in registers (facts, draw masks and, in
+// bit-exact mode, generator states); 0: words walked at run time (fast mode
+// on large bands).
 // WT: 0 the uniform rules; 1 periodic weights (a.wper > 0), a per-site
 // threshold instead of thr[0]; 2 the lozenges' volume weight q
 // (qlozengekernel.cl), add below thr[2], remove in [2^22, thr[3]).  Separate
 // instantiations, so that the uniform kernel carries none of it.
-template <int FAM, int MAXW, bool PHILOX, int LB, int WT>
+// NL: lattices (2: coupled CFTP chains).
+template <int FAM, int MAXW, bool PHILOX, int LB, int WT, bool CLUSTER, int NL>
 __global__ void __launch_bounds__(LB, 1) word_kernel(const __grid_constant__ WalkArgs a) {
     using M = WordModel<FAM>;
     constexpr int NC = M::NC;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    unsigned char* lat = smem_raw + 16;
+    const int inbox_bytes = CLUSTER ? 4 * NL * a.xwords * 8 : 0;
+    unsigned char* lat = smem_raw + inbox_bytes + 16;
 
     const int BLOCK = blockDim.x;
     const int cta = blockIdx.x, nct = gridDim.x, tid = threadIdx.x;
     const int r0 = cta * a.rows_per_cta;
     const int r1 = min(a.rows, r0 + a.rows_per_cta);
     const int nrows = r1 - r0;
-    const int a0 = r0 + M::ROFF, a1 = r1 + M::ROFF;
+    const int a0 = r0 + M::ROFF;
     const int W = a.wpad;
     const int plane = (nrows + 2) * W;
     const int Gw = W >> 2;  // words per row (the fast mode's counter stride too)
     const int nwords = nrows * Gw;
     const int N = a.n;
+    const WordExchange<CLUSTER> xch{a, reinterpret_cast<unsigned long long*>(smem_raw), cta};
 
-    for (int l = 0; l < a.nlat; ++l)
+    if (CLUSTER) {
+        for (int e = tid; e < inbox_bytes / 8; e += BLOCK) xch.inbox[e] = 0ull;
+        __syncthreads();
+        cluster_sync_all();  // every inbox is clear before anyone writes into it
+    }
+    for (int l = 0; l < NL; ++l)
         for (int c = 0; c < NC; ++c) {
             const int8_t* g = static_cast<const int8_t*>(a.arr[l][c]);
             unsigned char* s = lat + (l * NC + c) * plane;
@@ -81,7 +171,6 @@ __global__ void __launch_bounds__(LB, 1) word_kernel(const __grid_constant__ Wal
         }
 
     const bool has_top = cta > 0, has_bot = cta + 1 < nct;
-    const bool bot_edge = has_bot && !(has_top && nrows == 1);
     // Update mask of band row rr / word w: rows 1..N-2, columns 1..width-2;
     // Rotate positions: columns COFF..COFF+cols-1 (all band rows).
     auto info_at = [&](int rr, int w) {
@@ -99,289 +188,257 @@ __global__ void __launch_bounds__(LB, 1) word_kernel(const __grid_constant__ Wal
         }
         if (!(i >= 1 && i <= N - 2)) ub = 0;
         wi.um = lane_bytes(ub) * 0xffu;
-        wi.vm = lane_bytes(vb);
+        wi.vm = lane_bytes(vb) << 7;
         return wi;
     };
-    auto is_edge = [&](int u) {
-        const int rr = u / Gw;
-        return (has_top && rr == 0) || (bot_edge && rr == nrows - 1);
-    };
-    // Lozenge column shifts for each colour t whose Update is applied.
-    uint32_t shift_tab[3] = {0u, 0u, 0u};
-    if (!M::DOM) {
-        shift_tab[0] = lozenge_shift_table(0);
-        shift_tab[1] = lozenge_shift_table(1);
-        shift_tab[2] = lozenge_shift_table(2);
-    }
-    // This thread's share of the halo exchange: words e = tid + x * BLOCK of
-    // [side][lattice][word] (one array per phase in these models).
-    const int per_side = a.nlat * a.xwords;
+    __shared__ WordPhase s_phase[kWordPhases];
+    __shared__ uint4 s_sel[kLozengeSel];
+    if (tid < kWordPhases) s_phase[tid] = word_phase_entry<FAM>(tid, plane);
+    if (tid < kLozengeSel) s_sel[tid] = lozenge_sel_entry(tid);
+    __shared__ int s_fail[2];
+    if (tid < 2) s_fail[tid] = 0;
+    const uint32_t nt0 = 0u - (WT == 2 ? a.thr[2] : a.thr[0]), nt1 = 0u - (WT == 2 ? a.thr[3] : a.thr[1]);
 
-    // The words u = tid + m * BLOCK (m < MAXW) of this thread, their facts
-    // and (bit-exact mode) their positions' TinyMT states, all in registers.
-    // MAXW = 0 (fast mode on large bands): words are walked at run time.
+    // The words u = tid + m * BLOCK (m < MAXW) of this thread.
     constexpr int NW = MAXW > 0 ? MAXW : 1;
     WordInfo winfo[NW];
+    int wcol[NW];  // word column
     TinyState st[PHILOX ? 1 : NW][4];
-    uint32_t wflags = 0;  // bit 2m: word m exists, bit 2m+1: it is an edge word
+    uint32_t wflags = 0;  // per word, 4 bits: it exists, it is in the band's first row / last row next to another CTA
     if (MAXW > 0) {
 #pragma unroll
         for (int m = 0; m < MAXW; ++m) {
             const int u = tid + m * BLOCK;
             if (u < nwords) {
-                winfo[m] = info_at(u / Gw, u % Gw);
-                wflags |= (1u << (2 * m)) | ((is_edge(u) ? 1u : 0u) << (2 * m + 1));
+                const int rr = u / Gw;
+                wcol[m] = u - rr * Gw;
+                winfo[m] = info_at(rr, wcol[m]);
+                wflags |= (1u | (has_top && rr == 0 ? 2u : 0u) | (has_bot && rr == nrows - 1 ? 4u : 0u)) << (4 * m);
             } else {
                 winfo[m] = WordInfo{0, 0, 0u, 0u};
+                wcol[m] = 0;
             }
         }
     }
     const TinyParams tp{a.mat1, a.mat2, a.tmat};
 
-    // One word per thread: the owner of word w of the band's first row polls
-    // word w of the row above, the owner of word w of its last row the row
-    // below, and only the warps that hold edge words meet at the halo
-    // barrier -- the other warps' words overlap the whole exchange.
-    bool poll_top = false, poll_bot = false, in_group = false;
-    int gthreads = 0;
-    if (MAXW == 1) {
-        const int rr = tid / Gw;
-        poll_top = tid < nwords && has_top && rr == 0;
-        poll_bot = tid < nwords && has_bot && rr == nrows - 1;
-        in_group = __any_sync(0xffffffffu, poll_top || poll_bot);
-        gthreads = 32 * __syncthreads_count((tid & 31) == 0 && in_group);
-    }
-    // The split only pays when some warps hold no edge word.
-    const bool split = MAXW == 1 && gthreads < BLOCK;
-
     int epoch = -1;
     int64_t next_epoch = a.nepochs > 0 ? a.epoch_start[0] : INT64_MAX;
     uint32_t key0 = 0, key1 = 0;
     int64_t dstep = 0;
-    uint32_t d = a.nphases > 0 ? __ldg(a.phases) : 0u;
-    uint32_t d_prev = 0u;
-
-    __syncthreads();
-    for (int64_t ph = 0; ph < a.nphases; ++ph) {
-        const uint32_t d_next = ph + 1 < a.nphases ? __ldg(a.phases + ph + 1) : 0u;
-        if (ph == next_epoch) {
-            while (epoch + 1 < a.nepochs && a.epoch_start[epoch + 1] == ph) ++epoch;
-            next_epoch = epoch + 1 < a.nepochs ? a.epoch_start[epoch + 1] : INT64_MAX;
-            const uint64_t eseed = a.epoch_seed[epoch];
-            if (PHILOX) {
-                key0 = (uint32_t)eseed;
-                key1 = (uint32_t)(eseed >> 32);
-                dstep = 0;
-            } else {
-#pragma unroll
-                for (int m = 0; m < NW; ++m) {
-                    if (!(wflags & (1u << (2 * m)))) continue;
-                    const int rpos = r0 + winfo[m].off / W - 1;  // position row
-                    const int jw = winfo[m].off % W;             // 4 * word
-#pragma unroll
-                    for (int b = 0; b < 4; ++b) {
-                        if (!(winfo[m].vm & (1u << (8 * b)))) continue;
-                        const uint32_t sid = (uint32_t)(jw + b - M::COFF) + (uint32_t)a.cols * (uint32_t)rpos;
-                        tiny_seed(st[m][b], tp, (uint32_t)eseed + sid);
-                    }
-                }
-            }
-        }
-        const bool draws = (d & PH_DRAWS) != 0u;
-        const WordPhase P = word_phase_of<FAM>(d, lat, plane, shift_tab);
-        const int lat1 = NC * plane;  // second lattice (coupled CFTP chains)
-        auto apply = [&](const WordInfo& wi, const uint32_t (&k)[4]) {
-            uint32_t m0 = 0, m1 = 0;
-            if (draws) {
-                if (WT == 1 && FAM == FAM_DOMINO_HB) {
-                    // weighted heat bath: a threshold per site from its vertex (i, j);
-                    // array column c of the rotated array A is vertex column 2 c + ((i + A) & 1)
-                    const int i = a0 + wi.off / W - 1, c0 = wi.off % W, par = (i + 1 - (int)ph_a(d)) & 1;
-#pragma unroll
-                    for (int b = 0; b < 4; ++b)
-                        m0 |= (uint32_t)(k[b] < weight_thr(a, i, 2 * (c0 + b) + par)) << (8 * b);
-                } else if (WT == 1 && FAM == FAM_LOZENGE8) {
-                    // weighted lozenges: the add threshold of each site's vertex; array
-                    // column c of colour C is vertex column 3 c + (C + i) mod 3
-                    const int i = a0 + wi.off / W - 1, c0 = wi.off % W, rem = ((int)ph_a(d) + i) % 3;
-#pragma unroll
-                    for (int b = 0; b < 4; ++b)
-                        m0 |= (uint32_t)(k[b] < weight_thr(a, i, 3 * (c0 + b) + rem)) << (8 * b);
-                } else if (WT == 2) {
-                    m0 = below4(k, a.thr[2]);
-                } else {
-                    m0 = below4(k, a.thr[0]);
-                }
-                if (WT == 2)
-                    m1 = below4(k, a.thr[3]) & ~below4(k, 1u << 22);
-                else if (!M::DOM)
-                    m1 = below4(k, a.thr[1]) & ~m0;
-            }
-            word_phase<FAM>(P, 0, W, wi, m0, m1);
-            if (a.nlat > 1) word_phase<FAM>(P, lat1, W, wi, m0, m1);
-        };
-        // Word m of this thread (u = tid + m * BLOCK of the band).
-        auto own_word = [&](int m) {
-            uint32_t k[4] = {0u, 0u, 0u, 0u};
-            if (draws) {
-                if (PHILOX) {
-                    const int u = tid + m * BLOCK;
-                    const uint4 w4 = philox4((uint32_t)(a0 * Gw + u), (uint32_t)dstep, (uint32_t)((uint64_t)dstep >> 32),
-                                             a.chain, key0, key1);
-                    k[0] = w4.x >> 9;
-                    k[1] = w4.y >> 9;
-                    k[2] = w4.z >> 9;
-                    k[3] = w4.w >> 9;
-                } else {
-                    // The four generators advance side by side; a site that is
-                    // not a Rotate position keeps its state (and draws nothing).
-#pragma unroll
-                    for (int b = 0; b < 4; ++b) {
-                        TinyState& sb = st[PHILOX ? 0 : m][b];
-                        TinyState nx = sb;
-                        tiny_advance(nx, tp);
-                        const uint32_t out = tiny_output(nx, tp) >> 9;
-                        const bool on = (winfo[m].vm >> (8 * b)) & 1u;
-                        k[b] = on ? out : 0u;
-                        sb.s0 = on ? nx.s0 : sb.s0;
-                        sb.s1 = on ? nx.s1 : sb.s1;
-                        sb.s2 = on ? nx.s2 : sb.s2;
-                        sb.s3 = on ? nx.s3 : sb.s3;
-                    }
-                }
-            }
-            apply(winfo[m], k);
-        };
-        auto philox_word = [&](int rr, int w) {
-            const WordInfo wi = info_at(rr, w);
-            uint32_t k[4] = {0u, 0u, 0u, 0u};
-            if (draws) {
-                const uint4 w4 = philox4((uint32_t)((a0 + rr) * Gw + w), (uint32_t)dstep,
-                                         (uint32_t)((uint64_t)dstep >> 32), a.chain, key0, key1);
-                k[0] = w4.x >> 9;
-                k[1] = w4.y >> 9;
-                k[2] = w4.z >> 9;
-                k[3] = w4.w >> 9;
-            }
-            apply(wi, k);
-        };
-        // Fast mode: words u = lo + tid + x * BLOCK < hi, walked with an
-        // incremental (row, word) pair.
-        auto philox_range = [&](int lo, int hi) {
-            int u = lo + tid;
-            if (u >= hi) return;
-            int rr = u / Gw, w = u - rr * Gw;
-            const int drr = BLOCK / Gw, dw = BLOCK - drr * Gw;
-            for (; u < hi; u += BLOCK) {
-                philox_word(rr, w);
-                rr += drr;
-                w += dw;
-                if (w >= Gw) {
-                    w -= Gw;
-                    ++rr;
-                }
-            }
-        };
-
-        if (MAXW == 1 && split) {
-            bool fail = false;
-            if (!in_group) {
-                if (wflags & 1u) own_word(0);
-            } else {
-                if (ph > 0 && gthreads > 0) {
-                    // Halo words of the array the neighbours flipped in the previous phase.
-                    const uint32_t mask = M::written(d_prev);
-                    bool ok = true;
-                    if (mask && (poll_top || poll_bot)) {
-                        const int arr = __ffs(mask) - 1;
-                        const int par = (int)((ph - 1) & 1);
-                        const uint32_t tag = (uint32_t)ph;
-                        const int w = tid % Gw;
-                        for (int l = 0; l < a.nlat && ok; ++l) {
-                            uint32_t v;
-                            if (poll_top) {
-                                ok = wait_word(a, slot(a, cta - 1, 1, par, l, 0) + w, tag, &v);
-                                if (ok) sts(lat + (l * NC + arr) * plane + 4 * w, v);
-                            }
-                            if (poll_bot && ok) {
-                                ok = wait_word(a, slot(a, cta + 1, 0, par, l, 0) + w, tag, &v);
-                                if (ok) sts(lat + (l * NC + arr) * plane + (nrows + 1) * W + 4 * w, v);
-                            }
-                        }
-                    }
-                    fail = bar_red_or_n(1, gthreads, !ok);
-                }
-                if (!fail && wflags) own_word(0);  // the edge word, or a word of the row next to it
-            }
-            if (__syncthreads_or(fail)) return;
+    // Draws restart at phase `ph` when an epoch begins there.
+    auto begin_phase = [&](int64_t ph) {
+        if (ph != next_epoch) return;
+        while (epoch + 1 < a.nepochs && a.epoch_start[epoch + 1] == ph) ++epoch;
+        next_epoch = epoch + 1 < a.nepochs ? a.epoch_start[epoch + 1] : INT64_MAX;
+        const uint64_t eseed = a.epoch_seed[epoch];
+        if (PHILOX) {
+            key0 = (uint32_t)eseed;
+            key1 = (uint32_t)(eseed >> 32);
+            dstep = 0;
         } else {
-            // Words away from the band's edge rows first, overlapping the neighbours' progress.
-            if (MAXW == 0) {
-                const int lo = has_top ? Gw : 0;
-                philox_range(lo, max(lo, nwords - (has_bot ? Gw : 0)));
-            } else {
+            // A site that is not a Rotate position has no stream; what its
+            // generator holds is never used.
 #pragma unroll
-                for (int m = 0; m < NW; ++m)
-                    if ((wflags >> (2 * m) & 3u) == 1u) own_word(m);
+            for (int m = 0; m < NW; ++m) {
+                if (!(wflags >> (4 * m) & 1u)) continue;
+                const int rpos = r0 + winfo[m].off / W - 1;  // position row
+                const int jw = winfo[m].off % W;             // 4 * word
+#pragma unroll
+                for (int b = 0; b < 4; ++b) {
+                    const uint32_t sid = (uint32_t)(jw + b - M::COFF) + (uint32_t)a.cols * (uint32_t)rpos;
+                    tiny_seed(st[PHILOX ? 0 : m][b], tp, (uint32_t)eseed + sid);
+                }
             }
-            if (ph > 0) {
-                // Halo rows of the array the neighbours flipped in the previous phase.
-                const uint32_t mask = M::written(d_prev);
-                bool ok = true;
-                if (mask) {
-                    const int arr = __ffs(mask) - 1;
-                    const int par = (int)((ph - 1) & 1);
-                    const uint32_t tag = (uint32_t)ph;
-                    for (int e = tid; e < 2 * per_side && ok; e += BLOCK) {
-                        const int side = e >= per_side;  // 0: row above (from cta-1), 1: row below (from cta+1)
-                        const int rem = e - side * per_side;
-                        const int l = rem >= a.xwords;
-                        const int w = rem - l * a.xwords;
-                        const int src = side == 0 ? cta - 1 : cta + 1;
-                        if (src < 0 || src >= nct) continue;
-                        uint32_t v;
-                        ok = wait_word(a, slot(a, src, 1 - side, par, l, 0) + w, tag, &v);
-                        if (ok) sts(lat + (l * NC + arr) * plane + (side == 0 ? 0 : nrows + 1) * W + 4 * w, v);
+        }
+    };
+    // What the draws of one step do, as byte masks (word_phase): combined into
+    // m0 / m1, which hold what the run's earlier steps did.  Within a run the
+    // sites' neighbours do not change, so a rotatable site stays rotatable:
+    // toggles add up modulo 2, and of the other rules' draws the last one that
+    // acts on a site decides.
+    auto combine = [&](uint32_t d, const WordInfo& wi, const uint32_t (&k)[4], uint32_t& m0, uint32_t& m1) {
+        uint32_t lo;
+        if (WT == 1) {
+            // Periodic weights: a threshold per site from its vertex (i, j); array
+            // column c of the rotated array A is vertex column 2 c + ((i + A) & 1)
+            // (dominoes) or 3 c + (A + i) mod 3 (lozenges).
+            const int i = a0 + wi.off / W - 1, c0 = wi.off % W;
+            const int step = M::DOM ? 2 : 3;
+            const int j0 = step * c0 + (M::DOM ? (i + 1 - (int)ph_a(d)) & 1 : ((int)ph_a(d) + i) % 3);
+            lo = below4(k, 0u - weight_thr(a, i, j0), 0u - weight_thr(a, i, j0 + step),
+                        0u - weight_thr(a, i, j0 + 2 * step), 0u - weight_thr(a, i, j0 + 3 * step));
+        } else {
+            lo = below4(k, nt0);
+        }
+        if (FAM == FAM_DOMINO) {
+            m0 ^= lo;
+        } else if (FAM == FAM_DOMINO_HB) {
+            m0 = lo;
+        } else {
+            const uint32_t rem = below4(k, nt1) & (WT == 2 ? ~below4(k, 0u - (1u << 22)) : ~lo);
+            m0 = lo | (m0 & ~rem);
+            m1 = rem | (m1 & ~lo);
+        }
+    };
+    auto philox_draws = [&](uint32_t d, int u, const WordInfo& wi, int64_t s, uint32_t& m0, uint32_t& m1) {
+        m0 = m1 = 0u;
+        if (!(d & PH_DRAWS)) return;
+        for (uint32_t c = 0; c < ph_steps(d); ++c, ++s) {
+            const uint4 w4 =
+                philox4((uint32_t)(a0 * Gw + u), (uint32_t)s, (uint32_t)((uint64_t)s >> 32), a.chain, key0, key1);
+            const uint32_t k[4] = {w4.x, w4.y, w4.z, w4.w};
+            combine(d, wi, k, m0, m1);
+        }
+    };
+    // The masks of this thread's words for phase descriptor d.  They depend on
+    // the draws alone, so they are made a phase ahead, while the rows the
+    // phase needs are on their way.
+    uint32_t mk0[NW], mk1[NW];
+    auto draw_masks = [&](uint32_t d) {
+#pragma unroll
+        for (int m = 0; m < NW; ++m) {
+            mk0[m] = mk1[m] = 0u;
+            if (!(wflags >> (4 * m) & 1u) || !(d & PH_DRAWS)) continue;
+            if (PHILOX) {
+                philox_draws(d, (winfo[m].off >> 2) - Gw, winfo[m], dstep, mk0[m], mk1[m]);
+            } else {
+#pragma unroll 1
+                for (uint32_t c = 0; c < ph_steps(d); ++c) {
+                    uint32_t k[4];
+#pragma unroll
+                    for (int b = 0; b < 4; ++b) k[b] = tiny_draw32(st[PHILOX ? 0 : m][b], tp);
+                    combine(d, winfo[m], k, mk0[m], mk1[m]);
+                }
+            }
+        }
+        if (PHILOX && (d & PH_DRAWS)) dstep += ph_steps(d);
+    };
+
+    // Phases that need more than the plain loop body: those that begin an
+    // epoch (a phase earlier where the draws are made ahead), the tests'
+    // withheld one and the last two.  Returns how many phases after `ph` the
+    // next one comes.
+    auto until_special = [&](int64_t ph) {
+        int64_t s = a.nphases - 2;
+        const int64_t e = MAXW > 0 ? next_epoch - 1 : next_epoch;
+        if (e >= ph) s = min(s, e);
+        if (cta == 0 && a.drop_phase >= ph) s = min(s, a.drop_phase);
+        return (int)min(max(s - ph, (int64_t)0), (int64_t)1 << 30);
+    };
+    uint32_t d = a.nphases > 0 ? __ldg(a.phases) : 0u;
+    uint32_t d_next = a.nphases > 1 ? __ldg(a.phases + 1) : 0u;
+    if (MAXW > 0 && a.nphases > 0) {
+        begin_phase(0);
+        draw_masks(d);
+    }
+    const uint32_t* ahead = a.phases + 2;  // the descriptor two phases on
+    const int lat1 = NC * plane;           // second lattice (coupled CFTP chains)
+    uint32_t p32 = 0;                      // phase number modulo 2^32
+    int until = until_special(0);
+    bool fail = false, more = a.nphases > 0;
+    __syncthreads();
+    WordPhase P = s_phase[word_phase_index(d)];
+    while (more) {
+        const int par = (int)(p32 & 1u);
+        const bool failed = *(volatile int*)&s_fail[1 - par] != 0;
+        const bool first = ahead == a.phases + 2;
+        // Rows are exchanged after every phase but the last, whether or not the
+        // next one has an Update pending: the waits keep the slots' order.
+        bool pub = true;
+        uint32_t d_after = 0u;
+        if (until-- > 0) {
+            d_after = __ldg(ahead);
+        } else {
+            const int64_t ph = ahead - a.phases - 2;
+            if (ph + 2 < a.nphases) d_after = __ldg(ahead);
+            more = ph + 1 < a.nphases;
+            pub = more && !(cta == 0 && ph == a.drop_phase);
+            if (MAXW == 0)
+                begin_phase(ph);
+            else if (more)
+                begin_phase(ph + 1);
+            until = until_special(ph + 1);
+        }
+        ++ahead;
+        // One word: flags bit 1 (2) -- it needs the row above (below) the band
+        // from the neighbour and publishes itself to it.
+        auto do_word = [&](const WordInfo& wi, int w, uint32_t flags, uint32_t m0, uint32_t m1) {
+#pragma unroll
+            for (int l = 0; l < NL; ++l) {
+                unsigned char* const L = lat + l * lat1;
+                WordOp<FAM> op;
+                WordNbr nb;
+                op.load_up(nb, L, P, wi, W);
+                op.load_dn(nb, L, P, wi, W);
+                if (flags && !first) {
+                    bool ok = true;
+                    if (flags & 2u) ok = xch.read(0, 1 - par, l, w, M::DOM ? w : min(w + 1, Gw - 1), p32, nb.up);
+                    if (ok && (flags & 4u)) ok = xch.read(1, 1 - par, l, w, M::DOM ? w : max(w - 1, 0), p32, nb.dn);
+                    if (!ok) {
+                        fail = true;
+                        return;
                     }
                 }
-                if (__syncthreads_or(!ok)) return;
-            }
-            if (MAXW == 0) {
-                if (has_top) philox_range(0, Gw);
-                if (bot_edge) philox_range(nwords - Gw, nwords);
-            } else {
-#pragma unroll
-                for (int m = 0; m < NW; ++m)
-                    if ((wflags >> (2 * m) & 3u) == 3u) own_word(m);
-            }
-            __syncthreads();
-        }
-        if (ph + 1 < a.nphases && !(cta == 0 && ph == a.drop_phase)) {
-            // Publish the band's first / last row of the array flipped in this phase.
-            const uint32_t mask = M::written(d);
-            if (mask) {
-                const int arr = __ffs(mask) - 1;
-                const int par = (int)(ph & 1);
-                const unsigned long long tag = (unsigned long long)(uint32_t)(ph + 1) << 32;
-                for (int e = tid; e < 2 * per_side; e += BLOCK) {
-                    const int side = e >= per_side;  // 0: first row (read by cta-1), 1: last row (read by cta+1)
-                    const int rem = e - side * per_side;
-                    const int l = rem >= a.xwords;
-                    const int w = rem - l * a.xwords;
-                    const int dst = side == 0 ? cta - 1 : cta + 1;
-                    if (dst < 0 || dst >= nct) continue;
-                    const unsigned char* row = lat + (l * NC + arr) * plane + (side == 0 ? 1 : nrows) * W;
-                    st_relaxed64(slot(a, cta, side, par, l, 0) + w, tag | lds(row + 4 * w));
+                op.begin(L, P, wi, s_sel);
+                op.finish(P, wi, nb, m0, m1);
+                if (pub) {
+                    if (flags & 2u) xch.write(0, par, l, w, p32 + 1u, op.v);
+                    if (flags & 4u) xch.write(1, par, l, w, p32 + 1u, op.v);
                 }
+                op.store(L, P, wi);
             }
+        };
+        if (MAXW > 0) {
+            // words away from the neighbours first
+#pragma unroll
+            for (int m = 0; m < NW; ++m)
+                if ((wflags >> (4 * m) & 7u) == 1u) do_word(winfo[m], 0, 0u, mk0[m], mk1[m]);
+#pragma unroll
+            for (int m = 0; m < NW; ++m)
+                if (wflags >> (4 * m) & 6u) do_word(winfo[m], wcol[m], wflags >> (4 * m) & 6u, mk0[m], mk1[m]);
+            draw_masks(d_next);  // none after the last phase
+        } else {
+            // Words walked with an incremental (row, word) pair; the edge rows last.
+            auto range = [&](int u_lo, int u_hi, uint32_t flags) {
+                int u = u_lo + tid;
+                if (u >= u_hi) return;
+                int rr = u / Gw, w = u - rr * Gw;
+                const int drr = BLOCK / Gw, dw = BLOCK - drr * Gw;
+                for (; u < u_hi; u += BLOCK) {
+                    const WordInfo wi = info_at(rr, w);
+                    uint32_t m0, m1;
+                    philox_draws(d, u, wi, dstep, m0, m1);
+                    do_word(wi, w, flags, m0, m1);
+                    rr += drr;
+                    w += dw;
+                    if (w >= Gw) {
+                        w -= Gw;
+                        ++rr;
+                    }
+                }
+            };
+            const bool one = has_top && has_bot && nrows == 1;
+            range(has_top ? Gw : 0, nwords - (has_bot ? Gw : 0), 0u);
+            if (has_top) range(0, Gw, one ? 6u : 2u);
+            if (has_bot && !one) range(nwords - Gw, nwords, 4u);
+            if (d & PH_DRAWS) dstep += ph_steps(d);
         }
-        if (PHILOX && draws) ++dstep;
-        d_prev = d;
         d = d_next;
+        d_next = d_after;
+        P = s_phase[word_phase_index(d)];
+        // A wait that ran out is seen by every thread one phase later: the flag
+        // of this phase is read after its barrier and acted on before the next
+        // one, and not written again until then.
+        if (fail) s_fail[par] = 1;
+        if (failed) break;
+        __syncthreads();
+        ++p32;
     }
-
     __syncthreads();
-    for (int l = 0; l < a.nlat; ++l)
+    if (CLUSTER) cluster_sync_all();  // no CTA leaves while another may write into its inbox
+    if (s_fail[0] | s_fail[1]) return;
+    for (int l = 0; l < NL; ++l)
         for (int c = 0; c < NC; ++c) {
             int8_t* g = static_cast<int8_t*>(a.arr[l][c]);
             const unsigned char* s = lat + (l * NC + c) * plane;
@@ -394,45 +451,59 @@ __global__ void __launch_bounds__(LB, 1) word_kernel(const __grid_constant__ Wal
 
 using KernelFn = void (*)(WalkArgs);
 
-template <int FAM, int WT>
-static KernelFn word_fn(int maxw, bool philox) {
+// One word per thread, up to `block` threads: blocks of at most kWordBlockMid
+// threads have 96 registers a thread instead of 64.
+template <int FAM, bool PHILOX, int WT, bool CLUSTER, int NL>
+static KernelFn word_fn1(int block) {
+    return block <= kWordBlockMid ? word_kernel<FAM, 1, PHILOX, kWordBlockMid, WT, CLUSTER, NL>
+                                  : word_kernel<FAM, 1, PHILOX, 1024, WT, CLUSTER, NL>;
+}
+template <int FAM, int WT, int NL>
+static KernelFn word_fn(int maxw, int block, bool philox, bool cluster) {
+    if (maxw == 1) {
+        if (cluster) return philox ? word_fn1<FAM, true, WT, true, NL>(block) : word_fn1<FAM, false, WT, true, NL>(block);
+        return philox ? word_fn1<FAM, true, WT, false, NL>(block) : word_fn1<FAM, false, WT, false, NL>(block);
+    }
+    if (cluster) return nullptr;  // clusters are planned for one word per thread
     if (philox) {
         switch (maxw) {
-            case 0: return word_kernel<FAM, 0, true, 1024, WT>;
-            case 1: return word_kernel<FAM, 1, true, 1024, WT>;
-            case 2: return word_kernel<FAM, 2, true, 1024, WT>;
-            case 4: return word_kernel<FAM, 4, true, 1024, WT>;
+            case 0: return word_kernel<FAM, 0, true, 1024, WT, false, NL>;
+            case 2: return word_kernel<FAM, 2, true, 1024, WT, false, NL>;
+            case 4: return word_kernel<FAM, 4, true, 1024, WT, false, NL>;
             default: return nullptr;
         }
     }
     switch (maxw) {
-        case 1: return word_kernel<FAM, 1, false, 1024, WT>;
-        case 2: return word_kernel<FAM, 2, false, 512, WT>;
-        case 4: return word_kernel<FAM, 4, false, 512, WT>;
+        case 2: return word_kernel<FAM, 2, false, 512, WT, false, NL>;
+        case 4: return word_kernel<FAM, 4, false, 512, WT, false, NL>;
         default: return nullptr;
     }
 }
 
-static KernelFn word_kernel_for(int family, int maxw, bool philox, bool weighted) {
+template <int NL>
+static KernelFn word_kernel_for(int family, int maxw, int block, bool philox, bool weighted, bool cluster) {
     switch (family) {
-        case FAM_DOMINO: return word_fn<FAM_DOMINO, 0>(maxw, philox);
+        case FAM_DOMINO:  // not monotone: no coupled chains
+            return NL == 1 ? word_fn<FAM_DOMINO, 0, 1>(maxw, block, philox, cluster) : nullptr;
         case FAM_DOMINO_HB:
-            return weighted ? word_fn<FAM_DOMINO_HB, 1>(maxw, philox) : word_fn<FAM_DOMINO_HB, 0>(maxw, philox);
+            return weighted ? word_fn<FAM_DOMINO_HB, 1, NL>(maxw, block, philox, cluster)
+                            : word_fn<FAM_DOMINO_HB, 0, NL>(maxw, block, philox, cluster);
         case FAM_LOZENGE8:
-            return weighted ? word_fn<FAM_LOZENGE8, 1>(maxw, philox) : word_fn<FAM_LOZENGE8, 0>(maxw, philox);
-        case FAM_QLOZENGE8: return weighted ? nullptr : word_fn<FAM_LOZENGE8, 2>(maxw, philox);
+            return weighted ? word_fn<FAM_LOZENGE8, 1, NL>(maxw, block, philox, cluster)
+                            : word_fn<FAM_LOZENGE8, 0, NL>(maxw, block, philox, cluster);
+        case FAM_QLOZENGE8: return weighted ? nullptr : word_fn<FAM_LOZENGE8, 2, NL>(maxw, block, philox, cluster);
         default: return nullptr;
     }
 }
 
 bool word_family(int family) { return family == FAM_DOMINO || family == FAM_DOMINO_HB || family == FAM_LOZENGE8; }
 
-rt_status plan_word_walk(int family, int device, int nlat, int rows, int width, bool philox, int ctas_hint,
-                         WalkPlan* plan, std::string* err, bool weighted) {
-    if (!word_family(family) && family != FAM_QLOZENGE8) {
-        *err = "no word kernel for this model";
-        return RT_E_INVAL;
-    }
+constexpr int kClusterMax = 16;  // CTAs of the largest thread-block cluster (non-portable size)
+
+// Plans the walk on (at most) `ctas` CTAs: one cluster, or any number of
+// co-resident CTAs.
+static rt_status plan_word_grid(int family, int device, int nlat, int rows, int width, bool philox, int ctas,
+                                bool cluster, bool weighted, WalkPlan* plan, std::string* err) {
     int sms = 0, smem_optin = 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
         cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) != cudaSuccess) {
@@ -442,9 +513,9 @@ rt_status plan_word_walk(int family, int device, int nlat, int rows, int width, 
     const int nc = family == FAM_LOZENGE8 || family == FAM_QLOZENGE8 ? 3 : 2;
     const int wpad = (width + 3) & ~3;
     const int gw = wpad / 4;
-    int ctas = std::max(1, std::min(ctas_hint > 0 ? ctas_hint : sms, rows));
     const int rpc = (rows + ctas - 1) / ctas;
     ctas = (rows + rpc - 1) / rpc;
+    cluster = cluster && ctas > 1 && ctas <= kClusterMax;
     const int words = rpc * gw;
     // One word per thread up to 1024 threads; bit-exact mode then keeps 2
     // or 4 words' generator states per thread in registers (512 threads).
@@ -465,20 +536,47 @@ rt_status plan_word_walk(int family, int device, int nlat, int rows, int width, 
         }
         block = ((words + maxw - 1) / maxw + 31) / 32 * 32;
     }
-    const size_t smem = 32 + (size_t)nlat * nc * (rpc + 2) * wpad;
+    const size_t smem =
+        32 + (size_t)nlat * nc * (rpc + 2) * wpad + (cluster ? (size_t)4 * nlat * gw * 8 : (size_t)0);
     if (smem > (size_t)smem_optin) {
         *err = "band does not fit in shared memory";
         return RT_E_INVAL;
     }
-    KernelFn fn = word_kernel_for(family, maxw, philox, weighted);
+    KernelFn fn = nlat == 1 ? word_kernel_for<1>(family, maxw, block, philox, weighted, cluster)
+                            : word_kernel_for<2>(family, maxw, block, philox, weighted, cluster);
     if (!fn) {
         *err = "no word kernel for this configuration";
         return RT_E_INVAL;
     }
     if (cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-        cudaSuccess) {
+            cudaSuccess ||
+        (cluster && cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
+                        cudaSuccess)) {
         *err = "cudaFuncSetAttribute failed";
         return RT_E_CUDA;
+    }
+    plan->items = maxw;
+    plan->block = block;
+    plan->rows_per_cta = rpc;
+    plan->ctas = ctas;
+    plan->smem = smem;
+    plan->wpad = wpad;
+    plan->xwords = gw;
+    plan->xslots = 1;
+    plan->cluster = cluster;
+    plan->merge_runs = true;
+    plan->fn = (const void*)fn;
+    if (cluster) {
+        int active = 0;
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute attr[1];
+        walk_launch_config(*plan, &cfg, attr);
+        if (cudaOccupancyMaxActiveClusters(&active, (const void*)fn, &cfg) != cudaSuccess || active < 1) {
+            cudaGetLastError();
+            *err = "word-kernel cluster cannot be resident";
+            return RT_E_INVAL;
+        }
+        return RT_OK;
     }
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)fn, block, smem) != cudaSuccess) {
@@ -489,16 +587,45 @@ rt_status plan_word_walk(int family, int device, int nlat, int rows, int width, 
         *err = "word-kernel grid cannot be co-resident";
         return RT_E_INVAL;
     }
-    plan->items = maxw;
-    plan->block = block;
-    plan->rows_per_cta = rpc;
-    plan->ctas = ctas;
-    plan->smem = smem;
-    plan->wpad = wpad;
-    plan->xwords = wpad / 4;
-    plan->xslots = 1;
-    plan->fn = (const void*)fn;
     return RT_OK;
+}
+
+rt_status plan_word_walk(int family, int device, int nlat, int rows, int width, bool philox, int ctas_hint,
+                         WalkPlan* plan, std::string* err, bool weighted) {
+    if (!word_family(family) && family != FAM_QLOZENGE8) {
+        *err = "no word kernel for this model";
+        return RT_E_INVAL;
+    }
+    int sms = 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) {
+        *err = "cudaDeviceGetAttribute failed";
+        return RT_E_CUDA;
+    }
+    // Microseconds per step (Aztec diamonds TinyMT / hexagons TinyMT / hexagons
+    // Philox; words = 32-bit words of one colour array):
+    //   CTAs     378-432 words     945-1326          9,156            13,366-13,872
+    //   1        0.34 0.58 0.75    1.09 1.07 1.40    -                -
+    //   16       0.47 0.76 1.02    0.35 0.53 0.72    -    0.82 1.14   0.79 1.08 1.62
+    //   74       0.63 1.12 1.63    0.75 1.33 1.96    -    0.89 1.37   0.55 0.90 1.34
+    //   148      0.63 1.12 1.62    0.67 1.17 1.75    -    0.88 1.32   0.51 0.86 1.26
+    // So: one CTA (no exchange) while three warps a scheduler hold the lattice;
+    // one cluster of 16 (rows exchanged through distributed shared memory)
+    // while that leaves each CTA about 600 words; else the whole GPU, with
+    // bands of three rows or more, whose first and last rows are different
+    // warps' (258 rows: 0.71 at two rows a band, 0.54 at four).
+    const int64_t words = (int64_t)rows * ((width + 3) / 4);
+    int ctas = ctas_hint;
+    bool cluster = ctas_hint > 0 && ctas_hint <= kClusterMax;
+    if (ctas_hint <= 0) {
+        cluster = words <= (int64_t)kClusterMax * 600;
+        ctas = words <= 384 ? 1 : cluster ? kClusterMax : std::min(sms, rows / 3);
+    }
+    ctas = std::max(1, std::min(ctas, rows));
+    if (cluster &&
+        plan_word_grid(family, device, nlat, rows, width, philox, ctas, true, weighted, plan, err) == RT_OK)
+        return RT_OK;
+    if (ctas_hint <= 0) ctas = std::max(1, std::min(sms, rows / 3));
+    return plan_word_grid(family, device, nlat, rows, width, philox, ctas, false, weighted, plan, err);
 }
 
 }  // namespace rtb

@@ -9,64 +9,27 @@
 
 namespace rtb {
 
-// 0x01 in every byte of v equal to the same byte of pat (bytes < 0x80).
-__device__ __forceinline__ uint32_t eq_bytes(uint32_t v, uint32_t pat) {
-    const uint32_t x = v ^ pat;
-    return (~(x + 0x7f7f7f7fu) >> 7) & 0x01010101u;
+// 0xff in byte b iff (w[b] >> 9) < thr_b: the top byte of the difference of
+// two numbers up to 2^23 is its sign.  n_b = -thr_b.
+__device__ __forceinline__ uint32_t below4(const uint32_t (&w)[4], uint32_t n0, uint32_t n1, uint32_t n2, uint32_t n3) {
+    const uint32_t lo = __byte_perm((w[0] >> 9) + n0, (w[1] >> 9) + n1, 0x0073);
+    const uint32_t hi = __byte_perm((w[2] >> 9) + n2, (w[3] >> 9) + n3, 0x7300);
+    return __byte_perm(lo, hi, 0x7610);
 }
-
-// 0x01 in byte b iff k_b < thr.
-__device__ __forceinline__ uint32_t below4(const uint32_t (&k)[4], uint32_t thr) {
-    return (uint32_t)(k[0] < thr) | ((uint32_t)(k[1] < thr) << 8) | ((uint32_t)(k[2] < thr) << 16) |
-           ((uint32_t)(k[3] < thr) << 24);
-}
+__device__ __forceinline__ uint32_t below4(const uint32_t (&w)[4], uint32_t n) { return below4(w, n, n, n, n); }
 
 __device__ __forceinline__ uint32_t lds(const unsigned char* p) { return *reinterpret_cast<const uint32_t*>(p); }
 __device__ __forceinline__ void sts(unsigned char* p, uint32_t v) { *reinterpret_cast<uint32_t*>(p) = v; }
-
-// Domino UpdateTiles (dominokernel.cl:22-31) for the four sites of a word:
-// edge bits 1 up, 2 down, 4 towards j-1, 8 towards j+1 from the flipped array
-// `src`; the neighbour towards j+1 shares the column in rows with
-// p = (i + t) odd, towards j-1 in the others.
-__device__ __forceinline__ uint32_t domino_refresh(const unsigned char* src, int off, int W, int p) {
-    const uint32_t up = lds(src + off - W), dn = lds(src + off + W);
-    const uint32_t l = lds(src + off - 4), c = lds(src + off), r = lds(src + off + 4);
-    const uint32_t west = p ? c : __funnelshift_l(l, c, 8);
-    const uint32_t east = p ? __funnelshift_r(c, r, 8) : c;
-    return ((up & 0x02020202u) >> 1) | ((dn & 0x01010101u) << 1) | ((west & 0x08080808u) >> 1) |
-           ((east & 0x04040404u) << 1);
-}
-
-// Lozenge UpdateTiles (lozengekernel.cl:36-54) for four sites: colour t+1
-// keeps all but bits {2,4,32} and takes them from f[i-1][j+sa], f[i][j-sw],
-// f[i+1][j]; colour t+2 keeps all but {1,8,16} and takes them from f[i-1][j],
-// f[i][j+se], f[i+1][j-sa].  The bit fields never overlap, so the reference's
-// sums are ORs.
-__device__ __forceinline__ void lozenge_refresh(const unsigned char* f, int off, int W, uint32_t sh, uint32_t a_old,
-                                                uint32_t b_old, uint32_t& na, uint32_t& nb) {
-    const uint32_t u0 = lds(f + off - W), u1 = lds(f + off - W + 4);
-    const uint32_t ml = lds(f + off - 4), m0 = lds(f + off), mr = lds(f + off + 4);
-    const uint32_t dl = lds(f + off + W - 4), d0 = lds(f + off + W);
-    const uint32_t sa = sh & 1u, sw = (sh >> 1) & 1u, se = (sh >> 2) & 1u;
-    const uint32_t fu_sa = sa ? __funnelshift_r(u0, u1, 8) : u0;
-    const uint32_t fw = sw ? __funnelshift_l(ml, m0, 8) : m0;
-    const uint32_t fe = se ? __funnelshift_r(m0, mr, 8) : m0;
-    const uint32_t fd_sa = sa ? __funnelshift_l(dl, d0, 8) : d0;
-    na = (a_old & 0xd9d9d9d9u) | ((fu_sa & 0x10101010u) >> 3) | ((fw & 0x08080808u) >> 1) |
-         ((d0 & 0x01010101u) << 5);
-    nb = (b_old & 0xe6e6e6e6u) | ((u0 & 0x20202020u) >> 5) | ((fe & 0x04040404u) << 1) |
-         ((fd_sa & 0x02020202u) << 3);
-}
-
+// old where mask is clear, nw where it is set
 __device__ __forceinline__ uint32_t merge(uint32_t old, uint32_t nw, uint32_t mask) { return (old & ~mask) | (nw & mask); }
 
-// Fixed facts of one word of the band: its byte offset in a colour plane,
-// its colour-array row i, and two byte masks: `um` (0xff) marks the sites an
-// Update refreshes (1 <= i <= N-2, 1 <= j <= width-2), `vm` (0x01) the sites
-// that are Rotate positions.
+// Fixed facts of one word of the band: its byte offset in a colour plane, its
+// row's class (lozenges: i mod 3; dominoes: i mod 2), and two byte masks: `um`
+// (0xff) marks the sites an Update refreshes (1 <= i <= N-2, 1 <= j <=
+// width-2), `vm` (0x80) the sites that are Rotate positions.
 struct WordInfo {
     int off;
-    int cls;  // lozenges: i mod 3; dominoes: i mod 2
+    int cls;
     uint32_t um;
     uint32_t vm;
 };
@@ -83,16 +46,160 @@ struct WordModel {
     }
 };
 
-// Per-phase decoded descriptor: which planes a word reads and writes.
-struct WordPhase {
-    bool step, upd, keep_a;
-    int par;                // dominoes: parity t of the pending Update
-    uint32_t shifts;        // lozenges: column shifts per row class (3 bits each)
-    unsigned char* dst;     // dominoes: array written; lozenges: colour flipped (STEP)
-    const unsigned char* src;  // flipped array whose neighbours are read (Update)
-    unsigned char* pa;      // lozenges: colours t+1, t+2 of the Update
-    unsigned char* pb;
+// Decoded phase descriptor.  dst: byte offset of the plane written (dominoes:
+// the array flipped or, at the end, refreshed; lozenges: the colour flipped
+// or, at the end, t+1); src: of the flipped colour t whose Update is pending;
+// oth (lozenges): of the other colour that Update refreshes.  flags: the
+// WP_* bits, the pending Update's colour t in bits 8..9.
+enum : uint32_t { WP_STEP = 1u, WP_UPD = 2u, WP_NEXT = 4u /* dst is colour t+1 */ };
+struct __align__(16) WordPhase {
+    int dst, src, oth;
+    uint32_t flags;
+    __device__ __forceinline__ int t() const { return (int)(flags >> 8) & 3; }
 };
+
+// Phases take few values, so they are decoded once, into a table.
+constexpr int kWordPhases = 32;
+__device__ __forceinline__ int word_phase_index(uint32_t d) {
+    return (int)(((d & OP_FINAL) << 3) | ((d >> 6) & 12u) | ((d >> 16) & 3u));
+}
+// Entry `idx` of the table for planes of `plane` bytes.
+template <int FAM>
+__device__ __forceinline__ WordPhase word_phase_entry(int idx, int plane) {
+    const bool step = !(idx & 16);
+    const int ca = (idx >> 2) & 3, cb = idx & 3;  // cb = 3: none
+    const bool upd = step ? (cb != 3 && cb != ca) : true;
+    const int t = step ? (upd ? cb : 0) : ca;
+    WordPhase P;
+    P.flags = (step ? WP_STEP : 0u) | (upd ? WP_UPD : 0u) | ((uint32_t)t << 8);
+    if (FAM != FAM_LOZENGE8) {
+        // Reference colour r flips array 1 - r, then refreshes array r from it.
+        const int dst = step ? 1 - ca : ca;
+        P.dst = dst * plane;
+        P.src = (1 - dst) * plane;
+        P.oth = 0;
+    } else {
+        const int t1 = t == 2 ? 0 : t + 1, t2 = t == 0 ? 2 : t - 1;
+        const bool next = !step || ca == t1;
+        P.dst = (step ? ca : t1) * plane;
+        P.src = t * plane;
+        P.oth = (next ? t2 : t1) * plane;
+        if (next) P.flags |= WP_NEXT;
+    }
+    return P;
+}
+
+// Byte selectors of the lozenge column shifts for pending colour t and row
+// class i mod 3 (index 3 t + class): the reads from the row above (x: words
+// w, w+1), the row below (y: w-1, w), the left (z: w-1, w) and the right
+// (w: w, w+1).  Exactly one of the three shifts applies in a row.
+constexpr int kLozengeSel = 9;
+__device__ __forceinline__ uint4 lozenge_sel_entry(int e) {
+    const int t = e / 3, cls = e % 3;
+    const bool sa = cls == (2 * t + 1) % 3, sw = cls == (2 * t + 2) % 3, se = cls == (2 * t) % 3;
+    return make_uint4(sa ? 0x4321u : 0x3210u, sa ? 0x6543u : 0x7654u, sw ? 0x6543u : 0x7654u, se ? 0x4321u : 0x3210u);
+}
+
+// The words of the flipped colour in the rows next to a word's row, as its
+// Update reads them: dominoes up[0] and dn[0] (same column); lozenges also
+// up[1] (the next word of the row above) and dn[1] (the previous word of the
+// row below).
+struct WordNbr {
+    uint32_t up[2], dn[2];
+};
+
+// One phase on one word of one lattice (planes at `lat`, a pending Update or
+// none), in two parts: `begin` reads the word and its own row, `finish` takes
+// the rows next to it.  m0 / m1: byte masks (0xff) of the phase's draws --
+// dominoes: m0 where the site toggles (heat bath: becomes 12, else 3);
+// lozenges: m0 where a cube is added, m1 where one is removed.
+template <int FAM>
+struct WordOp {
+    static constexpr bool DOM = FAM != FAM_LOZENGE8;
+    uint32_t v, o;    // the word written; lozenges: the other refreshed colour's
+    uint32_t ta, tb;  // the own row's share of the refreshed bits (dominoes: ta)
+    uint4 sel;
+
+    __device__ __forceinline__ void begin(const unsigned char* lat, const WordPhase& P, const WordInfo& wi,
+                                          const uint4* sel_tab) {
+        v = lds(lat + P.dst + wi.off);
+        if (!(P.flags & WP_UPD)) return;
+        const unsigned char* f = lat + P.src + wi.off;
+        const uint32_t l = lds(f - 4), c = lds(f), r = lds(f + 4);
+        if (DOM) {
+            // UpdateTiles (dominokernel.cl:22-31): edge bits 1 up, 2 down, 4 towards
+            // j-1, 8 towards j+1; the neighbour towards j+1 shares the column in rows
+            // with i + t odd, towards j-1 in the others.
+            const uint32_t p = (uint32_t)((wi.cls ^ P.t()) & 1) * 0x1111u;
+            const uint32_t west = __byte_perm(l, c, 0x6543u + p), east = __byte_perm(c, r, 0x3210u + p);
+            ta = ((west >> 1) & 0x04040404u) | ((east << 1) & 0x08080808u);
+        } else {
+            // UpdateTiles (lozengekernel.cl:36-54): colour t+1 keeps all but bits
+            // {2,4,32} and takes them from f[i-1][j+sa], f[i][j-sw], f[i+1][j]; colour
+            // t+2 keeps all but {1,8,16} and takes them from f[i-1][j], f[i][j+se],
+            // f[i+1][j-sa].  The bit fields never overlap: sums are ORs.
+            sel = sel_tab[3 * P.t() + wi.cls];
+            o = lds(lat + P.oth + wi.off);
+            ta = (__byte_perm(l, c, sel.z) >> 1) & 0x04040404u;
+            tb = (__byte_perm(c, r, sel.w) << 1) & 0x08080808u;
+        }
+    }
+    // Rows above and below from the band in shared memory (row stride W).
+    __device__ __forceinline__ static void load_up(WordNbr& nb, const unsigned char* lat, const WordPhase& P,
+                                                   const WordInfo& wi, int W) {
+        const unsigned char* f = lat + P.src + wi.off - W;
+        nb.up[0] = lds(f);
+        nb.up[1] = DOM ? 0u : lds(f + 4);
+    }
+    __device__ __forceinline__ static void load_dn(WordNbr& nb, const unsigned char* lat, const WordPhase& P,
+                                                   const WordInfo& wi, int W) {
+        const unsigned char* f = lat + P.src + wi.off + W;
+        nb.dn[0] = lds(f);
+        nb.dn[1] = DOM ? 0u : lds(f - 4);
+    }
+    __device__ __forceinline__ void finish(const WordPhase& P, const WordInfo& wi, const WordNbr& nb, uint32_t m0,
+                                           uint32_t m1) {
+        if (P.flags & WP_UPD) {
+            if (DOM) {
+                const uint32_t x = ((nb.up[0] >> 1) & 0x01010101u) | ta;
+                v = merge(v, ((nb.dn[0] << 1) & 0x02020202u) | x, wi.um);
+            } else {
+                const uint32_t fu = __byte_perm(nb.up[0], nb.up[1], sel.x), fd = __byte_perm(nb.dn[1], nb.dn[0], sel.y);
+                const uint32_t na = ((nb.dn[0] << 5) & 0x20202020u) | (((fu >> 3) & 0x02020202u) | ta);
+                const uint32_t nbv = ((fd << 3) & 0x10101010u) | (((nb.up[0] >> 5) & 0x01010101u) | tb);
+                const uint32_t ma = wi.um & 0x26262626u, mb = wi.um & 0x19191919u;
+                const bool next = (P.flags & WP_NEXT) != 0u;
+                v = merge(v, next ? na : nbv, next ? ma : mb);
+                o = merge(o, next ? nbv : na, next ? mb : ma);
+            }
+        }
+        if (P.flags & WP_STEP) {
+            // bit 7 of a byte of z is clear iff the byte equals the pattern (bytes < 0x80)
+            uint32_t tog;
+            if (DOM) {
+                const uint32_t z3 = (v ^ 0x03030303u) + 0x7f7f7f7fu, z12 = (v ^ 0x0c0c0c0cu) + 0x7f7f7f7fu;
+                if (FAM == FAM_DOMINO_HB)  // dominokernelCFTP.cl:19-28
+                    tog = (~z3 & m0) | (~z12 & ~m0);
+                else  // dominokernel.cl:11-17
+                    tog = ~(z3 & z12) & m0;
+            } else {  // lozengekernel.cl:19-31: a cube is added (25 -> 38) or removed (38 -> 25)
+                const uint32_t z25 = (v ^ 0x19191919u) + 0x7f7f7f7fu, z38 = (v ^ 0x26262626u) + 0x7f7f7f7fu;
+                tog = (~z25 & m0) | (~z38 & m1);
+            }
+            // 0x80 per toggled site -> 15 or 63 per byte: the high word of a product
+            v ^= __umulhi(tog & wi.vm, (DOM ? 15u : 63u) << 25);
+        }
+    }
+    __device__ __forceinline__ void store(unsigned char* lat, const WordPhase& P, const WordInfo& wi) const {
+        sts(lat + P.dst + wi.off, v);
+        if (!DOM && (P.flags & WP_UPD)) sts(lat + P.oth + wi.off, o);
+    }
+};
+
+// 0x01 per byte of the bits set in mask, one bit per byte index.
+__device__ __forceinline__ uint32_t lane_bytes(uint32_t bits) {
+    return (bits & 1u) | ((bits & 2u) << 7) | ((bits & 4u) << 14) | ((bits & 8u) << 21);
+}
 
 __device__ __forceinline__ uint32_t lozenge_shift_table(int t) {
     uint32_t tab = 0;
@@ -102,96 +209,6 @@ __device__ __forceinline__ uint32_t lozenge_shift_table(int t) {
         tab |= (sa | (sw << 1) | (se << 2)) << (3 * rr);
     }
     return tab;
-}
-
-// One phase on one word of one lattice; `lo` is the byte offset of the
-// lattice's planes from those the phase descriptor points at.
-// m0 / m1: per-byte draw masks (0x01) -- dominoes: k < thr[0]; lozenges:
-// k < thr[0] (add a cube) and thr[0] <= k < thr[1] (remove one).
-template <int FAM>
-__device__ __forceinline__ void word_phase(const WordPhase& P, int lo, int W, const WordInfo& wi, uint32_t m0,
-                                           uint32_t m1) {
-    const int off = wi.off + lo;
-    if (FAM != FAM_LOZENGE8) {
-        uint32_t v = lds(P.dst + off);
-        if (P.upd) v = merge(v, domino_refresh(P.src, off, W, (wi.cls ^ P.par) & 1), wi.um);
-        if (P.step) {
-            const uint32_t e3 = eq_bytes(v, 0x03030303u), e12 = eq_bytes(v, 0x0c0c0c0cu);
-            uint32_t tog;
-            if (FAM == FAM_DOMINO_HB)  // dominokernelCFTP.cl:19-28: k < 2^22 -> 12, else -> 3
-                tog = (e3 & m0) | (e12 & ~m0);
-            else  // dominokernel.cl:11-17: k < thr toggles 3 <-> 12
-                tog = (e3 | e12) & m0;
-            v ^= (tog & wi.vm) * 15u;
-        }
-        sts(P.dst + off, v);
-    } else {
-        if (P.step) {
-            uint32_t v;
-            if (P.upd) {
-                const uint32_t ao = lds(P.pa + off), bo = lds(P.pb + off);
-                uint32_t na, nb;
-                lozenge_refresh(P.src, off, W, (P.shifts >> (3 * wi.cls)) & 7u, ao, bo, na, nb);
-                na = merge(ao, na, wi.um);
-                nb = merge(bo, nb, wi.um);
-                if (P.keep_a) {
-                    v = na;
-                    sts(P.pb + off, nb);
-                } else {
-                    v = nb;
-                    sts(P.pa + off, na);
-                }
-            } else {
-                v = lds(P.dst + off);
-            }
-            // lozengekernel.cl:19-31: k < thr0 turns 25 into 38, thr0 <= k < thr1 turns 38 into 25.
-            const uint32_t tog = (eq_bytes(v, 0x19191919u) & m0) | (eq_bytes(v, 0x26262626u) & m1);
-            v ^= (tog & wi.vm) * 63u;
-            sts(P.dst + off, v);
-        } else {
-            const uint32_t ao = lds(P.pa + off), bo = lds(P.pb + off);
-            uint32_t na, nb;
-            lozenge_refresh(P.src, off, W, (P.shifts >> (3 * wi.cls)) & 7u, ao, bo, na, nb);
-            sts(P.pa + off, merge(ao, na, wi.um));
-            sts(P.pb + off, merge(bo, nb, wi.um));
-        }
-    }
-}
-
-// 0x01 per byte of the bits set in mask, one bit per byte index.
-__device__ __forceinline__ uint32_t lane_bytes(uint32_t bits) {
-    return (bits & 1u) | ((bits & 2u) << 7) | ((bits & 4u) << 14) | ((bits & 8u) << 21);
-}
-
-// Decodes phase descriptor d for a lattice whose NC planes start at `lat`
-// (`plane` bytes each); tabs = lozenge_shift_table(0..2).
-template <int FAM>
-__device__ __forceinline__ WordPhase word_phase_of(uint32_t d, unsigned char* lat, int plane, const uint32_t* tabs) {
-    WordPhase P;
-    const int op = (int)ph_op(d), ca = (int)ph_a(d), cb = (int)ph_b(d);
-    P.step = op == (int)OP_STEP;
-    P.upd = P.step ? (cb != (int)NO_COLOUR && cb != ca) : true;
-    const int tt = P.step ? (P.upd ? cb : 0) : ca;
-    if (FAM != FAM_LOZENGE8) {
-        // Reference colour r flips array 1 - r, then refreshes array r from it.
-        const int flip_arr = P.step ? 1 - ca : ca;
-        P.dst = lat + flip_arr * plane;
-        P.src = lat + (1 - flip_arr) * plane;
-        P.par = tt & 1;
-        P.keep_a = false;
-        P.shifts = 0u;
-        P.pa = P.pb = nullptr;
-    } else {
-        const int t1 = tt == 2 ? 0 : tt + 1, t2 = tt == 0 ? 2 : tt - 1;
-        P.dst = lat + ca * plane;
-        P.src = lat + tt * plane;
-        P.pa = lat + t1 * plane;
-        P.pb = lat + t2 * plane;
-        P.keep_a = P.step && P.upd && t1 == ca;
-        P.shifts = tt == 0 ? tabs[0] : tt == 1 ? tabs[1] : tabs[2];
-        P.par = 0;
-    }
-    return P;
 }
 
 }  // namespace rtb
