@@ -1,20 +1,26 @@
 // rt_mlp.cu -- training and inference kernels of the coordinate MLP
 // (include/rt_b200_mlp.h).
 //
-// Layers 1 and 2 (128 x 128) run on the fifth-generation tensor cores: a CTA
-// of four warps computes a 128 x 128 tile of C = A * B with tcgen05.mma
-// (BF16 inputs, FP32 accumulator in tensor memory), A and B staged through
-// shared memory 64 columns of K at a time; each GEMM names its operands'
-// layouts, so one kernel serves the forward product X * W^T, the input
-// gradient dZ * W and the weight gradient dZ^T * X (the last split over K,
-// reduced with FP32 atomics).  Operands contiguous along K are staged with
-// 16-byte asynchronous copies, the others as 8 x 8 core matrices transposed
-// in registers.  Epilogues, read from tensor memory with tcgen05.ld and
-// turned through shared memory so that global accesses run along rows, fuse
-// bias + GELU (forward) and the GELU derivative (backward).
+// One kernel takes tiles of 128 rows through the whole network: the rows are
+// gathered into shared memory, layer 0 runs in FP32, layers 1 and 2 (128 x
+// 128) on the fifth-generation tensor cores (tcgen05.mma, BF16 inputs, FP32
+// accumulators in tensor memory), layer 3 in FP32; with gradients, the whole
+// backward pass follows in the same CTA.  Activations live in shared memory
+// as BF16 tiles that serve as the operands of every product they enter: the
+// same 8 x 16-byte core matrices are read K-major (X W^T, dZ W) or MN-major
+// (dZ^T X), so nothing is transposed or written to global memory.  GELU and
+// its derivative share one tanh; the derivative waits in tensor memory or
+// registers for the backward pass.
+//
+// Weight gradients of the 128 x 128 layers are sums over ranges of up to 256
+// rows, each accumulated in tensor memory by a pair of CTAs in row order; a
+// second kernel adds the ranges, sums the other gradients over the rows in a
+// fixed order from the rows' FP32 values, and applies Adam.  No sum depends on
+// timing, so training repeats bit for bit.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -40,74 +46,54 @@ __device__ __forceinline__ float gelu(float z) {
     const float u = 0.7978845608f * (z + 0.044715f * z * z * z);
     return 0.5f * z * (1.0f + tanhf(u));
 }
-__device__ __forceinline__ float gelu_grad(float z) {
+// gelu(z), and its derivative in `grad`.
+__device__ __forceinline__ float gelu_both(float z, float& grad) {
     const float u = 0.7978845608f * (z + 0.044715f * z * z * z);
     const float t = tanhf(u);
-    return 0.5f * (1.0f + t) + 0.5f * z * (1.0f - t * t) * 0.7978845608f * (1.0f + 3.0f * 0.044715f * z * z);
+    grad = 0.5f * (1.0f + t) + 0.5f * z * (1.0f - t * t) * 0.7978845608f * (1.0f + 3.0f * 0.044715f * z * z);
+    return 0.5f * z * (1.0f + t);
 }
 
 // ---------------------------------------------------------------------------
-// Operand access.  A matrix operand is (ptr, ld, trans): element (r, c) of
-// the logical matrix is ptr[r * ld + c], or ptr[c * ld + r] when trans.
+// Tiles.  An operand tile is 128 x 128 BF16 in shared memory, core matrices of
+// 8 rows x 16 bytes (8 columns): element (r, c) at tile_off(r, c / 8) + 2 (c
+// mod 8).  Read K-major (MN = rows, K = columns) the next core matrix along K
+// is 128 bytes on (leading byte offset) and the next 8 rows 2 KB on (stride
+// byte offset); read MN-major (MN = columns, K = rows) the next 8 columns are
+// 128 bytes on (stride) and the next 8 rows 2 KB on (leading).
 // ---------------------------------------------------------------------------
-struct Op {
-    const __nv_bfloat16* p;
-    int ld;
-    int trans;
-};
-__device__ __forceinline__ __nv_bfloat16 op_at(const Op& o, int r, int c) {
-    return o.trans ? o.p[(size_t)c * o.ld + r] : o.p[(size_t)r * o.ld + c];
-}
-
-enum Epi : int {
-    EPI_FWD = 0,     // z = acc + bias[n]; out_f = z; out_h = bf16(gelu(z))
-    EPI_DGELU = 1,   // d = acc * gelu'(zin[m][n]); out_f = d; out_h = bf16(d)
-    EPI_ATOMIC = 2   // out_f[m][n] += acc (weight gradients, split over K)
-};
-
-struct GemmArgs {
-    Op A, B;        // C[M][N] = A[M][K] * B[K][N], N = 128
-    int M, N, K;
-    int ksplit;     // K range per blockIdx.z
-    int epi;
-    const float* bias;
-    const float* zin;   // EPI_DGELU: pre-activation [M][N]
-    float* out_f;       // [M][N]
-    __nv_bfloat16* out_h;  // [M][N] (EPI_FWD, EPI_DGELU)
-    int* err;           // set to 1 when a bounded wait gives up
-};
-
-// ---------------------------------------------------------------------------
-// tcgen05 GEMM.  A CTA of four warps computes a 128 x 128 tile of C in a
-// tensor-memory accumulator (128 lanes = rows, 128 FP32 columns).  K is
-// walked in chunks of 64: all threads stage the A chunk (128 x 64) and the B
-// chunk (as 128 n-rows x 64 k) into shared memory in the canonical K-major
-// layout without swizzle -- core matrices of 8 rows x 16 bytes, the 8 core
-// matrices of a row group side by side (leading byte offset 128 B, stride
-// byte offset 1 KB) -- then one thread issues the four K = 16 MMAs
-// (tcgen05.mma kind::f16, BF16 A and B, FP32 accumulate) and commits them to
-// an mbarrier that every thread waits on before the next chunk overwrites
-// the operands.  The epilogue reads the accumulator with tcgen05.ld (warp w
-// owns lanes 32w..32w+31, i.e. rows) 32 columns at a time.
-// ---------------------------------------------------------------------------
-constexpr int TBM = 128, TBN = 128, TBK = 64;
-constexpr uint32_t kTmemCols = 128;
+constexpr int TR = 128;                 // rows of a tile
+constexpr int kTile = TR * H * 2;       // bytes of an operand tile
+constexpr int kPart = 2 * H * H;        // floats of one CTA's partial dW1, dW2
 // Instruction descriptor (PTX ISA, kind::f16): D = F32 (bits 4-5 = 1), A = B =
-// BF16 (bits 7-9, 10-12 = 1), both K-major, N >> 3 at bits 17-22, M >> 4 at
-// bits 24-28.
-constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TBN >> 3) << 17) | ((uint32_t)(TBM >> 4) << 24);
-constexpr unsigned long long kWaitLimit = 1ull << 28;  // mbarrier polls before giving up
+// BF16 (bits 7-9, 10-12 = 1), N >> 3 at bits 17-22, M >> 4 at bits 24-28; bits
+// 15 / 16 mark A / B as MN-major.
+constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(H >> 3) << 17) | ((uint32_t)(TR >> 4) << 24);
+constexpr unsigned long long kWaitLimit = 1ull << 26;  // mbarrier polls before giving up
 
-// Shared-memory matrix descriptor (K-major, no swizzle): start address,
-// leading byte offset 128 B (next core matrix along K), stride byte offset
-// 1 KB (next group of 8 rows), version 1.
-__device__ __forceinline__ uint64_t smem_desc(uint32_t saddr) {
-    return (uint64_t)((saddr >> 4) & 0x3FFFu) | ((uint64_t)(128 >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) |
-           (1ull << 46);
+__device__ __forceinline__ uint32_t tile_off(int r, int c8) {
+    return (uint32_t)(((r >> 3) * (H / 8) + c8) * 128 + (r & 7) * 16);
 }
-// Byte offset of element (row r, k) of a 128 x 64 operand chunk in that layout.
-__device__ __forceinline__ uint32_t chunk_off(int r, int k) {
-    return (uint32_t)(((r >> 3) * (TBK / 8) + (k >> 3)) * 128 + (r & 7) * 16 + (k & 7) * 2);
+// Shared-memory matrix descriptor, no swizzle, version 1.
+__device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, bool mn_major) {
+    const uint32_t lead = mn_major ? 2048u : 128u, stride = mn_major ? 128u : 2048u;
+    return (uint64_t)((saddr >> 4) & 0x3FFFu) | ((uint64_t)(lead >> 4) << 16) | ((uint64_t)(stride >> 4) << 32) | (1ull << 46);
+}
+
+// D (128 x 128) = or += A B over K = 128, eight MMAs of K = 16; one thread.
+__device__ __forceinline__ void mma_tile(uint32_t d, uint32_t a, bool a_mn, uint32_t b, bool b_mn, bool accumulate) {
+    const uint32_t idesc = kIdesc | (a_mn ? 1u << 15 : 0u) | (b_mn ? 1u << 16 : 0u);
+#pragma unroll
+    for (int k = 0; k < H / 16; ++k) {
+        const uint64_t da = smem_desc(a + (a_mn ? 4096u : 256u) * k, a_mn), db = smem_desc(b + (b_mn ? 4096u : 256u) * k, b_mn);
+        const uint32_t acc = (accumulate || k > 0) ? 1u : 0u;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "setp.ne.b32 p, %4, 0;\n\t"
+            "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
+            ::"r"(d), "l"(da), "l"(db), "r"(idesc), "r"(acc)
+            : "memory");
+    }
 }
 
 __device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity) {
@@ -125,96 +111,116 @@ __device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity) {
     return false;
 }
 
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, uint32_t src_bytes) {
-    // src_bytes 0: the 16 bytes are zero-filled and nothing is read
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(src_bytes) : "memory");
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
 
-// Stages rows [r0, r0 + 128) x k [k0, k_end) of a logical operand whose
-// element (r, k) is p[r * ld + k] into the canonical K-major layout: every
-// 16-byte group of 8 consecutive k is one asynchronous copy (zero-filled
-// for rows >= rlim), so all of a chunk's loads are in flight together; a
-// group cut by k_end is assembled element by element.
-__device__ __forceinline__ void stage_kcontig(uint32_t sdst, unsigned char* dst, const __nv_bfloat16* p, int ld,
-                                              int r0, int rlim, int k0, int k_end) {
-    const uint16_t* q = reinterpret_cast<const uint16_t*>(p);
-    for (int e = threadIdx.x; e < TBM * (TBK / 8); e += 128) {
-        const int r = e / (TBK / 8), k8 = (e % (TBK / 8)) * 8;
-        const int gr = r0 + r, gk = k0 + k8;
-        const uint32_t off = chunk_off(r, k8);
-        if (gr >= rlim || gk + 8 <= k_end) {
-            const bool in = gr < rlim;
-            cp_async16(sdst + off, in ? (const void*)(q + (size_t)gr * ld + gk) : (const void*)q, in ? 16u : 0u);
-        } else {
-            uint32_t w[4];
+// Eight columns of this warp's 32 tensor-memory lanes.
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&f)[8]) {
+    uint32_t v[8];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+                 : "r"(taddr)
+                 : "memory");
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-            for (int x = 0; x < 4; ++x) {
-                const uint32_t lo = gk + 2 * x < k_end ? q[(size_t)gr * ld + gk + 2 * x] : 0u;
-                const uint32_t hi = gk + 2 * x + 1 < k_end ? q[(size_t)gr * ld + gk + 2 * x + 1] : 0u;
-                w[x] = lo | hi << 16;
-            }
-            *reinterpret_cast<uint4*>(dst + off) = make_uint4(w[0], w[1], w[2], w[3]);
-        }
+    for (int i = 0; i < 8; ++i) f[i] = __uint_as_float(v[i]);
+}
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const float (&f)[8]) {
+    uint32_t v[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = __float_as_uint(f[i]);
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%8], {%0,%1,%2,%3,%4,%5,%6,%7};" ::"r"(v[0]), "r"(v[1]),
+                 "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(taddr)
+                 : "memory");
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+
+// Columns 8 c8 .. 8 c8 + 7 of row r, rounded to BF16, into an operand tile; and back.
+__device__ __forceinline__ void store8(unsigned char* tile, int r, int c8, const float (&f)[8]) {
+    __nv_bfloat162 w[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        w[i].x = __float2bfloat16(f[2 * i]);
+        w[i].y = __float2bfloat16(f[2 * i + 1]);
+    }
+    *reinterpret_cast<uint4*>(tile + tile_off(r, c8)) = *reinterpret_cast<uint4*>(w);
+}
+__device__ __forceinline__ void load8(const unsigned char* tile, int r, int c8, float (&f)[8]) {
+    const uint4 q = *reinterpret_cast<const uint4*>(tile + tile_off(r, c8));
+    const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        f[2 * i] = __uint_as_float(w[i] << 16);
+        f[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
     }
 }
 
-// The same chunk of an operand stored the other way, element (r, k) at
-// p[k * ld + r].  Thread t builds core matrix (t / 8, t % 8) -- rows
-// 8 (t / 8) .. +7, k 8 (t % 8) .. +7: eight 16-byte loads along r, an 8 x 8
-// transpose of 16-bit values in registers, eight 16-byte stores that fill
-// the core matrix's 128 contiguous bytes.
-__device__ __forceinline__ void stage_mncontig(unsigned char* dst, const __nv_bfloat16* p, int ld, int r0, int rlim,
-                                               int k0, int k_end) {
-    const uint16_t* q = reinterpret_cast<const uint16_t*>(p);
-    const int rg = threadIdx.x >> 3, kg = threadIdx.x & 7;
-    const int gr = r0 + 8 * rg, gkb = k0 + 8 * kg;
-    uint32_t w[8][4];  // w[kk]: r = gr .. gr + 7 at k = gkb + kk, two per word
-#pragma unroll
-    for (int kk = 0; kk < 8; ++kk) {
-        const int gk = gkb + kk;
-        if (gk < k_end && gr + 8 <= rlim) {
-            const uint4 v = *reinterpret_cast<const uint4*>(q + (size_t)gk * ld + gr);
-            w[kk][0] = v.x, w[kk][1] = v.y, w[kk][2] = v.z, w[kk][3] = v.w;
-        } else {
-#pragma unroll
-            for (int x = 0; x < 4; ++x) {
-                const uint32_t lo = (gk < k_end && gr + 2 * x < rlim) ? q[(size_t)gk * ld + gr + 2 * x] : 0u;
-                const uint32_t hi = (gk < k_end && gr + 2 * x + 1 < rlim) ? q[(size_t)gk * ld + gr + 2 * x + 1] : 0u;
-                w[kk][x] = lo | hi << 16;
-            }
-        }
-    }
-#pragma unroll
-    for (int rr = 0; rr < 8; ++rr) {
-        uint32_t o[4];
-#pragma unroll
-        for (int x = 0; x < 4; ++x) {
-            const uint32_t a = (w[2 * x][rr >> 1] >> (16 * (rr & 1))) & 0xFFFFu;
-            const uint32_t b = (w[2 * x + 1][rr >> 1] >> (16 * (rr & 1))) & 0xFFFFu;
-            o[x] = a | b << 16;
-        }
-        *reinterpret_cast<uint4*>(dst + chunk_off(8 * rg + rr, 8 * kg)) = make_uint4(o[0], o[1], o[2], o[3]);
-    }
+struct NetArgs {
+    const float* P;                 // FP32 parameters
+    const __nv_bfloat16 *w1, *w2;   // BF16 copies of W1, W2
+    const float *x, *t;             // rows (IN features each) and, for gradients, targets
+    int n;                          // rows of this call
+    int range;                      // gradients: rows of a range (a pair of CTAs), 64 .. 256
+    int chain;                      // gradients: every pair has one range (see net_kernel)
+    int64_t pool;                   // > 0: row b is row floor(u pool) of x, t, with u from Philox (seed, step)
+    uint64_t seed;
+    int64_t step;
+    float* y;      // forward: predictions
+    float* part;   // gradients: partial dW1, dW2 (kPart floats) of each CTA
+    float4* rows;  // gradients: dy h3, dz2, dz1, dz0 of every row (kRowArrays arrays, row_at)
+    int64_t row_array;   // float4s of one of them
+    float *dy, *xb, *err2;  // gradients, by tile: dy of the rows, their features ([IN][TR]), their shares of the loss
+    int* err;      // set to 1 when a bounded wait gives up
+};
+constexpr int kRowArrays = 4;
+// Columns 4 c4 .. 4 c4 + 3 of row r of a tile: a warp's rows side by side.
+__host__ __device__ __forceinline__ int64_t row_at(int64_t tile, int c4, int r) { return (tile * (H / 4) + c4) * TR + r; }
+
+// Shared memory: W1, W2 and one activation tile (forward) or h1, h2, dz2 and
+// dz1 (gradients), then the FP32 parts.
+struct NetSmall {
+    float w0[H * IN], b0[H], b1[H], b2[H], w3[H];
+    float x[TR * IN], t[TR];
+    float y[8][TR];
+    float w3h[32 * TR];  // gradients: a third of the products h3 W3
+};
+constexpr size_t net_smem(bool grad) {
+    return (size_t)(grad ? 6 : 3) * kTile + sizeof(NetSmall) - (grad ? 0 : sizeof(NetSmall::w3h));
 }
 
-__global__ void __launch_bounds__(128, 1) gemm_tc(const __grid_constant__ GemmArgs g) {
-    // A and B chunks; after the last MMA the epilogue's per-warp staging
-    __shared__ __align__(128) unsigned char sAB[(TBM + TBN) * TBK * 2];
-    unsigned char* sA = sAB;
-    unsigned char* sB = sAB + TBM * TBK * 2;
+// Thread (warp w, lane l) owns row 32 (w mod 4) + l -- the tensor-memory lanes
+// its warp can reach -- and, of every 128 x 128 array, the 8 NCH columns of
+// column group w / 4, taken eight at a time in loops that are not unrolled
+// across each other: with 32 columns at once in registers the kernel was
+// three times as much code and waited for instructions.
+//
+// Gradients run as clusters of two CTAs, one per half of a range.  With one
+// range per pair (chain; batches of up to 74 ranges), the second CTA starts
+// its dW1, dW2 accumulators from the first one's results, so a range is one
+// sum in row order.  With more ranges than pairs, each CTA adds its tiles'
+// products to its own partial.
+template <bool GRAD, int THREADS>
+__global__ void __launch_bounds__(THREADS, GRAD ? 1 : 2) net_kernel(const __grid_constant__ NetArgs g) {
+    constexpr int GROUPS = THREADS / TR, NCH = H / 8 / GROUPS;
+    extern __shared__ __align__(128) unsigned char smem[];
+    unsigned char *sW1 = smem, *sH1 = smem + 2 * kTile, *sH2 = GRAD ? sH1 + kTile : sH1, *sDz2 = sH1 + 2 * kTile,
+                  *sDz1 = sH1 + 3 * kTile;
+    NetSmall& S = *reinterpret_cast<NetSmall*>(smem + (GRAD ? 6 : 3) * kTile);
     __shared__ __align__(8) unsigned long long mbar;
     __shared__ uint32_t tmem_slot;
     __shared__ int s_fail;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int m0 = blockIdx.y * TBM;
-    const int k_begin = blockIdx.z * g.ksplit, k_end = min(g.K, k_begin + g.ksplit);
-    const uint32_t sa = (uint32_t)__cvta_generic_to_shared(sA), sb = (uint32_t)__cvta_generic_to_shared(sB);
+    const int cg = warp >> 2, r = 32 * (warp & 3) + lane, b0 = NCH * cg;  // columns 8 b0 .. 8 (b0 + NCH) - 1
+    constexpr uint32_t kCols = GRAD ? 512 : 128;
     const uint32_t mb = (uint32_t)__cvta_generic_to_shared(&mbar);
+    const uint32_t aW1 = (uint32_t)__cvta_generic_to_shared(sW1), aW2 = aW1 + kTile;
+    const uint32_t aH1 = (uint32_t)__cvta_generic_to_shared(sH1), aH2 = (uint32_t)__cvta_generic_to_shared(sH2),
+                   aDz2 = (uint32_t)__cvta_generic_to_shared(sDz2), aDz1 = (uint32_t)__cvta_generic_to_shared(sDz1);
 
     if (warp == 0) {
         const uint32_t slot = (uint32_t)__cvta_generic_to_shared(&tmem_slot);
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot), "r"(kTmemCols)
-                     : "memory");
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot), "r"(kCols) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     if (tid == 0) {
@@ -222,223 +228,286 @@ __global__ void __launch_bounds__(128, 1) gemm_tc(const __grid_constant__ GemmAr
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         s_fail = 0;
     }
+    for (int e = tid; e < TR * (H / 8); e += THREADS) {
+        const int o = e / (H / 8), k8 = e % (H / 8);
+        cp_async16(aW1 + tile_off(o, k8), g.w1 + o * H + 8 * k8);
+        cp_async16(aW2 + tile_off(o, k8), g.w2 + o * H + 8 * k8);
+    }
+    for (int e = tid; e < H * IN; e += THREADS) S.w0[e] = g.P[OW0 + e];
+    for (int e = tid; e < H; e += THREADS) {
+        S.b0[e] = g.P[OB0 + e];
+        S.b1[e] = g.P[OB1 + e];
+        S.b2[e] = g.P[OB2 + e];
+        S.w3[e] = g.P[OW3 + e];
+    }
+    const float b3 = g.P[OB3];
+    asm volatile("cp.async.wait_all;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = tmem_slot;
+    // D1: z1, then gelu'(z1); D2: z2, then gelu'(z2), dz2 W2, dz1 W1; dW1, dW2.
+    // gelu'(z0) waits where dW1 goes at the end of a tile.
+    const uint32_t D1 = tmem, D2 = GRAD ? tmem + H : tmem, DW1 = tmem + 2 * H, DW2 = tmem + 3 * H;
+    const uint32_t mine = ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(8 * b0);  // this warp's lanes and columns
 
     uint32_t parity = 0;
-    bool first = true;
-    for (int k0 = k_begin; k0 < k_end; k0 += TBK) {
-        // Stage A as (m, k) and B as (n, k) = B[k][n]; zero outside the matrices.
-        // A(m, k) is contiguous along k unless A is transposed; B(k, n) as (n, k)
-        // is contiguous along k when B is transposed.
-        if (g.A.trans == 0)
-            stage_kcontig(sa, sA, g.A.p, g.A.ld, m0, g.M, k0, k_end);
-        else
-            stage_mncontig(sA, g.A.p, g.A.ld, m0, g.M, k0, k_end);
-        if (g.B.trans != 0)
-            stage_kcontig(sb, sB, g.B.p, g.B.ld, 0, g.N, k0, k_end);
-        else
-            stage_mncontig(sB, g.B.p, g.B.ld, 0, g.N, k0, k_end);
-        asm volatile("cp.async.wait_all;" ::: "memory");
-        // shared-memory writes -> visible to the tensor core's async proxy
+    // Operands written by everyone -> products issued by one thread (`issue`)
+    // -> accumulators readable by everyone.  False when a wait gave up.
+    auto products = [&](auto issue) {
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncthreads();
         if (tid == 0) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-#pragma unroll
-            for (int kk = 0; kk < TBK / 16; ++kk) {
-                // K = 16 per MMA: two core matrices along K = 256 bytes
-                const uint64_t da = smem_desc(sa + 256u * kk), db = smem_desc(sb + 256u * kk);
-                const uint32_t acc = (first && kk == 0) ? 0u : 1u;
-                asm volatile(
-                    "{\n\t.reg .pred p;\n\t"
-                    "setp.ne.b32 p, %4, 0;\n\t"
-                    "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
-                    ::"r"(tmem), "l"(da), "l"(db), "r"(kIdesc), "r"(acc)
-                    : "memory");
-            }
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mb)
-                         : "memory");
+            issue();
+            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mb) : "memory");
         }
-        first = false;
         if (!mbar_wait(mb, parity)) {
             s_fail = 1;  // racy but every writer writes 1
             atomicOr(g.err, 1);
         }
         parity ^= 1u;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        return !__syncthreads_or(*(volatile int*)&s_fail);
+    };
+    // dW2 (+)= dz2^T h2, dW1 (+)= dz1^T h1 of the tile in shared memory
+    auto weight_products = [&](bool acc) {
+        return products([&] {
+            mma_tile(DW2, aDz2, true, aH2, true, acc);
+            mma_tile(DW1, aDz1, true, aH1, true, acc);
+        });
+    };
+    // The accumulators dW1, dW2 and this CTA's partial, [k / 4][o][k mod 4], so
+    // that a warp's accesses are contiguous.  `f` sees eight values and the two
+    // float4s they belong to.
+    auto each_part = [&](int cta, auto f) {
+        float4* part = reinterpret_cast<float4*>(g.part + (int64_t)cta * kPart);
+#pragma unroll 1
+        for (int e = 0; e < 2 * NCH; ++e) {
+            const int which = e >= NCH, ch = e - which * NCH;
+            float4* at = part + which * (H * H / 4) + 2 * (b0 + ch) * H + r;
+            f((which ? DW2 : DW1) + mine + 8 * ch, at, at + H);
+        }
+    };
+    auto store_part = [&](bool add) {
+        each_part((int)blockIdx.x, [&](uint32_t taddr, float4* lo, float4* hi) {
+            float v[8];
+            tmem_ld8(taddr, v);
+            if (add) {
+                const float4 a = __ldcg(lo), b = __ldcg(hi);
+                v[0] += a.x, v[1] += a.y, v[2] += a.z, v[3] += a.w;
+                v[4] += b.x, v[5] += b.y, v[6] += b.z, v[7] += b.w;
+            }
+            __stcg(lo, make_float4(v[0], v[1], v[2], v[3]));
+            __stcg(hi, make_float4(v[4], v[5], v[6], v[7]));
+        });
+    };
+
+    // Forward: tiles blockIdx.x, + gridDim.x, ...  Gradients: pair p takes the
+    // ranges p, + pairs, ...; CTA 0 of it rows 0 .. 127 of the range, CTA 1 the rest.
+    const int rank = GRAD ? (int)(blockIdx.x & 1) : 0, pair = GRAD ? (int)(blockIdx.x >> 1) : (int)blockIdx.x;
+    const int pairs = GRAD ? (int)(gridDim.x >> 1) : (int)gridDim.x;
+    const int span = GRAD ? g.range : TR, units = (g.n + span - 1) / span;
+    for (int u = pair; u < units; u += pairs) {
+        const int row0 = u * span + TR * rank, rows = max(0, min(min(span - TR * rank, TR), g.n - row0));
+        const int tile = GRAD ? 2 * u + rank : u;
+        const bool live = r < rows;
+        if (tid < TR) {
+            const int b = row0 + tid;
+            float4 lo = make_float4(0, 0, 0, 0), hi = lo;
+            float t = 0.0f;
+            if (tid < rows) {
+                int64_t src = b;
+                if (GRAD && g.pool > 0) {
+                    // batch rows drawn with replacement
+                    const uint4 w = philox4((uint32_t)b, (uint32_t)g.step, (uint32_t)((uint64_t)g.step >> 32), 0x4d4c50u,
+                                            (uint32_t)g.seed, (uint32_t)(g.seed >> 32));
+                    src = (int64_t)((((uint64_t)w.x << 32) | w.y) % (uint64_t)g.pool);
+                }
+                lo = *reinterpret_cast<const float4*>(g.x + src * IN);
+                hi = *reinterpret_cast<const float4*>(g.x + src * IN + 4);
+                if (GRAD) t = g.t[src];
+            }
+            *reinterpret_cast<float4*>(S.x + tid * IN) = lo;
+            *reinterpret_cast<float4*>(S.x + tid * IN + 4) = hi;
+            S.t[tid] = t;
+            if (GRAD) {
+                float* xb = g.xb + (int64_t)tile * IN * TR + tid;
+                xb[0] = lo.x, xb[TR] = lo.y, xb[2 * TR] = lo.z, xb[3 * TR] = lo.w;
+                xb[4 * TR] = hi.x, xb[5 * TR] = hi.y, xb[6 * TR] = hi.z, xb[7 * TR] = hi.w;
+            }
+        }
         __syncthreads();
-        if (s_fail) break;
+        float x[IN];
+#pragma unroll
+        for (int k = 0; k < IN; ++k) x[k] = S.x[r * IN + k];
+        // The layers: z (layer 0 from x, the others from tensor memory), h =
+        // gelu(z) rounded to BF16 into its tile, gelu'(z) into tensor memory.
+        bool ok = true;
+        float ysum = 0.0f;
+#pragma unroll 1
+        for (int layer = 0; layer < 3; ++layer) {
+            const uint32_t src = (layer == 1 ? D1 : D2) + mine, dst = (layer == 0 ? DW1 : layer == 1 ? D1 : D2) + mine;
+            const float* bias = layer == 0 ? S.b0 : layer == 1 ? S.b1 : S.b2;
+            unsigned char* tile_h = layer == 0 ? sH1 : layer == 1 ? sH2 : sDz1;  // h3 waits where dz1 goes
+#pragma unroll 1
+            for (int ch = 0; ch < NCH; ++ch) {
+                const int c = 8 * (b0 + ch);
+                float z[8], h[8], d[GRAD ? 8 : 1];
+                if (layer == 0) {
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        const float4 wa = *reinterpret_cast<const float4*>(S.w0 + (c + i) * IN);
+                        const float4 wb = *reinterpret_cast<const float4*>(S.w0 + (c + i) * IN + 4);
+                        z[i] = bias[c + i];
+                        z[i] += wa.x * x[0], z[i] += wa.y * x[1], z[i] += wa.z * x[2], z[i] += wa.w * x[3];
+                        z[i] += wb.x * x[4], z[i] += wb.y * x[5], z[i] += wb.z * x[6], z[i] += wb.w * x[7];
+                    }
+                } else {
+                    tmem_ld8(src + 8 * ch, z);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) z[i] += bias[c + i];
+                }
+#pragma unroll
+                for (int i = 0; i < 8; ++i) h[i] = GRAD ? gelu_both(z[i], d[GRAD ? i : 0]) : gelu(z[i]);
+                if (GRAD || layer < 2) {
+                    store8(tile_h, r, b0 + ch, h);
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) ysum += __bfloat162float(__float2bfloat16(h[i])) * S.w3[c + i];
+                }
+                if constexpr (GRAD) tmem_st8(dst + 8 * ch, d);
+            }
+            if (layer == 0) ok = products([&] { mma_tile(D1, aH1, false, aW1, false, false); });  // z1 = h1 W1^T
+            if (layer == 1) ok = products([&] { mma_tile(D2, aH2, false, aW2, false, false); });  // z2 = h2 W2^T
+            if (!ok) break;
+        }
+        if (!ok) break;
+        if constexpr (!GRAD) {
+            S.y[cg][r] = ysum;
+            __syncthreads();
+            if (cg == 0 && live) g.y[row0 + r] = ((S.y[0][r] + S.y[1][r]) + (S.y[2][r] + S.y[3][r])) + b3;
+        } else {
+            // y = h3 W3 + b3: the products of columns c, c + 32, c + 64 and c + 96 in
+            // turn, then pairwise over c mod 32.  y - t cancels, so the order of this
+            // sum shows in every gradient.  Columns 32 .. 127 pass through dz2's tile
+            // and w3h as [c][row].
+            float* const p1 = reinterpret_cast<float*>(sDz2);
+#pragma unroll 1
+            for (int ch = 0; ch < NCH; ++ch) {
+                const int c = 8 * (b0 + ch);
+                if (c < 32) continue;
+                float h[8];
+                load8(sDz1, r, b0 + ch, h);
+                float* p = c < 96 ? p1 + (c - 32) * TR : S.w3h + (c - 96) * TR;
+#pragma unroll
+                for (int i = 0; i < 8; ++i) p[i * TR + r] = h[i] * S.w3[c + i];
+            }
+            __syncthreads();
+            if (cg == 0) {
+                float q[32];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    float h[8];
+                    load8(sDz1, r, k, h);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) q[8 * k + i] = h[i] * S.w3[8 * k + i];
+                }
+#pragma unroll
+                for (int i = 0; i < 32; ++i) {
+                    q[i] = q[i] + p1[i * TR + r];
+                    q[i] = q[i] + p1[(32 + i) * TR + r];
+                    q[i] = q[i] + S.w3h[i * TR + r];
+                }
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+                    for (int i = 0; i < o; ++i) q[i] += q[i + o];
+                S.y[0][r] = q[0];
+            }
+            __syncthreads();
+            const float e = S.y[0][r] + b3 - S.t[r];
+            const float dy = live ? 2.0f * e / (float)g.n : 0.0f;
+            if (cg == 0) {
+                g.dy[(int64_t)tile * TR + r] = dy;
+                g.err2[(int64_t)tile * TR + r] = live ? e * e / (float)g.n : 0.0f;
+            }
+            // Eight of this thread's values of row array `which`.
+            auto put = [&](int which, int ch, const float (&f)[8]) {
+                float4* dst = g.rows + which * g.row_array + row_at(tile, 2 * (b0 + ch), r);
+                __stcg(dst, make_float4(f[0], f[1], f[2], f[3]));
+                __stcg(dst + TR, make_float4(f[4], f[5], f[6], f[7]));
+            };
+#pragma unroll 1
+            for (int ch = 0; ch < NCH; ++ch) {
+                float v[8], d[8];
+                load8(sDz1, r, b0 + ch, v);
+                tmem_ld8(D2 + mine + 8 * ch, d);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    v[i] = dy * v[i];                              // dy h3
+                    d[i] = dy * S.w3[8 * (b0 + ch) + i] * d[i];    // dz2
+                }
+                store8(sDz2, r, b0 + ch, d);
+                put(0, ch, v);
+                put(1, ch, d);
+            }
+            if (!products([&] { mma_tile(D2, aDz2, false, aW2, true, false); })) break;  // dz2 W2
+#pragma unroll 1
+            for (int ch = 0; ch < NCH; ++ch) {
+                float v[8], d[8];
+                tmem_ld8(D2 + mine + 8 * ch, v);
+                tmem_ld8(D1 + mine + 8 * ch, d);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) d[i] = v[i] * d[i];  // dz1
+                store8(sDz1, r, b0 + ch, d);
+                put(2, ch, d);
+            }
+            if (!products([&] { mma_tile(D2, aDz1, false, aW1, true, false); })) break;  // dz1 W1
+#pragma unroll 1
+            for (int ch = 0; ch < NCH; ++ch) {
+                float v[8], d[8];
+                tmem_ld8(D2 + mine + 8 * ch, v);
+                tmem_ld8(DW1 + mine + 8 * ch, d);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) v[i] = v[i] * d[i];  // dz0
+                put(3, ch, v);
+            }
+            if (!(g.chain && rank == 1)) {
+                if (!weight_products(false)) break;
+                store_part(u != pair);
+            }
+        }
+        __syncthreads();
     }
 
-    if (!s_fail && !first) {
-        // Epilogue: this warp's 32 rows (TMEM lanes 32w .. 32w + 31), 32
-        // columns per tcgen05.ld (lane = row), turned through shared memory
-        // (32 x 33 floats per warp) so that the global loads and stores run
-        // along rows: lane = column.
-        float* stg = reinterpret_cast<float*>(sAB) + warp * (32 * 33);
-        const int mrow = m0 + 32 * warp;
-#pragma unroll 1
-        for (int c0 = 0; c0 < TBN; c0 += 32) {
-            uint32_t v[32];
-            const uint32_t taddr = tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)c0;
-            asm volatile(
-                "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-                "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
-                "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-                : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-                  "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]),
-                  "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]),
-                  "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]),
-                  "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-                : "r"(taddr)
-                : "memory");
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-            for (int x = 0; x < 32; ++x) stg[lane * 33 + x] = __uint_as_float(v[x]);
-            __syncwarp();
-            const int n = c0 + lane;
-            const float b = (g.epi == EPI_FWD && n < g.N) ? g.bias[n] : 0.0f;
-#pragma unroll 4
-            for (int rr = 0; rr < 32; ++rr) {
-                const int m = mrow + rr;
-                if (m >= g.M || n >= g.N) continue;
-                const float acc = stg[rr * 33 + lane];
-                const size_t at = (size_t)m * g.N + n;
-                if (g.epi == EPI_FWD) {
-                    const float z = acc + b;
-                    g.out_f[at] = z;
-                    g.out_h[at] = __float2bfloat16(gelu(z));
-                } else if (g.epi == EPI_DGELU) {
-                    const float dd = acc * gelu_grad(g.zin[at]);
-                    g.out_f[at] = dd;
-                    g.out_h[at] = __float2bfloat16(dd);
-                } else {
-                    atomicAdd(g.out_f + at, acc);
-                }
-            }
-            __syncwarp();
+    if (GRAD && g.chain) {
+        // both CTAs pass here, whatever happened to either
+        __threadfence();
+        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+        if (rank == 1 && !s_fail) {
+            each_part((int)blockIdx.x - 1, [&](uint32_t taddr, float4* lo, float4* hi) {
+                const float4 a = __ldcg(lo), b = __ldcg(hi);
+                const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+                tmem_st8(taddr, v);
+            });
+            if (weight_products(true)) store_part(false);
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == 0) {
         if (s_fail) {
-            // the MMAs may still be running: wait for them (bounded) before freeing their accumulator
+            // the MMAs may still be running: wait for them (bounded) before freeing their accumulators
             mbar_wait(mb, parity ^ 1u);
         }
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kCols) : "memory");
     }
 }
+constexpr int kFwdThreads = 512, kGradThreads = 512;
 
-// Layer 0 (IN -> H), FP32: z0 = x W0^T + b0, h1 = bf16(gelu(z0)).
-__global__ void layer0_fwd(const float* __restrict__ x, const float* __restrict__ P, int n, float* z0,
-                           __nv_bfloat16* h1) {
-    const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= (int64_t)n * H) return;
-    const int r = (int)(e / H), o = (int)(e % H);
-    float z = P[OB0 + o];
-#pragma unroll
-    for (int k = 0; k < IN; ++k) z += P[OW0 + o * IN + k] * x[(size_t)r * IN + k];
-    z0[e] = z;
-    h1[e] = __float2bfloat16(gelu(z));
-}
-
-// Layer 3 (H -> 1), FP32, one warp per row: y = h3 . W3 + b3; with a target,
-// also dy = 2 (y - t) / n and the mean squared error (one atomic per block).
-__global__ void layer3_fwd(const __nv_bfloat16* __restrict__ h3, const float* __restrict__ P, int n, float* y,
-                           const float* __restrict__ target, float* dy, float* loss) {
-    const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    __shared__ float part[32];
-    float err = 0.0f;
-    if (row < n) {
-        float s = 0.0f;
-        for (int k = lane; k < H; k += 32) s += __bfloat162float(h3[(size_t)row * H + k]) * P[OW3 + k];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        const float v = s + P[OB3];
-        if (lane == 0) {
-            if (y) y[row] = v;
-            if (target) {
-                const float e = v - target[row];
-                dy[row] = 2.0f * e / (float)n;
-                err = e * e / (float)n;
-            }
-        }
-    }
-    if (!target) return;
-    if (lane == 0) part[threadIdx.x >> 5] = err;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        float t = 0.0f;
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += part[w];
-        atomicAdd(loss, t);
-    }
-}
-
-// Backward of layer 3, elementwise: dz2 = dy W3 * gelu'(z2) (FP32 and BF16).
-__global__ void layer3_bwd(const float* __restrict__ z2, const float* __restrict__ dy, const float* __restrict__ P,
-                           int n, float* dz2, __nv_bfloat16* dz2h) {
-    const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= (int64_t)n * H) return;
-    const int r = (int)(e / H), k = (int)(e % H);
-    const float g = dy[r] * P[OW3 + k] * gelu_grad(z2[e]);
-    dz2[e] = g;
-    dz2h[e] = __float2bfloat16(g);
-}
-
-// Output-layer weights: G[W3][k] = sum_r dy[r] h3[r][k] (block k < H), and
-// G[b3] = sum_r dy[r] (block H).
-__global__ void layer3_wgrad(const __nv_bfloat16* __restrict__ h3, const float* __restrict__ dy, int n, float* G) {
-    const int k = blockIdx.x;
-    float s = 0.0f;
-    for (int r = threadIdx.x; r < n; r += blockDim.x)
-        s += dy[r] * (k < H ? __bfloat162float(h3[(size_t)r * H + k]) : 1.0f);
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    __shared__ float part[32];
-    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        float t = 0.0f;
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += part[w];
-        G[k < H ? OW3 + k : OB3] += t;
-    }
-}
-
-// Bias gradient: G[off + c] += sum_r d[r][c].
-__global__ void bias_grad(const float* __restrict__ d, int n, float* G, int off) {
-    const int c = blockIdx.x;
-    float s = 0.0f;
-    for (int r = threadIdx.x; r < n; r += blockDim.x) s += d[(size_t)r * H + c];
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    __shared__ float part[32];
-    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        float t = 0.0f;
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += part[w];
-        G[off + c] += t;
-    }
-}
-
-// Layer 0 weights: G[W0] += dz0^T x, G[b0] by bias_grad.
-__global__ void layer0_wgrad(const float* __restrict__ dz0, const float* __restrict__ x, int n, float* G) {
-    const int o = blockIdx.x, k = threadIdx.x & 7, part = threadIdx.x >> 3;  // 256 threads: 32 parts x 8 inputs
-    float s = 0.0f;
-    for (int r = part; r < n; r += 32) s += dz0[(size_t)r * H + o] * x[(size_t)r * IN + k];
-    __shared__ float red[32][IN];
-    red[part][k] = s;
-    __syncthreads();
-    if (part == 0) {
-        float t = 0.0f;
-        for (int p = 0; p < 32; ++p) t += red[p][k];
-        G[OW0 + o * IN + k] += t;
-    }
-}
-
-// BF16 copies of W1, W2 for the tensor-core GEMMs.
+// BF16 copies of W1, W2 for the tensor-core products.
 __global__ void to_bf16(const float* __restrict__ P, __nv_bfloat16* w1, __nv_bfloat16* w2) {
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= H * H) return;
@@ -446,31 +515,224 @@ __global__ void to_bf16(const float* __restrict__ P, __nv_bfloat16* w1, __nv_bfl
     w2[e] = __float2bfloat16(P[OW2 + e]);
 }
 
-__global__ void adam(float* P, const float* __restrict__ G, float* m1, float* m2, int n, float lr, float b1t,
-                     float b2t) {
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= n) return;
-    const float g = G[e];
-    const float a = 0.9f * m1[e] + 0.1f * g;
-    const float b = 0.999f * m2[e] + 0.001f * g * g;
-    m1[e] = a;
-    m2[e] = b;
-    const float mh = a / (1.0f - b1t), vh = b / (1.0f - b2t);
-    P[e] -= lr * mh / (sqrtf(vh) + 1e-8f);
+// The second kernel of a gradient.  Blocks by role, 256 threads each, the
+// longest first:
+//   dW0, four rows and two inputs a block (128): lane p of warps 0 and 1 sums
+//     the rows p, p + 32, ... of an input, staged through shared memory by the
+//     block -- one chain of n / 32 additions a lane, and 384 KB of a batch of
+//     16,384 through each block;
+//   dW1, dW2 (128): the sum of the partials;
+//   dW3, db2, db1, db0, four columns a block (128): thread s sums the rows
+//     s, s + 256, ... of its columns, then the block the threads (within warps,
+//     then warp by warp);
+//   db3 and the loss (1).
+// Rows that a tile does not have were written as zeros.  ADAM: the step, and
+// the BF16 copies; else the gradient.  It reads 92 MB at batch 16,384, just
+// written and still in L2: 18 us, 10 of them for the roles after the first.
+struct SumArgs {
+    const float* part;
+    int parts, part_first, part_step;  // partials part_first, + part_step, ...
+    const float4* rows;
+    int64_t row_array;
+    const float *dy, *xb, *err2;
+    int n, range;
+    float *P, *M1, *M2, *G, *loss;
+    __nv_bfloat16 *w1, *w2;
+    float lr, b1t, b2t;
+};
+constexpr int kW0Inputs = 2;  // dW0: inputs of a block
+constexpr int kSumBlocks = 128 + 32 * kRowArrays + 32 * (IN / kW0Inputs) + 1;
+constexpr int kStage = 8;  // dW0: tiles of a stage
+constexpr int kBufs = 4;   // stages, three of them on their way
+constexpr int kSumSmem = kBufs * kStage * TR * (16 + kW0Inputs * 4);
+
+template <bool ADAM>
+__device__ __forceinline__ void take_gradient(const SumArgs& a, int at, float grad) {
+    if (!ADAM) {
+        a.G[at] = grad;
+        return;
+    }
+    const float m = 0.9f * a.M1[at] + 0.1f * grad;
+    const float v = 0.999f * a.M2[at] + 0.001f * grad * grad;
+    a.M1[at] = m;
+    a.M2[at] = v;
+    const float mh = m / (1.0f - a.b1t), vh = v / (1.0f - a.b2t);
+    const float np = a.P[at] - a.lr * mh / (sqrtf(vh) + 1e-8f);
+    a.P[at] = np;
+    if (at >= OW1 && at < OB1) a.w1[at - OW1] = __float2bfloat16(np);
+    if (at >= OW2 && at < OB2) a.w2[at - OW2] = __float2bfloat16(np);
 }
 
-// Batch rows drawn with replacement: row = floor(u * rows) with u from
-// Philox keyed by (seed, step).
-__global__ void gather_batch(const float* __restrict__ X, const float* __restrict__ T, int64_t rows, int batch,
-                             uint64_t seed, int64_t step, float* xb, float* tb) {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= batch) return;
-    const uint4 w = philox4((uint32_t)b, (uint32_t)step, (uint32_t)((uint64_t)step >> 32), 0x4d4c50u,
-                            (uint32_t)seed, (uint32_t)(seed >> 32));
-    const uint64_t r64 = (((uint64_t)w.x << 32) | w.y) % (uint64_t)rows;
+__device__ __forceinline__ float4 add4(float4 a, float4 b) {
+    return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
+}
+__device__ __forceinline__ float4 shfl_xor4(float4 a, int o) {
+    return make_float4(__shfl_xor_sync(0xffffffffu, a.x, o), __shfl_xor_sync(0xffffffffu, a.y, o),
+                       __shfl_xor_sync(0xffffffffu, a.z, o), __shfl_xor_sync(0xffffffffu, a.w, o));
+}
+
+template <bool ADAM>
+__global__ void __launch_bounds__(256) sum_kernel(const __grid_constant__ SumArgs a) {
+    extern __shared__ __align__(16) unsigned char sum_smem[];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    int role = blockIdx.x;
+    // Place of row `row` among the tiles: tile * TR + row of the tile.
+    auto place = [&](int row, int64_t* tile, int* r) {
+        const int u = row / a.range, rem = row - u * a.range;
+        *tile = 2 * (int64_t)u + (rem >= TR);
+        *r = rem & (TR - 1);
+    };
+    const int ranges = (a.n + a.range - 1) / a.range;
+    __shared__ float4 s_part[8];
+    if (role < 32 * (IN / kW0Inputs)) {
+        const int c4 = role & 31, k0 = kW0Inputs * (role >> 5);
+        float4(*s_d)[kStage * TR] = reinterpret_cast<float4(*)[kStage * TR]>(sum_smem);
+        float(*s_x)[kW0Inputs * kStage * TR] = reinterpret_cast<float(*)[kW0Inputs * kStage * TR]>(sum_smem + kBufs * kStage * TR * 16);
+        const float4* src = a.rows + 3 * a.row_array;
+        const int tiles = 2 * ranges, stages = (tiles + kStage - 1) / kStage;
+        auto load = [&](int st) {
+            if (st < stages) {
+                const int buf = st % kBufs, n = min(kStage, tiles - st * kStage);
+                for (int e = tid; e < n * TR; e += 256)
+                    cp_async16((uint32_t)__cvta_generic_to_shared(&s_d[buf][e]),
+                               src + row_at((int64_t)st * kStage + e / TR, c4, e % TR));
+                constexpr int kQuads = kW0Inputs * TR / 4;  // the inputs of a tile are side by side
+                for (int e = tid; e < n * kQuads; e += 256)
+                    cp_async16((uint32_t)__cvta_generic_to_shared(&s_x[buf][4 * e]),
+                               a.xb + (((int64_t)st * kStage + e / kQuads) * IN + k0) * TR + 4 * (e % kQuads));
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+        float4 s = make_float4(0, 0, 0, 0);
+        for (int st = 0; st < kBufs - 1; ++st) load(st);
+        for (int st = 0; st < stages; ++st) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(kBufs - 2) : "memory");
+            __syncthreads();  // the stage has arrived, and everyone is done with the one before
+            load(st + kBufs - 1);
+            if (warp >= kW0Inputs) continue;
+            const int buf = st % kBufs, n = min(kStage, tiles - st * kStage);
+            const float4* d = s_d[buf] + lane;
+            const float* x = s_x[buf] + warp * TR + lane;
+            auto product = [&](int e) {
+                const float4 v = d[(e >> 2) * TR + 32 * (e & 3)];
+                const float w = x[(e >> 2) * kW0Inputs * TR + 32 * (e & 3)];
+                return make_float4(v.x * w, v.y * w, v.z * w, v.w * w);
+            };
+            if (n == kStage) {
+                float4 v[4 * kStage];
 #pragma unroll
-    for (int k = 0; k < IN; ++k) xb[(size_t)b * IN + k] = X[r64 * IN + k];
-    tb[b] = T[r64];
+                for (int e = 0; e < 4 * kStage; ++e) v[e] = product(e);
+#pragma unroll
+                for (int e = 0; e < 4 * kStage; ++e) s = add4(s, v[e]);
+            } else {
+                for (int e = 0; e < 4 * n; ++e) s = add4(s, product(e));
+            }
+        }
+        if (warp >= kW0Inputs) return;
+        float4 t = make_float4(0, 0, 0, 0);
+        for (int p = 0; p < 32; ++p)
+            t = add4(t, make_float4(__shfl_sync(0xffffffffu, s.x, p), __shfl_sync(0xffffffffu, s.y, p),
+                                    __shfl_sync(0xffffffffu, s.z, p), __shfl_sync(0xffffffffu, s.w, p)));
+        if (lane < 4)
+            take_gradient<ADAM>(a, OW0 + (4 * c4 + lane) * IN + k0 + warp,
+                                lane == 0 ? t.x : lane == 1 ? t.y : lane == 2 ? t.z : t.w);
+        return;
+    }
+    role -= 32 * (IN / kW0Inputs);
+    if (role < 128) {
+        // four lanes share four consecutive floats, each lane a quarter of the partials
+        const int e4 = role * 64 + (tid >> 2), sub = tid & 3;
+        const float4* p = reinterpret_cast<const float4*>(a.part) + e4;
+        float4 s = make_float4(0, 0, 0, 0);
+        p += (int64_t)a.part_first * (kPart / 4);
+        const int64_t step = (int64_t)a.part_step * (kPart / 4);
+        int b = sub;
+        for (; b + 28 < a.parts; b += 32) {
+            float4 v[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) v[k] = __ldcg(p + (b + 4 * k) * step);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) s = add4(s, v[k]);
+        }
+        for (; b < a.parts; b += 4) s = add4(s, __ldcg(p + b * step));
+        s = add4(s, shfl_xor4(s, 1));
+        s = add4(s, shfl_xor4(s, 2));
+        const float grad = sub == 0 ? s.x : sub == 1 ? s.y : sub == 2 ? s.z : s.w;
+        const int which = e4 >= H * H / 4, e = e4 - which * (H * H / 4);  // e = (k / 4) H + o
+        take_gradient<ADAM>(a, (which ? OW2 : OW1) + (e & (H - 1)) * H + (e / H) * 4 + sub, grad);
+        return;
+    }
+    role -= 128;
+    if (role < 32 * kRowArrays) {
+        const int which = role >> 5, c4 = role & 31;
+        const float4* src = a.rows + which * a.row_array;
+        float4 s = make_float4(0, 0, 0, 0);
+        if (a.range == 256) {
+            const float4* q = src + row_at(tid >> 7, c4, tid & (TR - 1));
+            int u = 0;
+            for (; u + 16 <= ranges; u += 16) {
+                float4 v[16];
+#pragma unroll
+                for (int k = 0; k < 16; ++k) v[k] = __ldcg(q + (u + k) * row_at(2, 0, 0));
+#pragma unroll
+                for (int k = 0; k < 16; ++k) s = add4(s, v[k]);
+            }
+            for (; u < ranges; ++u) s = add4(s, __ldcg(q + u * row_at(2, 0, 0)));
+        } else {
+            for (int row = tid; row < a.n; row += 256) {
+                int64_t tile;
+                int r;
+                place(row, &tile, &r);
+                s = add4(s, __ldcg(src + row_at(tile, c4, r)));
+            }
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s = add4(s, shfl_xor4(s, o));
+        if (lane == 0) s_part[warp] = s;
+        __syncthreads();
+        if (tid < 4) {
+            float t = 0.0f;
+            for (int w = 0; w < 8; ++w) t += reinterpret_cast<const float*>(s_part + w)[tid];
+            take_gradient<ADAM>(a, (which == 0 ? OW3 : which == 1 ? OB2 : which == 2 ? OB1 : OB0) + 4 * c4 + tid, t);
+        }
+        return;
+    }
+    float s = 0.0f, loss = 0.0f;
+    if (a.range == 256) {
+        int u = 0;
+        for (; u + 16 <= ranges; u += 16) {
+            float v[16], w[16];
+#pragma unroll
+            for (int k = 0; k < 16; ++k) v[k] = __ldcg(a.dy + (u + k) * 256 + tid), w[k] = __ldcg(a.err2 + (u + k) * 256 + tid);
+#pragma unroll
+            for (int k = 0; k < 16; ++k) s += v[k], loss += w[k];
+        }
+        for (; u < ranges; ++u) {
+            s += __ldcg(a.dy + u * 256 + tid);
+            loss += __ldcg(a.err2 + u * 256 + tid);
+        }
+    } else {
+        for (int row = tid; row < a.n; row += 256) {
+            int64_t tile;
+            int r;
+            place(row, &tile, &r);
+            s += __ldcg(a.dy + tile * TR + r);
+            loss += __ldcg(a.err2 + tile * TR + r);
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        s += __shfl_xor_sync(0xffffffffu, s, o);
+        loss += __shfl_xor_sync(0xffffffffu, loss, o);
+    }
+    if (lane == 0) s_part[warp] = make_float4(s, loss, 0.0f, 0.0f);
+    __syncthreads();
+    if (tid == 0) {
+        float t = 0.0f, l = 0.0f;
+        for (int w = 0; w < 8; ++w) t += s_part[w].x, l += s_part[w].y;
+        take_gradient<ADAM>(a, OB3, t);
+        *a.loss = l;
+    }
 }
 
 }  // namespace mlp
@@ -484,39 +746,33 @@ struct rt_mlp {
     float *P = nullptr, *G = nullptr, *M1 = nullptr, *M2 = nullptr;
     __nv_bfloat16 *w1 = nullptr, *w2 = nullptr;
     int64_t adam_t = 0;
-    // workspace for batches of up to `cap` rows
+    // workspace: up to `cap` rows from the host; gradients of up to `gtiles` tiles on `sms` CTAs
     int64_t cap = 0;
-    float *x = nullptr, *t = nullptr, *y = nullptr, *dy = nullptr, *z0 = nullptr, *z1 = nullptr, *z2 = nullptr,
-          *d0 = nullptr, *d1 = nullptr, *d2 = nullptr, *loss = nullptr;
-    __nv_bfloat16 *h1 = nullptr, *h2 = nullptr, *h3 = nullptr, *d1h = nullptr, *d2h = nullptr;
+    float *x = nullptr, *t = nullptr, *y = nullptr, *loss = nullptr;
+    float *part = nullptr, *dy = nullptr, *xb = nullptr, *err2 = nullptr;
+    float4* rowvals = nullptr;
+    int64_t gtiles = 0;
+    int sms = 0;
     float *X = nullptr, *T = nullptr;
     int64_t rows = 0;
-    int* err = nullptr;  // device: set when a GEMM's bounded wait gave up
+    int* err = nullptr;  // device: set when a bounded wait gave up
 };
 
 namespace {
 
 void free_ws(rt_mlp* m) {
-    void* ps[] = {m->x, m->t, m->y, m->dy, m->z0, m->z1, m->z2, m->d0, m->d1, m->d2, m->h1, m->h2, m->h3, m->d1h, m->d2h};
+    void* ps[] = {m->x, m->t, m->y};
     for (void* p : ps)
         if (p) cudaFree(p);
-    m->x = m->t = m->y = m->dy = m->z0 = m->z1 = m->z2 = m->d0 = m->d1 = m->d2 = nullptr;
-    m->h1 = m->h2 = m->h3 = m->d1h = m->d2h = nullptr;
+    m->x = m->t = m->y = nullptr;
     m->cap = 0;
 }
 
 bool reserve(rt_mlp* m, int64_t n) {
     if (n <= m->cap) return true;
     free_ws(m);
-    const size_t nh = (size_t)n * H;
     bool ok = cudaMalloc(&m->x, (size_t)n * IN * 4) == cudaSuccess && cudaMalloc(&m->t, (size_t)n * 4) == cudaSuccess &&
-              cudaMalloc(&m->y, (size_t)n * 4) == cudaSuccess && cudaMalloc(&m->dy, (size_t)n * 4) == cudaSuccess &&
-              cudaMalloc(&m->z0, nh * 4) == cudaSuccess && cudaMalloc(&m->z1, nh * 4) == cudaSuccess &&
-              cudaMalloc(&m->z2, nh * 4) == cudaSuccess && cudaMalloc(&m->d0, nh * 4) == cudaSuccess &&
-              cudaMalloc(&m->d1, nh * 4) == cudaSuccess && cudaMalloc(&m->d2, nh * 4) == cudaSuccess &&
-              cudaMalloc(&m->h1, nh * 2) == cudaSuccess && cudaMalloc(&m->h2, nh * 2) == cudaSuccess &&
-              cudaMalloc(&m->h3, nh * 2) == cudaSuccess && cudaMalloc(&m->d1h, nh * 2) == cudaSuccess &&
-              cudaMalloc(&m->d2h, nh * 2) == cudaSuccess;
+              cudaMalloc(&m->y, (size_t)n * 4) == cudaSuccess;
     if (!ok) {
         free_ws(m);
         return false;
@@ -525,81 +781,111 @@ bool reserve(rt_mlp* m, int64_t n) {
     return true;
 }
 
-GemmArgs gemm(Op A, Op B, int M, int N, int K, int epi) {
-    GemmArgs g;
+NetArgs net_args(const rt_mlp* m, int n) {
+    NetArgs g;
     std::memset(&g, 0, sizeof g);
-    g.A = A;
-    g.B = B;
-    g.M = M;
-    g.N = N;
-    g.K = K;
-    g.ksplit = K;
-    g.epi = epi;
+    g.P = m->P;
+    g.w1 = m->w1;
+    g.w2 = m->w2;
+    g.x = m->x;
+    g.t = m->t;
+    g.n = n;
+    g.y = m->y;
+    g.err = m->err;
     return g;
 }
 
-// N is always the hidden width (128 = one tile); M rows in tiles of 128, K
-// split over blockIdx.z for the weight gradients.
-void launch_gemm(rt_mlp* m, GemmArgs g, int splits, cudaStream_t s) {
-    g.err = m->err;
-    dim3 grid(1, (g.M + TBM - 1) / TBM, splits);
-    gemm_tc<<<grid, 128, 0, s>>>(g);
+// Predictions of the n rows in m->x into m->y: two CTAs a SM.
+void forward(rt_mlp* m, int n) {
+    const int tiles = (n + TR - 1) / TR;
+    net_kernel<false, kFwdThreads><<<std::min(tiles, 2 * m->sms), kFwdThreads, net_smem(false), m->s>>>(net_args(m, n));
 }
 
-// Forward pass of the n rows in m->x; with `with_target`, also the loss and
-// dy.  Returns y in m->y.
-void forward(rt_mlp* m, int n, bool with_target) {
-    cudaStream_t s = m->s;
-    const int nh = n * H;
-    layer0_fwd<<<(nh + 255) / 256, 256, 0, s>>>(m->x, m->P, n, m->z0, m->h1);
-    // z1 = h1 W1^T + b1: A = h1 [n][H], B(k, o) = W1[o][k] -> (w1, H, trans)
-    GemmArgs g = gemm(Op{m->h1, H, 0}, Op{m->w1, H, 1}, n, H, H, EPI_FWD);
-    g.bias = m->P + OB1;
-    g.out_f = m->z1;
-    g.out_h = m->h2;
-    launch_gemm(m, g, 1, s);
-    g = gemm(Op{m->h2, H, 0}, Op{m->w2, H, 1}, n, H, H, EPI_FWD);
-    g.bias = m->P + OB2;
-    g.out_f = m->z2;
-    g.out_h = m->h3;
-    launch_gemm(m, g, 1, s);
-    if (with_target) cudaMemsetAsync(m->loss, 0, 4, s);
-    layer3_fwd<<<(n + 7) / 8, 256, 0, s>>>(m->h3, m->P, n, m->y, with_target ? m->t : nullptr, m->dy, m->loss);
+// Rows of a range: 256, or less where that evens out the ranges (a multiple of 64).
+int range_rows(int n) {
+    const int ranges = (n + 255) / 256;
+    return ((n + ranges - 1) / ranges + 63) / 64 * 64;
 }
 
-// Gradient of the loss over the batch in m->x / m->t into m->G (zeroed here).
-void backward(rt_mlp* m, int n) {
-    cudaStream_t s = m->s;
-    const int nh = n * H;
-    cudaMemsetAsync(m->G, 0, NPARAM * 4, s);
-    layer3_wgrad<<<H + 1, 256, 0, s>>>(m->h3, m->dy, n, m->G);
-    layer3_bwd<<<(nh + 255) / 256, 256, 0, s>>>(m->z2, m->dy, m->P, n, m->d2, m->d2h);
-    const int splits = (n + 255) / 256;  // weight-gradient GEMMs: K = rows, 256 per CTA
-    const int ks = ((n + splits - 1) / splits + TBK - 1) / TBK * TBK;
-    // dW2 = dz2^T h2: A(o, r) = dz2[r][o] -> (d2h, H, trans); B(r, k) = h2[r][k]
-    GemmArgs g = gemm(Op{m->d2h, H, 1}, Op{m->h2, H, 0}, H, H, n, EPI_ATOMIC);
-    g.ksplit = ks;
-    g.out_f = m->G + OW2;
-    launch_gemm(m, g, splits, s);
-    bias_grad<<<H, 256, 0, s>>>(m->d2, n, m->G, OB2);
-    // dz1 = (dz2 W2) * gelu'(z1): A = dz2 [n][H], B(o, k) = W2[o][k]
-    g = gemm(Op{m->d2h, H, 0}, Op{m->w2, H, 0}, n, H, H, EPI_DGELU);
-    g.zin = m->z1;
-    g.out_f = m->d1;
-    g.out_h = m->d1h;
-    launch_gemm(m, g, 1, s);
-    g = gemm(Op{m->d1h, H, 1}, Op{m->h1, H, 0}, H, H, n, EPI_ATOMIC);
-    g.ksplit = ks;
-    g.out_f = m->G + OW1;
-    launch_gemm(m, g, splits, s);
-    bias_grad<<<H, 256, 0, s>>>(m->d1, n, m->G, OB1);
-    g = gemm(Op{m->d1h, H, 0}, Op{m->w1, H, 0}, n, H, H, EPI_DGELU);
-    g.zin = m->z0;
-    g.out_f = m->d0;
-    g.out_h = m->h3;  // scratch: the BF16 copy of dz0 is not needed
-    launch_gemm(m, g, 1, s);
-    layer0_wgrad<<<H, 256, 0, s>>>(m->d0, m->x, n, m->G);
-    bias_grad<<<H, 256, 0, s>>>(m->d0, n, m->G, OB0);
+void free_gradient_ws(rt_mlp* m) {
+    void* ps[] = {m->part, m->dy, m->xb, m->err2, m->rowvals};
+    for (void* p : ps)
+        if (p) cudaFree(p);
+    m->part = m->dy = m->xb = m->err2 = nullptr;
+    m->rowvals = nullptr;
+    m->gtiles = 0;
+}
+
+bool reserve_gradient(rt_mlp* m, int n) {
+    const int range = range_rows(n);
+    const int64_t tiles = 2 * (((int64_t)n + range - 1) / range);
+    if (tiles <= m->gtiles) return true;
+    free_gradient_ws(m);
+    const size_t rows = (size_t)tiles * TR;
+    const bool ok = cudaMalloc(&m->part, (size_t)m->sms * kPart * 4) == cudaSuccess &&
+                    cudaMalloc(&m->dy, rows * 4) == cudaSuccess && cudaMalloc(&m->err2, rows * 4) == cudaSuccess &&
+                    cudaMalloc(&m->xb, rows * IN * 4) == cudaSuccess &&
+                    cudaMalloc(&m->rowvals, rows * kRowArrays * H * 4) == cudaSuccess;
+    if (!ok) {
+        free_gradient_ws(m);
+        cudaGetLastError();
+        return false;
+    }
+    m->gtiles = tiles;
+    return true;
+}
+
+// Loss and gradient of g's rows: into m->G and m->loss, or an Adam step.
+void gradient(rt_mlp* m, NetArgs g, bool adam, float lr, float b1t, float b2t) {
+    g.range = range_rows(g.n);
+    const int ranges = (g.n + g.range - 1) / g.range, pairs = std::min(ranges, m->sms / 2);
+    g.chain = ranges == pairs;
+    g.part = m->part;
+    g.rows = m->rowvals;
+    g.row_array = m->gtiles * TR * (H / 4);
+    g.dy = m->dy;
+    g.xb = m->xb;
+    g.err2 = m->err2;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(2 * pairs));
+    cfg.blockDim = dim3(kGradThreads);
+    cfg.dynamicSmemBytes = net_smem(true);
+    cfg.stream = m->s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, net_kernel<true, kGradThreads>, g);
+    SumArgs a;
+    std::memset(&a, 0, sizeof a);
+    a.part = m->part;
+    a.parts = g.chain ? pairs : 2 * pairs;  // a chain's sum is its second CTA's
+    a.part_first = g.chain ? 1 : 0;
+    a.part_step = g.chain ? 2 : 1;
+    a.rows = g.rows;
+    a.row_array = g.row_array;
+    a.dy = g.dy;
+    a.xb = g.xb;
+    a.err2 = g.err2;
+    a.n = g.n;
+    a.range = g.range;
+    a.P = m->P;
+    a.M1 = m->M1;
+    a.M2 = m->M2;
+    a.G = m->G;
+    a.loss = m->loss;
+    a.w1 = m->w1;
+    a.w2 = m->w2;
+    a.lr = lr;
+    a.b1t = b1t;
+    a.b2t = b2t;
+    if (adam)
+        sum_kernel<true><<<kSumBlocks, 256, kSumSmem, m->s>>>(a);
+    else
+        sum_kernel<false><<<kSumBlocks, 256, kSumSmem, m->s>>>(a);
 }
 
 rt_status sync(rt_mlp* m) {
@@ -625,7 +911,16 @@ rt_status rt_mlp_create(int32_t device, uint64_t seed, rt_mlp** out) {
                   cudaMalloc(&m->M1, NPARAM * 4) == cudaSuccess && cudaMalloc(&m->M2, NPARAM * 4) == cudaSuccess &&
                   cudaMalloc(&m->w1, H * H * 2) == cudaSuccess && cudaMalloc(&m->w2, H * H * 2) == cudaSuccess &&
                   cudaMalloc(&m->loss, 4) == cudaSuccess && cudaMalloc(&m->err, sizeof(int)) == cudaSuccess &&
-                  cudaMemset(m->err, 0, sizeof(int)) == cudaSuccess;
+                  cudaMemset(m->err, 0, sizeof(int)) == cudaSuccess &&
+                  cudaDeviceGetAttribute(&m->sms, cudaDevAttrMultiProcessorCount, device) == cudaSuccess &&
+                  cudaFuncSetAttribute((const void*)net_kernel<false, kFwdThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)net_smem(false)) == cudaSuccess &&
+                  cudaFuncSetAttribute((const void*)net_kernel<true, kGradThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)net_smem(true)) == cudaSuccess &&
+                  cudaFuncSetAttribute((const void*)sum_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       kSumSmem) == cudaSuccess &&
+                  cudaFuncSetAttribute((const void*)sum_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       kSumSmem) == cudaSuccess;
         if (!ok) {
             rt_mlp_destroy(m);
             return RT_E_NOMEM;
@@ -654,6 +949,7 @@ rt_status rt_mlp_destroy(rt_mlp* m) {
         cudaSetDevice(m->device);
         if (m->s) cudaStreamSynchronize(m->s);
         free_ws(m);
+        free_gradient_ws(m);
         void* ps[] = {m->P, m->G, m->M1, m->M2, m->w1, m->w2, m->loss, m->X, m->T, m->err};
         for (void* p : ps)
             if (p) cudaFree(p);
@@ -694,7 +990,7 @@ rt_status rt_mlp_predict(rt_mlp* m, const float* x, int64_t n, float* y) {
             const int rn = (int)std::min<int64_t>(chunk, n - r0);
             if (!reserve(m, rn)) return RT_E_NOMEM;
             cudaMemcpyAsync(m->x, x + r0 * IN, (size_t)rn * IN * 4, cudaMemcpyHostToDevice, m->s);
-            forward(m, rn, false);
+            forward(m, rn);
             cudaMemcpyAsync(y + r0, m->y, (size_t)rn * 4, cudaMemcpyDeviceToHost, m->s);
             rt_status st = sync(m);
             if (st != RT_OK) return st;
@@ -707,11 +1003,10 @@ rt_status rt_mlp_loss_grad(rt_mlp* m, const float* x, const float* target, int64
     return guarded([&]() -> rt_status {
         if (!m || !x || !target || n <= 0 || n > (1 << 22)) return RT_E_INVAL;
         cudaSetDevice(m->device);
-        if (!reserve(m, n)) return RT_E_NOMEM;
+        if (!reserve(m, n) || !reserve_gradient(m, (int)n)) return RT_E_NOMEM;
         cudaMemcpyAsync(m->x, x, (size_t)n * IN * 4, cudaMemcpyHostToDevice, m->s);
         cudaMemcpyAsync(m->t, target, (size_t)n * 4, cudaMemcpyHostToDevice, m->s);
-        forward(m, (int)n, true);
-        backward(m, (int)n);
+        gradient(m, net_args(m, (int)n), false, 0.0f, 0.0f, 0.0f);
         if (loss) cudaMemcpyAsync(loss, m->loss, 4, cudaMemcpyDeviceToHost, m->s);
         if (grad) cudaMemcpyAsync(grad, m->G, NPARAM * 4, cudaMemcpyDeviceToHost, m->s);
         return sync(m);
@@ -749,15 +1044,16 @@ rt_status rt_mlp_train(rt_mlp* m, int64_t steps, int32_t batch, float lr, uint64
     return guarded([&]() -> rt_status {
         if (!m || steps < 0 || batch <= 0 || batch > (1 << 22) || !m->X || !m->T || m->rows <= 0) return RT_E_INVAL;
         cudaSetDevice(m->device);
-        if (!reserve(m, batch)) return RT_E_NOMEM;
+        if (!reserve_gradient(m, batch)) return RT_E_NOMEM;
+        NetArgs g = net_args(m, batch);
+        g.x = m->X;
+        g.t = m->T;
+        g.pool = m->rows;
+        g.seed = seed;
         for (int64_t k = 0; k < steps; ++k) {
-            gather_batch<<<(batch + 255) / 256, 256, 0, m->s>>>(m->X, m->T, m->rows, batch, seed, m->adam_t, m->x, m->t);
-            forward(m, batch, true);
-            backward(m, batch);
-            ++m->adam_t;
+            g.step = m->adam_t++;
             const float b1t = std::pow(0.9f, (float)m->adam_t), b2t = std::pow(0.999f, (float)m->adam_t);
-            adam<<<(NPARAM + 255) / 256, 256, 0, m->s>>>(m->P, m->G, m->M1, m->M2, NPARAM, lr, b1t, b2t);
-            to_bf16<<<(H * H + 255) / 256, 256, 0, m->s>>>(m->P, m->w1, m->w2);
+            gradient(m, g, true, lr, b1t, b2t);
         }
         if (loss) cudaMemcpyAsync(loss, m->loss, 4, cudaMemcpyDeviceToHost, m->s);
         return sync(m);
