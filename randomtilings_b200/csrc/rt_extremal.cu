@@ -28,6 +28,7 @@
 #include <vector>
 
 #include "../../include/rt_b200_extremal.h"
+#include "rt_domain.cuh"
 #include "rt_internal.h"
 #include "rt_guard.h"
 
@@ -53,41 +54,14 @@ __constant__ int c_ddi[4] = {1, -1, 0, 0};
 __constant__ int c_ddj[4] = {0, 0, 1, -1};
 __constant__ int c_dbit[4] = {2, 1, 8, 4};
 
-__device__ __forceinline__ int dface(const int32_t* __restrict__ d, int m, int i, int j) {
-    return (i >= 0 && j >= 0 && i < m && j < m) ? d[(int64_t)i * m + j] : 0;
-}
-__device__ __forceinline__ int lface(const int32_t* __restrict__ d, int m, int r, int c) {
-    return (r >= 0 && c >= 0 && r < m && c < 2 * m) ? d[(int64_t)r * 2 * m + c] : 0;
-}
-
-// Vertex kinds (DomainToVertices, DominoTiler.cpp:479-506,
-// LozengeTiler.cpp:405-430) and the initial heights.
+// Vertex kinds and the initial heights.
 template <bool DOM>
 __global__ void ext_classify(const int32_t* __restrict__ d, int m, uint8_t* kind, int32_t* hx, int32_t* hn) {
     const int n = m + 1;
     const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= (int64_t)n * n) return;
     const int i = (int)(v / n), j = (int)(v % n);
-    int k;
-    if (DOM) {
-        if (i == 0 || j == 0 || i == m || j == m) {
-            const int i0 = i - (i == m), i1 = i - 1 + (i == 0), j0 = j - (j == m), j1 = j - 1 + (j == 0);
-            k = (dface(d, m, i0, j0) || dface(d, m, i1, j0) || dface(d, m, i0, j1) || dface(d, m, i1, j1)) ? 2 : 0;
-        } else {
-            const int s = (dface(d, m, i - 1, j - 1) != 0) + (dface(d, m, i - 1, j) != 0) +
-                          (dface(d, m, i, j - 1) != 0) + (dface(d, m, i, j) != 0);
-            k = s == 4 ? 1 : s > 0 ? 2 : 0;
-        }
-    } else {
-        k = 0;
-        if (i >= 1 && j >= 1 && i < m && j < m) {
-            const int s = (lface(d, m, i, 2 * j) != 0) + (lface(d, m, i, 2 * j - 1) != 0) +
-                          (lface(d, m, i, 2 * j - 2) != 0) + (lface(d, m, i - 1, 2 * j) != 0) +
-                          (lface(d, m, i - 1, 2 * j + 1) != 0) + (lface(d, m, i - 1, 2 * j - 1) != 0);
-            k = s == 6 ? 1 : s > 0 ? 2 : 0;
-        }
-    }
-    kind[v] = (uint8_t)k;
+    kind[v] = (uint8_t)vertex_kind<DOM>(d, m, i, j);
     hx[v] = kBig;
     hn[v] = -kBig;
 }

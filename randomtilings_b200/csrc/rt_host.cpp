@@ -1055,6 +1055,15 @@ namespace rtb {
 // direction whose edge touches the domain with both ends inside it.
 // Directions: dominoes (i+1, j), (i-1, j), (i, j+1), (i, j-1); lozenges
 // (i, j+1), (i-1, j+1), (i-1, j), (i, j-1), (i+1, j-1), (i+1, j).
+int domain_side(int model, int64_t dlen) {
+    if (model == RT_DOMINO) {
+        const int m = isqrt_exact(dlen);
+        return m < 1 ? -1 : m;
+    }
+    const int m = isqrt_exact(dlen / 2);
+    return m < 2 || (int64_t)2 * m * m != dlen ? -1 : m;
+}
+
 bool lipschitz_graph(int model, const int32_t* d, int64_t dlen, int* n_out, std::vector<uint8_t>* kind,
                      std::vector<uint8_t>* edges) {
     if (!d) return false;

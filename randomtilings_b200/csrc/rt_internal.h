@@ -89,8 +89,12 @@ uint32_t below_threshold(double x);
 // Integer acceptance thresholds of a kernel family on the 23-bit draw.
 void family_thresholds(int family, double q, int qcmp, uint32_t thr[4]);
 
+// Faces M of a side of a domain of `dlen` entries (dominoes M x M, lozenges M
+// x 2M), -1 if there is no such domain (rt_host.cpp).
+int domain_side(int model, int64_t dlen);
+
 // Vertex kinds and in-domain edge bits of a domino / lozenge domain
-// (rt_host.cpp), the graph of the height-function projection.
+// (rt_host.cpp), the graph of the height plans.
 bool lipschitz_graph(int model, const int32_t* d, int64_t dlen, int* n_out, std::vector<uint8_t>* kind,
                      std::vector<uint8_t>* edges);
 
