@@ -25,8 +25,7 @@
 #include "rt_internal.h"
 #include "rt_guard.h"
 #include "rt_models.cuh"
-#include "rt_tdplane.cuh"
-#include "rt_tridimer.cuh"
+#include "rt_tdwalk.cuh"
 #include "rt_word.cuh"
 
 using rtb::guarded;
@@ -310,53 +309,9 @@ __global__ void __launch_bounds__(1024, 1) batch_site_kernel(const __grid_consta
     }
 }
 
-// One phase of op OP over the band rows [r0, r0 + nrows) of a triangle-dimer
-// chain held as bit planes: only the rows TriDimerRule::live_rows admits, one
-// 32-site word per work item.  Drawing ops take the fast mode's draws: quad
-// cq of array row r is Philox4x32-10 of (r Gw + cq, step, chain), and a site
-// flips when its output word is below 2^31 (k = word >> 9 below 2^22).
-template <uint32_t OP, int T, int B = -1>
-__device__ __forceinline__ void tdp_phase(uint32_t* planes, int ps, int rs, int row0, uint32_t a, uint32_t b, int m,
-                                          int width, int r0, int nrows, int wb, int tid, int BLOCK, int64_t dstep,
-                                          uint32_t chain, uint32_t key0, uint32_t key1) {
-    constexpr bool DRAWS = OP == TD_ROT_LOZ || OP == TD_ROT_TRI || OP == TD_ROT_BFLY;
-    int S, o;
-    TriDimerRule::live_rows<OP>(a, b, &S, &o);
-    const int first = r0 + ((o - r0) % S + S) % S;
-    if (first >= r0 + nrows) return;
-    const int nlive = (r0 + nrows - first + S - 1) / S;
-    const int items = nlive * wb;
-    const int Gw = (width + 3) >> 2;
-    for (int u = tid; u < items; u += BLOCK) {
-        const int rr = u / wb, c = u - rr * wb;
-        const int r = first + S * rr;
-        uint32_t draw = 0u;
-        if (DRAWS) {
-#pragma unroll
-            for (int q = 0; q < 8; ++q) {
-                const int cq = 8 * c + q;
-                if (cq < Gw) {
-                    const uint4 w4 = philox4((uint32_t)(r * Gw + cq), (uint32_t)dstep, (uint32_t)((uint64_t)dstep >> 32),
-                                             chain, key0, key1);
-                    draw |= ((~w4.x >> 31) | ((~w4.y >> 31) << 1) | ((~w4.z >> 31) << 2) | ((~w4.w >> 31) << 3))
-                            << (4 * q);
-                }
-            }
-        }
-        const tdp::View v{planes, ps, rs, row0, r, c};
-        tdp::word_op<OP, T, B>(v, a, b, m, width, draw);
-    }
-}
-
-// ---------------------------------------------------------------------------
-// Triangle dimers: the eight arrays as 51 bit planes (rt_tdplane.cuh), 32
-// sites per word.  Shared memory: one zero word, then per plane (rpc + 2)
-// rows of wb + 1 words (the last word of a row stays zero), wb = words per
-// array row.  Rows move between global int32 arrays and planes one warp per
-// 32 columns, with a ballot per bit.
-// ---------------------------------------------------------------------------
+// Triangle dimers: the eight arrays as bit planes, 32 sites per word
+// (rt_tdwalk.cuh), through the phases of the schedule (rt_tdschedule.h).
 __global__ void __launch_bounds__(512, 1) batch_td_kernel(const __grid_constant__ BatchArgs b) {
-    using R = TriDimerRule;
     cg::cluster_group cluster = cg::this_cluster();
     const int CL = (int)cluster.num_blocks();
     const int rank = (int)cluster.block_rank();
@@ -369,115 +324,23 @@ __global__ void __launch_bounds__(512, 1) batch_td_kernel(const __grid_constant_
 
     for (int q = cid; q < b.nchains; q += ncl) {
         const BatchChain& ch = b.chains[b.order[q]];
-        const int rows = ch.rows, width = ch.width;
-        const int rpc = (rows + CL - 1) / CL;
-        const int r0 = min(rows, rank * rpc), r1 = min(rows, r0 + rpc);
-        const int nrows = r1 - r0;
-        const int wb = (width + 31) >> 5, rs = wb + 1, ps = (rpc + 2) * rs;
-        uint32_t* planes = sm + 1;
-        for (int e = tid; e < 1 + tdp::kPlanes * ps; e += BLOCK) sm[e] = 0u;
+        TdBand band(sm, ch.rows, ch.width, ch.n / 2, rank, CL, td_halo_cap(true), tid, BLOCK);
+        for (int e = tid; e < (int)td_band_words(ch.rows, ch.width, band.ctas, td_halo_cap(true)); e += BLOCK) sm[e] = 0u;
         __syncthreads();
-        // global int32 rows r0 - 1 .. r1 -> planes
-        for (int it = warp; it < (nrows + 2) * 8 * wb; it += nwarps) {
-            const int sr = it / (8 * wb), rem = it - sr * 8 * wb, arr = rem / wb, c = rem - arr * wb;
-            const int rr = r0 - 1 + sr, j = 32 * c + lane;
-            int32_t v = 0;
-            if (rr >= 0 && rr < ch.arows && j < width) v = static_cast<const int32_t*>(ch.arr[arr])[(size_t)rr * width + j];
-            for (int k = 0; k < tdp::bits_of(arr); ++k) {
-                const uint32_t w = __ballot_sync(0xffffffffu, (v >> k) & 1);
-                if (lane == 0) planes[(tdp::plane_of(arr) + k) * ps + sr * rs + c] = w;
-            }
-        }
+        td_load(band, ch.arr, ch.arows, warp, nwarps, lane);
         __syncthreads();
 
-        const uint32_t key0 = (uint32_t)ch.key, key1 = (uint32_t)(ch.key >> 32);
-        const int m = ch.n / 2, row0 = r0 - 1;
-        int64_t dstep = *b.step0 + b.step_add;
+        TdPhilox draw{(ch.width + 3) >> 2, *b.step0 + b.step_add, ch.chain, (uint32_t)ch.key, (uint32_t)(ch.key >> 32)};
+        uint32_t d = b.nphases > 0 ? __ldg(b.phases) : 0u;
         for (int64_t ph = 0; ph < b.nphases; ++ph) {
-            const uint32_t d = __ldg(b.phases + ph);
-            const bool draws = (d & PH_DRAWS) != 0u;
-            const uint32_t op = ph_op(d), pa = ph_a(d), pb = ph_b(d);
-#define RT_TDP_ARGS planes, ps, rs, row0, pa, pb, m, width, r0, nrows, wb, tid, BLOCK, dstep, ch.chain, key0, key1
-            switch (op) {
-#define RT_TD_PHASE(OPC)                           \
-    case OPC:                                      \
-        if (pa == 0)                               \
-            tdp_phase<OPC, 0>(RT_TDP_ARGS);        \
-        else if (pa == 1)                          \
-            tdp_phase<OPC, 1>(RT_TDP_ARGS);        \
-        else                                       \
-            tdp_phase<OPC, 2>(RT_TDP_ARGS);        \
-        break;
-                RT_TD_PHASE(TD_ROT_LOZ)
-                RT_TD_PHASE(TD_LOZ_FLIPPED)
-                RT_TD_PHASE(TD_LOZ_OTHER)
-                RT_TD_PHASE(TD_UP_FROM_LOZ)
-                case TD_TRI_OTHER:  // (a, b) in {(0, 7), (0, 0), (1, 0)} in the phase program
-                    if (pa == 0 && pb == 7)
-                        tdp_phase<TD_TRI_OTHER, 0, 7>(RT_TDP_ARGS);
-                    else if (pa == 0 && pb == 0)
-                        tdp_phase<TD_TRI_OTHER, 0, 0>(RT_TDP_ARGS);
-                    else if (pa == 1 && pb == 0)
-                        tdp_phase<TD_TRI_OTHER, 1, 0>(RT_TDP_ARGS);
-                    else
-                        tdp_phase<TD_TRI_OTHER, -1>(RT_TDP_ARGS);
-                    break;
-                RT_TD_PHASE(TD_ROT_TRI)
-                RT_TD_PHASE(TD_TRI_FLIPPED)
-                RT_TD_PHASE(TD_LOZ_FROM_TRI)
-                case TD_BFLY_FROM_LOZ:  // (a, b) in {(0, 7), (1, 3), (1, 5), (1, 6)}
-                    if (pa == 0 && pb == 7)
-                        tdp_phase<TD_BFLY_FROM_LOZ, 0, 7>(RT_TDP_ARGS);
-                    else if (pa == 1 && pb == 3)
-                        tdp_phase<TD_BFLY_FROM_LOZ, 1, 3>(RT_TDP_ARGS);
-                    else if (pa == 1 && pb == 5)
-                        tdp_phase<TD_BFLY_FROM_LOZ, 1, 5>(RT_TDP_ARGS);
-                    else if (pa == 1 && pb == 6)
-                        tdp_phase<TD_BFLY_FROM_LOZ, 1, 6>(RT_TDP_ARGS);
-                    else
-                        tdp_phase<TD_BFLY_FROM_LOZ, -1>(RT_TDP_ARGS);
-                    break;
-                RT_TD_PHASE(TD_ROT_BFLY)
-                RT_TD_PHASE(TD_BFLY_SAME)
-                RT_TD_PHASE(TD_BFLY_21)
-                RT_TD_PHASE(TD_BFLY_22)
-                RT_TD_PHASE(TD_BFLY_23_LOZ)
-#undef RT_TD_PHASE
-#undef RT_TDP_ARGS
-                default: break;
-            }
-            if (draws) ++dstep;
-            if (CL > 1) {
-                cluster.sync();
-                uint32_t mask = R::written(d);
-                if (nrows > 0) {
-                    while (mask) {
-                        const int arr = __ffs(mask) - 1;
-                        mask &= mask - 1;
-                        const int nb = tdp::bits_of(arr), p0 = tdp::plane_of(arr);
-                        for (int e = tid; e < 2 * nb * wb; e += BLOCK) {
-                            const int side = e >= nb * wb, rem = e - side * nb * wb, k = rem / wb, c = rem - k * wb;
-                            if ((side == 0 && rank == 0) || (side == 1 && r1 >= rows)) continue;
-                            const int mine = (p0 + k) * ps + (side == 0 ? 0 : nrows + 1) * rs + c;
-                            const int theirs = (p0 + k) * ps + (side == 0 ? rpc : 1) * rs + c;
-                            planes[mine] = *cluster.map_shared_rank(planes + theirs, rank + (side == 0 ? -1 : 1));
-                        }
-                    }
-                }
-                cluster.sync();
-            } else {
-                __syncthreads();
-            }
+            const uint32_t d_next = ph + 1 < b.nphases ? __ldg(b.phases + ph + 1) : 0u;
+            if (band.ctas > 1 && band.depth < td_reach(d)) band.exchange(cluster);
+            td_phase(d, band, draw);
+            if (d & PH_DRAWS) ++draw.step;
+            __syncthreads();
+            d = d_next;
         }
-        // planes -> global int32 rows r0 .. r1 - 1
-        for (int it = warp; it < nrows * 8 * wb; it += nwarps) {
-            const int sr = 1 + it / (8 * wb), rem = it - (sr - 1) * 8 * wb, arr = rem / wb, c = rem - arr * wb;
-            const int j = 32 * c + lane;
-            int32_t v = 0;
-            for (int k = 0; k < tdp::bits_of(arr); ++k)
-                v |= (int32_t)((planes[(tdp::plane_of(arr) + k) * ps + sr * rs + c] >> lane) & 1u) << k;
-            if (j < width) static_cast<int32_t*>(ch.arr[arr])[(size_t)(r0 - 1 + sr) * width + j] = v;
-        }
+        td_store(band, ch.arr, warp, nwarps, lane);
         cluster_or_block_sync(cluster, CL);
     }
 }
@@ -569,10 +432,7 @@ size_t smem_for(const Chain& c, int cl) {
     if (word_fam(c.fam)) {
         return 16 + (size_t)c.ncol * (rpc + 2) * wpad + 16 + (size_t)((2 * rpc + 3) & ~3) + 2 * 4 * (size_t)(wpad / 4);
     }
-    if (c.fam == FAM_TRIDIMER) {  // batch_td_kernel: one zero word, then 51 planes of (rpc + 2) x (wb + 1) words
-        const size_t wb = (size_t)(c.width + 31) / 32;
-        return 4 * (1 + (size_t)tdp::kPlanes * (rpc + 2) * (wb + 1));
-    }
+    if (c.fam == FAM_TRIDIMER) return 4 * td_band_words(c.rows, c.width, std::min(cl, c.rows), td_halo_cap(true));
     return (size_t)c.ncol * (rpc + 2) * wpad * 4;
 }
 
@@ -774,11 +634,11 @@ rt_status upload(rt_batch* b) {
             if (c.kind == 3) {
                 std::vector<int32_t> arrays((size_t)8 * c.arows * c.width);
                 td_split_host(c.start.data(), c.n, arrays.data());
-                // batch_td_kernel keeps array a as tdp::bits_of(a) bit planes
+                // dimer covers only
                 const size_t per = (size_t)c.arows * c.width;
                 for (size_t e = 0; e < 8 * per; ++e) {
                     const int32_t v = arrays[e];
-                    if (v < 0 || v >= (1 << tdp::bits_of((int)(e / per))))
+                    if (v < 0 || v >= (1 << tdp::cover_bits_of((int)(e / per))))
                         return b->fail(RT_E_INVAL, "triangle-dimer state out of range for the bit planes");
                 }
                 for (int a = 0; a < 8; ++a)

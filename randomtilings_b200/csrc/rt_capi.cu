@@ -21,6 +21,8 @@
 #include "rt_internal.h"
 #include "rt_guard.h"
 #include "rt_models.cuh"
+#include "rt_tdplane.cuh"
+#include "rt_tdschedule.h"
 #include "rt_tridimer.cuh"
 
 using rtb::guarded;
@@ -88,44 +90,15 @@ uint32_t below_threshold(double x) {
     return (uint32_t)s;
 }
 
-// Phases of one triangle-dimer step (TriangleDimerTiler.cpp:243-347): the
-// flip family `kind` (0 lozenges, 1 triangles, 2 butterflies), orientation /
-// class r1, kind or parity r2, and for butterflies the slice p1 and parity p2.
-int64_t td_step_phases(uint32_t* ph, int64_t at, uint32_t kind, uint32_t r1, uint32_t r2, uint32_t p1, uint32_t p2) {
-    if (kind == 0) {  // lozenge flips, :243-278
-        ph[at++] = make_phase(TD_ROT_LOZ, r1, r2, true);
-        ph[at++] = make_phase(TD_LOZ_FLIPPED, r1, r2, false);
-        ph[at++] = make_phase(TD_LOZ_OTHER, r1, 0, false);
-        ph[at++] = make_phase(TD_UP_FROM_LOZ, 0, 0, false);
-        ph[at++] = make_phase(TD_TRI_OTHER, 0, 7, false);
-    } else if (kind == 1) {  // triangle flips, :279-305
-        ph[at++] = make_phase(TD_ROT_TRI, r2, r1, true);
-        ph[at++] = make_phase(TD_TRI_FLIPPED, r2, r1, false);
-        ph[at++] = make_phase(TD_TRI_OTHER, r2, 0, false);
-        ph[at++] = make_phase(TD_LOZ_FROM_TRI, 0, 0, false);
-        ph[at++] = make_phase(TD_BFLY_FROM_LOZ, 0, 7, false);
-    } else {  // butterfly flips, :306-347
-        ph[at++] = make_phase(TD_ROT_BFLY, r1, p1 | (p2 << 2), true);
-        ph[at++] = make_phase(TD_BFLY_SAME, r1, p1 | (p2 << 2), false);
-        ph[at++] = make_phase(TD_BFLY_21, r1, p1, false);
-        ph[at++] = make_phase(TD_BFLY_22, r1, p1, false);
-        ph[at++] = make_phase(TD_BFLY_23_LOZ, r1, p1, false);
-        ph[at++] = make_phase(TD_BFLY_FROM_LOZ, 1, 7u & ~(1u << r1), false);
-        ph[at++] = make_phase(TD_TRI_OTHER, 0, 0, false);
-    }
-    return at;
-}
-
 // Fast-mode step s of an epoch: dominoes flip the black array (0) on even
 // steps and the white one on odd steps (reference colour r flips array
 // 1 - r); lozenges and rectangle-triangles flip colour s mod 3; triangle
 // dimers make move s mod 30 of a sweep over every flip class.
-int64_t fast_step_phases(int kind, int64_t s, uint32_t* ph, int64_t at, uint32_t* prev) {
+int64_t fast_step_phases(int kind, int64_t s, uint32_t* ph, int64_t at, uint32_t* prev, TdSchedule* td) {
     if (kind == 3) {
-        const uint32_t mv = (uint32_t)(s % 30);
-        if (mv < 6) return td_step_phases(ph, at, 0, mv / 2, mv % 2, 0, 0);
-        if (mv < 12) return td_step_phases(ph, at, 1, (mv - 6) % 3, (mv - 6) / 3, 0, 0);
-        return td_step_phases(ph, at, 2, (mv - 12) / 6, 0, ((mv - 12) / 2) % 3, (mv - 12) % 2);
+        td_fast_move(*td, (uint32_t)(s % 30),
+                     [&](uint32_t op, uint32_t a, uint32_t b, bool draws) { ph[at++] = make_phase(op, a, b, draws); });
+        return at;
     }
     const uint32_t r = kind == 0 ? (uint32_t)(1 - (s & 1)) : (uint32_t)(s % 3);
     ph[at++] = make_phase(OP_STEP, r, *prev, true);
@@ -145,22 +118,28 @@ int64_t colour_step_phase(uint32_t colour, bool merge, int64_t first, uint32_t* 
 
 void fast_phases(int kind, int64_t steps, std::vector<uint32_t>& ph) {
     const size_t base = ph.size();
-    ph.resize(base + (size_t)(kind == 3 ? 7 * steps : steps + 1));
+    ph.resize(base + (size_t)(kind == 3 ? TdSchedule::kMaxPhases * (steps + 1) : steps + 1));
     int64_t at = (int64_t)base;
     uint32_t prev = NO_COLOUR;
-    for (int64_t s = 0; s < steps; ++s) at = fast_step_phases(kind, s, ph.data(), at, &prev);
-    if (kind != 3 && steps > 0) ph[at++] = make_phase(OP_FINAL, prev, NO_COLOUR, false);
+    TdSchedule td;
+    for (int64_t s = 0; s < steps; ++s) at = fast_step_phases(kind, s, ph.data(), at, &prev, &td);
+    if (kind == 3)
+        td.flush([&](uint32_t op, uint32_t a, uint32_t b, bool draws) { ph[at++] = make_phase(op, a, b, draws); });
+    else if (steps > 0) ph[at++] = make_phase(OP_FINAL, prev, NO_COLOUR, false);
     ph.resize((size_t)at);
 }
 
 rt_status choose_plan(int family, int device, int nlat, int rows, int cols, int width, bool uniform, bool fast,
-                      bool planes, bool weighted, int kernel_choice, int ctas_hint, int depth_hint, WalkPlan* plan,
-                      std::string* err) {
+                      bool planes, bool weighted, bool td_fits, int kernel_choice, int ctas_hint, int depth_hint,
+                      WalkPlan* plan, std::string* err) {
     if (planes) return plan_plane_walk(family, device, nlat, rows, width, ctas_hint, depth_hint, plan, err);
     rt_status s = RT_E_INVAL;
     if (kernel_choice != 1 && uniform && (word_family(family) || family == FAM_QLOZENGE8))
         s = plan_word_walk(family, device, nlat, rows, width, fast, ctas_hint, plan, err, weighted);
+    if (kernel_choice == 0 && td_fits && family == FAM_TRIDIMER)
+        s = plan_td_walk(device, rows, width, fast, ctas_hint, plan, err);
     if (s == RT_OK || kernel_choice == 2) return s;
+    *plan = WalkPlan();
     return plan_walk(family, device, nlat, rows, cols, width, uniform, fast, plan, err);
 }
 
@@ -229,6 +208,8 @@ struct rt_tiler {
     int plan_rows = -1, plan_cols = -1, plan_nlat = -1;
     bool plan_uniform = true;
     bool plan_weighted = false;
+    bool plan_td_fits = false;
+    bool td_fits = false;   // triangle dimers: the uploaded arrays' values fit the bit planes
     int kernel_choice = 0;  // 0 auto, 1 generic walk kernel only, 2 word kernel only (RT_WALK_KERNEL)
     int ctas_hint = 0;      // word kernel grid (RT_WALK_CTAS; 0 = one CTA per SM)
     int depth_hint = 0;     // bit-plane kernel: phases per halo exchange (RT_PLANE_DEPTH; 0 = up to 8)
@@ -536,6 +517,11 @@ rt_status rt_upload(rt_tiler* h, const int32_t* tiling, int32_t n) {
             // (TriangleDimerTiler.cpp:90-133) and copied up as they are.
             std::vector<int32_t> arrays((size_t)8 * arows * width);
             td_split_host(tiling, n, arrays.data());
+            const size_t per = (size_t)arows * width;
+            uint32_t over = 0;
+            for (int c = 0; c < 8; ++c)
+                for (size_t e = 0; e < per; ++e) over |= (uint32_t)arrays[c * per + e] >> tdp::bits_of(c);
+            h->td_fits = over == 0;
             for (int c = 0; c < 8 && e == cudaSuccess; ++c)
                 e = cudaMemcpy(h->d_arr[0][c], arrays.data() + (size_t)c * arows * width, per_arr, cudaMemcpyHostToDevice);
             if (e != cudaSuccess) return h->cuda_fail(e, "upload of the triangle-dimer arrays");
@@ -647,19 +633,19 @@ static rt_status run_schedule(rt_tiler* h, const int64_t* steps, const int64_t* 
     // The tests' withheld row needs a neighbour to withhold it from.
     const int ctas_hint = h->drop_phase >= 0 && h->ctas_hint == 0 ? 2 : h->ctas_hint;
     if (h->plan_rows != h->rows || h->plan_cols != h->cols || h->plan_nlat != h->nlat || h->plan_uniform != uniform ||
-        h->plan_weighted != weighted) {
+        h->plan_weighted != weighted || h->plan_td_fits != h->td_fits) {
         rt_status s = choose_plan(h->family, h->cfg.device, h->nlat, h->rows, h->cols, width, uniform, fast, planes,
-                                  weighted, h->kernel_choice, ctas_hint, h->depth_hint, &h->plan, &h->err);
+                                  weighted, h->td_fits, h->kernel_choice, ctas_hint, h->depth_hint, &h->plan, &h->err);
         if (s != RT_OK) return s;
         h->plan_rows = h->rows;
         h->plan_cols = h->cols;
         h->plan_nlat = h->nlat;
         h->plan_uniform = uniform;
         h->plan_weighted = weighted;
+        h->plan_td_fits = h->td_fits;
     }
-    // At most 7 phases per triangle-dimer step; one per step + the final
-    // Update for the colour models.
-    const int64_t cap_ph = h->kind == 3 ? 7 * total : total + 1;
+    // One phase per step + the final Update for the colour models.
+    const int64_t cap_ph = h->kind == 3 ? TdSchedule::kMaxPhases * (total + 1) : total + 1;
     // The staging buffers may still feed the previous run's copies.
     cudaEventSynchronize(h->ev_staged);
     if (!h->h_phases.reserve((size_t)cap_ph * 4) || !h->d_phases.reserve((size_t)cap_ph * 4) ||
@@ -671,11 +657,13 @@ static rt_status run_schedule(rt_tiler* h, const int64_t* steps, const int64_t* 
     uint64_t* sd = static_cast<uint64_t*>(h->h_epoch_seed.p);
     int64_t at = 0;
     uint32_t prev = NO_COLOUR;
+    TdSchedule td;
+    auto emit = [&](uint32_t op, uint32_t a, uint32_t b, bool draws) { ph[at++] = make_phase(op, a, b, draws); };
     for (int e = 0; e < k; ++e) {
         es[e] = at;
         if (fast) {
             sd[e] = (uint64_t)seeds[e];
-            for (int64_t s = 0; s < steps[e]; ++s) at = fast_step_phases(h->kind, s, ph, at, &prev);
+            for (int64_t s = 0; s < steps[e]; ++s) at = fast_step_phases(h->kind, s, ph, at, &prev, &td);
         } else if (h->kind == 0) {
             std::mt19937 mt_rand(seeds[e]);
             sd[e] = single_walk ? (uint32_t)mt_rand() : (uint32_t)seeds[e];  // DominoTiler.cpp:31-32 vs :81-82
@@ -699,7 +687,12 @@ static rt_status run_schedule(rt_tiler* h, const int64_t* steps, const int64_t* 
                     p1 = (uint32_t)d1(generator);
                     p2 = (uint32_t)d2(generator);
                 }
-                at = td_step_phases(ph, at, kind, r1, r2, p1, p2);
+                if (kind == 0)
+                    td.lozenges(r1, r2, emit);
+                else if (kind == 1)
+                    td.triangles(r2, r1, emit);
+                else
+                    td.butterflies(r1, p1, p2, emit);
             }
         } else {
             std::default_random_engine generator;
@@ -712,7 +705,10 @@ static rt_status run_schedule(rt_tiler* h, const int64_t* steps, const int64_t* 
             }
         }
     }
-    if (h->kind != 3) ph[at++] = make_phase(OP_FINAL, prev, NO_COLOUR, false);
+    if (h->kind == 3)
+        td.flush(emit);
+    else
+        ph[at++] = make_phase(OP_FINAL, prev, NO_COLOUR, false);
     const int64_t nph = at;
 
     const int64_t ids = (int64_t)h->rows * h->cols;

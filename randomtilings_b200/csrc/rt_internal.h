@@ -58,6 +58,9 @@ bool word_family(int family);
 // weighted: the instantiation that reads per-site thresholds (WalkArgs::wper > 0).
 rt_status plan_word_walk(int family, int device, int nlat, int rows, int width, bool philox, int ctas_hint,
                          WalkPlan* plan, std::string* err, bool weighted = false);
+// Bit-plane kernel of a single triangle-dimer walk (rt_td.cu), for arrays whose
+// values fit its planes, on one cluster of ctas_hint CTAs (<= 0: by size).
+rt_status plan_td_walk(int device, int rows, int width, bool philox, int ctas_hint, WalkPlan* plan, std::string* err);
 // Bit-plane kernel of the int8 models (rt_plane.cu, RT_RNG_PLANES).
 // ctas_hint / depth_hint <= 0: one CTA per SM / the largest depth up to 8.
 rt_status plan_plane_walk(int family, int device, int nlat, int rows, int width, int ctas_hint, int depth_hint,
@@ -65,11 +68,13 @@ rt_status plan_plane_walk(int family, int device, int nlat, int rows, int width,
 // The kernel a walk runs on, as every walk entry point chooses it: the
 // bit-plane kernel in RT_RNG_PLANES mode; otherwise the word kernel for the
 // int8 models with uniform generator parameters (unless kernel_choice = 1),
-// falling back to the generic walk kernel for every other case and for any
-// band the word kernel cannot hold (kernel_choice = 2 forbids the fallback).
+// and the triangle dimers' bit-plane kernel for arrays whose values fit it
+// (td_fits); falling back to the generic walk kernel for every other case and
+// for any band those kernels cannot hold (kernel_choice = 2 forbids the
+// fallback).
 rt_status choose_plan(int family, int device, int nlat, int rows, int cols, int width, bool uniform, bool fast,
-                      bool planes, bool weighted, int kernel_choice, int ctas_hint, int depth_hint, WalkPlan* plan,
-                      std::string* err);
+                      bool planes, bool weighted, bool td_fits, int kernel_choice, int ctas_hint, int depth_hint,
+                      WalkPlan* plan, std::string* err);
 // kind: 0 domino, 1 lozenge, 2 rect-triangle, 3 triangle-dimer (merge only).
 rt_status launch_split(bool merge, int elem_bytes, int kind, int ncol, int n, int32_t* tiling, void* const* arr,
                        cudaStream_t stream, std::string* err);
@@ -77,8 +82,10 @@ rt_status launch_split(bool merge, int elem_bytes, int kind, int ncol, int n, in
 // Fast-mode schedules (rt_capi.cu).  kind: 0 domino, 1 lozenge,
 // 2 rect-triangle, 3 triangle dimer.  fast_step_phases appends the phases of
 // step s of an epoch; fast_phases appends a whole walk of `steps` steps
-// (with the final Update of the colour models).
-int64_t fast_step_phases(int kind, int64_t s, uint32_t* ph, int64_t at, uint32_t* prev);
+// (with the final Update of the colour models, or the triangle dimers' pending
+// refreshes).
+class TdSchedule;
+int64_t fast_step_phases(int kind, int64_t s, uint32_t* ph, int64_t at, uint32_t* prev, TdSchedule* td);
 // Appends a bit-exact colour step of a two- or three-colour model: a phase of
 // its own, or (merge) one more step of the run that `ph` ends with, if that
 // run began at or after index `first`, the epoch's first phase.

@@ -149,7 +149,8 @@ extern "C" rt_status rt_walk_device_noalloc(const rt_config* cfg, int32_t* d_til
         WalkPlan plan;
         // The kernel rt_walk would run for this walk (word kernel for the int8
         // models, the generic walk kernel otherwise).
-        s = choose_plan(family, cfg->device, 1, rows, cols, width, true, false, false, false, 0, 0, 0, &plan, &perr);
+        s = choose_plan(family, cfg->device, 1, rows, cols, width, true, false, false, false, false, 0, 0, 0, &plan,
+                        &perr);
         if (s != RT_OK) {
             say(errbuf, errcap, "%s", perr.c_str());
             return s;

@@ -3,14 +3,16 @@
 // The eight state arrays of TriDimerRule (rt_tridimer.cuh) hold small
 // integers: the lozenge arrays H, L, R four bits, the triangle arrays U, D
 // three base-4 digits (six bits), the butterfly arrays BH, BL, BR four base-4
-// digits and a centre bit (nine bits).  Here every bit of every array is a
-// plane of its own, 32 sites of a row per 32-bit word, 51 planes in all, and
-// each phase op is written as boolean algebra on the words: one work item
-// updates 32 sites of a row at once.  A neighbour at column j +- 1 is a
+// digits and a centre bit (nine bits).  The rules' digit sums can carry out of
+// these only on states that are no dimer covers, by at most one bit, which the
+// planes keep too: any start whose values fit the planes gives the integer
+// rule's values.  Every bit of every array is a plane of its own, 32 sites of
+// a row per 32-bit word, 56 planes in all, and each phase op is written as
+// boolean algebra on the words: one work item updates 32 sites of a row at
+// once.  A neighbour at column j +- 1 is a
 // funnel shift of two adjacent words.  Sums of weighted conditions (the
 // digits a + 2 b + 3 c of the reference's rules) use a bit-sliced ripple
-// adder, so every value is the one the integer rule computes, modulo the
-// array's width (states reached from a valid tiling never exceed it).
+// adder, so every value is the one the integer rule computes.
 //
 // Sites outside an op's mask keep their bits; within one phase no op reads a
 // site it writes (the reference's parallel kernels rely on the same), so the
@@ -31,12 +33,33 @@
 namespace rtb {
 namespace tdp {
 
-constexpr int kPlanes = 51;
+constexpr int kPlanes = 56;
 
 // First plane and bit count of array `arr` (0 H, 1 L, 2 R, 3 U, 4 D, 5 BH, 6 BL, 7 BR).
-TDP_HD constexpr int plane_of(int arr) { return arr < 3 ? 4 * arr : arr < 5 ? 12 + 6 * (arr - 3) : 24 + 9 * (arr - 5); }
-TDP_HD constexpr int bits_of(int arr) { return arr < 3 ? 4 : arr < 5 ? 6 : 9; }
+TDP_HD constexpr int plane_of(int arr) { return arr < 3 ? 4 * arr : arr < 5 ? 12 + 7 * (arr - 3) : 26 + 10 * (arr - 5); }
+TDP_HD constexpr int bits_of(int arr) { return arr < 3 ? 4 : arr < 5 ? 7 : 10; }
+// Bits of the values a dimer cover's arrays hold.
+TDP_HD constexpr int cover_bits_of(int arr) { return arr < 3 ? 4 : arr < 5 ? 6 : 9; }
 
+// ---- lane masks -------------------------------------------------------------
+TDP_HD int mod3(int x) { return ((x % 3) + 3) % 3; }
+// lanes of word c whose column j = 32 c + l has j mod 2 == r
+TDP_HD uint32_t col_par(int r) { return (r & 1) ? 0xAAAAAAAAu : 0x55555555u; }
+// lanes of word c whose column has j mod 3 == r (32 = 2 mod 3)
+TDP_HD uint32_t col_mod3(int r, int c) {
+    const int k = mod3(r - 2 * c);
+    return k == 0 ? 0x49249249u : k == 1 ? 0x92492492u : 0x24924924u;
+}
+// lanes of word c whose column lies in [lo, hi]
+TDP_HD uint32_t col_range(int c, int lo, int hi) {
+    int a = lo - 32 * c, b = hi - 32 * c;
+    if (b < 0 || a > 31 || a > b) return 0u;
+    a = a < 0 ? 0 : a;
+    b = b > 31 ? 31 : b;
+    const uint32_t upto = b >= 31 ? 0xFFFFFFFFu : ((1u << (b + 1)) - 1u);
+    const uint32_t below = (1u << a) - 1u;
+    return upto & ~below;
+}
 // The planes of one chain (or one band of it) and the work item (array row
 // i, word c covering columns 32 c .. 32 c + 31).  Layout: plane-major, then
 // rows (row 0 = array row row0), then words; the word before a row's first
@@ -61,27 +84,13 @@ struct View {
         uint32_t* q = word(plane_of(arr) + bit, 0);
         *q = (*q & ~m) | (v & m);
     }
+    // Lanes whose column is inside the lattice's border, in use, = r (mod 3).
+    // A view that visits one word column may know them (rt_tdwalk.cuh).
+    TDP_HD uint32_t inner_cols(int m) const { return col_range(c, 1, m - 2); }
+    TDP_HD uint32_t used_cols(int width) const { return col_range(c, 0, width - 1); }
+    TDP_HD uint32_t cols_mod3(int r) const { return col_mod3(r, c); }
 };
 
-// ---- lane masks -------------------------------------------------------------
-TDP_HD int mod3(int x) { return ((x % 3) + 3) % 3; }
-// lanes of word c whose column j = 32 c + l has j mod 2 == r
-TDP_HD uint32_t col_par(int r) { return (r & 1) ? 0xAAAAAAAAu : 0x55555555u; }
-// lanes of word c whose column has j mod 3 == r (32 = 2 mod 3)
-TDP_HD uint32_t col_mod3(int r, int c) {
-    const int k = mod3(r - 2 * c);
-    return k == 0 ? 0x49249249u : k == 1 ? 0x92492492u : 0x24924924u;
-}
-// lanes of word c whose column lies in [lo, hi]
-TDP_HD uint32_t col_range(int c, int lo, int hi) {
-    int a = lo - 32 * c, b = hi - 32 * c;
-    if (b < 0 || a > 31 || a > b) return 0u;
-    a = a < 0 ? 0 : a;
-    b = b > 31 ? 31 : b;
-    const uint32_t upto = b >= 31 ? 0xFFFFFFFFu : ((1u << (b + 1)) - 1u);
-    const uint32_t below = (1u << a) - 1u;
-    return upto & ~below;
-}
 TDP_HD uint32_t all_if(bool x) { return x ? 0xFFFFFFFFu : 0u; }
 
 // ---- bit-sliced small integers -------------------------------------------------
@@ -112,11 +121,11 @@ TDP_HD void wsum(uint32_t (&out)[3], int w1, uint32_t a, int w2, uint32_t b, int
 TDP_HD uint32_t deq(uint32_t lo, uint32_t hi, int v) {
     return ((v & 1) ? lo : ~lo) & ((v & 2) ? hi : ~hi);
 }
-// t1 + 4 t4 + 16 t16 + 64 t64 + 256 c (each t three bits) into nine planes.
-TDP_HD void pack(uint32_t (&out)[9], const uint32_t (&t1)[3], const uint32_t (&t4)[3], const uint32_t (&t16)[3],
+// t1 + 4 t4 + 16 t16 + 64 t64 + 256 c (each t three bits, at most 6).
+TDP_HD void pack(uint32_t (&out)[10], const uint32_t (&t1)[3], const uint32_t (&t4)[3], const uint32_t (&t16)[3],
                  const uint32_t (&t64)[3], uint32_t c) {
 #pragma unroll
-    for (int k = 0; k < 9; ++k) out[k] = 0u;
+    for (int k = 0; k < 10; ++k) out[k] = 0u;
     add_at(out, t1, 3, 0);
     add_at(out, t4, 3, 2);
     add_at(out, t16, 3, 4);
@@ -145,7 +154,8 @@ TDP_HD void const3(uint32_t (&out)[3], int v) {
 // ---- values built from the lozenge arrays ---------------------------------------
 // Butterfly state of orientation `which` from the lozenges
 // (UpdateButterflys{H,L,R}FromLozenge, triangledimerkernel.cl:118-189).
-TDP_HD void bfly_from_loz(uint32_t (&out)[9], const View& v, int which) {
+template <class V>
+TDP_HD void bfly_from_loz(uint32_t (&out)[10], const V& v, int which) {
     uint32_t t1[3], t4[3], t16[3], t64[3], c;
     if (which == 0) {
         c = v.ld(1, 2, -1, 1);
@@ -170,20 +180,22 @@ TDP_HD void bfly_from_loz(uint32_t (&out)[9], const View& v, int which) {
 }
 
 // Up-triangle state from the lozenges (UpdateTriangleUFromLozenges, :96-116).
-TDP_HD void up_from_loz(uint32_t (&out)[6], const View& v) {
+template <class V>
+TDP_HD void up_from_loz(uint32_t (&out)[7], const V& v) {
     uint32_t x[3], y[3], z[3];
     wsum(x, 1, v.ld(1, 0, 0, 0), 2, v.ld(0, 3, 0, 0), 3, v.ld(0, 0, 1, 0));
     wsum(y, 1, v.ld(1, 0, 0, 1), 2, v.ld(0, 1, 1, 0), 3, v.ld(1, 1, 0, 1));
     wsum(z, 1, v.ld(1, 2, 0, 1), 2, v.ld(0, 3, 1, 0), 3, v.ld(0, 2, 1, 0));
 #pragma unroll
-    for (int k = 0; k < 6; ++k) out[k] = 0u;
+    for (int k = 0; k < 7; ++k) out[k] = 0u;
     add_at(out, x, 3, 0);
     add_at(out, y, 3, 2);
     add_at(out, z, 3, 4);
 }
 
 // TriDimerRule::tri_digit of the triangle value at (di, dj) of array arr.
-TDP_HD void tri_digit(uint32_t (&out)[3], const View& v, int arr, int di, int dj) {
+template <class V>
+TDP_HD void tri_digit(uint32_t (&out)[3], const V& v, int arr, int di, int dj) {
     const uint32_t A = v.ld(arr, 4, di, dj) & ~v.ld(arr, 5, di, dj);  // (x & 48) == 16
     const uint32_t B = v.ld(arr, 0, di, dj) & v.ld(arr, 1, di, dj);   // (x & 3) == 3
     const uint32_t C = ~v.ld(arr, 2, di, dj) & v.ld(arr, 3, di, dj);  // (x & 12) == 8
@@ -196,10 +208,14 @@ TDP_HD uint32_t cls2(int t, int i, int r) {
     return t == 0 ? all_if((i & 1) == (r & 1)) : t == 1 ? col_par(r) : col_par((r - i) & 1);
 }
 // (j + 2 i) mod 3 == r
-TDP_HD uint32_t cls3(int i, int c, int r) { return col_mod3(mod3(r - 2 * i), c); }
+template <class V>
+TDP_HD uint32_t cls3(const V& v, int r) {
+    return v.cols_mod3(mod3(r - 2 * v.i));
+}
 // TriDimerRule::slice(t, i, j) == r
-TDP_HD uint32_t slice3(int t, int i, int c, int r) {
-    return t == 0 ? all_if(mod3(i) == r) : t == 1 ? col_mod3(r, c) : col_mod3(mod3(r - i), c);
+template <class V>
+TDP_HD uint32_t slice3(int t, const V& v, int r) {
+    return t == 0 ? all_if(mod3(v.i) == r) : t == 1 ? v.cols_mod3(r) : v.cols_mod3(mod3(r - v.i));
 }
 // TriDimerRule::bpar(t, i, j) == r
 TDP_HD uint32_t bpar2(int t, int i, int r) { return t == 1 ? all_if((i & 1) == (r & 1)) : col_par(r); }
@@ -208,32 +224,70 @@ TDP_HD uint32_t bpar2(int t, int i, int r) { return t == 1 ? all_if((i & 1) == (
 struct Dig {
     uint32_t lo, hi;
 };
-TDP_HD Dig bdig(const View& v, int arr, int k, int di, int dj) { return {v.ld(arr, 2 * k, di, dj), v.ld(arr, 2 * k + 1, di, dj)}; }
+template <class V>
+TDP_HD Dig bdig(const V& v, int arr, int k, int di, int dj) { return {v.ld(arr, 2 * k, di, dj), v.ld(arr, 2 * k + 1, di, dj)}; }
 TDP_HD void d3(uint32_t (&out)[3], Dig d) { dig3(out, d.lo, d.hi); }
 TDP_HD void d3(uint32_t (&out)[3], uint32_t lo, uint32_t hi) { dig3(out, lo, hi); }
+
+// ---- the rotations --------------------------------------------------------------------
+// Lanes a drawing op flips where their draw is below 2^22: of its class, in
+// use, and in one of the two states it swaps.
+template <uint32_t OP, int T = -1, class V>
+TDP_HD uint32_t rot_mask(const V& v, uint32_t a, uint32_t b, int width) {
+    const int t = T >= 0 ? T : (int)a;
+    const int i = v.i;
+    const uint32_t VAL = v.used_cols(width);
+    if (OP == TD_ROT_LOZ) {  // :4-22
+        const uint32_t x0 = v.ld(t, 0, 0, 0), x1 = v.ld(t, 1, 0, 0), x2 = v.ld(t, 2, 0, 0), x3 = v.ld(t, 3, 0, 0);
+        return cls2(t, i, (int)b) & VAL & ((x0 & ~x1 & x2 & ~x3) | (~x0 & x1 & ~x2 & x3));  // 5, 10
+    }
+    if (OP == TD_ROT_TRI) {  // :191-211
+        const int arr = t == 1 ? 4 : 3;
+        uint32_t x[7];
+#pragma unroll
+        for (int k = 0; k < 7; ++k) x[k] = v.ld(arr, k, 0, 0);
+        const uint32_t eq45 = x[0] & ~x[1] & x[2] & x[3] & ~x[4] & x[5];
+        const uint32_t eq54 = ~x[0] & x[1] & x[2] & ~x[3] & x[4] & x[5];
+        return cls3(v, (int)b) & VAL & (eq45 | eq54) & ~x[6];
+    }
+    // TD_ROT_BFLY, :331-353
+    const int p1 = (int)(b & 3), p2 = (int)(b >> 2);
+    const uint32_t cond = t == 0   ? all_if(mod3(i) == p1) & col_par(p2)
+                          : t == 1 ? v.cols_mod3(p1) & all_if((i & 1) == p2)
+                                   : v.cols_mod3(mod3(p1 - i)) & col_par(p2);
+    uint32_t x[10];
+#pragma unroll
+    for (int k = 0; k < 10; ++k) x[k] = v.ld(5 + t, k, 0, 0);
+    // 170 = bits 1, 3, 5, 7; 85 = bits 0, 2, 4, 6; the centre bit clear in both
+    const uint32_t odd = x[1] & x[3] & x[5] & x[7], even = x[0] & x[2] & x[4] & x[6];
+    const uint32_t nodd = ~x[1] & ~x[3] & ~x[5] & ~x[7], neven = ~x[0] & ~x[2] & ~x[4] & ~x[6];
+    return cond & VAL & ~x[8] & ~x[9] & ((odd & neven) | (even & nodd));
+}
+// Swaps the two states in the lanes of F, a part of the op's rot_mask.
+template <uint32_t OP, int T = -1, class V>
+TDP_HD void rot_flip(const V& v, uint32_t a, uint32_t F) {
+    const int t = T >= 0 ? T : (int)a;
+    const int arr = OP == TD_ROT_LOZ ? t : OP == TD_ROT_TRI ? (t == 1 ? 4 : 3) : 5 + t;
+    const uint32_t bits = OP == TD_ROT_LOZ ? 0xfu : OP == TD_ROT_TRI ? 0x1bu : 0xffu;
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+        if (bits >> k & 1u) *v.word(plane_of(arr) + k, 0) ^= F;
+}
 
 // ---- the ops ------------------------------------------------------------------------
 // One 32-site word of phase (OP, a, b) at the view's row and word.  T >= 0
 // / B >= 0 fix a / b at compile time.  m: array side; width: columns in
 // use; draw: lanes whose draw k is below 2^22 (drawing ops only).
-template <uint32_t OP, int T = -1, int B = -1>
-TDP_HD void word_op(const View& v, uint32_t a_, uint32_t b_, int m, int width, uint32_t draw) {
+template <uint32_t OP, int T = -1, int B = -1, class V>
+TDP_HD void word_op(const V& v, uint32_t a_, uint32_t b_, int m, int width, uint32_t draw) {
     const int t = T >= 0 ? T : (int)a_;
     const uint32_t bb = B >= 0 ? (uint32_t)B : b_;
-    const int i = v.i, c = v.c;
-    const uint32_t VAL = col_range(c, 0, width - 1);
-    const uint32_t INT = (i >= 1 && i <= m - 2) ? col_range(c, 1, m - 2) : 0u;
+    const int i = v.i;
+    const uint32_t INT = (i >= 1 && i <= m - 2) ? v.inner_cols(m) : 0u;
     switch (OP) {
-        case TD_ROT_LOZ: {  // :4-22
-            uint32_t x[4];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) x[k] = v.ld(t, k, 0, 0);
-            const uint32_t eq5 = x[0] & ~x[1] & x[2] & ~x[3], eq10 = ~x[0] & x[1] & ~x[2] & x[3];
-            const uint32_t F = cls2(t, i, (int)bb) & draw & VAL & (eq5 | eq10);
-#pragma unroll
-            for (int k = 0; k < 4; ++k) v.st(t, k, ~x[k], F);
+        case TD_ROT_LOZ:
+            rot_flip<TD_ROT_LOZ, T>(v, a_, rot_mask<TD_ROT_LOZ, T>(v, a_, bb, width) & draw);
             break;
-        }
         case TD_LOZ_FLIPPED: {  // :24-33
             const uint32_t M = INT & ~cls2(t, i, (int)bb);
             const int dj = t & 1, di = (2 - t) / 2;
@@ -269,52 +323,41 @@ TDP_HD void word_op(const View& v, uint32_t a_, uint32_t b_, int m, int width, u
             break;
         }
         case TD_UP_FROM_LOZ: {
-            uint32_t u[6];
+            uint32_t u[7];
             up_from_loz(u, v);
 #pragma unroll
-            for (int k = 0; k < 6; ++k) v.st(3, k, u[k], INT);
+            for (int k = 0; k < 7; ++k) v.st(3, k, u[k], INT);
             break;
         }
         case TD_TRI_OTHER: {  // :255-275, then :118-189 for the butterflies in b
             const int src = t == 0 ? 3 : 4, dst = t == 0 ? 4 : 3, p = t == 0 ? -1 : 1;
-            uint32_t d0[3], d1[3], d2[3], tv[6] = {0u, 0u, 0u, 0u, 0u, 0u};
+            uint32_t d0[3], d1[3], d2[3], tv[7] = {0u, 0u, 0u, 0u, 0u, 0u, 0u};
             tri_digit(d0, v, src, 0, -1 + t);
             tri_digit(d1, v, src, 0, t);
             tri_digit(d2, v, src, p, 0);
             add_at(tv, d0, 3, 0);
             add_at(tv, d1, 3, 2);
             add_at(tv, d2, 3, 4);
-            uint32_t bv[3][9];
+            uint32_t bv[3][10];
 #pragma unroll
             for (int w = 0; w < 3; ++w)
                 if (bb & (1u << w)) bfly_from_loz(bv[w], v, w);
 #pragma unroll
-            for (int k = 0; k < 6; ++k) v.st(dst, k, tv[k], INT);
+            for (int k = 0; k < 7; ++k) v.st(dst, k, tv[k], INT);
 #pragma unroll
             for (int w = 0; w < 3; ++w)
                 if (bb & (1u << w)) {
 #pragma unroll
-                    for (int k = 0; k < 9; ++k) v.st(5 + w, k, bv[w][k], INT);
+                    for (int k = 0; k < 10; ++k) v.st(5 + w, k, bv[w][k], INT);
                 }
             break;
         }
-        case TD_ROT_TRI: {  // :191-211
-            const int arr = t == 1 ? 4 : 3;
-            uint32_t x[6];
-#pragma unroll
-            for (int k = 0; k < 6; ++k) x[k] = v.ld(arr, k, 0, 0);
-            const uint32_t eq45 = x[0] & ~x[1] & x[2] & x[3] & ~x[4] & x[5];
-            const uint32_t eq54 = ~x[0] & x[1] & x[2] & ~x[3] & x[4] & x[5];
-            const uint32_t F = cls3(i, c, (int)bb) & draw & VAL & (eq45 | eq54);
-            v.st(arr, 0, ~x[0], F);
-            v.st(arr, 1, ~x[1], F);
-            v.st(arr, 3, ~x[3], F);
-            v.st(arr, 4, ~x[4], F);
+        case TD_ROT_TRI:
+            rot_flip<TD_ROT_TRI, T>(v, a_, rot_mask<TD_ROT_TRI, T>(v, a_, bb, width) & draw);
             break;
-        }
         case TD_TRI_FLIPPED: {  // :213-253
             const int arr = t == 1 ? 4 : 3;
-            const uint32_t M1 = INT & cls3(i, c, ((int)bb + 1) % 3), M2 = INT & cls3(i, c, ((int)bb + 2) % 3);
+            const uint32_t M1 = INT & cls3(v, ((int)bb + 1) % 3), M2 = INT & cls3(v, ((int)bb + 2) % 3);
             uint32_t vp[6], vq[6];
             // p: digit 1 of (0,-1), digit 2 of (-1,+1) [t = 1: (+1,0)], digit 0 of (+1,0) [t = 1: (-1,+1)]
             const int ai = t == 0 ? -1 : 1, aj = t == 0 ? 1 : 0, ci = t == 0 ? 1 : -1, cj = t == 0 ? 0 : 1;
@@ -334,6 +377,7 @@ TDP_HD void word_op(const View& v, uint32_t a_, uint32_t b_, int m, int width, u
             vq[5] = v.ld(arr, 3, gi, gj);
 #pragma unroll
             for (int k = 0; k < 6; ++k) v.st(arr, k, (vp[k] & M1) | (vq[k] & M2), M1 | M2);
+            v.st(arr, 6, 0u, M1 | M2);
             break;
         }
         case TD_LOZ_FROM_TRI: {  // :277-329
@@ -362,7 +406,7 @@ TDP_HD void word_op(const View& v, uint32_t a_, uint32_t b_, int m, int width, u
             break;
         }
         case TD_BFLY_FROM_LOZ: {
-            uint32_t bv[3][9], uv[6];
+            uint32_t bv[3][10], uv[7];
 #pragma unroll
             for (int w = 0; w < 3; ++w)
                 if (bb & (1u << w)) bfly_from_loz(bv[w], v, w);
@@ -371,34 +415,21 @@ TDP_HD void word_op(const View& v, uint32_t a_, uint32_t b_, int m, int width, u
             for (int w = 0; w < 3; ++w)
                 if (bb & (1u << w)) {
 #pragma unroll
-                    for (int k = 0; k < 9; ++k) v.st(5 + w, k, bv[w][k], INT);
+                    for (int k = 0; k < 10; ++k) v.st(5 + w, k, bv[w][k], INT);
                 }
             if (t) {
 #pragma unroll
-                for (int k = 0; k < 6; ++k) v.st(3, k, uv[k], INT);
+                for (int k = 0; k < 7; ++k) v.st(3, k, uv[k], INT);
             }
             break;
         }
-        case TD_ROT_BFLY: {  // :331-353
-            const int p1 = (int)(bb & 3), p2 = (int)(bb >> 2);
-            const uint32_t cond = t == 0   ? all_if(mod3(i) == p1) & col_par(p2)
-                                  : t == 1 ? col_mod3(p1, c) & all_if((i & 1) == p2)
-                                           : col_mod3(mod3(p1 - i), c) & col_par(p2);
-            uint32_t x[9];
-#pragma unroll
-            for (int k = 0; k < 9; ++k) x[k] = v.ld(5 + t, k, 0, 0);
-            // 170 = bits 1, 3, 5, 7; 85 = bits 0, 2, 4, 6; the centre bit clear in both
-            const uint32_t odd = x[1] & x[3] & x[5] & x[7], even = x[0] & x[2] & x[4] & x[6];
-            const uint32_t nodd = ~x[1] & ~x[3] & ~x[5] & ~x[7], neven = ~x[0] & ~x[2] & ~x[4] & ~x[6];
-            const uint32_t F = cond & draw & VAL & ~x[8] & ((odd & neven) | (even & nodd));
-#pragma unroll
-            for (int k = 0; k < 8; ++k) v.st(5 + t, k, ~x[k], F);
+        case TD_ROT_BFLY:
+            rot_flip<TD_ROT_BFLY, T>(v, a_, rot_mask<TD_ROT_BFLY, T>(v, a_, bb, width) & draw);
             break;
-        }
         case TD_BFLY_SAME: {  // UpdateButterflysFlipped{H,L,R}1
             const int p1 = (int)(bb & 3), p2 = (int)(bb >> 2);
             const int arr = 5 + t;
-            const uint32_t M = INT & slice3(t, i, c, p1) & ~bpar2(t, i, p2);
+            const uint32_t M = INT & slice3(t, v, p1) & ~bpar2(t, i, p2);
             Dig t1, t4, t16, t64;
             // cyc_up (0,1,2,3 -> 0,2,3,1): (lo, hi) -> (hi, hi ^ lo); cyc_dn (-> 0,3,1,2): -> (hi ^ lo, lo)
             auto up = [](Dig d) { return Dig{d.hi, d.hi ^ d.lo}; };
@@ -418,13 +449,14 @@ TDP_HD void word_op(const View& v, uint32_t a_, uint32_t b_, int m, int width, u
             const uint32_t out[8] = {t1.lo, t1.hi, t4.lo, t4.hi, t16.lo, t16.hi, t64.lo, t64.hi};
 #pragma unroll
             for (int k = 0; k < 8; ++k) v.st(arr, k, out[k], M);
+            v.st(arr, 9, 0u, M);
             break;
         }
         case TD_BFLY_21: {
             const int p1 = (int)bb;
             const int want = t == 0 ? (p1 + 1) % 3 : (p1 + 2) % 3;
             const int arr = 5 + t;
-            const uint32_t M = INT & slice3(t, i, c, want);
+            const uint32_t M = INT & slice3(t, v, want);
             const Dig f0 = bdig(v, arr, 0, 0, 0), f1 = bdig(v, arr, 1, 0, 0), f2 = bdig(v, arr, 2, 0, 0),
                       f3 = bdig(v, arr, 3, 0, 0);
             uint32_t t1[3], t4[3], t16[3], t64[3], cc, alt[3], k3[3];
@@ -454,17 +486,17 @@ TDP_HD void word_op(const View& v, uint32_t a_, uint32_t b_, int m, int width, u
                 d3(t16, f2);
                 d3(t64, f3);
             }
-            uint32_t out[9];
+            uint32_t out[10];
             pack(out, t1, t4, t16, t64, cc);
 #pragma unroll
-            for (int k = 0; k < 9; ++k) v.st(arr, k, out[k], M);
+            for (int k = 0; k < 10; ++k) v.st(arr, k, out[k], M);
             break;
         }
         case TD_BFLY_22: {
             const int p1 = (int)bb;
             const int want = t == 0 ? (p1 + 2) % 3 : (p1 + 1) % 3;
             const int arr = 5 + t;
-            const uint32_t M = INT & slice3(t, i, c, want);
+            const uint32_t M = INT & slice3(t, v, want);
             const Dig f0 = bdig(v, arr, 0, 0, 0), f1 = bdig(v, arr, 1, 0, 0), f2 = bdig(v, arr, 2, 0, 0),
                       f3 = bdig(v, arr, 3, 0, 0);
             uint32_t t1[3], t4[3], t16[3], t64[3], cc, alt[3], k3[3];
@@ -505,39 +537,49 @@ TDP_HD void word_op(const View& v, uint32_t a_, uint32_t b_, int m, int width, u
                 const3(k3, 1);
                 sel3(t64, deq(f3.lo, f3.hi, 1), k3, alt);
             }
-            uint32_t out[9];
+            uint32_t out[10];
             pack(out, t1, t4, t16, t64, cc);
 #pragma unroll
-            for (int k = 0; k < 9; ++k) v.st(arr, k, out[k], M);
+            for (int k = 0; k < 10; ++k) v.st(arr, k, out[k], M);
             break;
         }
-        case TD_BFLY_23_LOZ: {
+        case TD_BFLY_23_LOZ:  // pass 23, then UpdateLozengeFromButterflys{H,L,R} (:655-746), own site only
+            word_op<TD_BFLY_23, T, B>(v, a_, b_, m, width, draw);
+            word_op<TD_LOZ_FROM_BFLY, T, B>(v, a_, b_, m, width, draw);
+            break;
+        case TD_BFLY_23: {
             const int p1 = (int)bb;
             const int want = t == 0 ? (p1 + 1) % 3 : (p1 + 2) % 3;
             const int arr = 5 + t;
-            const uint32_t M = INT, S = INT & slice3(t, i, c, want);
-            Dig d[4];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) d[k] = bdig(v, arr, k, 0, 0);
-            const uint32_t cen = v.ld(arr, 8, 0, 0);
-            Dig nd[4] = {d[0], d[1], d[2], d[3]};
+            const uint32_t S = INT & slice3(t, v, want);
             if (t == 2) {
-                const uint32_t a = v.ld(arr, 8, -1, 0), b = v.ld(arr, 8, 0, -1);
-                // t1 = a ? 1 : (f0 != 1) * f0; t64 = b ? 2 : (f3 != 2) * f3
-                nd[0] = Dig{(a) | (d[0].lo & d[0].hi), ~a & d[0].hi};
-                nd[3] = Dig{~b & d[3].lo, b | (d[3].hi & d[3].lo)};
+                const uint32_t p = v.ld(arr, 8, -1, 0), q = v.ld(arr, 8, 0, -1);
+                const Dig d0 = bdig(v, arr, 0, 0, 0), d3v = bdig(v, arr, 3, 0, 0);
+                // t1 = p ? 1 : (f0 != 1) * f0; t64 = q ? 2 : (f3 != 2) * f3
+                v.st(arr, 0, p | (d0.lo & d0.hi), S);
+                v.st(arr, 1, ~p & d0.hi, S);
+                v.st(arr, 6, ~q & d3v.lo, S);
+                v.st(arr, 7, q | (d3v.hi & d3v.lo), S);
             } else {
                 const int n3i = 1, n3j = t == 0 ? 0 : -1, n4i = t == 0 ? 1 : 0, n4j = -1;
-                const uint32_t a = v.ld(arr, 8, n3i, n3j), b = v.ld(arr, 8, n4i, n4j);
-                // t16 = a ? 2 : (f2 != 2) * f2; t64 = b ? 1 : (f3 != 1) * f3
-                nd[2] = Dig{~a & d[2].lo, a | (d[2].hi & d[2].lo)};
-                nd[3] = Dig{b | (d[3].lo & d[3].hi), ~b & d[3].hi};
+                const uint32_t p = v.ld(arr, 8, n3i, n3j), q = v.ld(arr, 8, n4i, n4j);
+                const Dig d2 = bdig(v, arr, 2, 0, 0), d3v = bdig(v, arr, 3, 0, 0);
+                // t16 = p ? 2 : (f2 != 2) * f2; t64 = q ? 1 : (f3 != 1) * f3
+                v.st(arr, 4, ~p & d2.lo, S);
+                v.st(arr, 5, p | (d2.hi & d2.lo), S);
+                v.st(arr, 6, q | (d3v.lo & d3v.hi), S);
+                v.st(arr, 7, ~q & d3v.hi, S);
             }
-            // the butterfly array after pass 23 (centre bit unchanged)
+            v.st(arr, 9, 0u, S);  // the other digits and the centre bit stay
+            break;
+        }
+        case TD_LOZ_FROM_BFLY: {
+            const int arr = 5 + t;
+            const uint32_t M = INT;
             Dig e[4];
 #pragma unroll
-            for (int k = 0; k < 4; ++k) e[k] = Dig{(nd[k].lo & S) | (d[k].lo & ~S), (nd[k].hi & S) | (d[k].hi & ~S)};
-            // UpdateLozengeFromButterflys{H,L,R} (:655-746), own site only
+            for (int k = 0; k < 4; ++k) e[k] = bdig(v, arr, k, 0, 0);
+            const uint32_t cen = v.ld(arr, 8, 0, 0);
             const uint32_t o0 = deq(e[0].lo, e[0].hi, 3), o1 = deq(e[1].lo, e[1].hi, 3), o2 = deq(e[2].lo, e[2].hi, 3),
                            o3 = deq(e[3].lo, e[3].hi, 3);
             uint32_t H[4], L[4], R[4];
@@ -553,11 +595,6 @@ TDP_HD void word_op(const View& v, uint32_t a_, uint32_t b_, int m, int width, u
                 R[0] = o0, R[1] = o1, R[2] = o2, R[3] = o3;
                 H[0] = deq(e[0].lo, e[0].hi, 1), H[1] = deq(e[0].lo, e[0].hi, 2), H[2] = cen, H[3] = o3;
                 L[0] = o0, L[1] = cen, L[2] = deq(e[3].lo, e[3].hi, 1), L[3] = deq(e[3].lo, e[3].hi, 2);
-            }
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                v.st(arr, 2 * k, e[k].lo, S);
-                v.st(arr, 2 * k + 1, e[k].hi, S);
             }
 #pragma unroll
             for (int k = 0; k < 4; ++k) {

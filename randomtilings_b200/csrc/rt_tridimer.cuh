@@ -30,8 +30,8 @@ struct TriDimerRule {
         return (uint32_t)c + (uint32_t)(a.n / 2) * (uint32_t)r;
     }
     // Arrays a phase writes (bit k = array k); their halo rows are exchanged.
-    TD_HD static uint32_t written(uint32_t d) {
-        const uint32_t op = ph_op(d), a = ph_a(d), b = ph_b(d);
+    TD_HD static uint32_t written(uint32_t d) { return written_arrays(ph_op(d), ph_a(d), ph_b(d)); }
+    TD_HD static constexpr uint32_t written_arrays(uint32_t op, uint32_t a, uint32_t b) {
         switch (op) {
             case TD_ROT_LOZ:
             case TD_LOZ_FLIPPED: return 1u << a;
@@ -45,8 +45,10 @@ struct TriDimerRule {
             case TD_ROT_BFLY:
             case TD_BFLY_SAME:
             case TD_BFLY_21:
-            case TD_BFLY_22: return 1u << (5 + a);
+            case TD_BFLY_22:
+            case TD_BFLY_23: return 1u << (5 + a);
             case TD_BFLY_23_LOZ: return (1u << (5 + a)) | 7u;
+            case TD_LOZ_FROM_BFLY: return 7u;
             default: return 0u;
         }
     }
@@ -324,27 +326,32 @@ struct TriDimerRule {
                 put(arr, i, j, pack(t1, t4, t16, t64, c));
                 break;
             }
-            case TD_BFLY_23_LOZ: {
-                if (!interior) break;
+            case TD_BFLY_23_LOZ:  // pass 23, then the lozenges, own site only
+                site_op<TD_BFLY_23, T, B>(x, i, j, k);
+                site_op<TD_LOZ_FROM_BFLY, T, B>(x, i, j, k);
+                break;
+            case TD_BFLY_23: {
                 const int p1 = (int)x.b;
                 const int want = t == 0 ? (p1 + 1) % 3 : (p1 + 2) % 3;
+                if (!interior || slice(t, i, j) != want) break;
                 const int arr = 5 + t;
-                if (slice(t, i, j) == want) {
-                    const int32_t f = at(arr, i, j);
-                    int t1 = dg(f, 0), t4 = dg(f, 1), t16 = dg(f, 2), t64 = dg(f, 3);
-                    if (t == 2) {
-                        t1 = (at(arr, i - 1, j) & 256) ? 1 : (dg(f, 0) != 1) * dg(f, 0);
-                        t64 = (at(arr, i, j - 1) & 256) ? 2 : (dg(f, 3) != 2) * dg(f, 3);
-                    } else {
-                        const int32_t n3 = t == 0 ? at(arr, i + 1, j) : at(arr, i + 1, j - 1);
-                        const int32_t n4 = t == 0 ? at(arr, i + 1, j - 1) : at(arr, i, j - 1);
-                        t16 = (n3 & 256) ? 2 : (dg(f, 2) != 2) * dg(f, 2);
-                        t64 = (n4 & 256) ? 1 : (dg(f, 3) != 1) * dg(f, 3);
-                    }
-                    put(arr, i, j, pack(t1, t4, t16, t64, (f >> 8) & 1));
+                const int32_t f = at(arr, i, j);
+                int t1 = dg(f, 0), t4 = dg(f, 1), t16 = dg(f, 2), t64 = dg(f, 3);
+                if (t == 2) {
+                    t1 = (at(arr, i - 1, j) & 256) ? 1 : (dg(f, 0) != 1) * dg(f, 0);
+                    t64 = (at(arr, i, j - 1) & 256) ? 2 : (dg(f, 3) != 2) * dg(f, 3);
+                } else {
+                    const int32_t n3 = t == 0 ? at(arr, i + 1, j) : at(arr, i + 1, j - 1);
+                    const int32_t n4 = t == 0 ? at(arr, i + 1, j - 1) : at(arr, i, j - 1);
+                    t16 = (n3 & 256) ? 2 : (dg(f, 2) != 2) * dg(f, 2);
+                    t64 = (n4 & 256) ? 1 : (dg(f, 3) != 1) * dg(f, 3);
                 }
-                // UpdateLozengeFromButterflys{H,L,R} (:655-746), own site only.
-                const int32_t bf = at(arr, i, j);
+                put(arr, i, j, pack(t1, t4, t16, t64, (f >> 8) & 1));
+                break;
+            }
+            case TD_LOZ_FROM_BFLY: {  // UpdateLozengeFromButterflys{H,L,R} (:655-746)
+                if (!interior) break;
+                const int32_t bf = at(5 + t, i, j);
                 const int d0 = dg(bf, 0), d1 = dg(bf, 1), d2 = dg(bf, 2), d3 = dg(bf, 3), c = (bf >> 8) & 1;
                 const int32_t own = (d0 == 3) + 2 * (d1 == 3) + 4 * (d2 == 3) + 8 * (d3 == 3);
                 if (t == 0) {
@@ -383,6 +390,8 @@ struct TriDimerRule {
             case TD_BFLY_21: site_op<TD_BFLY_21>(x, i, j, k); break;
             case TD_BFLY_22: site_op<TD_BFLY_22>(x, i, j, k); break;
             case TD_BFLY_23_LOZ: site_op<TD_BFLY_23_LOZ>(x, i, j, k); break;
+            case TD_BFLY_23: site_op<TD_BFLY_23>(x, i, j, k); break;
+            case TD_LOZ_FROM_BFLY: site_op<TD_LOZ_FROM_BFLY>(x, i, j, k); break;
             default: break;
         }
     }
@@ -405,6 +414,7 @@ struct TriDimerRule {
         }
         if (OP == TD_BFLY_21 && t == 0) *S = 3, *o = ((int)b + 1) % 3;
         if (OP == TD_BFLY_22 && t == 0) *S = 3, *o = ((int)b + 2) % 3;
+        if (OP == TD_BFLY_23 && t == 0) *S = 3, *o = ((int)b + 1) % 3;
     }
 };
 
