@@ -25,6 +25,7 @@
 #include "rt_internal.h"
 #include "rt_guard.h"
 #include "rt_models.cuh"
+#include "rt_rtmoves.cuh"
 #include "rt_tdwalk.cuh"
 #include "rt_word.cuh"
 
@@ -53,6 +54,7 @@ struct BatchArgs {
     int64_t step_add;      // colour steps of this run made by the family's earlier launches in it
     uint32_t thr[4];
     float weights[16];
+    int table;  // rectangle-triangles: shared memory begins with a RectTriMoves
 };
 
 __device__ __forceinline__ void cluster_or_block_sync(cg::cluster_group& cluster, int CL) {
@@ -197,75 +199,88 @@ __global__ void __launch_bounds__(1024, 1) batch_word_kernel(const __grid_consta
 }
 
 // ---------------------------------------------------------------------------
-// int32 models (rectangle-triangles, triangle dimers): the per-site rules of
-// the generic walk kernel, positions taken in quads of one Philox call.
-// Shared memory: NC planes of (rpc + 2) x wpad int32.
+// Rectangle-triangles: quads of four sites of one Philox call; as in
+// rt_recttri.cu a phase refreshes only the colour it flips, and the moves come
+// from a table (64 chains of side 135, 200 sweeps: 1.92 ms; 4.10 with the rule
+// evaluated in place and all colours refreshed).
+// Shared memory: three planes of (rpc + 2) x wpad int32.
 // ---------------------------------------------------------------------------
-template <class Model>
-__global__ void __launch_bounds__(1024, 1) batch_site_kernel(const __grid_constant__ BatchArgs b) {
-    using T = typename Model::Elem;
-    constexpr int NC = Model::NCOL;
+__global__ void __launch_bounds__(1024, 1) batch_recttri_kernel(const __grid_constant__ BatchArgs b) {
     cg::cluster_group cluster = cg::this_cluster();
     const int CL = (int)cluster.num_blocks();
     const int rank = (int)cluster.block_rank();
     const int ncl = gridDim.x / CL;
     const int cid = blockIdx.x / CL;
     const int BLOCK = blockDim.x, tid = threadIdx.x;
-    __shared__ WalkArgs wa;  // the fields the site rules read: n, wpad, thr, weights
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    T* lat = reinterpret_cast<T*>(smem_raw);
+    RectTriMoves& moves = *reinterpret_cast<RectTriMoves*>(smem_raw);
+    int* lat = reinterpret_cast<int*>(smem_raw + (b.table ? sizeof(RectTriMoves) : 0));
 
+    if (b.table) {
+        moves.clear(tid, BLOCK);
+        __syncthreads();
+        moves.fill(b, tid, BLOCK);
+    }
     for (int q = cid; q < b.nchains; q += ncl) {
         const BatchChain& ch = b.chains[b.order[q]];
-        const int rows = ch.rows, W = ch.wpad, cols = ch.cols, width = ch.width;
+        const int rows = ch.rows, W = ch.wpad, width = ch.width, n = ch.n;
         const int rpc = (rows + CL - 1) / CL;
         const int r0 = min(rows, rank * rpc), r1 = min(rows, r0 + rpc);
         const int nrows = r1 - r0;
-        const int a0 = r0 + Model::ROFF;
         const int plane = (rpc + 2) * W;
-        if (tid == 0) {
-            wa.n = ch.n;
-            wa.wpad = W;
-            for (int x = 0; x < 4; ++x) wa.thr[x] = b.thr[x];
-            for (int x = 0; x < 16; ++x) wa.weights[x] = b.weights[x];
-            wa.wper = 0;  // no weighted dominoes in batches
-        }
-        for (int c = 0; c < NC; ++c) {
-            const T* g = static_cast<const T*>(ch.arr[c]);
-            T* s = lat + c * plane;
+        for (int c = 0; c < 3; ++c) {
+            const int* g = static_cast<const int*>(ch.arr[c]);
+            int* s = lat + c * plane;
             for (int e = tid; e < (nrows + 2) * W; e += BLOCK) {
-                const int rr = a0 - 1 + e / W, j = e % W;
-                T v = (T)0;
-                if (rr >= 0 && rr < ch.arows && j < width) v = g[(size_t)rr * width + j];
-                s[e] = v;
+                const int rr = r0 - 1 + e / W, j = e % W;
+                s[e] = rr >= 0 && rr < ch.arows && j < width ? g[(size_t)rr * width + j] : 0;
             }
         }
         __syncthreads();
 
         const uint32_t key0 = (uint32_t)ch.key, key1 = (uint32_t)(ch.key >> 32);
         int64_t dstep = *b.step0 + b.step_add;
-        const int Gw = (width + 3) >> 2;
-        const int qlo = Model::COFF >> 2;
-        const int G = ((Model::COFF + cols - 1) >> 2) - qlo + 1;
+        const int G = (width + 3) >> 2;  // quads per row
         const int nq = nrows * G;
         const int drr = BLOCK / G, dq = BLOCK - drr * G;
         for (int64_t ph = 0; ph < b.nphases; ++ph) {
             const uint32_t d = __ldg(b.phases + ph);
             const bool draws = (d & PH_DRAWS) != 0u;
-            const typename Model::Ctx x0 = Model::ctx(wa, lat, plane, d, a0 - 1);
+            const bool step = ph_op(d) == OP_STEP;
+            const int ca = (int)ph_a(d), cb = (int)ph_b(d);
+            const bool upd = !step || (cb != (int)NO_COLOUR && cb != ca);
+            const int t = step ? (upd ? cb : 0) : ca;
+            const int t1 = t == 2 ? 0 : t + 1, t2 = t == 0 ? 2 : t - 1;
             int rr = tid / G, cq = tid - (tid / G) * G;
             for (int u = tid; u < nq; u += BLOCK) {
-                const int qq = qlo + cq, r = r0 + rr;
+                const int i = r0 + rr, cls = i % 3;
+                const int s1 = cls == t, s2 = cls == t1, s3 = cls == t2;  // column shifts of the reads
                 uint4 w4 = make_uint4(0u, 0u, 0u, 0u);
                 if (draws)
-                    w4 = philox4((uint32_t)((r + Model::ROFF) * Gw + qq), (uint32_t)dstep,
-                                 (uint32_t)((uint64_t)dstep >> 32), ch.chain, key0, key1);
+                    w4 = philox4((uint32_t)(i * G + cq), (uint32_t)dstep, (uint32_t)((uint64_t)dstep >> 32), ch.chain,
+                                 key0, key1);
 #pragma unroll
                 for (int bb = 0; bb < 4; ++bb) {
-                    const int c = 4 * qq + bb - Model::COFF;
-                    if (c >= 0 && c < cols) {
-                        const int i = r + Model::ROFF, j = c + Model::COFF;
-                        Model::site(wa, x0, (rr + 1) * W + j, i, j, quad_word(w4, bb) >> 9);
+                    const int j = 4 * cq + bb;
+                    if (j >= width) break;
+                    const int off = (rr + 1) * W + j;
+                    const bool inner = i >= 1 && i <= n - 2 && j >= 1 && j <= width - 2;
+                    const int* f = lat + t * plane + off;
+                    if (step) {
+                        int* cur = lat + ca * plane + off;
+                        int v;
+                        if (upd && inner)
+                            v = ca == t1 ? rt_next(f[-W], f[s1], f[W - s2]) : rt_next2(f[-s3], f[s2 - W], f[W]);
+                        else
+                            v = *cur;
+                        if (draws) {
+                            const uint32_t k = quad_word(w4, bb) >> 9;
+                            v = b.table ? moves.flip(v, RectTriMoves::prepare(k)) : RectTriRule::flip(v, k, b);
+                        }
+                        *cur = v;
+                    } else if (inner) {
+                        lat[t1 * plane + off] = rt_next(f[-W], f[s1], f[W - s2]);
+                        lat[t2 * plane + off] = rt_next2(f[-s3], f[s2 - W], f[W]);
                     }
                 }
                 rr += drr;
@@ -278,18 +293,13 @@ __global__ void __launch_bounds__(1024, 1) batch_site_kernel(const __grid_consta
             if (draws) ++dstep;
             if (CL > 1) {
                 cluster.sync();
-                uint32_t mask = Model::written(d);
-                if (nrows > 0) {
-                    while (mask) {
-                        const int arr = __ffs(mask) - 1;
-                        mask &= mask - 1;
-                        for (int e = tid; e < 2 * W; e += BLOCK) {
-                            const int side = e >= W, x = e - side * W;
-                            if ((side == 0 && rank == 0) || (side == 1 && r1 >= rows)) continue;
-                            T* mine = lat + arr * plane + (side == 0 ? 0 : nrows + 1) * W + x;
-                            T* theirs = lat + arr * plane + (side == 0 ? rpc : 1) * W + x;
-                            *mine = *cluster.map_shared_rank(theirs, rank + (side == 0 ? -1 : 1));
-                        }
+                if (step && nrows > 0) {
+                    for (int e = tid; e < 2 * W; e += BLOCK) {
+                        const int side = e >= W, x = e - side * W;
+                        if ((side == 0 && rank == 0) || (side == 1 && r1 >= rows)) continue;
+                        int* mine = lat + ca * plane + (side == 0 ? 0 : nrows + 1) * W + x;
+                        int* theirs = lat + ca * plane + (side == 0 ? rpc : 1) * W + x;
+                        *mine = *cluster.map_shared_rank(theirs, rank + (side == 0 ? -1 : 1));
                     }
                 }
                 cluster.sync();
@@ -297,12 +307,12 @@ __global__ void __launch_bounds__(1024, 1) batch_site_kernel(const __grid_consta
                 __syncthreads();
             }
         }
-        for (int c = 0; c < NC; ++c) {
-            T* g = static_cast<T*>(ch.arr[c]);
-            const T* s = lat + c * plane;
+        for (int c = 0; c < 3; ++c) {
+            int* g = static_cast<int*>(ch.arr[c]);
+            const int* s = lat + c * plane;
             for (int e = tid; e < nrows * width; e += BLOCK) {
                 const int rr = e / width, j = e % width;
-                g[(size_t)(a0 + rr) * width + j] = s[(rr + 1) * W + j];
+                g[(size_t)(r0 + rr) * width + j] = s[(rr + 1) * W + j];
             }
         }
         cluster_or_block_sync(cluster, CL);
@@ -352,7 +362,7 @@ static BatchFn batch_fn(int family) {
         case FAM_DOMINO: return batch_word_kernel<FAM_DOMINO>;
         case FAM_DOMINO_HB: return batch_word_kernel<FAM_DOMINO_HB>;
         case FAM_LOZENGE8: return batch_word_kernel<FAM_LOZENGE8>;
-        case FAM_RECTTRI: return batch_site_kernel<ThreeColour<int32_t, RectTriRule>>;
+        case FAM_RECTTRI: return batch_recttri_kernel;
         case FAM_TRIDIMER: return batch_td_kernel;
         default: return nullptr;
     }
@@ -397,6 +407,7 @@ struct Dev {
 struct Plan {
     int cl = 1, block = 256, clusters = 1;
     size_t smem = 0;
+    bool table = false;  // rectangle-triangles: the moves' table is in shared memory
     int64_t spl = 0;  // sweeps per launch: a run of S sweeps is S / spl launches (+ one for the rest); 0 = one
 };
 
@@ -495,6 +506,7 @@ rt_status launch_family(rt_batch* b, int f, const Plan& p, const void* recs, cud
                         int64_t step_add = 0, bool rest = false) {
     BatchFn fn = batch_fn(f);
     BatchArgs a = args_for(b, f, recs, step_add, rest);
+    a.table = p.table;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(p.clusters * p.cl));
     cfg.blockDim = dim3((unsigned)p.block);
@@ -529,6 +541,9 @@ bool fill_plan(rt_batch* b, int f, int cl, int block, Plan* p) {
     // bit-plane triangle-dimer kernel: 512); it then runs with its maximum.
     block = std::min(block, fa.maxThreadsPerBlock);
     if (smem + fa.sharedSizeBytes > (size_t)optin) return false;
+    // The table of moves goes in front of the lattice where there is room left.
+    p->table = f == FAM_RECTTRI && smem + sizeof(RectTriMoves) + fa.sharedSizeBytes <= (size_t)optin;
+    if (p->table) smem += sizeof(RectTriMoves);
     if (cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
         return false;
     if (cl > 8 && cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)

@@ -138,6 +138,8 @@ rt_status choose_plan(int family, int device, int nlat, int rows, int cols, int 
         s = plan_word_walk(family, device, nlat, rows, width, fast, ctas_hint, plan, err, weighted);
     if (kernel_choice == 0 && td_fits && family == FAM_TRIDIMER)
         s = plan_td_walk(device, rows, width, fast, ctas_hint, plan, err);
+    if (kernel_choice == 0 && nlat == 1 && family == FAM_RECTTRI)
+        s = plan_recttri_walk(device, rows, width, fast, ctas_hint, plan, err);
     if (s == RT_OK || kernel_choice == 2) return s;
     *plan = WalkPlan();
     return plan_walk(family, device, nlat, rows, cols, width, uniform, fast, plan, err);

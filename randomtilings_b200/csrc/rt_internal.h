@@ -61,6 +61,10 @@ rt_status plan_word_walk(int family, int device, int nlat, int rows, int width, 
 // Bit-plane kernel of a single triangle-dimer walk (rt_td.cu), for arrays whose
 // values fit its planes, on one cluster of ctas_hint CTAs (<= 0: by size).
 rt_status plan_td_walk(int device, int rows, int width, bool philox, int ctas_hint, WalkPlan* plan, std::string* err);
+// Rectangle-triangle kernel (rt_recttri.cu), one site per thread: bands of up to
+// 1,024 sites.  ctas_hint <= 0: by size.
+rt_status plan_recttri_walk(int device, int rows, int width, bool philox, int ctas_hint, WalkPlan* plan,
+                            std::string* err);
 // Bit-plane kernel of the int8 models (rt_plane.cu, RT_RNG_PLANES).
 // ctas_hint / depth_hint <= 0: one CTA per SM / the largest depth up to 8.
 rt_status plan_plane_walk(int family, int device, int nlat, int rows, int width, int ctas_hint, int depth_hint,
@@ -68,8 +72,8 @@ rt_status plan_plane_walk(int family, int device, int nlat, int rows, int width,
 // The kernel a walk runs on, as every walk entry point chooses it: the
 // bit-plane kernel in RT_RNG_PLANES mode; otherwise the word kernel for the
 // int8 models with uniform generator parameters (unless kernel_choice = 1),
-// and the triangle dimers' bit-plane kernel for arrays whose values fit it
-// (td_fits); falling back to the generic walk kernel for every other case and
+// the triangle dimers' bit-plane kernel for arrays whose values fit it
+// (td_fits), and the rectangle-triangle kernel; falling back to the generic walk kernel for every other case and
 // for any band those kernels cannot hold (kernel_choice = 2 forbids the
 // fallback).
 rt_status choose_plan(int family, int device, int nlat, int rows, int cols, int width, bool uniform, bool fast,

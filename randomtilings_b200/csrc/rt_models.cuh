@@ -297,7 +297,8 @@ struct RectTriRule {
         nb = (digit(west, 3) << 20) | (digit(upr, 2) << 16) | (digit(upr, 1) << 12) | (digit(west, 0) << 8) |
              (digit(down, 5) << 4) | digit(down, 4);
     }
-    __device__ static float weight(const WalkArgs& a, int x) {
+    template <class A>  // the kernel's arguments: .weights
+    __device__ static float weight(const A& a, int x) {
         float p = a.weights[digit(x, 5)];
         p = __fmul_rn(p, a.weights[digit(x, 4)]);
         p = __fmul_rn(p, a.weights[digit(x, 3)]);
@@ -311,14 +312,8 @@ struct RectTriRule {
     // standing in for 0x122133); one of six pair states toggles to its
     // partner.  The move is kept iff weight(new)/weight(old) >= the draw
     // rescaled to [0,1).  IEEE float arithmetic, as on the host CPU.
-    __device__ static int flip(int v, uint32_t k, const WalkArgs& a) {
-        const float bs = 0.9f;
-        float rd = __fsub_rn(__uint_as_float(k | 0x3f800000u), 1.0f);
-        if (!(rd < bs)) return v;
-        rd = __fdiv_rn(rd, bs);
-        const int quarter = rd < 0.25f ? 0 : rd < 0.5f ? 1 : rd < 0.75f ? 2 : 3;
-        float sc = (float)quarter * 0.25f;
-        int nv = v;
+    // The move proposed in a quarter (0: v never moves, 1: cycle, 2: pair).
+    __device__ static int propose(int v, int quarter, int& nv) {
         switch (v) {
             case 0x122133:
             case 0x331221:
@@ -327,25 +322,40 @@ struct RectTriRule {
             case 0xa7dd7a: {
                 const int pick = quarter == 0 ? 0xa7dd7a : quarter == 1 ? 0xfc99cf : quarter == 2 ? 0x8ebbe8 : 0x331221;
                 nv = pick == v ? 0x122133 : pick;
-                break;
+                return 1;
             }
-            case 0x47d47a: nv = 0xd22a33; sc = 1.0f; break;
-            case 0xd22a33: nv = 0x47d47a; sc = 1.0f; break;
-            case 0xa74d74: nv = 0x33a22d; sc = 1.0f; break;
-            case 0x33a22d: nv = 0xa74d74; sc = 1.0f; break;
-            case 0x8eb558: nv = 0x331eb1; sc = 1.0f; break;
-            case 0x331eb1: nv = 0x8eb558; sc = 1.0f; break;
-            case 0x855be8: nv = 0x1be133; sc = 1.0f; break;
-            case 0x1be133: nv = 0x855be8; sc = 1.0f; break;
-            case 0x6699cf: nv = 0xcf1221; sc = 1.0f; break;
-            case 0xcf1221: nv = 0x6699cf; sc = 1.0f; break;
-            case 0xfc9966: nv = 0x1221fc; sc = 1.0f; break;
-            case 0x1221fc: nv = 0xfc9966; sc = 1.0f; break;
-            default: return v;
+            case 0x47d47a: nv = 0xd22a33; return 2;
+            case 0xd22a33: nv = 0x47d47a; return 2;
+            case 0xa74d74: nv = 0x33a22d; return 2;
+            case 0x33a22d: nv = 0xa74d74; return 2;
+            case 0x8eb558: nv = 0x331eb1; return 2;
+            case 0x331eb1: nv = 0x8eb558; return 2;
+            case 0x855be8: nv = 0x1be133; return 2;
+            case 0x1be133: nv = 0x855be8; return 2;
+            case 0x6699cf: nv = 0xcf1221; return 2;
+            case 0xcf1221: nv = 0x6699cf; return 2;
+            case 0xfc9966: nv = 0x1221fc; return 2;
+            case 0x1221fc: nv = 0xfc9966; return 2;
+            default: return 0;
         }
-        const float ratio = __fdiv_rn(weight(a, nv), weight(a, v));
-        const float x = sc == 1.0f ? rd : __fmul_rn(__fsub_rn(rd, sc), 4.0f);
-        return ratio >= x ? nv : v;
+    }
+    __device__ static float scaled(uint32_t k) {
+        return __fdiv_rn(__fsub_rn(__uint_as_float(k | 0x3f800000u), 1.0f), 0.9f);
+    }
+    // Whether the move of kind `kind` of draw k, in `quarter`, is kept.
+    __device__ static bool kept(float ratio, int kind, int quarter, uint32_t k) {
+        const float rd = scaled(k);
+        return ratio >= (kind == 2 ? rd : __fmul_rn(__fsub_rn(rd, (float)quarter * 0.25f), 4.0f));
+    }
+    template <class A>
+    __device__ static int flip(int v, uint32_t k, const A& a) {
+        if (!(__fsub_rn(__uint_as_float(k | 0x3f800000u), 1.0f) < 0.9f)) return v;
+        const float rd = scaled(k);
+        const int quarter = rd < 0.25f ? 0 : rd < 0.5f ? 1 : rd < 0.75f ? 2 : 3;
+        int nv = v;
+        const int kind = propose(v, quarter, nv);
+        if (kind == 0) return v;
+        return kept(__fdiv_rn(weight(a, nv), weight(a, v)), kind, quarter, k) ? nv : v;
     }
 };
 

@@ -148,7 +148,7 @@ extern "C" rt_status rt_walk_device_noalloc(const rt_config* cfg, int32_t* d_til
         std::string perr;  // filled only on a failure path
         WalkPlan plan;
         // The kernel rt_walk would run for this walk (word kernel for the int8
-        // models, the generic walk kernel otherwise).
+        // models, the rectangle-triangle kernel, the generic one for what they do not hold).
         s = choose_plan(family, cfg->device, 1, rows, cols, width, true, false, false, false, false, 0, 0, 0, &plan,
                         &perr);
         if (s != RT_OK) {

@@ -38,88 +38,6 @@ namespace rtb {
 constexpr int kWordBlockMax = 512;  // threads that keep 2 or 4 words' generator states each
 constexpr int kWordBlockMid = 640;  // 65,536 registers / 96, in whole warps
 
-// ---------------------------------------------------------------------------
-// Exchange of the rows next to a band.  A row of the colour flipped in phase
-// p is published as tagged 64-bit words (32 bits of lattice, p + 1), double
-// buffered by the parity of p; its reader is the thread that owns the word
-// next to it, which polls the words it needs in phase p + 1 (never a copy of
-// the row in shared memory), so a wait costs its own warp and no barrier.  A
-// CTA publishes phase p + 2 only after it read its neighbour's phase p + 1,
-// which the neighbour published after reading phase p: a slot is rewritten
-// only after it was read.
-//   CLUSTER = false: slots in global memory (any number of co-resident CTAs).
-//   CLUSTER = true: the CTAs are one thread-block cluster and a row is written
-//   straight into its reader's shared memory.
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t cluster_addr(uint32_t saddr, int rank) {
-    uint32_t r;
-    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
-    return r;
-}
-
-template <bool CLUSTER>
-struct WordExchange {
-    const WalkArgs& a;
-    unsigned long long* inbox;  // CLUSTER: [side][parity][lattice][word] in this CTA's shared memory
-    int cta;
-
-    __device__ __forceinline__ int at(int side, int par, int l, int w) const {
-        return ((side * 2 + par) * a.nlat + l) * a.xwords + w;
-    }
-    __device__ __forceinline__ unsigned long long poll(const unsigned long long* p) const {
-        if (!CLUSTER) return ld_relaxed64(p);
-        unsigned long long x;
-        asm volatile("ld.relaxed.cluster.shared::cta.u64 %0, [%1];"
-                     : "=l"(x)
-                     : "r"((uint32_t)__cvta_generic_to_shared(p))
-                     : "memory");
-        return x;
-    }
-    // Words w and w2 (both polled in one round trip; w2 = w: one word) of the
-    // row above (side 0) or below (side 1) the band, tagged `tag`.
-    __device__ __forceinline__ bool read(int side, int par, int l, int w, int w2, uint32_t tag,
-                                         uint32_t (&out)[2]) const {
-        const unsigned long long* row =
-            CLUSTER ? inbox + at(side, par, l, 0) : slot(a, side == 0 ? cta - 1 : cta + 1, 1 - side, par, l, 0);
-        unsigned spins = 0;
-        uint64_t t0 = 0;
-        for (;;) {
-            const unsigned long long x = poll(row + w), y = w2 == w ? x : poll(row + w2);
-            if ((uint32_t)(x >> 32) == tag && (uint32_t)(y >> 32) == tag) {
-                out[0] = (uint32_t)x;
-                out[1] = (uint32_t)y;
-                return true;
-            }
-            if ((++spins & (CLUSTER ? 1023u : 63u)) == 0u) {
-                if (*(volatile int*)a.err) return false;
-                const uint64_t now = global_ns();
-                if (t0 == 0) {
-                    t0 = now;
-                } else if (now - t0 > a.timeout_ns) {
-                    atomicOr(a.err, ERR_TIMEOUT);
-                    return false;
-                }
-            }
-        }
-    }
-    // Word w of the band's first (side 0) or last (side 1) row for the CTA above / below.
-    __device__ __forceinline__ void write(int side, int par, int l, int w, uint32_t tag, uint32_t v) const {
-        const unsigned long long x = (unsigned long long)tag << 32 | v;
-        if (CLUSTER) {
-            // the upper CTA receives it as its row below, the lower one as its row above
-            const uint32_t mine = (uint32_t)__cvta_generic_to_shared(inbox + at(1 - side, par, l, w));
-            const uint32_t theirs = cluster_addr(mine, side == 0 ? cta - 1 : cta + 1);
-            asm volatile("st.relaxed.cluster.shared::cluster.u64 [%0], %1;" ::"r"(theirs), "l"(x) : "memory");
-        } else {
-            st_relaxed64(slot(a, cta, side, par, l, 0) + w, x);
-        }
-    }
-};
-
-__device__ __forceinline__ void cluster_sync_all() {
-    asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
-}
-
 // Shared memory: the inbox (CLUSTER), 16 bytes of slack, then for each lattice
 // NC colour planes of (band rows + 2) x wpad bytes, then 16 bytes of slack
 // (the funnel shifts read one word beyond a row; those bytes only reach sites
