@@ -48,10 +48,23 @@ __device__ __forceinline__ void unpack_word(T* row, int w, uint32_t v) {
         row[w] = (T)v;
 }
 
-// Waits for one tagged word; returns false on timeout (a.timeout_ns from the
-// first check of this wait's clock) or when another CTA already reported an
+// Whether a wait goes on: false on timeout (a.timeout_ns from the first check
+// of this wait's clock t0, 0 before it) or when another CTA already reported an
 // error.  The clock starts at this wait, so a walk may run for any length of
 // time; only a single wait is bounded.
+__device__ __forceinline__ bool wait_more(const WalkArgs& a, uint64_t& t0) {
+    if (*(volatile int*)a.err) return false;
+    const uint64_t now = global_ns();
+    if (t0 == 0) {
+        t0 = now;
+    } else if (now - t0 > a.timeout_ns) {
+        atomicOr(a.err, ERR_TIMEOUT);
+        return false;
+    }
+    return true;
+}
+
+// Waits for one tagged word; returns false where wait_more does.
 __device__ __forceinline__ bool wait_word(const WalkArgs& a, const unsigned long long* p, uint32_t tag,
                                           uint32_t* out) {
     unsigned spins = 0;
@@ -62,16 +75,7 @@ __device__ __forceinline__ bool wait_word(const WalkArgs& a, const unsigned long
             *out = (uint32_t)x;
             return true;
         }
-        if ((++spins & 63u) == 0u) {
-            if (*(volatile int*)a.err) return false;
-            const uint64_t now = global_ns();
-            if (t0 == 0) {
-                t0 = now;
-            } else if (now - t0 > a.timeout_ns) {
-                atomicOr(a.err, ERR_TIMEOUT);
-                return false;
-            }
-        }
+        if ((++spins & 63u) == 0u && !wait_more(a, t0)) return false;
     }
 }
 
@@ -127,16 +131,7 @@ struct WordExchange {
                 out[1] = (uint32_t)y;
                 return true;
             }
-            if ((++spins & (CLUSTER ? 1023u : 63u)) == 0u) {
-                if (*(volatile int*)a.err) return false;
-                const uint64_t now = global_ns();
-                if (t0 == 0) {
-                    t0 = now;
-                } else if (now - t0 > a.timeout_ns) {
-                    atomicOr(a.err, ERR_TIMEOUT);
-                    return false;
-                }
-            }
+            if ((++spins & (CLUSTER ? 1023u : 63u)) == 0u && !wait_more(a, t0)) return false;
         }
     }
     // Word w of the band's first (side 0) or last (side 1) row for the CTA above / below.

@@ -1,4 +1,6 @@
-// rt_plane.cu -- the bit-plane walk kernel of the int8 models (RT_RNG_PLANES).
+// rt_plane.cu -- the bit-plane walk kernel of the int8 models (RT_RNG_PLANES)
+// for bands of more than 2,048 words of a plane; smaller ones, which is most,
+// run the kernel of rt_planeband.cu by the same rules.
 //
 // Dominoes and uniform lozenges keep 4 / 6 edge bits per site.  Here a
 // colour array lives in shared memory as 4 / 6 bit planes, one 32-bit word
@@ -34,36 +36,16 @@
 #include "rt_exchange.cuh"
 #include "rt_internal.h"
 #include "rt_models.cuh"
+#include "rt_plane.cuh"
 #include "rt_word.cuh"
 
 namespace rtb {
 
-template <int FAM>
-struct PlaneModel {
-    static constexpr bool DOM = FAM != FAM_LOZENGE8;
-    static constexpr int NC = DOM ? 2 : 3;  // colour arrays
-    static constexpr int NP = DOM ? 4 : 6;  // bit planes per colour
-    static constexpr int ROFF = DOM ? 1 : 0;
-    static constexpr int COFF = DOM ? 1 : 0;
-};
-
-__device__ __forceinline__ uint32_t col_next(uint32_t cur, uint32_t nxt) { return __funnelshift_r(cur, nxt, 1); }
-__device__ __forceinline__ uint32_t col_prev(uint32_t prv, uint32_t cur) { return __funnelshift_l(prv, cur, 1); }
-
-// Bits [lo, hi) of the 32 columns starting at column 32 w.
-__device__ __forceinline__ uint32_t col_mask(int w, int lo, int hi) {
-    const int a = max(lo - 32 * w, 0), b = min(hi - 32 * w, 32);
-    if (b <= a) return 0u;
-    const uint32_t upper = b >= 32 ? 0xffffffffu : ((1u << b) - 1u);
-    return upper & ~((1u << a) - 1u);
-}
-
 // Shared memory: planes [lattice][colour][plane][stored row][RS words];
 // stored row s is colour-array row a0 - H + s; word 0 and word WW + 1 of a
 // row are zero padding for the funnel shifts; then two masks per word.
-// WPT: words per work item -- 1 (small bands: the most parallelism; the
-// four words of a Philox call each recompute it) or 4 (one call per item).
-template <int FAM, int LB, int WPT>
+// A work item is the four words of a Philox call.
+template <int FAM, int LB>
 __global__ void __launch_bounds__(LB, 1) plane_kernel(const __grid_constant__ WalkArgs a) {
     using M = PlaneModel<FAM>;
     constexpr int NC = M::NC, NP = M::NP;
@@ -195,7 +177,7 @@ __global__ void __launch_bounds__(LB, 1) plane_kernel(const __grid_constant__ Wa
             // rows computed in this phase (global band-row index g)
             const int g_lo = max(0, r0 - H + k + 1), g_hi = min(a.rows, r1 + H - k - 1);
             const int s_lo = g_lo - (r0 - H);
-            const int IPR = WPT == 1 ? WW : QPR;  // work items per row
+            const int IPR = QPR;  // work items per row
             const int items = (g_hi - g_lo) * IPR;
             // Plane offsets (32-bit shared-memory word indices) used by this phase,
             // lattice 0; lattice l adds l * LAT.
@@ -220,7 +202,7 @@ __global__ void __launch_bounds__(LB, 1) plane_kernel(const __grid_constant__ Wa
                 const int i = a0 - H + s;  // colour-array row
                 uint4 r1 = make_uint4(0u, 0u, 0u, 0u), r2 = make_uint4(0u, 0u, 0u, 0u);
                 if (draws) {
-                    const uint32_t c0 = (uint32_t)((i - M::ROFF) * QPR + (WPT == 1 ? (it >> 2) : it));
+                    const uint32_t c0 = (uint32_t)((i - M::ROFF) * QPR + it);
                     r1 = philox4(c0, (uint32_t)dstep, (uint32_t)((uint64_t)dstep >> 32), a.chain, key0, key1);
                     if (FAM == FAM_DOMINO)
                         r2 = philox4(c0 | 0x80000000u, (uint32_t)dstep, (uint32_t)((uint64_t)dstep >> 32), a.chain,
@@ -230,8 +212,8 @@ __global__ void __launch_bounds__(LB, 1) plane_kernel(const __grid_constant__ Wa
                 const int p = (i ^ tt) & 1;                                                  // dominoes
                 const uint32_t sh = M::DOM ? 0u : (shifts >> (9 * tt + 3 * (i % 3))) & 7u;  // lozenges
 #pragma unroll
-                for (int x4 = 0; x4 < WPT; ++x4) {
-                const int w = WPT == 1 ? it : 4 * it + x4;
+                for (int x4 = 0; x4 < 4; ++x4) {
+                const int w = 4 * it + x4;
                 if (w >= WW) break;
                 const int o = s * RS + w + 1;
                 const uint32_t um = row_upd ? um_col[w] : 0u;
@@ -391,16 +373,15 @@ __global__ void __launch_bounds__(LB, 1) plane_kernel(const __grid_constant__ Wa
 using PlaneFn = void (*)(WalkArgs);
 
 template <int FAM>
-static PlaneFn plane_fn_of(int block, int wpt) {
-    if (wpt == 4) return block > 512 ? plane_kernel<FAM, 1024, 4> : plane_kernel<FAM, 512, 4>;
-    return block > 512 ? plane_kernel<FAM, 1024, 1> : plane_kernel<FAM, 512, 1>;
+static PlaneFn plane_fn_of(int block) {
+    return block > 512 ? plane_kernel<FAM, 1024> : plane_kernel<FAM, 512>;
 }
 
-static PlaneFn plane_fn(int family, int block, int wpt) {
+static PlaneFn plane_fn(int family, int block) {
     switch (family) {
-        case FAM_DOMINO: return plane_fn_of<FAM_DOMINO>(block, wpt);
-        case FAM_DOMINO_HB: return plane_fn_of<FAM_DOMINO_HB>(block, wpt);
-        case FAM_LOZENGE8: return plane_fn_of<FAM_LOZENGE8>(block, wpt);
+        case FAM_DOMINO: return plane_fn_of<FAM_DOMINO>(block);
+        case FAM_DOMINO_HB: return plane_fn_of<FAM_DOMINO_HB>(block);
+        case FAM_LOZENGE8: return plane_fn_of<FAM_LOZENGE8>(block);
         default: return nullptr;
     }
 }
@@ -411,6 +392,7 @@ rt_status plan_plane_walk(int family, int device, int nlat, int rows, int width,
         *err = "bit-plane walks exist for dominoes and uniform lozenges";
         return RT_E_INVAL;
     }
+    if (plan_plane_band(family, device, nlat, rows, width, ctas_hint, depth_hint, plan, err) == RT_OK) return RT_OK;
     int sms = 0, smem_optin = 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
         cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) != cudaSuccess) {
@@ -433,15 +415,11 @@ rt_status plan_plane_walk(int family, int device, int nlat, int rows, int width,
         *err = "band does not fit in shared memory";
         return RT_E_INVAL;
     }
-    // Work items of the widest phase (band + 2 (depth - 1) rows): one word
-    // each while that keeps 1024 threads busy at most twice, else four words
-    // (one Philox call each).  The halo exchange uses every thread, so small
-    // bands still launch 512.
-    const int words = (rpc + 2 * (depth - 1)) * ww;
-    const int wpt = words > 2048 ? 4 : 1;
-    const int items = wpt == 4 ? (rpc + 2 * (depth - 1)) * ((ww + 3) / 4) : words;
+    // Work items of the widest phase (band + 2 (depth - 1) rows).  The halo
+    // exchange uses every thread, so small bands still launch 512.
+    const int items = (rpc + 2 * (depth - 1)) * ((ww + 3) / 4);
     const int block = items > 512 ? 1024 : 512;
-    PlaneFn fn = plane_fn(family, block, wpt);
+    PlaneFn fn = plane_fn(family, block);
     if (cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
         *err = "cudaFuncSetAttribute failed";
         return RT_E_CUDA;
