@@ -52,7 +52,8 @@ __device__ __forceinline__ void unpack_word(T* row, int w, uint32_t v) {
 // of this wait's clock t0, 0 before it) or when another CTA already reported an
 // error.  The clock starts at this wait, so a walk may run for any length of
 // time; only a single wait is bounded.
-__device__ __forceinline__ bool wait_more(const WalkArgs& a, uint64_t& t0) {
+template <class A>  // the kernel's arguments: err, timeout_ns
+__device__ __forceinline__ bool wait_more(const A& a, uint64_t& t0) {
     if (*(volatile int*)a.err) return false;
     const uint64_t now = global_ns();
     if (t0 == 0) {

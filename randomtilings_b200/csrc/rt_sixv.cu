@@ -21,10 +21,12 @@
 #include <cstring>
 #include <random>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/rt_b200_sixv.h"
 #include "rt_device.cuh"
+#include "rt_exchange.cuh"
 #include "rt_internal.h"
 #include "rt_guard.h"
 
@@ -65,20 +67,31 @@ __global__ void __launch_bounds__(256) sixv_step_kernel(const __grid_constant__ 
 }
 
 // ---------------------------------------------------------------------------
-// The heights on chip for a whole epoch: CTA c owns face rows [r0, r1) of
-// every lattice in shared memory (row stride sp = n + 1 rounded up to even,
-// plus the rows r0 - 1 and r1 as halo).  Each colour step updates the band's
-// faces of its class exactly as sixv_step_kernel does (same draws, same
-// rule).  Steps 2t and 2t + 1 update rows of one parity, so the halo rows
-// (the other parity) cannot change between them: after each odd step the
-// band's first and last rows go to the neighbours through tagged 64-bit
-// global slots (32 bits of heights and the step + 1), double-buffered by
-// the parity of the exchange's number, and a CTA reads its halo rows before
-// each even step.  A CTA publishes exchange t + 1 only after it read
-// exchange t, which each neighbour published after reading exchange t - 1
-// from it, so a slot is rewritten only after it was read.  Every wait is
-// bounded: past timeout_ns the CTA sets ERR_TIMEOUT in *err and returns, and
-// the others see it.  The launch is cooperative, so every CTA is resident.
+// The heights on chip for a whole epoch.  CTA c owns face rows [r0, r1) of
+// every lattice and keeps them, with H rows above and below, in shared memory
+// as two planes: the even columns and the odd ones (4 Q halfwords a row each,
+// column 2 x + parity at x).  The four faces of a work item, and the same
+// columns of any row, are then one 64-bit access, and faces go two to a
+// register: with m the height above a face, the others are compared by
+// exclusive or, and the diagonals, which differ from m by one where it matters,
+// by a subtraction whose borrow a set top bit keeps out of the other half.
+//
+// Steps 2t and 2t + 1 update rows of one parity from themselves and the rows
+// next to them, so after a pair of steps one row less on each side of the band
+// is current: H pairs run between two exchanges, the halo rows recomputed by
+// both CTAs (the draws depend on the face and the step only).  Then the band's
+// first and last H rows go to the neighbours through tagged 64-bit global slots
+// (32 bits of heights and the exchange's number), double-buffered by its
+// parity.  A CTA publishes exchange t + 1 only after it read exchange t, which
+// each neighbour published after reading exchange t - 1 from it, so a slot is
+// rewritten only after it was read.  Every wait is bounded: past timeout_ns the
+// CTA sets ERR_TIMEOUT in *err and returns, and the others see it.  The launch
+// is cooperative, so every CTA is resident.
+//
+// What bounds it: the arithmetic -- a Philox call a quad (73 issue cycles a warp),
+// the logic of the rule at half rate -- and the latency of a step (0.26 us at n =
+// 10).  n = 1000: 400 steps take 0.38 ms (0.9 us a step; 2.4 with int16 accesses
+// one by one and an exchange every two steps).
 // ---------------------------------------------------------------------------
 struct SixvBandArgs {
     int16_t* h[2];
@@ -86,7 +99,7 @@ struct SixvBandArgs {
     uint32_t chain, k0, k1;
     uint32_t thr[16];
     int64_t steps;
-    int rows_per_cta, sp, xwords;
+    int rows_max, H, xwords;   // most rows of a CTA; halo rows; slot words of a side: H rows x 4 Q
     unsigned long long* xbuf;  // [cta][side][parity][lattice][xwords]
     int* err;
     uint64_t timeout_ns;
@@ -96,122 +109,175 @@ __device__ __forceinline__ unsigned long long* sixv_slot(const SixvBandArgs& a, 
     return a.xbuf + ((((size_t)cta * 2 + side) * 2 + par) * a.nlat + l) * a.xwords;
 }
 
-__device__ __forceinline__ bool sixv_wait(const SixvBandArgs& a, const unsigned long long* p, uint32_t tag,
-                                          uint32_t* out) {
-    unsigned spins = 0;
-    uint64_t t0 = 0;
-    for (;;) {
-        unsigned long long x;
-        asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(x) : "l"(p) : "memory");
-        if ((uint32_t)(x >> 32) == tag) {
-            *out = (uint32_t)x;
-            return true;
-        }
-        if ((++spins & 63u) == 0u) {
-            if (*(volatile int*)a.err) return false;
-            const uint64_t now = global_ns();
-            if (t0 == 0) {
-                t0 = now;
-            } else if (now - t0 > a.timeout_ns) {
-                atomicOr(a.err, ERR_TIMEOUT);
-                return false;
-            }
-        }
-    }
-}
-
-template <int NLAT>
+// ONE: the sixteen thresholds are equal, and neither 0 nor 2^23 (as with equal
+// weights): the diagonals need not be looked at.
+template <int NLAT, bool ONE>
 __global__ void __launch_bounds__(1024, 1) sixv_band_kernel(const __grid_constant__ SixvBandArgs a) {
-    extern __shared__ __align__(16) int16_t sh[];
-    const int S = a.n + 1, sp = a.sp, X = a.xwords;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ uint32_t s_thr[16];
+    int16_t* const sh = reinterpret_cast<int16_t*>(smem_raw);
+    const int S = a.n + 1, Q = a.Q, ST = 4 * Q, H = a.H, X = a.xwords;
     const int cta = blockIdx.x, nct = gridDim.x, tid = threadIdx.x, BLOCK = blockDim.x;
-    const int r0 = min(S, cta * a.rows_per_cta), r1 = min(S, r0 + a.rows_per_cta), nrows = r1 - r0;
-    const int plane = (a.rows_per_cta + 2) * sp;  // per lattice; band row i sits at row i - r0 + 1
+    const int r0 = (int)((int64_t)cta * S / nct), r1 = (int)((int64_t)(cta + 1) * S / nct), nrows = r1 - r0;
+    const int base = r0 - H;                         // face row of stored row 0
+    const int plane = (a.rows_max + 2 * H) * ST;     // halfwords of one parity
+    const bool has_top = cta > 0, has_bot = cta + 1 < nct;
+    if (tid < 16) s_thr[tid] = a.thr[tid];
     for (int l = 0; l < NLAT; ++l)
-        for (int e = tid; e < (nrows + 2) * sp; e += BLOCK) {
-            const int rr = r0 - 1 + e / sp, j = e % sp;
-            sh[l * plane + e] = rr >= 0 && rr < S && j < S ? a.h[l][(size_t)rr * S + j] : (int16_t)0;
+        for (int e = tid; e < (nrows + 2 * H) * 2 * ST; e += BLOCK) {
+            const int rr = e / (2 * ST), j = e - rr * 2 * ST, i = base + rr;
+            sh[(2 * l + (j & 1)) * plane + rr * ST + (j >> 1)] =
+                i >= 0 && i < S && j < S ? a.h[l][(size_t)i * S + j] : (int16_t)0;
         }
+
+    // The launch has a multiple of Q threads: a thread keeps its column.
+    const int q = tid % Q, rr0 = tid / Q, dr = BLOCK / Q;
+    // the faces of the quad that move, two to a register, by column parity
+    auto inside = [&](int j) { return (j >= 1 && j < a.n ? 0x2u : 0u) | (j + 2 < a.n ? 0x20000u : 0u); };
+    const uint32_t in0[2] = {inside(8 * q), inside(8 * q + 1)}, in2[2] = {inside(8 * q + 4), inside(8 * q + 5)};
+    auto draws = [&](int i, int64_t st) {
+        return philox4((uint32_t)(i * Q + q), (uint32_t)st, (uint32_t)((uint64_t)st >> 32), a.chain, a.k0, a.k1);
+    };
+
+    const uint32_t one = a.thr[0] << 9;
+    // The four faces (i, 8 q + PJ + 2 b) of every lattice.
+    auto item = [&](auto pj, int i, const uint4& w4) {
+        constexpr int PJ = decltype(pj)::value;
+#pragma unroll
+        for (int l = 0; l < NLAT; ++l) {
+            int16_t* const P = sh + (2 * l + PJ) * plane + (i - base) * ST + 4 * q;
+            const int16_t* const O = sh + (2 * l + 1 - PJ) * plane + (i - base) * ST + 4 * q;
+            const uint2 up = *reinterpret_cast<const uint2*>(P - ST), dn = *reinterpret_cast<const uint2*>(P + ST);
+            const uint2 old = *reinterpret_cast<const uint2*>(P);
+            // the columns left and right of the faces, in the rows above, at and below
+            uint32_t L01[3], L23[3], R01[3], R23[3];
+#pragma unroll
+            for (int y = 0; y < 3; ++y) {
+                if (ONE && y != 1) continue;
+                const int16_t* const row = O + (y - 1) * ST;
+                const uint2 v = *reinterpret_cast<const uint2*>(row);
+                // beyond a row's ends this is another row's face, which only masked ones see
+                const uint32_t ext = (uint16_t)row[PJ ? 4 : -1];
+                const uint32_t mid = __byte_perm(v.x, v.y, 0x5432);
+                L01[y] = PJ ? v.x : __byte_perm(ext, v.x, 0x5410);
+                L23[y] = PJ ? v.y : mid;
+                R01[y] = PJ ? mid : v.x;
+                R23[y] = PJ ? __byte_perm(v.y, ext, 0x5432) : v.y;
+            }
+            // Neighbours of a face differ from one another by 0 or 2, and what
+            // differs by 2 differs in bit 1: so one logic operation compares two
+            // pairs of them.
+            auto two = [&](uint32_t m, uint32_t below, const uint32_t(&L)[3], const uint32_t(&R)[3], uint32_t in,
+                           uint32_t was, uint32_t wa, uint32_t wb) -> uint32_t {
+                const uint32_t flat = ~((below ^ m) | (L[1] ^ m) | (R[1] ^ m)) & in;  // bit 1 of each half
+                const uint32_t high = m + 0x00010001u;
+                bool la, lb;  // the draw takes m - 1
+                if (ONE) {
+                    la = wa >= one;
+                    lb = wb >= one;
+                } else {
+                    // a diagonal is m + 1 where its bit 1 is that of m + 1
+                    const uint32_t d0 = ~(L[0] ^ high) & 0x00020002u, d1 = ~(R[0] ^ high) & 0x00020002u;
+                    const uint32_t d2 = ~(L[2] ^ high) & 0x00020002u, d3 = ~(R[2] ^ high) & 0x00020002u;
+                    const uint32_t p = d0 + 2u * d1 + 4u * d2 + 8u * d3;
+                    la = wa >> 9 >= s_thr[p >> 1 & 15u];
+                    lb = wb >> 9 >= s_thr[p >> 17];
+                }
+                // m >= 1 in every flat face: no borrow
+                const uint32_t v = high - (((la ? 0x2u : 0u) | (lb ? 0x20000u : 0u)) & flat);
+                const uint32_t mask = (flat >> 1) * 0xffffu;
+                return (was & ~mask) | (v & mask);
+            };
+            uint2 out;
+            out.x = two(up.x, dn.x, L01, R01, in0[PJ], old.x, w4.x, w4.y);
+            out.y = two(up.y, dn.y, L23, R23, in2[PJ], old.y, w4.z, w4.w);
+            *reinterpret_cast<uint2*>(P) = out;
+        }
+    };
+    using C0 = std::integral_constant<int, 0>;
+    using C1 = std::integral_constant<int, 1>;
+
     __syncthreads();
-    for (int64_t s = 0; s < a.steps; ++s) {
-        if (s > 0 && (s & 1) == 0) {
-            // halo rows: the neighbours' edge rows after step s - 1 (exchange s / 2)
-            bool ok = true;
-            const int par = (int)((s >> 1) & 1);
-            const uint32_t tag = (uint32_t)s;
-            for (int e = tid; e < 2 * NLAT * X && ok; e += BLOCK) {
-                const int side = e >= NLAT * X, rem = e - side * NLAT * X, l = rem / X, w = rem - l * X;
-                const int from = side == 0 ? cta - 1 : cta + 1;
-                if (from < 0 || from >= nct || nrows <= 0) continue;
-                uint32_t v;
-                ok = sixv_wait(a, sixv_slot(a, from, 1 - side, par, l) + w, tag, &v);
-                if (ok)
-                    reinterpret_cast<uint32_t*>(sh + l * plane + (side == 0 ? 0 : nrows + 1) * sp)[w] = v;
-            }
-            if (__syncthreads_or(!ok)) return;
-        }
-        // this step's class: row parity (s mod 4) / 2, column parity s mod 2
-        const int pi = (int)((s & 3) >> 1), pj = (int)(s & 1);
-        const int par_row = pi == 0 ? 0 : 1;  // rows 2, 4, .. or 1, 3, .. up to n - 1
-        const int lo = max(r0, 1), hi = min(r1, a.n);
-        const int first = lo + ((lo & 1) != par_row);
+    int k = 0;          // pairs of steps since the last exchange
+    uint32_t blk = 0;   // exchanges made
+    for (int64_t s = 0; s < a.steps; s += 2) {
+        // rows of the pair's parity that are computed: within the lattice, one
+        // less on each side with every pair
+        const int odd = (int)(s >> 1 & 1);  // the first pair takes the even rows
+        const int lo = max(1, has_top ? base + 1 + k : r0), hi = min(a.n, has_bot ? r1 + H - 1 - k : r1);
+        const int first = lo + ((lo & 1) != odd);
         const int nlive = first < hi ? (hi - first + 1) / 2 : 0;
-        const uint32_t s_lo = (uint32_t)s, s_hi = (uint32_t)((uint64_t)s >> 32);
-        for (int u = tid; u < nlive * a.Q; u += BLOCK) {
-            const int rr = u / a.Q, q = u - rr * a.Q;
-            const int i = first + 2 * rr;
-            const uint4 w4 = philox4((uint32_t)(i * a.Q + q), s_lo, s_hi, a.chain, a.k0, a.k1);
-            const int j0 = 8 * q + pj;  // the faces j0, j0 + 2, j0 + 4, j0 + 6
-            // Columns j0 - 1 .. j0 + 7 clamped to the row: a clamped column
-            // serves only faces outside 1 .. n - 1, which are skipped.  All
-            // reads come before the writes (no face of the class is another's
-            // neighbour), so they need not wait on them.
-            int col[9];
-#pragma unroll
-            for (int t = 0; t < 9; ++t) col[t] = min(max(j0 - 1 + t, 0), sp - 1);
-#pragma unroll
-            for (int l = 0; l < NLAT; ++l) {
-                int16_t* row = sh + l * plane + (i - r0 + 1) * sp;
-                int up[9], dn[9], md[5];
-#pragma unroll
-                for (int t = 0; t < 9; ++t) {
-                    up[t] = row[col[t] - sp];
-                    dn[t] = row[col[t] + sp];
-                }
-#pragma unroll
-                for (int t = 0; t < 5; ++t) md[t] = row[col[2 * t]];
-#pragma unroll
-                for (int b = 0; b < 4; ++b) {
-                    const int j = j0 + 2 * b, m = up[2 * b + 1];
-                    if (j < 1 || j > a.n - 1 || dn[2 * b + 1] != m || md[b] != m || md[b + 1] != m) continue;
-                    const int p = (up[2 * b] > m) | ((up[2 * b + 2] > m) << 1) | ((dn[2 * b] > m) << 2) |
-                                  ((dn[2 * b + 2] > m) << 3);
-                    const uint32_t k = quad_word(w4, b) >> 9;
-                    row[j] = (int16_t)(k < a.thr[p] ? m + 1 : m - 1);
-                }
+        if (nlive <= dr) {
+            // one item a thread: the draws of both steps are made together
+            const int i = first + 2 * rr0;
+            uint4 w0, w1;
+            if (rr0 < nlive) {
+                w0 = draws(i, s);
+                w1 = draws(i, s + 1);
+                item(C0{}, i, w0);
             }
+            __syncthreads();
+            if (rr0 < nlive) item(C1{}, i, w1);
+        } else {
+            for (int rr = rr0; rr < nlive; rr += dr) item(C0{}, first + 2 * rr, draws(first + 2 * rr, s));
+            __syncthreads();
+            for (int rr = rr0; rr < nlive; rr += dr) item(C1{}, first + 2 * rr, draws(first + 2 * rr, s + 1));
         }
         __syncthreads();
-        if ((s & 1) && s + 1 < a.steps && nrows > 0) {
-            // the band's first and last rows, for the neighbours' next two steps
-            const int par = (int)(((s + 1) >> 1) & 1);
-            const unsigned long long tag = (unsigned long long)(uint32_t)(s + 1) << 32;
-            for (int e = tid; e < 2 * NLAT * X; e += BLOCK) {
-                const int side = e >= NLAT * X, rem = e - side * NLAT * X, l = rem / X, w = rem - l * X;
-                const int to = side == 0 ? cta - 1 : cta + 1;
-                if (to < 0 || to >= nct) continue;
-                const uint32_t v =
-                    reinterpret_cast<const uint32_t*>(sh + l * plane + (side == 0 ? 1 : nrows) * sp)[w];
-                unsigned long long* dst = sixv_slot(a, cta, side, par, l) + w;
-                asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(dst), "l"(tag | v) : "memory");
+        ++k;
+        if (nct == 1 || k < H || s + 2 >= a.steps) continue;
+
+        // Row y of a side's H rows, quad q: slot words (4 y + z) Q + q, z = 0, 1 the
+        // quad's even columns, 2, 3 its odd ones.
+        const int par = (int)(blk & 1u);
+        const uint32_t tag = blk + 1u;
+#pragma unroll
+        for (int l = 0; l < NLAT; ++l)
+            for (int yy = rr0; yy < 2 * H; yy += dr) {
+                const int side = yy >= H, y = yy - side * H;
+                if (side == 0 ? !has_top : !has_bot) continue;
+                const int16_t* const row = sh + 2 * l * plane + ((side == 0 ? H : nrows) + y) * ST + 4 * q;
+                const uint2 ev = *reinterpret_cast<const uint2*>(row), od = *reinterpret_cast<const uint2*>(row + plane);
+                unsigned long long* const to = sixv_slot(a, cta, side, par, l) + 4 * y * Q + q;
+                const unsigned long long t = (unsigned long long)tag << 32;
+                st_relaxed64(to, t | ev.x);
+                st_relaxed64(to + Q, t | ev.y);
+                st_relaxed64(to + 2 * Q, t | od.x);
+                st_relaxed64(to + 3 * Q, t | od.y);
             }
-        }
+        bool ok = true;
+#pragma unroll
+        for (int l = 0; l < NLAT; ++l)
+            for (int yy = rr0; yy < 2 * H; yy += dr) {
+                const int side = yy >= H, y = yy - side * H;
+                if (side == 0 ? !has_top : !has_bot) continue;
+                const unsigned long long* const from =
+                    sixv_slot(a, side == 0 ? cta - 1 : cta + 1, 1 - side, par, l) + 4 * y * Q + q;
+                // the four words in one round trip, again until the last one is there
+                unsigned long long v[4];
+                unsigned spins = 0;
+                uint64_t t0 = 0;
+                for (;;) {
+                    bool here = true;
+#pragma unroll
+                    for (int z = 0; z < 4; ++z) v[z] = ld_relaxed64(from + z * Q);
+#pragma unroll
+                    for (int z = 0; z < 4; ++z) here = here && (uint32_t)(v[z] >> 32) == tag;
+                    if (here || !ok) break;
+                    if ((++spins & 63u) == 0u) ok = wait_more(a, t0);
+                }
+                int16_t* const row = sh + 2 * l * plane + ((side == 0 ? 0 : H + nrows) + y) * ST + 4 * q;
+                *reinterpret_cast<uint2*>(row) = make_uint2((uint32_t)v[0], (uint32_t)v[1]);
+                *reinterpret_cast<uint2*>(row + plane) = make_uint2((uint32_t)v[2], (uint32_t)v[3]);
+            }
+        if (__syncthreads_or(!ok)) return;
+        k = 0;
+        ++blk;
     }
-    __syncthreads();
     for (int l = 0; l < NLAT; ++l)
         for (int e = tid; e < nrows * S; e += BLOCK) {
             const int rr = e / S, j = e - rr * S;
-            a.h[l][(size_t)(r0 + rr) * S + j] = sh[l * plane + (rr + 1) * sp + j];
+            a.h[l][(size_t)(r0 + rr) * S + j] = sh[(2 * l + (j & 1)) * plane + (H + rr) * ST + (j >> 1)];
         }
 }
 
@@ -358,17 +424,29 @@ rt_status run_epoch(rt_sixv* h, int n, int nlat, int64_t sweeps, uint64_t key, u
     {
         // The band kernel, when every CTA's rows (and halo) fit shared memory.
         int dev = 0, sms = 0, optin = 0;
-        const int S = n + 1, sp = (S + 1) & ~1;
+        const int S = n + 1;
         if (cudaGetDevice(&dev) == cudaSuccess &&
             cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
             cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) == cudaSuccess && sms > 0) {
-            int ctas = std::min(sms, S);
-            const int rpc = (S + ctas - 1) / ctas;
-            ctas = (S + rpc - 1) / rpc;
-            const size_t smem = (size_t)nlat * (rpc + 2) * sp * sizeof(int16_t);
-            const size_t xbytes = (size_t)ctas * 2 * 2 * nlat * (sp / 2) * sizeof(unsigned long long);
-            const void* band_fn = nlat == 2 ? (const void*)sixv_band_kernel<2> : (const void*)sixv_band_kernel<1>;
-            bool ready = smem <= (size_t)optin &&
+            // Microseconds per step: n = 30 0.28 on one CTA, 0.37 on four; n = 64
+            // 0.44 on one, 0.39 on eight; n = 200 0.49 with bands of six rows, 0.45
+            // of four; n = 400 0.66 and 0.52.  An exchange takes 1.5 us or so: n =
+            // 1000 (bands of 7 rows) 0.97 with H = 1, 0.93 with 2, 0.91 with 3 or 4,
+            // 1.0 with 6; n = 2000 (14 rows) 2.24 with 1, 1.99 with 2, 2.41 with 4;
+            // n = 3500 5.2 with 1, 4.4 with 2.
+            int ctas = (int64_t)S / 2 * a.Q <= 128 ? 1 : std::min(sms, std::max(1, S / 4));
+            auto rows_max = [&]() { return (S + ctas - 1) / ctas; };
+            int H = ctas == 1 ? 1 : std::min(rows_max() <= 8 ? 4 : 2, S / ctas);
+            auto bytes = [&]() { return (size_t)nlat * (rows_max() + 2 * H) * 8 * a.Q * sizeof(int16_t); };
+            while (H > 1 && bytes() > (size_t)optin) --H;
+            const size_t smem = bytes();
+            const size_t xbytes = (size_t)ctas * 2 * 2 * nlat * (H * 4 * a.Q) * sizeof(unsigned long long);
+            bool one = h->thr[0] > 0 && h->thr[0] < 1u << 23;
+            for (int t = 1; t < 16; ++t) one = one && h->thr[t] == h->thr[0];
+            const void* band_fn = nlat == 2 ? (one ? (const void*)sixv_band_kernel<2, true> : (const void*)sixv_band_kernel<2, false>)
+                                            : (one ? (const void*)sixv_band_kernel<1, true> : (const void*)sixv_band_kernel<1, false>);
+            const int block = std::max(1, 1024 / a.Q) * a.Q;
+            bool ready = block <= 1024 && smem + sizeof(uint32_t[16]) <= (size_t)optin &&
                          cudaFuncSetAttribute(band_fn,
                                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess;
             if (ready && xbytes > h->xcap) {
@@ -392,9 +470,9 @@ rt_status run_epoch(rt_sixv* h, int n, int nlat, int64_t sweeps, uint64_t key, u
                 b.k1 = a.k1;
                 std::memcpy(b.thr, a.thr, sizeof b.thr);
                 b.steps = 4 * sweeps;
-                b.rows_per_cta = rpc;
-                b.sp = sp;
-                b.xwords = sp / 2;
+                b.rows_max = rows_max();
+                b.H = H;
+                b.xwords = H * 4 * a.Q;
                 b.xbuf = h->d_xbuf;
                 b.err = h->d_err;
                 b.timeout_ns = 5000000000ull;
@@ -402,8 +480,8 @@ rt_status run_epoch(rt_sixv* h, int n, int nlat, int64_t sweeps, uint64_t key, u
                 cudaError_t e = cudaMemsetAsync(h->d_xbuf, 0, xbytes, h->stream);
                 if (e == cudaSuccess) e = cudaMemsetAsync(h->d_err, 0, sizeof(int), h->stream);
                 if (e == cudaSuccess)
-                    e = cudaLaunchCooperativeKernel(band_fn, dim3((unsigned)ctas), dim3(1024),
-                                                    args, smem, h->stream);
+                    e = cudaLaunchCooperativeKernel(band_fn, dim3((unsigned)ctas), dim3((unsigned)block), args, smem,
+                                                    h->stream);
                 if (e == cudaSuccess) {
                     int flag = 0;
                     e = cudaMemcpyAsync(&flag, h->d_err, sizeof flag, cudaMemcpyDeviceToHost, h->stream);
