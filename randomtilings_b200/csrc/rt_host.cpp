@@ -1177,4 +1177,32 @@ bool boundary_walk(int model, const int32_t* d, int64_t dlen, int* n_out, std::v
     return true;
 }
 
+// ---- six-vertex rows -------------------------------------------------------
+// Compiled for wide vectors too: a row is 16 bits a face, and these three passes
+// are most of what a short walk of a large lattice waits for.
+#define RT_WIDE __attribute__((target_clones("avx2", "default")))
+
+RT_WIDE void sixv_narrow_row(const int32_t* __restrict__ from, int count, int16_t* __restrict__ to) {
+    for (int j = 0; j < count; ++j) to[j] = (int16_t)std::min(32767, std::max(-32768, from[j]));
+}
+
+RT_WIDE bool sixv_row_ok(const int16_t* row_, const int16_t* above_, int n, int i) {
+    const uint16_t* const row = reinterpret_cast<const uint16_t*>(row_);
+    const uint16_t* const above = reinterpret_cast<const uint16_t*>(above_);
+    uint16_t bad = (uint16_t)((row[0] ^ i) | (row[n] ^ (n - i)));
+    if (i == 0)
+        for (int j = 0; j <= n; ++j) bad |= (uint16_t)(row[j] ^ j);
+    if (i == n)
+        for (int j = 0; j <= n; ++j) bad |= (uint16_t)(row[j] ^ (n - j));
+    // a difference d is +-1 iff d + 1 is 0 or 2
+    for (int j = 0; j < n; ++j) bad |= (uint16_t)((uint16_t)(row[j + 1] - row[j] + 1) & 0xfffd);
+    if (above)
+        for (int j = 0; j <= n; ++j) bad |= (uint16_t)((uint16_t)(row[j] - above[j] + 1) & 0xfffd);
+    return bad == 0;
+}
+
+RT_WIDE void sixv_widen(const int16_t* __restrict__ from, size_t count, int32_t* __restrict__ to) {
+    for (size_t j = 0; j < count; ++j) to[j] = from[j];
+}
+
 }  // namespace rtb

@@ -115,6 +115,16 @@ bool lipschitz_graph(int model, const int32_t* d, int64_t dlen, int* n_out, std:
 bool boundary_walk(int model, const int32_t* d, int64_t dlen, int* n_out, std::vector<int64_t>* idx,
                    std::vector<int32_t>* h);
 
+// Six-vertex height rows on the host (rt_host.cpp).  Narrowing saturates.
+// sixv_row_ok: row i (and `above`, row i - 1, null for i = 0) of the heights of an
+// n x n domain wall: boundary values, and edges that join heights differing by 1.
+// Rows that all pass are exactly a domain-wall height function: every face then
+// lies within n / 2 edges of the boundary's 0..n <= 32,000 and, modulo 2^16,
+// between the extremal heights, which no saturated value is.
+void sixv_narrow_row(const int32_t* from, int count, int16_t* to);
+bool sixv_row_ok(const int16_t* row, const int16_t* above, int n, int i);
+void sixv_widen(const int16_t* from, size_t count, int32_t* to);
+
 // Host split of a triangle-dimer tiling into its eight M x M arrays
 // (H, L, R, U, D, BH, BL, BR), rt_host.cpp.
 void td_split_host(const int32_t* t, int n, int32_t* arrays);
