@@ -170,34 +170,8 @@ __global__ void __launch_bounds__(LB, 1) word_kernel(const __grid_constant__ Wal
             }
         }
     };
-    // What the draws of one step do, as byte masks (word_phase): combined into
-    // m0 / m1, which hold what the run's earlier steps did.  Within a run the
-    // sites' neighbours do not change, so a rotatable site stays rotatable:
-    // toggles add up modulo 2, and of the other rules' draws the last one that
-    // acts on a site decides.
     auto combine = [&](uint32_t d, const WordInfo& wi, const uint32_t (&k)[4], uint32_t& m0, uint32_t& m1) {
-        uint32_t lo;
-        if (WT == 1) {
-            // Periodic weights: a threshold per site from its vertex (i, j); array
-            // column c of the rotated array A is vertex column 2 c + ((i + A) & 1)
-            // (dominoes) or 3 c + (A + i) mod 3 (lozenges).
-            const int i = a0 + wi.off / W - 1, c0 = wi.off % W;
-            const int step = M::DOM ? 2 : 3;
-            const int j0 = step * c0 + (M::DOM ? (i + 1 - (int)ph_a(d)) & 1 : ((int)ph_a(d) + i) % 3);
-            lo = below4(k, 0u - weight_thr(a, i, j0), 0u - weight_thr(a, i, j0 + step),
-                        0u - weight_thr(a, i, j0 + 2 * step), 0u - weight_thr(a, i, j0 + 3 * step));
-        } else {
-            lo = below4(k, nt0);
-        }
-        if (FAM == FAM_DOMINO) {
-            m0 ^= lo;
-        } else if (FAM == FAM_DOMINO_HB) {
-            m0 = lo;
-        } else {
-            const uint32_t rem = below4(k, nt1) & (WT == 2 ? ~below4(k, 0u - (1u << 22)) : ~lo);
-            m0 = lo | (m0 & ~rem);
-            m1 = rem | (m1 & ~lo);
-        }
+        word_combine<FAM, WT>(a, d, a0 + wi.off / W - 1, wi.off % W, k, nt0, nt1, m0, m1);
     };
     auto philox_draws = [&](uint32_t d, int u, const WordInfo& wi, int64_t s, uint32_t& m0, uint32_t& m1) {
         m0 = m1 = 0u;
@@ -514,6 +488,8 @@ rt_status plan_word_walk(int family, int device, int nlat, int rows, int width, 
         *err = "no word kernel for this model";
         return RT_E_INVAL;
     }
+    // The fast mode's small and middle lattices run on bands with halos.
+    if (philox && plan_word_band(family, device, nlat, rows, width, ctas_hint, weighted, plan, err) == RT_OK) return RT_OK;
     int sms = 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) {
         *err = "cudaDeviceGetAttribute failed";

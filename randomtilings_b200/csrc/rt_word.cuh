@@ -201,6 +201,39 @@ __device__ __forceinline__ uint32_t lane_bytes(uint32_t bits) {
     return (bits & 1u) | ((bits & 2u) << 7) | ((bits & 4u) << 14) | ((bits & 8u) << 21);
 }
 
+// What the draws k of one step do to the word at array row i, columns c0 .. c0 + 3,
+// as the byte masks of WordOp: combined into m0 / m1, which hold what the run's
+// earlier steps did.  Within a run the sites' neighbours do not change, so a
+// rotatable site stays rotatable: toggles add up modulo 2, and of the other
+// rules' draws the last one that acts on a site decides.  nt0, nt1: the negated
+// thresholds (WT: rt_word.cu).
+template <int FAM, int WT>
+__device__ __forceinline__ void word_combine(const WalkArgs& a, uint32_t d, int i, int c0, const uint32_t (&k)[4],
+                                             uint32_t nt0, uint32_t nt1, uint32_t& m0, uint32_t& m1) {
+    constexpr bool DOM = FAM != FAM_LOZENGE8;
+    uint32_t lo;
+    if (WT == 1) {
+        // Periodic weights: a threshold per site from its vertex (i, j); array
+        // column c of the rotated array A is vertex column 2 c + ((i + A) & 1)
+        // (dominoes) or 3 c + (A + i) mod 3 (lozenges).
+        const int step = DOM ? 2 : 3;
+        const int j0 = step * c0 + (DOM ? (i + 1 - (int)ph_a(d)) & 1 : ((int)ph_a(d) + i) % 3);
+        lo = below4(k, 0u - weight_thr(a, i, j0), 0u - weight_thr(a, i, j0 + step), 0u - weight_thr(a, i, j0 + 2 * step),
+                    0u - weight_thr(a, i, j0 + 3 * step));
+    } else {
+        lo = below4(k, nt0);
+    }
+    if (FAM == FAM_DOMINO) {
+        m0 ^= lo;
+    } else if (FAM == FAM_DOMINO_HB) {
+        m0 = lo;
+    } else {
+        const uint32_t rem = below4(k, nt1) & (WT == 2 ? ~below4(k, 0u - (1u << 22)) : ~lo);
+        m0 = lo | (m0 & ~rem);
+        m1 = rem | (m1 & ~lo);
+    }
+}
+
 __device__ __forceinline__ uint32_t lozenge_shift_table(int t) {
     uint32_t tab = 0;
 #pragma unroll
