@@ -647,19 +647,19 @@ rt_status upload(rt_batch* b) {
             void* arr[8] = {};
             for (int a = 0; a < c.ncol; ++a) arr[a] = base + a * c.per_arr;
             if (c.kind == 3) {
-                std::vector<int32_t> arrays((size_t)8 * c.arows * c.width);
-                td_split_host(c.start.data(), c.n, arrays.data());
-                // dimer covers only
-                const size_t per = (size_t)c.arows * c.width;
-                for (size_t e = 0; e < 8 * per; ++e) {
-                    const int32_t v = arrays[e];
-                    if (v < 0 || v >= (1 << tdp::cover_bits_of((int)(e / per))))
-                        return b->fail(RT_E_INVAL, "triangle-dimer state out of range for the bit planes");
-                }
-                for (int a = 0; a < 8; ++a)
-                    cudaMemcpyAsync(arr[a], arrays.data() + (size_t)a * c.arows * c.width,
-                                    (size_t)c.arows * c.width * 4, cudaMemcpyHostToDevice, b->stream);
-                cudaStreamSynchronize(b->stream);
+                const size_t tb = (size_t)c.n * c.n * 4;
+                if (!tmp.reserve(tb + 256)) return b->fail(RT_E_NOMEM, "staging buffer");
+                uint32_t* const over = reinterpret_cast<uint32_t*>(static_cast<char*>(tmp.p) + tb);
+                cudaMemcpyAsync(tmp.p, c.start.data(), tb, cudaMemcpyHostToDevice, b->stream);
+                std::string e;
+                if (launch_td_split(static_cast<int32_t*>(tmp.p), c.n, true, static_cast<int32_t*>(arr[0]), c.per_arr / 4,
+                                    over, b->stream, &e) != RT_OK)
+                    return b->fail(RT_E_CUDA, e);
+                uint32_t bad = 0;
+                cudaMemcpyAsync(&bad, over, sizeof bad, cudaMemcpyDeviceToHost, b->stream);
+                const cudaError_t ce = cudaStreamSynchronize(b->stream);
+                if (ce != cudaSuccess) return b->fail(RT_E_CUDA, std::string("batch upload: ") + cudaGetErrorString(ce));
+                if (bad) return b->fail(RT_E_INVAL, "triangle-dimer state out of range for the bit planes");  // dimer covers only
             } else {
                 const size_t tb = (size_t)c.n * c.n * 4;
                 if (!tmp.reserve(tb)) return b->fail(RT_E_NOMEM, "staging buffer");

@@ -515,18 +515,16 @@ rt_status rt_upload(rt_tiler* h, const int32_t* tiling, int32_t n) {
         e = cudaMemcpyAsync(h->d_tiling.p, tiling, (size_t)n * n * 4, cudaMemcpyHostToDevice, h->stream);
         if (e != cudaSuccess) return h->cuda_fail(e, "upload");
         if (h->kind == 3) {
-            // The eight triangle-dimer arrays are derived on the host
-            // (TriangleDimerTiler.cpp:90-133) and copied up as they are.
-            std::vector<int32_t> arrays((size_t)8 * arows * width);
-            td_split_host(tiling, n, arrays.data());
-            const size_t per = (size_t)arows * width;
-            uint32_t over = 0;
-            for (int c = 0; c < 8; ++c)
-                for (size_t e = 0; e < per; ++e) over |= (uint32_t)arrays[c * per + e] >> tdp::bits_of(c);
-            h->td_fits = over == 0;
-            for (int c = 0; c < 8 && e == cudaSuccess; ++c)
-                e = cudaMemcpy(h->d_arr[0][c], arrays.data() + (size_t)c * arows * width, per_arr, cudaMemcpyHostToDevice);
+            // The eight triangle-dimer arrays are derived from the tiling
+            // (TriangleDimerTiler.cpp:90-133).
+            if (!h->d_err.reserve(sizeof(int)) || !h->h_err.reserve(sizeof(int))) return h->fail(RT_E_NOMEM, "error word");
+            s = launch_td_split(static_cast<int32_t*>(h->d_tiling.p), n, false, static_cast<int32_t*>(h->d_arr[0][0]),
+                                per_arr_al / 4, static_cast<uint32_t*>(h->d_err.p), h->stream, &h->err);
+            if (s != RT_OK) return s;
+            e = cudaMemcpyAsync(h->h_err.p, h->d_err.p, sizeof(int), cudaMemcpyDeviceToHost, h->stream);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
             if (e != cudaSuccess) return h->cuda_fail(e, "upload of the triangle-dimer arrays");
+            h->td_fits = *static_cast<int*>(h->h_err.p) == 0;
         } else {
             s = launch_split(false, h->elem, h->kind, h->ncol, n, static_cast<int32_t*>(h->d_tiling.p), h->d_arr[0],
                              h->stream, &h->err);

@@ -24,6 +24,7 @@
 #include "../../include/rt_b200.h"
 #include "../../include/rt_b200_host.h"
 #include "rt_guard.h"
+#include "rt_tdderive.h"
 
 using rtb::guarded;
 
@@ -852,85 +853,14 @@ rt_status rt_tridimer_test_butterfly(int32_t kind, int32_t* out, int64_t cap, in
 }  // extern "C"
 
 namespace rtb {
-// Triangle-flip states ((N/2) x N) and butterfly-flip states (N x N) of a
-// tiling (TilingToTriangleFlips / TilingToButterflyFlips,
-// TriangleDimerTiler.cpp:385-460).
+// Triangle-flip states ((N/2) x N) and butterfly-flip states (N x N) of a tiling.
 void td_derived_states(const int32_t* t, int n, int32_t* tri, int32_t* bfl) {
-    auto T = [&](int i, int j) { return t[(size_t)i * n + j]; };
-    std::fill(tri, tri + (size_t)(n / 2) * n, 0);
-    std::fill(bfl, bfl + (size_t)n * n, 0);
-    auto b = [](int32_t x, int k) { return (x >> k) & 1; };
-    for (int i = 1; i < n / 2 - 1; ++i)
-        for (int j = 1; j < n - 1; ++j) {
-            const int32_t a = T(2 * i + 1, j), c = T(2 * i + 1, j + 1);
-            int d0, d1, d2;
-            if (j % 2 == 0) {  // down triangle
-                const int32_t u = T(2 * i, j + 1);
-                d0 = b(a, 2) + 2 * b(a, 3) + 3 * b(c, 3);
-                d1 = b(c, 2) + 2 * b(a, 1) + 3 * b(c, 1);
-                d2 = 2 * b(u, 0) + b(a, 0) + 3 * b(u, 1);
-            } else {  // up triangle
-                const int32_t w = T(2 * i + 2, j);
-                d0 = b(a, 0) + 2 * b(a, 3) + 3 * b(c, 3);
-                d1 = b(c, 0) + 2 * b(a, 1) + 3 * b(c, 1);
-                d2 = 2 * b(w, 3) + 3 * b(w, 2) + b(a, 2);
-            }
-            tri[(size_t)i * n + j] = d0 + 4 * d1 + 16 * d2;
-        }
-    for (int i = 2; i < n - 2; ++i)
-        for (int j = 2; j < n - 2; ++j) {
-            const int32_t x = T(i, j);
-            int f1, f4, f16, f64, c;
-            if (i % 2 == 0) {
-                if (j % 2 == 0) continue;
-                const int32_t u = T(i - 1, j), ue = T(i - 1, j + 1), d = T(i + 1, j), dw = T(i + 1, j - 1);
-                f1 = b(u, 3) + 2 * b(u, 0) + 3 * b(x, 0);
-                f4 = b(ue, 0) + 2 * b(ue, 1) + 3 * b(x, 1);
-                f16 = b(d, 1) + 2 * b(d, 2) + 3 * b(x, 2);
-                f64 = b(dw, 2) + 2 * b(dw, 3) + 3 * b(x, 3);
-                c = b(ue, 2);
-            } else if (j % 2 == 0) {
-                const int32_t ue = T(i - 1, j + 1), e = T(i, j + 1), dw = T(i + 1, j - 1), w = T(i, j - 1);
-                f1 = b(ue, 0) + 2 * b(ue, 1) + 3 * b(x, 0);
-                f4 = b(e, 1) + 2 * b(e, 2) + 3 * b(x, 1);
-                f16 = b(dw, 2) + 2 * b(dw, 3) + 3 * b(x, 2);
-                f64 = b(w, 3) + 2 * b(w, 0) + 3 * b(x, 3);
-                c = b(e, 3);
-            } else {
-                const int32_t u = T(i - 1, j), e = T(i, j + 1), d = T(i + 1, j), w = T(i, j - 1);
-                f1 = b(u, 0) + 2 * b(u, 1) + 3 * b(x, 0);
-                f4 = b(e, 0) + 2 * b(e, 1) + 3 * b(x, 1);
-                f16 = b(d, 2) + 2 * b(d, 3) + 3 * b(x, 2);
-                f64 = b(w, 2) + 2 * b(w, 3) + 3 * b(x, 3);
-                c = b(e, 3);
-            }
-            bfl[(size_t)i * n + j] = f1 + 4 * f4 + 16 * f16 + 64 * f64 + 256 * c;
-        }
+    for (int i = 0; i < n / 2; ++i)
+        for (int j = 0; j < n; ++j) tri[(size_t)i * n + j] = td_triangle_state(t, n, i, j);
+    for (int i = 0; i < n; ++i)
+        for (int j = 0; j < n; ++j) bfl[(size_t)i * n + j] = td_butterfly_state(t, n, i, j);
 }
 
-// The eight M x M arrays the walk runs on (TriangleDimerTiler.cpp:107-133),
-// in the order H, L, R, U, D, BH, BL, BR.
-void td_split_host(const int32_t* t, int n, int32_t* arrays) {
-    const int m = n / 2;
-    const size_t mm = (size_t)m * m;
-    Vec tri((size_t)(n / 2) * n), bfl((size_t)n * n);
-    td_derived_states(t, n, tri.data(), bfl.data());
-    std::fill(arrays, arrays + 8 * mm, 0);
-    for (int i = 0; i < n; ++i)
-        for (int j = 0; j < n; ++j) {
-            const size_t at = (size_t)(i / 2) * m + j / 2;
-            const size_t src = (size_t)i * n + j;
-            if (i % 2 == 0) {
-                if (j % 2 == 1) arrays[0 * mm + at] = t[src], arrays[5 * mm + at] = bfl[src];
-            } else if (j % 2 == 0) {
-                arrays[1 * mm + at] = t[src], arrays[6 * mm + at] = bfl[src];
-            } else {
-                arrays[2 * mm + at] = t[src], arrays[7 * mm + at] = bfl[src];
-            }
-        }
-    for (int i = 0; i < n / 2; ++i)
-        for (int j = 0; j < n; ++j) arrays[(j % 2 == 0 ? 4 : 3) * mm + (size_t)i * m + j / 2] = tri[(size_t)i * n + j];
-}
 }  // namespace rtb
 
 extern "C" {

@@ -129,9 +129,11 @@ void sixv_narrow_row(const int32_t* from, int count, int16_t* to);
 bool sixv_row_ok(const int16_t* row, const int16_t* above, int n, int i);
 void sixv_widen(const int16_t* from, size_t count, int32_t* to);
 
-// Host split of a triangle-dimer tiling into its eight M x M arrays
-// (H, L, R, U, D, BH, BL, BR), rt_host.cpp.
-void td_split_host(const int32_t* t, int n, int32_t* arrays);
+// The eight arrays of a triangle-dimer tiling (device pointers; array c at
+// arrays + c stride), and in *over whether some value does not fit a dimer
+// cover's bits (cover) or the bit planes (rt_walk.cu).
+rt_status launch_td_split(const int32_t* tiling, int n, bool cover, int32_t* arrays, size_t stride, uint32_t* over,
+                          cudaStream_t stream, std::string* err);
 
 // Counts differing 32-bit words of a and b (bytes must be a multiple of 4).
 rt_status launch_count_diff(const void* a, const void* b, size_t bytes, unsigned long long* d_count,

@@ -10,6 +10,8 @@
 #include "rt_internal.h"
 #include "rt_models.cuh"
 #include "rt_exchange.cuh"
+#include "rt_tdderive.h"
+#include "rt_tdplane.cuh"
 #include "rt_tridimer.cuh"
 
 namespace rtb {
@@ -430,6 +432,50 @@ __global__ void merge_kernel(int32_t* __restrict__ t, int n, int ncol, int kind,
     }
     const T* src = c == 0 ? a0 : c == 1 ? a1 : a2;
     t[idx] = (int32_t)src[(int64_t)i * w + col];
+}
+
+// The eight m x m arrays (m = n / 2) the triangle-dimer walk runs on
+// (TriangleDimerTiler.cpp:107-133), in the order H, L, R, U, D, BH, BL, BR, one
+// thread a place; `over` gets the bits that no array of a dimer cover has, or
+// (cover = false) that the bit planes do not hold.  On the host the arrays of a
+// 272 x 272 tiling took 0.5 ms.
+__global__ void td_split_kernel(const int32_t* __restrict__ t, int n, bool cover, int32_t* arrays, size_t stride,
+                                uint32_t* over) {
+    const int m = n / 2, at = blockIdx.x * blockDim.x + threadIdx.x;
+    uint32_t high = 0;
+    if (at < m * m) {
+        const int i = at / m, j = at - i * m;
+        const int y[3] = {2 * i, 2 * i + 1, 2 * i + 1}, x[3] = {2 * j + 1, 2 * j, 2 * j + 1};
+        int32_t v[8];
+#pragma unroll
+        for (int o = 0; o < 3; ++o) {
+            v[o] = t[(size_t)y[o] * n + x[o]];
+            v[5 + o] = td_butterfly_state(t, n, y[o], x[o]);
+        }
+        v[3] = td_triangle_state(t, n, i, 2 * j + 1);
+        v[4] = td_triangle_state(t, n, i, 2 * j);
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+            arrays[c * stride + at] = v[c];
+            high |= (uint32_t)v[c] >> (cover ? tdp::cover_bits_of(c) : tdp::bits_of(c));
+        }
+    }
+    if (high) atomicOr(over, 1u);
+}
+
+rt_status launch_td_split(const int32_t* tiling, int n, bool cover, int32_t* arrays, size_t stride, uint32_t* over,
+                          cudaStream_t stream, std::string* err) {
+    const int64_t total = (int64_t)(n / 2) * (n / 2);
+    cudaError_t e = cudaMemsetAsync(over, 0, sizeof *over, stream);
+    if (e == cudaSuccess && total > 0) {
+        td_split_kernel<<<(unsigned)((total + 127) / 128), 128, 0, stream>>>(tiling, n, cover, arrays, stride, over);
+        e = cudaGetLastError();
+    }
+    if (e != cudaSuccess) {
+        *err = std::string("triangle-dimer split failed: ") + cudaGetErrorString(e);
+        return RT_E_CUDA;
+    }
+    return RT_OK;
 }
 
 rt_status launch_split(bool merge, int elem_bytes, int kind, int ncol, int n, int32_t* tiling, void* const* arr,
