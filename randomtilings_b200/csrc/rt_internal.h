@@ -58,9 +58,9 @@ bool word_family(int family);
 // weighted: the instantiation that reads per-site thresholds (WalkArgs::wper > 0).
 rt_status plan_word_walk(int family, int device, int nlat, int rows, int width, bool philox, int ctas_hint,
                          WalkPlan* plan, std::string* err, bool weighted = false);
-// The same in the fast mode, one word per thread, on bands with halo rows
-// (rt_wordband.cu); an error if the bands do not fit it.
-rt_status plan_word_band(int family, int device, int nlat, int rows, int width, int ctas_hint, bool weighted,
+// The same, one word per thread, on bands with halo rows (rt_wordband.cu); an
+// error if the bands do not fit it.
+rt_status plan_word_band(int family, int device, int nlat, int rows, int width, bool philox, int ctas_hint, bool weighted,
                          WalkPlan* plan, std::string* err);
 // Bit-plane kernel of a single triangle-dimer walk (rt_td.cu), for arrays whose
 // values fit its planes, on one cluster of ctas_hint CTAs (<= 0: by size).

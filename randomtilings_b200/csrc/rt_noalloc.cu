@@ -149,8 +149,12 @@ extern "C" rt_status rt_walk_device_noalloc(const rt_config* cfg, int32_t* d_til
         WalkPlan plan;
         // The kernel rt_walk would run for this walk (word kernel for the int8
         // models, the rectangle-triangle kernel, the generic one for what they do not hold).
-        s = choose_plan(family, cfg->device, 1, rows, cols, width, true, false, false, false, false, 0, 0, 0, &plan,
-                        &perr);
+        auto replan = [&](int ctas_hint) {
+            plan = WalkPlan();
+            return choose_plan(family, cfg->device, 1, rows, cols, width, true, false, false, false, false, 0, ctas_hint, 0,
+                               &plan, &perr);
+        };
+        s = replan(0);
         if (s != RT_OK) {
             say(errbuf, errcap, "%s", perr.c_str());
             return s;
@@ -162,7 +166,14 @@ extern "C" rt_status rt_walk_device_noalloc(const rt_config* cfg, int32_t* d_til
         const size_t off_ph = per_arr * ncol;
         const size_t off_ep = off_ph + align256((size_t)nph * 4);
         const size_t off_x = off_ep + 256;
-        const size_t xbytes = (size_t)plan.ctas * 2 * 2 * plan.xslots * plan.xwords * sizeof(unsigned long long);
+        auto slots = [&] { return (size_t)plan.ctas * 2 * 2 * plan.xslots * plan.xwords * sizeof(unsigned long long); };
+        // Bands with halos exchange several rows at a time; a walk that leaves no
+        // room for that takes the kernel that exchanges one.
+        if (off_x + align256(slots()) + 256 > kScratchBytes && replan(-1) != RT_OK) {
+            say(errbuf, errcap, "%s", perr.c_str());
+            return RT_E_INVAL;
+        }
+        const size_t xbytes = slots();
         const size_t off_err = off_x + align256(xbytes);
         const size_t need = off_err + 256;
         if (need > kScratchBytes) {

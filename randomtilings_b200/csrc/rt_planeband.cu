@@ -251,8 +251,8 @@ __global__ void __launch_bounds__(kBandBlock, 1) plane_band_kernel(const __grid_
     };
 
     __syncthreads();
-    int blk = 0;  // halo exchanges made (modulo 2^32, as the tags)
-    int k = 0;    // phases since the last one
+    uint32_t blk = 0;  // halo exchanges made (modulo 2^32, as the tags)
+    int k = 0;         // phases since the last one
     const int s_top = has_top ? 1 : H, s_bot = H + nrows + (has_bot ? H - 1 : 0);
     // After phase k of a block the rows within H - k - 1 of the band are
     // current; rows beyond them may hold anything until the next exchange.
@@ -280,8 +280,8 @@ __global__ void __launch_bounds__(kBandBlock, 1) plane_band_kernel(const __grid_
     // come from them.  A slot is rewritten two blocks later, after the
     // neighbour's next rows were read, which it sent after reading this one.
     auto exchange = [&]() -> bool {
-        const int par = blk & 1;
-        const uint32_t tag = (uint32_t)blk + 1u;
+        const int par = (int)(blk & 1u);
+        const uint32_t tag = blk + 1u;
         if (live && !(cta == 0 && blk == a.drop_phase)) {
             auto publish = [&](int side, int r, int j) {
 #pragma unroll

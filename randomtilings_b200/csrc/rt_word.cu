@@ -488,8 +488,10 @@ rt_status plan_word_walk(int family, int device, int nlat, int rows, int width, 
         *err = "no word kernel for this model";
         return RT_E_INVAL;
     }
-    // The fast mode's small and middle lattices run on bands with halos.
-    if (philox && plan_word_band(family, device, nlat, rows, width, ctas_hint, weighted, plan, err) == RT_OK) return RT_OK;
+    // Small and middle lattices run on bands with halos (ctas_hint < 0: not wanted).
+    if (ctas_hint >= 0 &&
+        plan_word_band(family, device, nlat, rows, width, philox, ctas_hint, weighted, plan, err) == RT_OK)
+        return RT_OK;
     int sms = 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) {
         *err = "cudaDeviceGetAttribute failed";
