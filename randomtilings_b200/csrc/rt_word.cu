@@ -20,9 +20,10 @@
 // What bounds it: the integer work of the draws (about 100 instructions a
 // word and step), the latency of one word's update, and the exchange.  On the
 // a = b = c = 500 hexagon (148 CTAs) a step takes 0.98 us, 1.83 with a phase
-// per step, a halo row copied through shared memory and a block-wide vote; on
-// the Aztec diamond of order 100 (one cluster of 16) 0.43 us, 1.35 before; of
-// order 24 (one CTA) 0.34 us, 1.33 before.
+// per step, a halo row copied through shared memory and a block-wide vote.
+// Lattices whose bands have room for halo rows run on rt_wordband.cu; on one
+// cluster of 16 this kernel takes 0.43 us on the Aztec diamond of order 100
+// (1.35 before, 0.38 there), on one CTA 0.34 at order 24 (1.33, 0.28).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -176,12 +177,11 @@ __global__ void __launch_bounds__(LB, 1) word_kernel(const __grid_constant__ Wal
     auto philox_draws = [&](uint32_t d, int u, const WordInfo& wi, int64_t s, uint32_t& m0, uint32_t& m1) {
         m0 = m1 = 0u;
         if (!(d & PH_DRAWS)) return;
-        for (uint32_t c = 0; c < ph_steps(d); ++c, ++s) {
-            const uint4 w4 =
-                philox4((uint32_t)(a0 * Gw + u), (uint32_t)s, (uint32_t)((uint64_t)s >> 32), a.chain, key0, key1);
-            const uint32_t k[4] = {w4.x, w4.y, w4.z, w4.w};
-            combine(d, wi, k, m0, m1);
-        }
+        // the fast mode's colours go round in turn: one step a phase
+        const uint4 w4 =
+            philox4((uint32_t)(a0 * Gw + u), (uint32_t)s, (uint32_t)((uint64_t)s >> 32), a.chain, key0, key1);
+        const uint32_t k[4] = {w4.x, w4.y, w4.z, w4.w};
+        combine(d, wi, k, m0, m1);
     };
     // The masks of this thread's words for phase descriptor d.  They depend on
     // the draws alone, so they are made a phase ahead, while the rows the
@@ -204,7 +204,7 @@ __global__ void __launch_bounds__(LB, 1) word_kernel(const __grid_constant__ Wal
                 }
             }
         }
-        if (PHILOX && (d & PH_DRAWS)) dstep += ph_steps(d);
+        if (PHILOX && (d & PH_DRAWS)) ++dstep;
     };
 
     // Phases that need more than the plain loop body: those that begin an
@@ -314,7 +314,7 @@ __global__ void __launch_bounds__(LB, 1) word_kernel(const __grid_constant__ Wal
             range(has_top ? Gw : 0, nwords - (has_bot ? Gw : 0), 0u);
             if (has_top) range(0, Gw, one ? 6u : 2u);
             if (has_bot && !one) range(nwords - Gw, nwords, 4u);
-            if (d & PH_DRAWS) dstep += ph_steps(d);
+            if (d & PH_DRAWS) ++dstep;
         }
         d = d_next;
         d_next = d_after;

@@ -275,7 +275,8 @@ rt_status plan_word_band(int family, int device, int nlat, int rows, int width, 
     // Philox: Aztec diamonds of order 24 0.41 / 0.52, 50 0.48 / 0.65, 100 0.58 /
     // 0.75, 200 0.78 / 1.03, 300 (bands of 4 rows, H = 4) 0.99 / 1.00, 400 (6 rows,
     // H = 2) 1.44 / 1.10; hexagons of side 30 0.46 / 1.03, 100 0.62 / 0.80, 250 0.84 /
-    // 1.38, 400 1.19 / 1.28; volume weight, 190 x 131 x 83 0.68 / 1.20.
+    // 1.38, 400 1.19 / 1.28, 450 (H = 3) 1.26 / 1.42, 500 (H = 2) 1.44 / 1.46; Aztec
+    // diamond of order 350 (H = 3) 1.12 / 1.04; volume weight, 190 x 131 x 83 0.68 / 1.20.
     // TinyMT: Aztec diamonds of order 8 0.18 / 0.20, 24 0.28 / 0.35, 50 0.32 / 0.34,
     // 100 0.38 / 0.43, 200 0.48 / 0.56, 300 (H = 2) 0.54 / 0.55, 400 (803 words)
     // 0.94 / 0.64; hexagons of side 30 0.37 / 0.74, 60 0.40 / 0.51, 100 0.44 / 0.56,
@@ -284,7 +285,8 @@ rt_status plan_word_band(int family, int device, int nlat, int rows, int width, 
     // words (order 24: 0.41 on 4 CTAs, 0.48 on 11; order 50: 0.58, 0.48, 0.52 on 8,
     // 16, 26); of two where TinyMT's draws would be the longer part (order 200: 0.47
     // on 148 CTAs with H = 2, 0.53 on 100, 0.62 there with H = 4).  Philox halos of
-    // fewer than four rows and TinyMT bands beyond 640 words stay on rt_word.cu.
+    // fewer than four rows (lozenges: three) and TinyMT bands beyond 640 words stay
+    // on rt_word.cu.
     int ctas = ctas_hint;
     if (ctas <= 0) {
         const int band = std::max(!philox && gw > 40 ? 2 : 4, std::min(16, (philox ? 90 : 64) / gw));
@@ -292,7 +294,7 @@ rt_status plan_word_band(int family, int device, int nlat, int rows, int width, 
     }
     ctas = std::max(1, std::min(ctas, rows));
     const int rpc = (rows + ctas - 1) / ctas;
-    const int most = philox ? 16 : 8, least = ctas == 1 ? 1 : philox ? 4 : 2, room = philox ? 1024 : kWbBlockMid;
+    const int most = philox ? 16 : 8, least = ctas == 1 ? 1 : !philox ? 2 : nc == 3 ? 3 : 4, room = philox ? 1024 : kWbBlockMid;
     int depth = ctas == 1 ? 1 : std::min(most, rows / ctas);
     while (depth > least && (int64_t)(rpc + 2 * depth) * gw > (philox ? room : 360)) --depth;
     const int64_t words = (int64_t)(rpc + 2 * depth) * gw;
