@@ -8,6 +8,8 @@ from __future__ import annotations
 import os
 import subprocess
 import sys
+import tempfile
+from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
@@ -16,7 +18,7 @@ LIB = os.path.join(HERE, "librt_b200.so")
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
     "-lineinfo", "-O3", "-std=c++17",
-    "-Xcompiler", "-fPIC", "-shared",
+    "-Xcompiler", "-fPIC",
     # IEEE single-precision division and no FMA contraction surprises: the
     # rect-triangle acceptance test must match the host CPU bit for bit.
     "-prec-div=true", "-fmad=false",
@@ -52,10 +54,19 @@ def build(force: bool = False, verbose: bool = False) -> str:
     if not force and not needs_build():
         return LIB
     tmp = LIB + ".tmp"
-    cmd = [nvcc(), *NVCC_FLAGS, "-o", tmp, *sources(), "-lcudart"]
-    if verbose:
-        print(" ".join(cmd), file=sys.stderr)
-    subprocess.run(cmd, check=True, cwd=CSRC)
+
+    def run(cmd: list[str]) -> None:
+        if verbose:
+            print(" ".join(cmd), file=sys.stderr)
+        subprocess.run(cmd, check=True, cwd=CSRC)
+
+    # One compiler per source file, on all cores: one after the other they take
+    # six minutes and more.
+    with tempfile.TemporaryDirectory() as objs:
+        todo = [(f, os.path.join(objs, os.path.basename(f) + ".o")) for f in sources()]
+        with ThreadPoolExecutor(max_workers=os.cpu_count() or 1) as pool:
+            list(pool.map(lambda x: run([nvcc(), *NVCC_FLAGS, "-c", "-o", x[1], x[0]]), todo))
+        run([nvcc(), *NVCC_FLAGS, "-shared", "-o", tmp, *[o for _, o in todo], "-lcudart"])
     os.replace(tmp, LIB)
     return LIB
 

@@ -116,7 +116,7 @@ __global__ void __launch_bounds__(1024, 1) sixv_band_kernel(const __grid_constan
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ uint32_t s_thr[16];
     int16_t* const sh = reinterpret_cast<int16_t*>(smem_raw);
-    const int S = a.n + 1, Q = a.Q, ST = 4 * Q, H = a.H, X = a.xwords;
+    const int S = a.n + 1, Q = a.Q, ST = 4 * Q, H = a.H;
     const int cta = blockIdx.x, nct = gridDim.x, tid = threadIdx.x, BLOCK = blockDim.x;
     const int r0 = (int)((int64_t)cta * S / nct), r1 = (int)((int64_t)(cta + 1) * S / nct), nrows = r1 - r0;
     const int base = r0 - H;                         // face row of stored row 0
