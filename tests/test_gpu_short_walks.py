@@ -1,0 +1,71 @@
+"""Walks that end before the first halo exchange: a band's rows are written only
+after the neighbours have read them.  A withheld flag ends the walk with a timeout;
+walks of one step to just beyond a block of phases, on many CTAs and again and
+again, equal the oracle."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from oracle import pyoracle as po
+
+pytestmark = pytest.mark.gpu
+
+RT_E_TIMEOUT = -5
+REPEATS = 40
+
+
+def _start(rt, model, size):
+    if model == "lozenge":
+        return rt.LozengeTiler.MinTiling(rt.LozengeTiler.Hexagon(size, size, size))
+    return rt.DominoTiler.MinTiling(rt.DominoTiler.AztecDiamond(size))
+
+
+def _check(tiler, t, want, steps, seed):
+    for _ in range(REPEATS):
+        a = np.array(t, dtype=np.int32)
+        tiler.Walk(a, steps, seed)
+        assert np.array_equal(a, want)
+
+
+def _withheld(monkeypatch, make, t):
+    """The first CTA withholds its flag: its neighbour may not write."""
+    import randomtilings_b200 as rt
+
+    monkeypatch.setenv("RT_TEST_DROP_PUBLISH", "0")
+    monkeypatch.setenv("RT_WAIT_TIMEOUT_MS", "100")
+    a = np.array(t, dtype=np.int32)
+    with pytest.raises(rt.RtError) as e:
+        make().Walk(a, 1, 3)
+    assert e.value.status == RT_E_TIMEOUT
+
+
+# Order 47: 94 rows; side 40: 81 rows.
+@pytest.mark.parametrize("model", ["domino", "lozenge"])
+@pytest.mark.parametrize("rng", ["tinymt", "philox"])
+def test_word_bands_wait_for_their_neighbours(monkeypatch, model, rng):
+    import randomtilings_b200 as rt
+
+    monkeypatch.setenv("RT_WALK_CTAS", "9")
+    cls = rt.DominoTiler if model == "domino" else rt.LozengeTiler
+    _withheld(monkeypatch, lambda: cls(rng=getattr(rt, f"RT_RNG_{rng.upper()}")),
+              _start(rt, model, 47 if model == "domino" else 40))
+
+
+@pytest.mark.parametrize("model", ["domino", "lozenge"])
+@pytest.mark.parametrize("rng", ["tinymt", "philox"])
+@pytest.mark.parametrize("ctas", [2, 9, 0])
+@pytest.mark.parametrize("steps", [1, 2, 5, 9, 17])
+def test_short_word_band_walks(monkeypatch, model, rng, ctas, steps):
+    import randomtilings_b200 as rt
+
+    if ctas:
+        monkeypatch.setenv("RT_WALK_CTAS", str(ctas))
+    t = _start(rt, model, 47 if model == "domino" else 40)
+    cls = rt.DominoTiler if model == "domino" else rt.LozengeTiler
+    tl = cls(rng=getattr(rt, f"RT_RNG_{rng.upper()}"))
+    if rng == "philox":
+        want = po.walk_fast(model, t, steps, 11)
+    else:
+        want = (po.domino_walk if model == "domino" else po.lozenge_walk)(t, steps, 11)
+    _check(tl, t, want, steps, 11)
