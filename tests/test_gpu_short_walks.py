@@ -69,3 +69,26 @@ def test_short_word_band_walks(monkeypatch, model, rng, ctas, steps):
     else:
         want = (po.domino_walk if model == "domino" else po.lozenge_walk)(t, steps, 11)
     _check(tl, t, want, steps, 11)
+
+
+# Order 130: 260 rows; side 90: 270 rows.
+@pytest.mark.parametrize("model", ["domino", "lozenge"])
+def test_plane_bands_wait_for_their_neighbours(monkeypatch, model):
+    import randomtilings_b200 as rt
+
+    monkeypatch.setenv("RT_WALK_CTAS", "12")
+    cls = rt.DominoTiler if model == "domino" else rt.LozengeTiler
+    _withheld(monkeypatch, lambda: cls(rng=rt.RT_RNG_PLANES), _start(rt, model, 130 if model == "domino" else 90))
+
+
+@pytest.mark.parametrize("model", ["domino", "lozenge"])
+@pytest.mark.parametrize("ctas", [2, 12, 0])
+@pytest.mark.parametrize("steps", [1, 3, 20, 33])
+def test_short_plane_band_walks(monkeypatch, model, ctas, steps):
+    import randomtilings_b200 as rt
+
+    if ctas:
+        monkeypatch.setenv("RT_WALK_CTAS", str(ctas))
+    t = _start(rt, model, 130 if model == "domino" else 90)
+    cls = rt.DominoTiler if model == "domino" else rt.LozengeTiler
+    _check(cls(rng=rt.RT_RNG_PLANES), t, po.walk_planes(model, t, steps, 11), steps, 11)
