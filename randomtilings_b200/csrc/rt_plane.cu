@@ -106,6 +106,11 @@ __global__ void __launch_bounds__(LB, 1) plane_kernel(const __grid_constant__ Wa
     uint32_t key0 = 0, key1 = 0;
     int64_t dstep = 0;
     __syncthreads();
+    const bool no_exchange = nct > 1 && a.nphases <= H;
+    if (no_exchange && tid == 0 && !(cta == 0 && a.drop_phase == 0)) {
+        if (cta > 0) raise_loaded(slot(a, cta, 0, 0, 0, 0));
+        if (cta + 1 < nct) raise_loaded(slot(a, cta, 1, 0, 0, 0));
+    }
 
     int64_t blk = 0;
     for (int64_t b0 = 0; b0 < a.nphases; b0 += H, ++blk) {
@@ -354,7 +359,12 @@ __global__ void __launch_bounds__(LB, 1) plane_kernel(const __grid_constant__ Wa
         }
     }
 
-    __syncthreads();
+    bool ok = true;
+    if (no_exchange && tid == 0) {  // the neighbours may still be reading this band's rows
+        if (cta > 0) ok = wait_loaded(a, slot(a, cta - 1, 1, 0, 0, 0));
+        if (cta + 1 < nct) ok = ok && wait_loaded(a, slot(a, cta + 1, 0, 0, 0, 0));
+    }
+    if (__syncthreads_or(!ok)) return;
     // Store the band rows back as bytes.
     for (int l = 0; l < a.nlat; ++l)
         for (int c = 0; c < NC; ++c) {

@@ -92,3 +92,30 @@ def test_short_plane_band_walks(monkeypatch, model, ctas, steps):
     t = _start(rt, model, 130 if model == "domino" else 90)
     cls = rt.DominoTiler if model == "domino" else rt.LozengeTiler
     _check(cls(rng=rt.RT_RNG_PLANES), t, po.walk_planes(model, t, steps, 11), steps, 11)
+
+
+# Bands of more than 2,048 words (rt_plane.cu): order 500 on 5 CTAs, 201 rows of
+# 16 words; side 500 on 5, 202 rows of 11 words (12 with padding).
+PLANE = {"domino": (500, 5), "lozenge": (500, 5)}
+
+
+@pytest.mark.parametrize("model", ["domino", "lozenge"])
+def test_large_plane_bands_wait_for_their_neighbours(monkeypatch, model):
+    import randomtilings_b200 as rt
+
+    size, ctas = PLANE[model]
+    monkeypatch.setenv("RT_WALK_CTAS", str(ctas))
+    cls = rt.DominoTiler if model == "domino" else rt.LozengeTiler
+    _withheld(monkeypatch, lambda: cls(rng=rt.RT_RNG_PLANES), _start(rt, model, size))
+
+
+@pytest.mark.parametrize("model", ["domino", "lozenge"])
+@pytest.mark.parametrize("steps", [1, 6, 8])
+def test_short_large_plane_band_walks(monkeypatch, model, steps):
+    import randomtilings_b200 as rt
+
+    size, ctas = PLANE[model]
+    monkeypatch.setenv("RT_WALK_CTAS", str(ctas))
+    t = _start(rt, model, size)
+    cls = rt.DominoTiler if model == "domino" else rt.LozengeTiler
+    _check(cls(rng=rt.RT_RNG_PLANES), t, po.walk_planes(model, t, steps, 11), steps, 11)
