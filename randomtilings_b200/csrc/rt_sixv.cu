@@ -18,6 +18,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstdlib>
 #include <cstring>
 #include <random>
 #include <string>
@@ -103,6 +104,7 @@ struct SixvBandArgs {
     unsigned long long* xbuf;  // [cta][side][parity][lattice][xwords]
     int* err;
     uint64_t timeout_ns;
+    int64_t drop_blk;  // an exchange whose rows CTA 0 withholds (bounded-wait tests); -1: none
 };
 
 __device__ __forceinline__ unsigned long long* sixv_slot(const SixvBandArgs& a, int cta, int side, int par, int l) {
@@ -198,6 +200,11 @@ __global__ void __launch_bounds__(1024, 1) sixv_band_kernel(const __grid_constan
     using C1 = std::integral_constant<int, 1>;
 
     __syncthreads();
+    const bool no_exchange = nct > 1 && (a.steps + 1) / 2 <= H;
+    if (no_exchange && tid == 0 && !(cta == 0 && a.drop_blk == 0)) {
+        if (has_top) raise_loaded(sixv_slot(a, cta, 0, 0, 0));
+        if (has_bot) raise_loaded(sixv_slot(a, cta, 1, 0, 0));
+    }
     int k = 0;          // pairs of steps since the last exchange
     uint32_t blk = 0;   // exchanges made
     for (int64_t s = 0; s < a.steps; s += 2) {
@@ -235,7 +242,7 @@ __global__ void __launch_bounds__(1024, 1) sixv_band_kernel(const __grid_constan
         for (int l = 0; l < NLAT; ++l)
             for (int yy = rr0; yy < 2 * H; yy += dr) {
                 const int side = yy >= H, y = yy - side * H;
-                if (side == 0 ? !has_top : !has_bot) continue;
+                if ((side == 0 ? !has_top : !has_bot) || (cta == 0 && blk == a.drop_blk)) continue;
                 const int16_t* const row = sh + 2 * l * plane + ((side == 0 ? H : nrows) + y) * ST + 4 * q;
                 const uint2 ev = *reinterpret_cast<const uint2*>(row), od = *reinterpret_cast<const uint2*>(row + plane);
                 unsigned long long* const to = sixv_slot(a, cta, side, par, l) + 4 * y * Q + q;
@@ -273,6 +280,12 @@ __global__ void __launch_bounds__(1024, 1) sixv_band_kernel(const __grid_constan
         if (__syncthreads_or(!ok)) return;
         k = 0;
         ++blk;
+    }
+    if (no_exchange) {  // the neighbours may still be reading this band's rows
+        bool ok = true;
+        if (tid == 0 && has_top) ok = wait_loaded(a, sixv_slot(a, cta - 1, 1, 0, 0));
+        if (tid == 0 && has_bot) ok = ok && wait_loaded(a, sixv_slot(a, cta + 1, 0, 0, 0));
+        if (__syncthreads_or(!ok)) return;
     }
     for (int l = 0; l < NLAT; ++l)
         for (int e = tid; e < nrows * S; e += BLOCK) {
@@ -333,6 +346,8 @@ struct rt_sixv {
     unsigned long long* d_xbuf = nullptr;  // band kernel: halo slots
     size_t xcap = 0;
     int* d_err = nullptr;                  // band kernel: error word
+    uint64_t timeout_ns = 5000000000ull;   // band kernel: limit of one wait
+    int64_t drop_blk = -1;                 // RT_TEST_DROP_PUBLISH
 
     rt_status fail(rt_status s, const std::string& m) {
         err = m;
@@ -493,7 +508,8 @@ rt_status run_epoch(rt_sixv* h, int n, int nlat, int64_t sweeps, uint64_t key, u
                 b.xwords = H * 4 * a.Q;
                 b.xbuf = h->d_xbuf;
                 b.err = h->d_err;
-                b.timeout_ns = 5000000000ull;
+                b.timeout_ns = h->timeout_ns;
+                b.drop_blk = h->drop_blk;
                 void* args[] = {&b};
                 cudaError_t e = cudaMemsetAsync(h->d_xbuf, 0, xbytes, h->stream);
                 if (e == cudaSuccess) e = cudaMemsetAsync(h->d_err, 0, sizeof(int), h->stream);
@@ -550,6 +566,11 @@ rt_status rt_sixv_create(int32_t device, rt_sixv** out) {
             return RT_E_CUDA;
         }
         sixv_thresholds(h->w, h->thr, &h->monotone);
+        if (const char* dp = std::getenv("RT_TEST_DROP_PUBLISH")) h->drop_blk = std::atoll(dp);
+        if (const char* t = std::getenv("RT_WAIT_TIMEOUT_MS")) {
+            const long ms = std::atol(t);
+            if (ms > 0) h->timeout_ns = (uint64_t)ms * 1000000ull;
+        }
         *out = h;
         return RT_OK;
     });

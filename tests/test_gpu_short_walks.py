@@ -119,3 +119,43 @@ def test_short_large_plane_band_walks(monkeypatch, model, steps):
     t = _start(rt, model, size)
     cls = rt.DominoTiler if model == "domino" else rt.LozengeTiler
     _check(cls(rng=rt.RT_RNG_PLANES), t, po.walk_planes(model, t, steps, 11), steps, 11)
+
+
+# Bands of four rows with halos of four, and of 7 to 11 rows with halos of four
+# and two: one sweep is two pairs of steps, and no exchange comes before the
+# third pair or the fifth.
+@pytest.mark.parametrize("n", [90, 333, 1000, 1601])
+@pytest.mark.parametrize("sweeps", [1, 2, 3])
+def test_short_six_vertex_walks(n, sweeps):
+    import randomtilings_b200 as rt
+
+    t = rt.SixVertexTiler()
+    h = np.array(rt.SixVertexTiler.MaxHeights(n), dtype=np.int32)
+    _check(t, h, np.asarray(po.sixv_walk(h, sweeps, 11)).reshape(-1), sweeps, 11)
+
+
+@pytest.mark.parametrize("n", [90, 1601])
+@pytest.mark.parametrize("sweeps", [1, 40])
+def test_six_vertex_bands_wait_for_their_neighbours(monkeypatch, n, sweeps):
+    """The first CTA withholds its flag, or its rows of the first exchange."""
+    import randomtilings_b200 as rt
+
+    h = np.array(rt.SixVertexTiler.MaxHeights(n), dtype=np.int32)
+    monkeypatch.setenv("RT_TEST_DROP_PUBLISH", "0")
+    monkeypatch.setenv("RT_WAIT_TIMEOUT_MS", "100")
+    a = h.copy()
+    with pytest.raises(rt.RtError) as e:
+        rt.SixVertexTiler().Walk(a, sweeps, 3)
+    assert e.value.status == RT_E_TIMEOUT
+    assert np.array_equal(a, h)
+
+
+def test_six_vertex_samples_from_epochs_of_one_sweep():
+    import randomtilings_b200 as rt
+
+    n, seed = 60, 4
+    t = rt.SixVertexTiler()
+    got, st = t.CFTP(n, first_sweeps=1, master_seed=seed)
+    want, trials, total, ok = po.sixv_cftp(n, 1, seed)
+    assert ok and st["coalesced"] and (st["trials"], st["sweeps"]) == (trials, total)
+    assert np.array_equal(np.asarray(got).reshape(-1), np.asarray(want).reshape(-1))
