@@ -132,6 +132,9 @@ void fast_phases(int kind, int64_t steps, std::vector<uint32_t>& ph) {
 rt_status choose_plan(int family, int device, int nlat, int rows, int cols, int width, bool uniform, bool fast,
                       bool planes, bool weighted, bool td_fits, int kernel_choice, int ctas_hint, int depth_hint,
                       WalkPlan* plan, std::string* err) {
+    // A planner sets the fields its kernel reads; what an earlier plan (or a
+    // planner that gave up) left in the others must not reach the launch.
+    *plan = WalkPlan();
     if (planes) return plan_plane_walk(family, device, nlat, rows, width, ctas_hint, depth_hint, plan, err);
     rt_status s = RT_E_INVAL;
     if (kernel_choice != 1 && uniform && (word_family(family) || family == FAM_QLOZENGE8))
@@ -634,9 +637,11 @@ static rt_status run_schedule(rt_tiler* h, const int64_t* steps, const int64_t* 
     const int ctas_hint = h->drop_phase >= 0 && h->ctas_hint == 0 ? 2 : h->ctas_hint;
     if (h->plan_rows != h->rows || h->plan_cols != h->cols || h->plan_nlat != h->nlat || h->plan_uniform != uniform ||
         h->plan_weighted != weighted || h->plan_td_fits != h->td_fits) {
+        WalkPlan plan;  // the handle keeps its plan, and the shape it is for, if this one fails
         rt_status s = choose_plan(h->family, h->cfg.device, h->nlat, h->rows, h->cols, width, uniform, fast, planes,
-                                  weighted, h->td_fits, h->kernel_choice, ctas_hint, h->depth_hint, &h->plan, &h->err);
+                                  weighted, h->td_fits, h->kernel_choice, ctas_hint, h->depth_hint, &plan, &h->err);
         if (s != RT_OK) return s;
+        h->plan = plan;
         h->plan_rows = h->rows;
         h->plan_cols = h->cols;
         h->plan_nlat = h->nlat;

@@ -150,7 +150,6 @@ extern "C" rt_status rt_walk_device_noalloc(const rt_config* cfg, int32_t* d_til
         // The kernel rt_walk would run for this walk (word kernel for the int8
         // models, the rectangle-triangle kernel, the generic one for what they do not hold).
         auto replan = [&](int ctas_hint) {
-            plan = WalkPlan();
             return choose_plan(family, cfg->device, 1, rows, cols, width, true, false, false, false, false, 0, ctas_hint, 0,
                                &plan, &perr);
         };
