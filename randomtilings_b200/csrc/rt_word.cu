@@ -110,9 +110,12 @@ __global__ void __launch_bounds__(LB, 1) word_kernel(const __grid_constant__ Wal
         wi.vm = lane_bytes(vb) << 7;
         return wi;
     };
-    __shared__ WordPhase s_phase[kWordPhases];
+    // Decoded phases: a table, or for the largest bands (MAXW = 0), where its 512
+    // bytes would cost the last sides that fit, this phase's and the next one's.
+    constexpr bool TABLE = MAXW > 0;
+    __shared__ WordPhase s_phase[TABLE ? kWordPhases : 2];
     __shared__ uint4 s_sel[kLozengeSel];
-    if (tid < kWordPhases) s_phase[tid] = word_phase_entry<FAM>(tid, plane);
+    if (TABLE && tid < kWordPhases) s_phase[TABLE ? tid : 0] = word_phase_entry<FAM>(tid, plane);
     if (tid < kLozengeSel) s_sel[tid] = lozenge_sel_entry(tid);
     __shared__ int s_fail[2];
     if (tid < 2) s_fail[tid] = 0;
@@ -229,11 +232,13 @@ __global__ void __launch_bounds__(LB, 1) word_kernel(const __grid_constant__ Wal
     uint32_t p32 = 0;                      // phase number modulo 2^32
     int until = until_special(0);
     bool fail = false, more = a.nphases > 0;
+    if (!TABLE && tid == 0) s_phase[0] = word_phase_entry<FAM>(word_phase_index(d), plane);
     __syncthreads();
-    WordPhase P = s_phase[word_phase_index(d)];
+    WordPhase P = s_phase[TABLE ? word_phase_index(d) : 0];
     while (more) {
         const int par = (int)(p32 & 1u);
         const bool failed = *(volatile int*)&s_fail[1 - par] != 0;
+        if (!TABLE && tid == 0) s_phase[1 - par] = word_phase_entry<FAM>(word_phase_index(d_next), plane);
         const bool first = ahead == a.phases + 2;
         // Rows are exchanged after every phase but the last, whether or not the
         // next one has an Update pending: the waits keep the slots' order.
@@ -318,13 +323,14 @@ __global__ void __launch_bounds__(LB, 1) word_kernel(const __grid_constant__ Wal
         }
         d = d_next;
         d_next = d_after;
-        P = s_phase[word_phase_index(d)];
+        if (TABLE) P = s_phase[TABLE ? word_phase_index(d) : 0];
         // A wait that ran out is seen by every thread one phase later: the flag
         // of this phase is read after its barrier and acted on before the next
         // one, and not written again until then.
         if (fail) s_fail[par] = 1;
         if (failed) break;
         __syncthreads();
+        if (!TABLE) P = s_phase[1 - par];
         ++p32;
     }
     __syncthreads();
@@ -430,14 +436,19 @@ static rt_status plan_word_grid(int family, int device, int nlat, int rows, int 
     }
     const size_t smem =
         32 + (size_t)nlat * nc * (rpc + 2) * wpad + (cluster ? (size_t)4 * nlat * gw * 8 : (size_t)0);
-    if (smem > (size_t)smem_optin) {
-        *err = "band does not fit in shared memory";
-        return RT_E_INVAL;
-    }
     KernelFn fn = nlat == 1 ? word_kernel_for<1>(family, maxw, block, philox, weighted, cluster)
                             : word_kernel_for<2>(family, maxw, block, philox, weighted, cluster);
     if (!fn) {
         *err = "no word kernel for this configuration";
+        return RT_E_INVAL;
+    }
+    cudaFuncAttributes fa;
+    if (cudaFuncGetAttributes(&fa, (const void*)fn) != cudaSuccess) {
+        *err = "cudaFuncGetAttributes failed";
+        return RT_E_CUDA;
+    }
+    if (smem + fa.sharedSizeBytes > (size_t)smem_optin) {
+        *err = "band does not fit in shared memory";
         return RT_E_INVAL;
     }
     if (cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
