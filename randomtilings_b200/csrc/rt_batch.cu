@@ -69,8 +69,10 @@ __device__ __forceinline__ void cluster_or_block_sync(cg::cluster_group& cluster
 // Shared memory: 16 B slack, NC planes of (rpc + 2) x wpad bytes, 16 B
 // slack, then per band row its class (i mod 3 or i mod 2) and "row can be
 // refreshed" flag, then per word column its update and position masks.
+// TABLE: decoded phases and column shifts are in (static) shared memory; the
+// largest lozenge chains leave no room for them (see fill_plan).
 // ---------------------------------------------------------------------------
-template <int FAM>
+template <int FAM, bool TABLE>
 __global__ void __launch_bounds__(1024, 1) batch_word_kernel(const __grid_constant__ BatchArgs b) {
     using M = WordModel<FAM>;
     constexpr int NC = M::NC;
@@ -82,9 +84,15 @@ __global__ void __launch_bounds__(1024, 1) batch_word_kernel(const __grid_consta
     const int BLOCK = blockDim.x, tid = threadIdx.x;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     unsigned char* lat = smem_raw + 16;
-    __shared__ WordPhase s_phase[kWordPhases];
-    __shared__ uint4 s_sel[kLozengeSel];
-    if (tid < kLozengeSel) s_sel[tid] = lozenge_sel_entry(tid);
+    WordPhase* s_phase = nullptr;
+    uint4* s_sel = nullptr;
+    if constexpr (TABLE) {
+        __shared__ WordPhase phase_table[kWordPhases];
+        __shared__ uint4 sel_table[kLozengeSel];
+        s_phase = phase_table;
+        s_sel = sel_table;
+        if (tid < kLozengeSel) s_sel[tid] = lozenge_sel_entry(tid);
+    }
 
     for (int q = cid; q < b.nchains; q += ncl) {
         const BatchChain& ch = b.chains[b.order[q]];
@@ -109,7 +117,7 @@ __global__ void __launch_bounds__(1024, 1) batch_word_kernel(const __grid_consta
                 s[e] = (unsigned char)v;
             }
         }
-        if (tid < kWordPhases) s_phase[tid] = word_phase_entry<FAM>(tid, plane);
+        if (TABLE && tid < kWordPhases) s_phase[tid] = word_phase_entry<FAM>(tid, plane);
         for (int rr = tid; rr < nrows; rr += BLOCK) {
             const int i = a0 + rr;
             row_cls[rr] = (unsigned char)(M::DOM ? (i & 1) : i % 3);
@@ -136,7 +144,8 @@ __global__ void __launch_bounds__(1024, 1) batch_word_kernel(const __grid_consta
         for (int64_t ph = 0; ph < b.nphases; ++ph) {
             const uint32_t d = __ldg(b.phases + ph);
             const bool draws = (d & PH_DRAWS) != 0u;
-            const WordPhase P = s_phase[word_phase_index(d)];
+            const int idx = word_phase_index(d);
+            const WordPhase P = TABLE ? s_phase[idx] : word_phase_entry<FAM>(idx, plane);
             int rr = tid / Gw, w = tid - (tid / Gw) * Gw;
             for (int u = tid; u < nwords; u += BLOCK) {
                 WordInfo wi;
@@ -357,13 +366,14 @@ __global__ void __launch_bounds__(512, 1) batch_td_kernel(const __grid_constant_
 
 using BatchFn = void (*)(BatchArgs);
 
-static BatchFn batch_fn(int family) {
+// lean: the kernel that needs less shared memory, null if there is none.
+static BatchFn batch_fn(int family, bool lean) {
     switch (family) {
-        case FAM_DOMINO: return batch_word_kernel<FAM_DOMINO>;
-        case FAM_DOMINO_HB: return batch_word_kernel<FAM_DOMINO_HB>;
-        case FAM_LOZENGE8: return batch_word_kernel<FAM_LOZENGE8>;
-        case FAM_RECTTRI: return batch_recttri_kernel;
-        case FAM_TRIDIMER: return batch_td_kernel;
+        case FAM_DOMINO: return lean ? nullptr : batch_word_kernel<FAM_DOMINO, true>;
+        case FAM_DOMINO_HB: return lean ? nullptr : batch_word_kernel<FAM_DOMINO_HB, true>;
+        case FAM_LOZENGE8: return lean ? batch_word_kernel<FAM_LOZENGE8, false> : batch_word_kernel<FAM_LOZENGE8, true>;
+        case FAM_RECTTRI: return lean ? nullptr : batch_recttri_kernel;
+        case FAM_TRIDIMER: return lean ? nullptr : batch_td_kernel;
         default: return nullptr;
     }
 }
@@ -405,6 +415,7 @@ struct Dev {
 };
 
 struct Plan {
+    BatchFn fn = nullptr;
     int cl = 1, block = 256, clusters = 1;
     size_t smem = 0;
     bool table = false;  // rectangle-triangles: the moves' table is in shared memory
@@ -504,7 +515,6 @@ BatchArgs args_for(rt_batch* b, int f, const void* recs, int64_t step_add = 0, b
 // priority: a CUDA stream priority (lower = scheduled first); 0 = default.
 rt_status launch_family(rt_batch* b, int f, const Plan& p, const void* recs, cudaStream_t s, int priority = 0,
                         int64_t step_add = 0, bool rest = false) {
-    BatchFn fn = batch_fn(f);
     BatchArgs a = args_for(b, f, recs, step_add, rest);
     a.table = p.table;
     cudaLaunchConfig_t cfg = {};
@@ -521,22 +531,28 @@ rt_status launch_family(rt_batch* b, int f, const Plan& p, const void* recs, cud
     attr[1].val.priority = priority;
     cfg.attrs = attr;
     cfg.numAttrs = 2;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, fn, a);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, p.fn, a);
     if (e != cudaSuccess) return b->fail(RT_E_CUDA, std::string("batch launch: ") + cudaGetErrorString(e));
     return RT_OK;
 }
 
 // Completes a plan (clusters that fit at once) for cluster size cl and CTA
-// size block; false if it cannot run.
+// size block; false if it cannot run.  A lean kernel runs only what the
+// family's first choice cannot hold: lozenge chains that fill shared memory to
+// within the 656 bytes of the tables (sides 1,899 and 1,902 on a cluster of 16).
 bool fill_plan(rt_batch* b, int f, int cl, int block, Plan* p) {
     FamilyState& F = b->fam[f];
     size_t smem = 0;
     for (int i : F.members) smem = std::max(smem, smem_for(b->chains[i], cl));
     int optin = 0;
     cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, b->device);
-    BatchFn fn = batch_fn(f);
+    BatchFn fn = batch_fn(f, false);
     cudaFuncAttributes fa;
     if (cudaFuncGetAttributes(&fa, (const void*)fn) != cudaSuccess) return false;
+    if (smem + fa.sharedSizeBytes > (size_t)optin) {
+        fn = batch_fn(f, true);
+        if (!fn || cudaFuncGetAttributes(&fa, (const void*)fn) != cudaSuccess) return false;
+    }
     // A family's kernel may be built for fewer threads than asked for (the
     // bit-plane triangle-dimer kernel: 512); it then runs with its maximum.
     block = std::min(block, fa.maxThreadsPerBlock);
@@ -564,6 +580,7 @@ bool fill_plan(rt_batch* b, int f, int cl, int block, Plan* p) {
         cudaGetLastError();
         return false;
     }
+    p->fn = fn;
     p->cl = cl;
     p->block = block;
     p->smem = smem;
@@ -746,7 +763,7 @@ rt_status plan_family(rt_batch* b, int f) {
     float best = 1e30f;
     for (const Plan& p : cand) {
         // Candidates set different shared-memory limits; this one's applies now.
-        cudaFuncSetAttribute((const void*)batch_fn(f), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem);
+        cudaFuncSetAttribute((const void*)p.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem);
         cudaMemcpyAsync(F.scratch.p, F.data.p, F.bytes, cudaMemcpyDeviceToDevice, b->stream);
         // one untimed run, then a timed one
         for (int rep = 0; rep < 2; ++rep) {
@@ -768,7 +785,7 @@ rt_status plan_family(rt_batch* b, int f) {
     // Sweeps per launch at the chosen shape: a run of 32 sweeps as one
     // launch, against four launches of 8 (each reloading the lattices from
     // global memory, with its own tail of uneven chains).
-    cudaFuncSetAttribute((const void*)batch_fn(f), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)F.plan.smem);
+    cudaFuncSetAttribute((const void*)F.plan.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)F.plan.smem);
     if ((s = stage_phases(b, f, 32)) != RT_OK || (s = stage_phases(b, f, 8, true)) != RT_OK) return s;
     float best_spl = 1e30f;
     for (const int64_t spl : {(int64_t)0, (int64_t)8}) {
@@ -961,7 +978,7 @@ rt_status rt_batch_run(rt_batch* b, int64_t sweeps) {
         if (!b->exec) {
             for (int f = 0; f < kFamilies; ++f)
                 if (!b->fam[f].members.empty())
-                    cudaFuncSetAttribute((const void*)batch_fn(f), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                    cudaFuncSetAttribute((const void*)b->fam[f].plan.fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)b->fam[f].plan.smem);
             // One graph: fork to a stream per family, one launch each, join.  The
             // family with the most work goes first at the highest priority, so its

@@ -109,7 +109,8 @@ struct WordNbr {
 };
 
 // One phase on one word of one lattice (planes at `lat`, a pending Update or
-// none), in two parts: `begin` reads the word and its own row, `finish` takes
+// none), in two parts: `begin` reads the word and its own row (sel_tab: the
+// column shifts, null where no table is at hand), `finish` takes
 // the rows next to it.  m0 / m1: byte masks (0xff) of the phase's draws --
 // dominoes: m0 where the site toggles (heat bath: becomes 12, else 3);
 // lozenges: m0 where a cube is added, m1 where one is removed.
@@ -138,7 +139,7 @@ struct WordOp {
             // {2,4,32} and takes them from f[i-1][j+sa], f[i][j-sw], f[i+1][j]; colour
             // t+2 keeps all but {1,8,16} and takes them from f[i-1][j], f[i][j+se],
             // f[i+1][j-sa].  The bit fields never overlap: sums are ORs.
-            sel = sel_tab[3 * P.t() + wi.cls];
+            sel = sel_tab ? sel_tab[3 * P.t() + wi.cls] : lozenge_sel_entry(3 * P.t() + wi.cls);
             o = lds(lat + P.oth + wi.off);
             ta = (__byte_perm(l, c, sel.z) >> 1) & 0x04040404u;
             tb = (__byte_perm(c, r, sel.w) << 1) & 0x08080808u;
