@@ -55,6 +55,7 @@ struct BatchArgs {
     uint32_t thr[4];
     float weights[16];
     int table;  // rectangle-triangles: shared memory begins with a RectTriMoves
+    int halo;   // triangle dimers: most halo rows of a band
 };
 
 __device__ __forceinline__ void cluster_or_block_sync(cg::cluster_group& cluster, int CL) {
@@ -330,6 +331,7 @@ __global__ void __launch_bounds__(1024, 1) batch_recttri_kernel(const __grid_con
 
 // Triangle dimers: the eight arrays as bit planes, 32 sites per word
 // (rt_tdwalk.cuh), through the phases of the schedule (rt_tdschedule.h).
+template <class BITS>
 __global__ void __launch_bounds__(512, 1) batch_td_kernel(const __grid_constant__ BatchArgs b) {
     cg::cluster_group cluster = cg::this_cluster();
     const int CL = (int)cluster.num_blocks();
@@ -343,8 +345,8 @@ __global__ void __launch_bounds__(512, 1) batch_td_kernel(const __grid_constant_
 
     for (int q = cid; q < b.nchains; q += ncl) {
         const BatchChain& ch = b.chains[b.order[q]];
-        TdBand band(sm, ch.rows, ch.width, ch.n / 2, rank, CL, td_halo_cap(true), tid, BLOCK);
-        for (int e = tid; e < (int)td_band_words(ch.rows, ch.width, band.ctas, td_halo_cap(true)); e += BLOCK) sm[e] = 0u;
+        TdBand<BITS> band(sm, ch.rows, ch.width, ch.n / 2, rank, CL, b.halo, tid, BLOCK);
+        for (int e = tid; e < (int)td_band_words(ch.rows, ch.width, band.ctas, b.halo, BITS::planes); e += BLOCK) sm[e] = 0u;
         __syncthreads();
         td_load(band, ch.arr, ch.arows, warp, nwarps, lane);
         __syncthreads();
@@ -373,7 +375,7 @@ static BatchFn batch_fn(int family, bool lean) {
         case FAM_DOMINO_HB: return lean ? nullptr : batch_word_kernel<FAM_DOMINO_HB, true>;
         case FAM_LOZENGE8: return lean ? batch_word_kernel<FAM_LOZENGE8, false> : batch_word_kernel<FAM_LOZENGE8, true>;
         case FAM_RECTTRI: return lean ? nullptr : batch_recttri_kernel;
-        case FAM_TRIDIMER: return lean ? nullptr : batch_td_kernel;
+        case FAM_TRIDIMER: return lean ? batch_td_kernel<tdp::CoverBits> : batch_td_kernel<tdp::AllBits>;
         default: return nullptr;
     }
 }
@@ -419,6 +421,7 @@ struct Plan {
     int cl = 1, block = 256, clusters = 1;
     size_t smem = 0;
     bool table = false;  // rectangle-triangles: the moves' table is in shared memory
+    int halo = 1;        // triangle dimers: most halo rows of a band
     int64_t spl = 0;  // sweeps per launch: a run of S sweeps is S / spl launches (+ one for the rest); 0 = one
 };
 
@@ -447,14 +450,16 @@ int elem_of(int fam) { return fam <= FAM_LOZENGE8 ? 1 : 4; }
 int steps_per_sweep(int kind) { return kind == 0 ? 2 : kind == 3 ? 30 : 3; }
 bool word_fam(int fam) { return fam <= FAM_LOZENGE8; }
 
-// Shared memory one CTA of a cluster of `cl` needs for chain c.
-size_t smem_for(const Chain& c, int cl) {
+// Shared memory one CTA of a cluster of `cl` needs for chain c; triangle dimers:
+// with up to `halo` halo rows, in the lean kernel's planes or in all.
+size_t smem_for(const Chain& c, int cl, int halo, bool lean) {
     const int rpc = (c.rows + cl - 1) / cl;
     const int wpad = (c.width + 3) & ~3;
     if (word_fam(c.fam)) {
         return 16 + (size_t)c.ncol * (rpc + 2) * wpad + 16 + (size_t)((2 * rpc + 3) & ~3) + 2 * 4 * (size_t)(wpad / 4);
     }
-    if (c.fam == FAM_TRIDIMER) return 4 * td_band_words(c.rows, c.width, std::min(cl, c.rows), td_halo_cap(true));
+    if (c.fam == FAM_TRIDIMER)
+        return 4 * td_band_words(c.rows, c.width, std::min(cl, c.rows), halo, lean ? tdp::CoverBits::planes : tdp::kPlanes);
     return (size_t)c.ncol * (rpc + 2) * wpad * 4;
 }
 
@@ -517,6 +522,7 @@ rt_status launch_family(rt_batch* b, int f, const Plan& p, const void* recs, cud
                         int64_t step_add = 0, bool rest = false) {
     BatchArgs a = args_for(b, f, recs, step_add, rest);
     a.table = p.table;
+    a.halo = p.halo;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(p.clusters * p.cl));
     cfg.blockDim = dim3((unsigned)p.block);
@@ -539,24 +545,32 @@ rt_status launch_family(rt_batch* b, int f, const Plan& p, const void* recs, cud
 // Completes a plan (clusters that fit at once) for cluster size cl and CTA
 // size block; false if it cannot run.  A lean kernel runs only what the
 // family's first choice cannot hold: lozenge chains that fill shared memory to
-// within the 656 bytes of the tables (sides 1,899 and 1,902 on a cluster of 16).
+// within the 656 bytes of the tables (sides 1,899 and 1,902 on a cluster of 16),
+// and triangle-dimer chains that leave no room for five planes more than dimer
+// covers need.  Their halos have as many rows as fit, up to the cap.
 bool fill_plan(rt_batch* b, int f, int cl, int block, Plan* p) {
     FamilyState& F = b->fam[f];
-    size_t smem = 0;
-    for (int i : F.members) smem = std::max(smem, smem_for(b->chains[i], cl));
     int optin = 0;
     cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, b->device);
-    BatchFn fn = batch_fn(f, false);
+    BatchFn fn = nullptr;
     cudaFuncAttributes fa;
-    if (cudaFuncGetAttributes(&fa, (const void*)fn) != cudaSuccess) return false;
-    if (smem + fa.sharedSizeBytes > (size_t)optin) {
-        fn = batch_fn(f, true);
+    size_t smem = 0;
+    int halo = 1;
+    bool fits = false;
+    for (int lean = 0; lean < 2 && !fits; ++lean) {
+        fn = batch_fn(f, lean != 0);
         if (!fn || cudaFuncGetAttributes(&fa, (const void*)fn) != cudaSuccess) return false;
+        for (halo = f == FAM_TRIDIMER ? td_halo_cap(true) : 1; halo >= 1; --halo) {
+            smem = 0;
+            for (int i : F.members) smem = std::max(smem, smem_for(b->chains[i], cl, halo, lean != 0));
+            fits = smem + fa.sharedSizeBytes <= (size_t)optin;
+            if (fits) break;
+        }
     }
+    if (!fits) return false;
     // A family's kernel may be built for fewer threads than asked for (the
     // bit-plane triangle-dimer kernel: 512); it then runs with its maximum.
     block = std::min(block, fa.maxThreadsPerBlock);
-    if (smem + fa.sharedSizeBytes > (size_t)optin) return false;
     // The table of moves goes in front of the lattice where there is room left.
     p->table = f == FAM_RECTTRI && smem + sizeof(RectTriMoves) + fa.sharedSizeBytes <= (size_t)optin;
     if (p->table) smem += sizeof(RectTriMoves);
@@ -581,6 +595,7 @@ bool fill_plan(rt_batch* b, int f, int cl, int block, Plan* p) {
         return false;
     }
     p->fn = fn;
+    p->halo = halo;
     p->cl = cl;
     p->block = block;
     p->smem = smem;

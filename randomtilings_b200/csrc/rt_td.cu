@@ -42,10 +42,10 @@ __global__ void __launch_bounds__(kTdBlock, 1) td_walk_kernel(const __grid_const
     uint32_t* st = td_smem;
     uint32_t* draws = st + (PHILOX ? 0 : 4 * 32 * slots);
     uint32_t* sm = draws + (PHILOX ? 0 : 2 * slots);
-    TdBand band(sm, a.rows, a.width, a.n / 2, rank, CL, td_halo_cap(PHILOX), min(tid, RUN - 1), RUN);
+    TdBand<tdp::AllBits> band(sm, a.rows, a.width, a.n / 2, rank, CL, td_halo_cap(PHILOX), min(tid, RUN - 1), RUN);
     const int first = max(0, band.row0), words = (min(a.rows, band.r1 + halo) - first) * wb;  // rows that draw
 
-    for (int e = tid; e < (int)td_band_words(a.rows, a.width, ctas, td_halo_cap(PHILOX)); e += BLOCK) sm[e] = 0u;
+    for (int e = tid; e < (int)td_band_words(a.rows, a.width, ctas, td_halo_cap(PHILOX), tdp::kPlanes); e += BLOCK) sm[e] = 0u;
     __syncthreads();
     td_load(band, a.arr[0], a.arows, tid >> 5, BLOCK >> 5, lane);
     __syncthreads();
@@ -170,7 +170,7 @@ rt_status plan_td_walk(int device, int rows, int width, bool philox, int ctas_hi
     ctas = std::min(ctas_hint > 0 ? ctas_hint : ctas, std::min(rows, 16));
     const int rpc = (rows + ctas - 1) / ctas;
     const size_t slots = (size_t)(rpc + 2 * td_halo(rows, ctas, td_halo_cap(philox))) * ((width + 31) / 32);
-    const size_t smem = 4 * (td_band_words(rows, width, ctas, td_halo_cap(philox)) + (philox ? 0 : (4 * 32 + 2) * slots));
+    const size_t smem = 4 * (td_band_words(rows, width, ctas, td_halo_cap(philox), tdp::kPlanes) + (philox ? 0 : (4 * 32 + 2) * slots));
     if (smem > (size_t)optin) {
         *err = "triangle-dimer band does not fit in shared memory";
         return RT_E_INVAL;

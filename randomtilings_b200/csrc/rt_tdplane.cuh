@@ -41,6 +41,19 @@ TDP_HD constexpr int bits_of(int arr) { return arr < 3 ? 4 : arr < 5 ? 7 : 10; }
 // Bits of the values a dimer cover's arrays hold.
 TDP_HD constexpr int cover_bits_of(int arr) { return arr < 3 ? 4 : arr < 5 ? 6 : 9; }
 
+// Which bits have a plane: all, or those of dimer covers (51 planes), whose
+// digit sums never carry out of them.
+struct AllBits {
+    static constexpr int planes = kPlanes;
+    TDP_HD static constexpr int plane_of(int arr) { return tdp::plane_of(arr); }
+    TDP_HD static constexpr int bits_of(int arr) { return tdp::bits_of(arr); }
+};
+struct CoverBits {
+    static constexpr int planes = 51;
+    TDP_HD static constexpr int plane_of(int arr) { return arr < 3 ? 4 * arr : arr < 5 ? 12 + 6 * (arr - 3) : 24 + 9 * (arr - 5); }
+    TDP_HD static constexpr int bits_of(int arr) { return cover_bits_of(arr); }
+};
+
 // ---- lane masks -------------------------------------------------------------
 TDP_HD int mod3(int x) { return ((x % 3) + 3) % 3; }
 // lanes of word c whose column j = 32 c + l has j mod 2 == r
@@ -65,8 +78,10 @@ TDP_HD uint32_t col_range(int c, int lo, int hi) {
 // rows (row 0 = array row row0), then words; the word before a row's first
 // word and the word after its last one read as zero (the columns outside
 // the array), e.g. rows of wb + 1 words whose last word stays zero, after
-// one zero word.
-struct View {
+// one zero word.  BITS: a bit without a plane reads as zero.
+template <class BITS>
+struct ViewOf {
+    using Bits = BITS;
     uint32_t* p;  // plane 0, row 0, word 0
     int ps, rs;   // plane and row strides in words
     int row0;
@@ -75,13 +90,15 @@ struct View {
     // Plane `bit` of array `arr` at row i + di, columns shifted by dj (-1, 0, +1):
     // lane l holds the site (i + di, 32 c + l + dj).
     TDP_HD uint32_t ld(int arr, int bit, int di, int dj) const {
-        const uint32_t* q = word(plane_of(arr) + bit, di);
+        if (BITS::planes < kPlanes && bit >= BITS::bits_of(arr)) return 0u;
+        const uint32_t* q = word(BITS::plane_of(arr) + bit, di);
         if (dj == 0) return q[0];
         if (dj > 0) return (q[0] >> 1) | (q[1] << 31);
         return (q[0] << 1) | (q[-1] >> 31);
     }
     TDP_HD void st(int arr, int bit, uint32_t v, uint32_t m) const {
-        uint32_t* q = word(plane_of(arr) + bit, 0);
+        if (BITS::planes < kPlanes && bit >= BITS::bits_of(arr)) return;
+        uint32_t* q = word(BITS::plane_of(arr) + bit, 0);
         *q = (*q & ~m) | (v & m);
     }
     // Lanes whose column is inside the lattice's border, in use, = r (mod 3).
@@ -90,6 +107,7 @@ struct View {
     TDP_HD uint32_t used_cols(int width) const { return col_range(c, 0, width - 1); }
     TDP_HD uint32_t cols_mod3(int r) const { return col_mod3(r, c); }
 };
+using View = ViewOf<AllBits>;
 
 TDP_HD uint32_t all_if(bool x) { return x ? 0xFFFFFFFFu : 0u; }
 
@@ -271,7 +289,7 @@ TDP_HD void rot_flip(const V& v, uint32_t a, uint32_t F) {
     const uint32_t bits = OP == TD_ROT_LOZ ? 0xfu : OP == TD_ROT_TRI ? 0x1bu : 0xffu;
 #pragma unroll
     for (int k = 0; k < 8; ++k)
-        if (bits >> k & 1u) *v.word(plane_of(arr) + k, 0) ^= F;
+        if (bits >> k & 1u) *v.word(V::Bits::plane_of(arr) + k, 0) ^= F;
 }
 
 // ---- the ops ------------------------------------------------------------------------

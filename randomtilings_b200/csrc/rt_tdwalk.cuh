@@ -36,9 +36,9 @@ __host__ __device__ inline int td_first_row(int rows, int ctas, int rank) {
 }
 // Words of shared memory a band takes: one zero word, then per plane its rows
 // and halo rows of wb + 1 words (the last word of a row stays zero).
-__host__ __device__ inline size_t td_band_words(int rows, int width, int ctas, int cap) {
+__host__ __device__ inline size_t td_band_words(int rows, int width, int ctas, int cap, int planes) {
     const int rpc = (rows + ctas - 1) / ctas;
-    return 1 + (size_t)tdp::kPlanes * (rpc + 2 * td_halo(rows, ctas, cap)) * (((width + 31) >> 5) + 1);
+    return 1 + (size_t)planes * (rpc + 2 * td_halo(rows, ctas, cap)) * (((width + 31) >> 5) + 1);
 }
 
 // Rows by which phase d's results depend on neighbouring rows.
@@ -52,7 +52,8 @@ __device__ __forceinline__ int td_reach(uint32_t d) {
 
 // The view of a thread's words: all of one word column, whose lane masks the
 // thread keeps.
-struct TdView : tdp::View {
+template <class BITS>
+struct TdView : tdp::ViewOf<BITS> {
     uint32_t inner, used;
     int c2;  // 2 c mod 3
     __device__ __forceinline__ uint32_t inner_cols(int) const { return inner; }
@@ -63,6 +64,7 @@ struct TdView : tdp::View {
     }
 };
 
+template <class BITS>
 struct TdBand {
     uint32_t* planes;  // plane 0, row 0 (array row row0), word 0
     int ps, rs, wb;    // plane and row strides in words, words per row
@@ -73,7 +75,7 @@ struct TdBand {
     // (idle: g beyond the threads that make up whole rows).
     int g, stride;
     bool idle;
-    TdView view;
+    TdView<BITS> view;
     // Its words of an exchange: column xc of halo row xh, of every xstride-th
     // plane from xp on; arrays written since the last exchange.
     int xc, xh, xp, xstride;
@@ -96,7 +98,7 @@ struct TdBand {
         const int c = tid % wb;
         g = tid / wb;
         idle = g >= stride || r0 == r1;
-        static_cast<tdp::View&>(view) = tdp::View{planes, ps, rs, row0, 0, c};
+        static_cast<tdp::ViewOf<BITS>&>(view) = tdp::ViewOf<BITS>{planes, ps, rs, row0, 0, c};
         view.inner = tdp::col_range(c, 1, m - 2);
         view.used = tdp::col_range(c, 0, width - 1);
         view.c2 = 2 * c % 3;
@@ -105,7 +107,7 @@ struct TdBand {
         xh = tid / wb % halo;
         xp = tid / per;
         xstride = BLOCK / per;  // 0: fewer threads than words
-        if (xp >= xstride) xp = tdp::kPlanes;
+        if (xp >= xstride) xp = BITS::planes;
         written = 0u;
     }
 
@@ -123,7 +125,7 @@ struct TdBand {
                 if (dn) dn[p * ps + h * rs + c] = mine[(r1 - r0 + h) * rs];
             };
             for (uint32_t w = written; w; w &= w - 1) {
-                const int arr = __ffs((int)w) - 1, p0 = tdp::plane_of(arr), n = tdp::bits_of(arr);
+                const int arr = __ffs((int)w) - 1, p0 = BITS::plane_of(arr), n = BITS::bits_of(arr);
                 if (xstride > 0)
                     for (int k = xp; k < n; k += xstride) word(p0 + k, xh, xc);
                 else if (!idle)
@@ -139,26 +141,28 @@ struct TdBand {
 
 // Global int32 rows of the band and its halo -> planes (cleared before); one
 // warp per 32 columns, with a ballot per bit.
-__device__ __forceinline__ void td_load(const TdBand& b, void* const* arr, int arows, int warp, int nwarps, int lane) {
+template <class BITS>
+__device__ __forceinline__ void td_load(const TdBand<BITS>& b, void* const* arr, int arows, int warp, int nwarps, int lane) {
     for (int it = warp; it < (b.r1 - b.r0 + 2 * b.halo) * 8 * b.wb; it += nwarps) {
         const int sr = it / (8 * b.wb), rem = it - sr * 8 * b.wb, a = rem / b.wb, c = rem - a * b.wb;
         const int rr = b.row0 + sr, j = 32 * c + lane;
         int32_t v = 0;
         if (rr >= 0 && rr < arows && j < b.width) v = static_cast<const int32_t*>(arr[a])[(size_t)rr * b.width + j];
-        for (int k = 0; k < tdp::bits_of(a); ++k) {
+        for (int k = 0; k < BITS::bits_of(a); ++k) {
             const uint32_t w = __ballot_sync(0xffffffffu, (v >> k) & 1);
-            if (lane == 0) b.planes[(tdp::plane_of(a) + k) * b.ps + sr * b.rs + c] = w;
+            if (lane == 0) b.planes[(BITS::plane_of(a) + k) * b.ps + sr * b.rs + c] = w;
         }
     }
 }
 // planes -> global int32 rows r0 .. r1 - 1
-__device__ __forceinline__ void td_store(const TdBand& b, void* const* arr, int warp, int nwarps, int lane) {
+template <class BITS>
+__device__ __forceinline__ void td_store(const TdBand<BITS>& b, void* const* arr, int warp, int nwarps, int lane) {
     for (int it = warp; it < (b.r1 - b.r0) * 8 * b.wb; it += nwarps) {
         const int rr = it / (8 * b.wb), sr = b.halo + rr, rem = it - rr * 8 * b.wb, a = rem / b.wb, c = rem - a * b.wb;
         const int j = 32 * c + lane;
         int32_t v = 0;
-        for (int k = 0; k < tdp::bits_of(a); ++k)
-            v |= (int32_t)((b.planes[(tdp::plane_of(a) + k) * b.ps + sr * b.rs + c] >> lane) & 1u) << k;
+        for (int k = 0; k < BITS::bits_of(a); ++k)
+            v |= (int32_t)((b.planes[(BITS::plane_of(a) + k) * b.ps + sr * b.rs + c] >> lane) & 1u) << k;
         if (j < b.width) static_cast<int32_t*>(arr[a])[(size_t)(b.r0 + rr) * b.width + j] = v;
     }
 }
@@ -186,12 +190,12 @@ struct TdPhilox {
 
 // Phase (OP, a, b) on rows lo .. hi - 1: only those TriDimerRule::live_rows
 // admits, one 32-site word per work item.
-template <uint32_t OP, int T, int B, class Draw>
-__device__ __forceinline__ void td_op(const TdBand& d, int lo, int hi, uint32_t a, uint32_t b, const Draw& draw) {
+template <uint32_t OP, int T, int B, class BITS, class Draw>
+__device__ __forceinline__ void td_op(const TdBand<BITS>& d, int lo, int hi, uint32_t a, uint32_t b, const Draw& draw) {
     constexpr bool DRAWS = OP == TD_ROT_LOZ || OP == TD_ROT_TRI || OP == TD_ROT_BFLY;
     int S, o;
     TriDimerRule::live_rows<OP>(T >= 0 ? (uint32_t)T : a, b, &S, &o);
-    TdView v = d.view;
+    TdView<BITS> v = d.view;
     for (v.i = lo + ((o - lo) % S + S) % S + S * d.g; v.i < hi; v.i += S * d.stride) {
         if (DRAWS) {
             uint32_t F = tdp::rot_mask<OP, T>(v, a, b, d.width);
@@ -203,8 +207,8 @@ __device__ __forceinline__ void td_op(const TdBand& d, int lo, int hi, uint32_t 
     }
 }
 
-template <class Draw>
-__device__ __forceinline__ void td_phase(uint32_t d, TdBand& band, const Draw& draw) {
+template <class BITS, class Draw>
+__device__ __forceinline__ void td_phase(uint32_t d, TdBand<BITS>& band, const Draw& draw) {
     const uint32_t pa = ph_a(d), pb = ph_b(d);
     // the band's rows and the halo rows that can be kept current
     const int keep = band.ctas == 1 ? 0 : band.depth - td_reach(d);
