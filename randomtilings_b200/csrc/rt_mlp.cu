@@ -22,6 +22,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstdlib>
 #include <cstring>
 #include <vector>
 
@@ -756,6 +757,7 @@ struct rt_mlp {
     float *X = nullptr, *T = nullptr;
     int64_t rows = 0;
     int* err = nullptr;  // device: set when a bounded wait gave up
+    size_t over = 0;     // RT_TEST_REFUSE_LAUNCH: bytes of shared memory asked for beyond what is allowed
 };
 
 namespace {
@@ -795,10 +797,31 @@ NetArgs net_args(const rt_mlp* m, int n) {
     return g;
 }
 
+// `pair`: clusters of two CTAs.
+template <class K, class A>
+bool launch(rt_mlp* m, K kernel, int grid, int block, size_t smem, bool pair, const A& args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = m->s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pair ? 1 : 0;
+    if (cudaLaunchKernelEx(&cfg, kernel, args) == cudaSuccess) return true;
+    cudaGetLastError();
+    return false;
+}
+
 // Predictions of the n rows in m->x into m->y: two CTAs a SM.
-void forward(rt_mlp* m, int n) {
+bool forward(rt_mlp* m, int n) {
     const int tiles = (n + TR - 1) / TR;
-    net_kernel<false, kFwdThreads><<<std::min(tiles, 2 * m->sms), kFwdThreads, net_smem(false), m->s>>>(net_args(m, n));
+    return launch(m, net_kernel<false, kFwdThreads>, std::min(tiles, 2 * m->sms), kFwdThreads, net_smem(false) + m->over, false,
+                  net_args(m, n));
 }
 
 // Rows of a range: 256, or less where that evens out the ranges (a multiple of 64).
@@ -835,8 +858,9 @@ bool reserve_gradient(rt_mlp* m, int n) {
     return true;
 }
 
-// Loss and gradient of g's rows: into m->G and m->loss, or an Adam step.
-void gradient(rt_mlp* m, NetArgs g, bool adam, float lr, float b1t, float b2t) {
+// Loss and gradient of g's rows: into m->G and m->loss, or an Adam step.  False
+// if a kernel did not start; the second one then does not either.
+bool gradient(rt_mlp* m, NetArgs g, bool adam, float lr, float b1t, float b2t) {
     g.range = range_rows(g.n);
     const int ranges = (g.n + g.range - 1) / g.range, pairs = std::min(ranges, m->sms / 2);
     g.chain = ranges == pairs;
@@ -846,19 +870,7 @@ void gradient(rt_mlp* m, NetArgs g, bool adam, float lr, float b1t, float b2t) {
     g.dy = m->dy;
     g.xb = m->xb;
     g.err2 = m->err2;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(2 * pairs));
-    cfg.blockDim = dim3(kGradThreads);
-    cfg.dynamicSmemBytes = net_smem(true);
-    cfg.stream = m->s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, net_kernel<true, kGradThreads>, g);
+    if (!launch(m, net_kernel<true, kGradThreads>, 2 * pairs, kGradThreads, net_smem(true) + m->over, true, g)) return false;
     SumArgs a;
     std::memset(&a, 0, sizeof a);
     a.part = m->part;
@@ -882,10 +894,8 @@ void gradient(rt_mlp* m, NetArgs g, bool adam, float lr, float b1t, float b2t) {
     a.lr = lr;
     a.b1t = b1t;
     a.b2t = b2t;
-    if (adam)
-        sum_kernel<true><<<kSumBlocks, 256, kSumSmem, m->s>>>(a);
-    else
-        sum_kernel<false><<<kSumBlocks, 256, kSumSmem, m->s>>>(a);
+    return adam ? launch(m, sum_kernel<true>, kSumBlocks, 256, kSumSmem, false, a)
+                : launch(m, sum_kernel<false>, kSumBlocks, 256, kSumSmem, false, a);
 }
 
 rt_status sync(rt_mlp* m) {
@@ -906,6 +916,7 @@ rt_status rt_mlp_create(int32_t device, uint64_t seed, rt_mlp** out) {
         if (cudaSetDevice(device) != cudaSuccess) return RT_E_NODEVICE;
         rt_mlp* m = new rt_mlp();
         m->device = device;
+        if (std::getenv("RT_TEST_REFUSE_LAUNCH")) m->over = 1024;
         bool ok = cudaStreamCreateWithFlags(&m->s, cudaStreamNonBlocking) == cudaSuccess &&
                   cudaMalloc(&m->P, NPARAM * 4) == cudaSuccess && cudaMalloc(&m->G, NPARAM * 4) == cudaSuccess &&
                   cudaMalloc(&m->M1, NPARAM * 4) == cudaSuccess && cudaMalloc(&m->M2, NPARAM * 4) == cudaSuccess &&
@@ -990,7 +1001,7 @@ rt_status rt_mlp_predict(rt_mlp* m, const float* x, int64_t n, float* y) {
             const int rn = (int)std::min<int64_t>(chunk, n - r0);
             if (!reserve(m, rn)) return RT_E_NOMEM;
             cudaMemcpyAsync(m->x, x + r0 * IN, (size_t)rn * IN * 4, cudaMemcpyHostToDevice, m->s);
-            forward(m, rn);
+            if (!forward(m, rn)) return RT_E_CUDA;
             cudaMemcpyAsync(y + r0, m->y, (size_t)rn * 4, cudaMemcpyDeviceToHost, m->s);
             rt_status st = sync(m);
             if (st != RT_OK) return st;
@@ -1006,7 +1017,7 @@ rt_status rt_mlp_loss_grad(rt_mlp* m, const float* x, const float* target, int64
         if (!reserve(m, n) || !reserve_gradient(m, (int)n)) return RT_E_NOMEM;
         cudaMemcpyAsync(m->x, x, (size_t)n * IN * 4, cudaMemcpyHostToDevice, m->s);
         cudaMemcpyAsync(m->t, target, (size_t)n * 4, cudaMemcpyHostToDevice, m->s);
-        gradient(m, net_args(m, (int)n), false, 0.0f, 0.0f, 0.0f);
+        if (!gradient(m, net_args(m, (int)n), false, 0.0f, 0.0f, 0.0f)) return RT_E_CUDA;
         if (loss) cudaMemcpyAsync(loss, m->loss, 4, cudaMemcpyDeviceToHost, m->s);
         if (grad) cudaMemcpyAsync(grad, m->G, NPARAM * 4, cudaMemcpyDeviceToHost, m->s);
         return sync(m);
@@ -1053,7 +1064,10 @@ rt_status rt_mlp_train(rt_mlp* m, int64_t steps, int32_t batch, float lr, uint64
         for (int64_t k = 0; k < steps; ++k) {
             g.step = m->adam_t++;
             const float b1t = std::pow(0.9f, (float)m->adam_t), b2t = std::pow(0.999f, (float)m->adam_t);
-            gradient(m, g, true, lr, b1t, b2t);
+            if (!gradient(m, g, true, lr, b1t, b2t)) {
+                --m->adam_t;
+                return RT_E_CUDA;
+            }
         }
         if (loss) cudaMemcpyAsync(loss, m->loss, 4, cudaMemcpyDeviceToHost, m->s);
         return sync(m);
