@@ -21,9 +21,7 @@
 // word and step), the latency of one word's update, and the exchange.  On the
 // a = b = c = 500 hexagon (148 CTAs) a step takes 0.98 us, 1.83 with a phase
 // per step, a halo row copied through shared memory and a block-wide vote.
-// Lattices whose bands have room for halo rows run on rt_wordband.cu; on one
-// cluster of 16 this kernel takes 0.43 us on the Aztec diamond of order 100
-// (1.35 before, 0.38 there), on one CTA 0.34 at order 24 (1.33, 0.28).
+// Lattices whose bands have room for halo rows run on rt_wordband.cu.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -39,10 +37,9 @@ namespace rtb {
 constexpr int kWordBlockMax = 512;  // threads that keep 2 or 4 words' generator states each
 constexpr int kWordBlockMid = 640;  // 65,536 registers / 96, in whole warps
 
-// Shared memory: the inbox (CLUSTER), 16 bytes of slack, then for each lattice
-// NC colour planes of (band rows + 2) x wpad bytes, then 16 bytes of slack
-// (the funnel shifts read one word beyond a row; those bytes only reach sites
-// outside the update / flip masks).
+// Shared memory: 16 bytes of slack, then for each lattice NC colour planes of
+// (band rows + 2) x wpad bytes, then 16 bytes of slack (the funnel shifts read one
+// word beyond a row; those bytes only reach sites outside the update / flip masks).
 // MAXW: words per thread kept in registers (facts, draw masks and, in
 // bit-exact mode, generator states); 0: words walked at run time (fast mode
 // on large bands).
@@ -51,13 +48,12 @@ constexpr int kWordBlockMid = 640;  // 65,536 registers / 96, in whole warps
 // (qlozengekernel.cl), add below thr[2], remove in [2^22, thr[3]).  Separate
 // instantiations, so that the uniform kernel carries none of it.
 // NL: lattices (2: coupled CFTP chains).
-template <int FAM, int MAXW, bool PHILOX, int LB, int WT, bool CLUSTER, int NL>
+template <int FAM, int MAXW, bool PHILOX, int LB, int WT, int NL>
 __global__ void __launch_bounds__(LB, 1) word_kernel(const __grid_constant__ WalkArgs a) {
     using M = WordModel<FAM>;
     constexpr int NC = M::NC;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int inbox_bytes = CLUSTER ? 4 * NL * a.xwords * 8 : 0;
-    unsigned char* lat = smem_raw + inbox_bytes + 16;
+    unsigned char* lat = smem_raw + 16;
 
     const int BLOCK = blockDim.x;
     const int cta = blockIdx.x, nct = gridDim.x, tid = threadIdx.x;
@@ -70,13 +66,7 @@ __global__ void __launch_bounds__(LB, 1) word_kernel(const __grid_constant__ Wal
     const int Gw = W >> 2;  // words per row (the fast mode's counter stride too)
     const int nwords = nrows * Gw;
     const int N = a.n;
-    const WordExchange<CLUSTER> xch{a, reinterpret_cast<unsigned long long*>(smem_raw), cta};
-
-    if (CLUSTER) {
-        for (int e = tid; e < inbox_bytes / 8; e += BLOCK) xch.inbox[e] = 0ull;
-        __syncthreads();
-        cluster_sync_all();  // every inbox is clear before anyone writes into it
-    }
+    const WordExchange<false> xch{a, nullptr, cta};
     for (int l = 0; l < NL; ++l)
         for (int c = 0; c < NC; ++c) {
             const int8_t* g = static_cast<const int8_t*>(a.arr[l][c]);
@@ -334,7 +324,6 @@ __global__ void __launch_bounds__(LB, 1) word_kernel(const __grid_constant__ Wal
         ++p32;
     }
     __syncthreads();
-    if (CLUSTER) cluster_sync_all();  // no CTA leaves while another may write into its inbox
     if (s_fail[0] | s_fail[1]) return;
     for (int l = 0; l < NL; ++l)
         for (int c = 0; c < NC; ++c) {
@@ -351,57 +340,50 @@ using KernelFn = void (*)(WalkArgs);
 
 // One word per thread, up to `block` threads: blocks of at most kWordBlockMid
 // threads have 96 registers a thread instead of 64.
-template <int FAM, bool PHILOX, int WT, bool CLUSTER, int NL>
+template <int FAM, bool PHILOX, int WT, int NL>
 static KernelFn word_fn1(int block) {
-    return block <= kWordBlockMid ? word_kernel<FAM, 1, PHILOX, kWordBlockMid, WT, CLUSTER, NL>
-                                  : word_kernel<FAM, 1, PHILOX, 1024, WT, CLUSTER, NL>;
+    return block <= kWordBlockMid ? word_kernel<FAM, 1, PHILOX, kWordBlockMid, WT, NL>
+                                  : word_kernel<FAM, 1, PHILOX, 1024, WT, NL>;
 }
 template <int FAM, int WT, int NL>
-static KernelFn word_fn(int maxw, int block, bool philox, bool cluster) {
-    if (maxw == 1) {
-        if (cluster) return philox ? word_fn1<FAM, true, WT, true, NL>(block) : word_fn1<FAM, false, WT, true, NL>(block);
-        return philox ? word_fn1<FAM, true, WT, false, NL>(block) : word_fn1<FAM, false, WT, false, NL>(block);
-    }
-    if (cluster) return nullptr;  // clusters are planned for one word per thread
+static KernelFn word_fn(int maxw, int block, bool philox) {
+    if (maxw == 1) return philox ? word_fn1<FAM, true, WT, NL>(block) : word_fn1<FAM, false, WT, NL>(block);
     if (philox) {
         switch (maxw) {
-            case 0: return word_kernel<FAM, 0, true, 1024, WT, false, NL>;
-            case 2: return word_kernel<FAM, 2, true, 1024, WT, false, NL>;
-            case 4: return word_kernel<FAM, 4, true, 1024, WT, false, NL>;
+            case 0: return word_kernel<FAM, 0, true, 1024, WT, NL>;
+            case 2: return word_kernel<FAM, 2, true, 1024, WT, NL>;
+            case 4: return word_kernel<FAM, 4, true, 1024, WT, NL>;
             default: return nullptr;
         }
     }
     switch (maxw) {
-        case 2: return word_kernel<FAM, 2, false, 512, WT, false, NL>;
-        case 4: return word_kernel<FAM, 4, false, 512, WT, false, NL>;
+        case 2: return word_kernel<FAM, 2, false, 512, WT, NL>;
+        case 4: return word_kernel<FAM, 4, false, 512, WT, NL>;
         default: return nullptr;
     }
 }
 
 template <int NL>
-static KernelFn word_kernel_for(int family, int maxw, int block, bool philox, bool weighted, bool cluster) {
+static KernelFn word_kernel_for(int family, int maxw, int block, bool philox, bool weighted) {
     switch (family) {
         case FAM_DOMINO:  // not monotone: no coupled chains
-            return NL == 1 ? word_fn<FAM_DOMINO, 0, 1>(maxw, block, philox, cluster) : nullptr;
+            return NL == 1 ? word_fn<FAM_DOMINO, 0, 1>(maxw, block, philox) : nullptr;
         case FAM_DOMINO_HB:
-            return weighted ? word_fn<FAM_DOMINO_HB, 1, NL>(maxw, block, philox, cluster)
-                            : word_fn<FAM_DOMINO_HB, 0, NL>(maxw, block, philox, cluster);
+            return weighted ? word_fn<FAM_DOMINO_HB, 1, NL>(maxw, block, philox)
+                            : word_fn<FAM_DOMINO_HB, 0, NL>(maxw, block, philox);
         case FAM_LOZENGE8:
-            return weighted ? word_fn<FAM_LOZENGE8, 1, NL>(maxw, block, philox, cluster)
-                            : word_fn<FAM_LOZENGE8, 0, NL>(maxw, block, philox, cluster);
-        case FAM_QLOZENGE8: return weighted ? nullptr : word_fn<FAM_LOZENGE8, 2, NL>(maxw, block, philox, cluster);
+            return weighted ? word_fn<FAM_LOZENGE8, 1, NL>(maxw, block, philox)
+                            : word_fn<FAM_LOZENGE8, 0, NL>(maxw, block, philox);
+        case FAM_QLOZENGE8: return weighted ? nullptr : word_fn<FAM_LOZENGE8, 2, NL>(maxw, block, philox);
         default: return nullptr;
     }
 }
 
 bool word_family(int family) { return family == FAM_DOMINO || family == FAM_DOMINO_HB || family == FAM_LOZENGE8; }
 
-constexpr int kClusterMax = 16;  // CTAs of the largest thread-block cluster (non-portable size)
-
-// Plans the walk on (at most) `ctas` CTAs: one cluster, or any number of
-// co-resident CTAs.
+// Plans the walk on (at most) `ctas` co-resident CTAs.
 static rt_status plan_word_grid(int family, int device, int nlat, int rows, int width, bool philox, int ctas,
-                                bool cluster, bool weighted, WalkPlan* plan, std::string* err) {
+                                bool weighted, WalkPlan* plan, std::string* err) {
     int sms = 0, smem_optin = 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
         cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) != cudaSuccess) {
@@ -413,7 +395,6 @@ static rt_status plan_word_grid(int family, int device, int nlat, int rows, int 
     const int gw = wpad / 4;
     const int rpc = (rows + ctas - 1) / ctas;
     ctas = (rows + rpc - 1) / rpc;
-    cluster = cluster && ctas > 1 && ctas <= kClusterMax;
     const int words = rpc * gw;
     // One word per thread up to 1024 threads; bit-exact mode then keeps 2
     // or 4 words' generator states per thread in registers (512 threads).
@@ -434,10 +415,9 @@ static rt_status plan_word_grid(int family, int device, int nlat, int rows, int 
         }
         block = ((words + maxw - 1) / maxw + 31) / 32 * 32;
     }
-    const size_t smem =
-        32 + (size_t)nlat * nc * (rpc + 2) * wpad + (cluster ? (size_t)4 * nlat * gw * 8 : (size_t)0);
-    KernelFn fn = nlat == 1 ? word_kernel_for<1>(family, maxw, block, philox, weighted, cluster)
-                            : word_kernel_for<2>(family, maxw, block, philox, weighted, cluster);
+    const size_t smem = 32 + (size_t)nlat * nc * (rpc + 2) * wpad;
+    KernelFn fn = nlat == 1 ? word_kernel_for<1>(family, maxw, block, philox, weighted)
+                            : word_kernel_for<2>(family, maxw, block, philox, weighted);
     if (!fn) {
         *err = "no word kernel for this configuration";
         return RT_E_INVAL;
@@ -451,10 +431,7 @@ static rt_status plan_word_grid(int family, int device, int nlat, int rows, int 
         *err = "band does not fit in shared memory";
         return RT_E_INVAL;
     }
-    if (cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-            cudaSuccess ||
-        (cluster && cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
-                        cudaSuccess)) {
+    if (cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
         *err = "cudaFuncSetAttribute failed";
         return RT_E_CUDA;
     }
@@ -466,21 +443,8 @@ static rt_status plan_word_grid(int family, int device, int nlat, int rows, int 
     plan->wpad = wpad;
     plan->xwords = gw;
     plan->xslots = 1;
-    plan->cluster = cluster;
     plan->merge_runs = true;
     plan->fn = (const void*)fn;
-    if (cluster) {
-        int active = 0;
-        cudaLaunchConfig_t cfg = {};
-        cudaLaunchAttribute attr[1];
-        walk_launch_config(*plan, &cfg, attr);
-        if (cudaOccupancyMaxActiveClusters(&active, (const void*)fn, &cfg) != cudaSuccess || active < 1) {
-            cudaGetLastError();
-            *err = "word-kernel cluster cannot be resident";
-            return RT_E_INVAL;
-        }
-        return RT_OK;
-    }
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)fn, block, smem) != cudaSuccess) {
         *err = "cudaOccupancyMaxActiveBlocksPerMultiprocessor failed";
@@ -508,31 +472,21 @@ rt_status plan_word_walk(int family, int device, int nlat, int rows, int width, 
         *err = "cudaDeviceGetAttribute failed";
         return RT_E_CUDA;
     }
-    // Microseconds per step (Aztec diamonds TinyMT / hexagons TinyMT / hexagons
-    // Philox; words = 32-bit words of one colour array):
+    // What gets here is larger than the bands' words, or (the walk of a program
+    // that owns the memory) has no scratch left for their slots.  Microseconds per
+    // step (Aztec diamonds TinyMT / hexagons TinyMT / hexagons Philox; words =
+    // 32-bit words of one colour array):
     //   CTAs     378-432 words     945-1326          9,156            13,366-13,872
     //   1        0.34 0.58 0.75    1.09 1.07 1.40    -                -
-    //   16       0.47 0.76 1.02    0.35 0.53 0.72    -    0.82 1.14   0.79 1.08 1.62
     //   74       0.63 1.12 1.63    0.75 1.33 1.96    -    0.89 1.37   0.55 0.90 1.34
     //   148      0.63 1.12 1.62    0.67 1.17 1.75    -    0.88 1.32   0.51 0.86 1.26
     // So: one CTA (no exchange) while three warps a scheduler hold the lattice;
-    // one cluster of 16 (rows exchanged through distributed shared memory)
-    // while that leaves each CTA about 600 words; else the whole GPU, with
-    // bands of three rows or more, whose first and last rows are different
-    // warps' (258 rows: 0.71 at two rows a band, 0.54 at four).
-    const int64_t words = (int64_t)rows * ((width + 3) / 4);
+    // else the whole GPU, with bands of three rows or more, whose first and last
+    // rows are different warps' (258 rows: 0.71 at two rows a band, 0.54 at four).
     int ctas = ctas_hint;
-    bool cluster = ctas_hint > 0 && ctas_hint <= kClusterMax;
-    if (ctas_hint <= 0) {
-        cluster = words <= (int64_t)kClusterMax * 600;
-        ctas = words <= 384 ? 1 : cluster ? kClusterMax : std::min(sms, rows / 3);
-    }
+    if (ctas_hint <= 0) ctas = (int64_t)rows * ((width + 3) / 4) <= 384 ? 1 : std::min(sms, rows / 3);
     ctas = std::max(1, std::min(ctas, rows));
-    if (cluster &&
-        plan_word_grid(family, device, nlat, rows, width, philox, ctas, true, weighted, plan, err) == RT_OK)
-        return RT_OK;
-    if (ctas_hint <= 0) ctas = std::max(1, std::min(sms, rows / 3));
-    return plan_word_grid(family, device, nlat, rows, width, philox, ctas, false, weighted, plan, err);
+    return plan_word_grid(family, device, nlat, rows, width, philox, ctas, weighted, plan, err);
 }
 
 }  // namespace rtb
