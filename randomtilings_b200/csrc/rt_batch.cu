@@ -574,8 +574,8 @@ bool fill_plan(rt_batch* b, int f, int cl, int block, Plan* p) {
     // The table of moves goes in front of the lattice where there is room left.
     p->table = f == FAM_RECTTRI && smem + sizeof(RectTriMoves) + fa.sharedSizeBytes <= (size_t)optin;
     if (p->table) smem += sizeof(RectTriMoves);
-    if (cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-        return false;
+    std::string err;
+    if (allow_shared((const void*)fn, b->device, smem, &err) != RT_OK) return false;
     if (cl > 8 && cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
         return false;
     cudaLaunchConfig_t cfg = {};
@@ -777,8 +777,6 @@ rt_status plan_family(rt_batch* b, int f) {
     if (s != RT_OK) return s;
     float best = 1e30f;
     for (const Plan& p : cand) {
-        // Candidates set different shared-memory limits; this one's applies now.
-        cudaFuncSetAttribute((const void*)p.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem);
         cudaMemcpyAsync(F.scratch.p, F.data.p, F.bytes, cudaMemcpyDeviceToDevice, b->stream);
         // one untimed run, then a timed one
         for (int rep = 0; rep < 2; ++rep) {
@@ -800,7 +798,6 @@ rt_status plan_family(rt_batch* b, int f) {
     // Sweeps per launch at the chosen shape: a run of 32 sweeps as one
     // launch, against four launches of 8 (each reloading the lattices from
     // global memory, with its own tail of uneven chains).
-    cudaFuncSetAttribute((const void*)F.plan.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)F.plan.smem);
     if ((s = stage_phases(b, f, 32)) != RT_OK || (s = stage_phases(b, f, 8, true)) != RT_OK) return s;
     float best_spl = 1e30f;
     for (const int64_t spl : {(int64_t)0, (int64_t)8}) {
@@ -991,10 +988,6 @@ rt_status rt_batch_run(rt_batch* b, int64_t sweeps) {
             if (s != RT_OK) return s;
         }
         if (!b->exec) {
-            for (int f = 0; f < kFamilies; ++f)
-                if (!b->fam[f].members.empty())
-                    cudaFuncSetAttribute((const void*)b->fam[f].plan.fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)b->fam[f].plan.smem);
             // One graph: fork to a stream per family, one launch each, join.  The
             // family with the most work goes first at the highest priority, so its
             // CTAs take the SMs and the smaller families fill the slots its last

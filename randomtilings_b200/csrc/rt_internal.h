@@ -49,6 +49,11 @@ struct WalkPlan {
 
 rt_status plan_walk(int family, int device, int nlat, int rows, int cols, int width, bool uniform, bool philox,
                     WalkPlan* plan, std::string* err);
+// Lets kernel `fn` use `smem` bytes of dynamic shared memory; an error if a block
+// cannot have them beside the kernel's static ones.  What is set is all there is:
+// the limit is the function's, so a plan that set its own size would take it from
+// the larger plan of another handle (or thread).
+rt_status allow_shared(const void* fn, int device, size_t smem, std::string* err);
 // Launch configuration of a one-cluster plan; `attr` outlives *cfg.
 void walk_launch_config(const WalkPlan& plan, cudaLaunchConfig_t* cfg, cudaLaunchAttribute (&attr)[1]);
 rt_status launch_walk(const WalkPlan& plan, WalkArgs& args, cudaStream_t stream, std::string* err);

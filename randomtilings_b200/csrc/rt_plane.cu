@@ -430,10 +430,7 @@ rt_status plan_plane_walk(int family, int device, int nlat, int rows, int width,
     const int items = (rpc + 2 * (depth - 1)) * ((ww + 3) / 4);
     const int block = items > 512 ? 1024 : 512;
     PlaneFn fn = plane_fn(family, block);
-    if (cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
-        *err = "cudaFuncSetAttribute failed";
-        return RT_E_CUDA;
-    }
+    if (const rt_status s = allow_shared((const void*)fn, device, smem, err); s != RT_OK) return s;
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)fn, block, smem) != cudaSuccess) {
         *err = "cudaOccupancyMaxActiveBlocksPerMultiprocessor failed";

@@ -493,10 +493,7 @@ rt_status plan_plane_band(int family, int device, int nlat, int rows, int width,
         *err = "no such bit-plane walk";
         return RT_E_INVAL;
     }
-    if (cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
-        *err = "cudaFuncSetAttribute failed";
-        return RT_E_CUDA;
-    }
+    if (const rt_status s = allow_shared((const void*)fn, device, smem, err); s != RT_OK) return s;
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)fn, block, smem) != cudaSuccess) {
         *err = "cudaOccupancyMaxActiveBlocksPerMultiprocessor failed";

@@ -218,10 +218,8 @@ static rt_status plan_recttri_grid(int device, int rows, int width, bool philox,
     else
         fn = cluster ? (philox ? recttri_kernel<true, true, 1024> : recttri_kernel<false, true, 1024>)
                      : (philox ? recttri_kernel<true, false, 1024> : recttri_kernel<false, false, 1024>);
-    if (cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-            cudaSuccess ||
-        (cluster && cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
-                        cudaSuccess)) {
+    if (const rt_status s = allow_shared((const void*)fn, device, smem, err); s != RT_OK) return s;
+    if (cluster && cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
         *err = "cudaFuncSetAttribute failed";
         return RT_E_CUDA;
     }

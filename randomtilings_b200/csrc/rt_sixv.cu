@@ -471,7 +471,7 @@ rt_status run_epoch(rt_sixv* h, int n, int nlat, int64_t sweeps, uint64_t key, u
             auto rows_max = [&]() { return (S + ctas - 1) / ctas; };
             int H = ctas == 1 ? 1 : std::min(rows_max() <= 8 ? 4 : 2, S / ctas);
             auto bytes = [&]() { return (size_t)nlat * (rows_max() + 2 * H) * 8 * a.Q * sizeof(int16_t); };
-            while (H > 1 && bytes() > (size_t)optin) --H;
+            while (H > 1 && bytes() + sizeof(uint32_t[16]) > (size_t)optin) --H;
             const size_t smem = bytes();
             const size_t xbytes = (size_t)ctas * 2 * 2 * nlat * (H * 4 * a.Q) * sizeof(unsigned long long);
             bool one = h->thr[0] > 0 && h->thr[0] < 1u << 23;
@@ -480,8 +480,9 @@ rt_status run_epoch(rt_sixv* h, int n, int nlat, int64_t sweeps, uint64_t key, u
                                             : (one ? (const void*)sixv_band_kernel<1, true> : (const void*)sixv_band_kernel<1, false>);
             const int block = std::max(1, 1024 / a.Q) * a.Q;
             bool ready = block <= 1024 && smem + sizeof(uint32_t[16]) <= (size_t)optin &&
-                         cudaFuncSetAttribute(band_fn,
-                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess;
+                         // all there is: the limit is the function's, for every handle and thread
+                         cudaFuncSetAttribute(band_fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                              optin - (int)sizeof(uint32_t[16])) == cudaSuccess;
             if (ready && xbytes > h->xcap) {
                 if (h->d_xbuf) cudaFree(h->d_xbuf);
                 h->d_xbuf = nullptr;

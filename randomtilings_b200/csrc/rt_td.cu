@@ -156,11 +156,6 @@ __global__ void __launch_bounds__(kTdBlock, 1) td_walk_kernel(const __grid_const
 
 // One cluster; ctas_hint > 0 sets its size.
 rt_status plan_td_walk(int device, int rows, int width, bool philox, int ctas_hint, WalkPlan* plan, std::string* err) {
-    int optin = 0;
-    if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) != cudaSuccess) {
-        *err = "cudaDeviceGetAttribute failed";
-        return RT_E_CUDA;
-    }
     const void* fn = philox ? (const void*)td_walk_kernel<true> : (const void*)td_walk_kernel<false>;
     // us per step on 1 / 8 / 16 CTAs (words of one plane): Philox 2.4 / 3.6 / 4.3
     // (90), 3.0 / 3.6 / 4.0 (261), 4.7 / 3.9 / 3.8 (680); TinyMT 3.1 / 4.5 / 5.1,
@@ -171,12 +166,8 @@ rt_status plan_td_walk(int device, int rows, int width, bool philox, int ctas_hi
     const int rpc = (rows + ctas - 1) / ctas;
     const size_t slots = (size_t)(rpc + 2 * td_halo(rows, ctas, td_halo_cap(philox))) * ((width + 31) / 32);
     const size_t smem = 4 * (td_band_words(rows, width, ctas, td_halo_cap(philox), tdp::kPlanes) + (philox ? 0 : (4 * 32 + 2) * slots));
-    if (smem > (size_t)optin) {
-        *err = "triangle-dimer band does not fit in shared memory";
-        return RT_E_INVAL;
-    }
-    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
-        cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+    if (const rt_status s = allow_shared(fn, device, smem, err); s != RT_OK) return s;
+    if (cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
         *err = "cudaFuncSetAttribute failed";
         return RT_E_CUDA;
     }

@@ -339,6 +339,25 @@ rt_status plan_walk(int family, int device, int nlat, int rows, int cols, int wi
     return RT_E_INVAL;
 }
 
+rt_status allow_shared(const void* fn, int device, size_t smem, std::string* err) {
+    int optin = 0;
+    cudaFuncAttributes fa;
+    if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) != cudaSuccess ||
+        cudaFuncGetAttributes(&fa, fn) != cudaSuccess) {
+        *err = "cudaFuncGetAttributes failed";
+        return RT_E_CUDA;
+    }
+    if (smem + fa.sharedSizeBytes > (size_t)optin) {
+        *err = "band does not fit in shared memory";
+        return RT_E_INVAL;
+    }
+    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)fa.sharedSizeBytes) != cudaSuccess) {
+        *err = "cudaFuncSetAttribute failed";
+        return RT_E_CUDA;
+    }
+    return RT_OK;
+}
+
 void walk_launch_config(const WalkPlan& plan, cudaLaunchConfig_t* cfg, cudaLaunchAttribute (&attr)[1]) {
     cfg->gridDim = dim3((unsigned)plan.ctas);
     cfg->blockDim = dim3((unsigned)plan.block);

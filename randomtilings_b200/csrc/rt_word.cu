@@ -384,9 +384,8 @@ bool word_family(int family) { return family == FAM_DOMINO || family == FAM_DOMI
 // Plans the walk on (at most) `ctas` co-resident CTAs.
 static rt_status plan_word_grid(int family, int device, int nlat, int rows, int width, bool philox, int ctas,
                                 bool weighted, WalkPlan* plan, std::string* err) {
-    int sms = 0, smem_optin = 0;
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
-        cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) != cudaSuccess) {
+    int sms = 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) {
         *err = "cudaDeviceGetAttribute failed";
         return RT_E_CUDA;
     }
@@ -422,19 +421,7 @@ static rt_status plan_word_grid(int family, int device, int nlat, int rows, int 
         *err = "no word kernel for this configuration";
         return RT_E_INVAL;
     }
-    cudaFuncAttributes fa;
-    if (cudaFuncGetAttributes(&fa, (const void*)fn) != cudaSuccess) {
-        *err = "cudaFuncGetAttributes failed";
-        return RT_E_CUDA;
-    }
-    if (smem + fa.sharedSizeBytes > (size_t)smem_optin) {
-        *err = "band does not fit in shared memory";
-        return RT_E_INVAL;
-    }
-    if (cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
-        *err = "cudaFuncSetAttribute failed";
-        return RT_E_CUDA;
-    }
+    if (const rt_status s = allow_shared((const void*)fn, device, smem, err); s != RT_OK) return s;
     plan->items = maxw;
     plan->block = block;
     plan->rows_per_cta = rpc;

@@ -47,3 +47,34 @@ def test_one_handle_walks_large_and_small_lattices(monkeypatch, ctas, orders):
     for order in orders:
         t = _aztec(rt, order)
         assert np.array_equal(_walk(tl, t, 60, 5), po.domino_walk(t, 60, 5))
+
+
+def _cases(rt):
+    D, L, R, T = rt.DominoTiler, rt.LozengeTiler, rt.RectTriangleTiler, rt.TriangleDimerTiler
+    philox, planes = rt.RT_RNG_PHILOX, rt.RT_RNG_PLANES
+    return {
+        "word bands": (lambda: D(rng=philox), [_aztec(rt, 200), _aztec(rt, 8)]),
+        "words": (lambda: D(rng=philox), [_aztec(rt, 900), _aztec(rt, 520)]),
+        "plane bands": (lambda: D(rng=planes), [_aztec(rt, 900), _aztec(rt, 8)]),
+        "rectangle-triangles": (lambda: R(rng=philox), [R.maxHex(60), R.maxHex(40)]),
+        "triangle dimers": (lambda: T(rng=philox), [T.BiboneHexagon(64), T.BiboneHexagon(9)]),
+        "triangle dimers, bit-exact": (lambda: T(), [T.BiboneHexagon(64), T.BiboneHexagon(9)]),
+    }
+
+
+@pytest.mark.parametrize("kind", ["word bands", "words", "plane bands", "rectangle-triangles", "triangle dimers",
+                                  "triangle dimers, bit-exact"])
+def test_handles_of_unequal_sizes_in_turn(kind):
+    """A handle's plan stays good while another handle plans a smaller lattice for
+    the same kernel."""
+    import randomtilings_b200 as rt
+
+    make, (large, small) = _cases(rt)[kind]
+    large, small = np.asarray(large, dtype=np.int32), np.asarray(small, dtype=np.int32)
+    alone = make()
+    want = _walk(alone, large, 40, 5)
+    alone.close()
+    a, b = make(), make()
+    assert np.array_equal(_walk(a, large, 40, 5), want)
+    _walk(b, small, 40, 5)
+    assert np.array_equal(_walk(a, large, 40, 5), want)
