@@ -81,28 +81,6 @@ __device__ __forceinline__ bool wait_word(const WalkArgs& a, const unsigned long
 }
 
 // ---------------------------------------------------------------------------
-// Bands with halo rows: a CTA reads its neighbours' rows of the lattice when it
-// starts and writes its own when it ends.  The rows of an exchange were sent
-// after their sender's loads, so a walk that made one may write.  A walk that
-// ends before the first exchange waits for the loads themselves: a CTA raises a
-// flag for either neighbour when its loads are done, and writes when both
-// neighbours' are up.  The flag is the first word of a slot, which such a walk
-// uses for nothing else; slots are zero at launch.
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ void raise_loaded(unsigned long long* slot) {
-    st_release(reinterpret_cast<unsigned*>(slot), 1u);
-}
-// One thread; false where wait_more is.
-template <class A>
-__device__ __forceinline__ bool wait_loaded(const A& a, const unsigned long long* slot) {
-    unsigned spins = 0;
-    uint64_t t0 = 0;
-    while (ld_acquire(reinterpret_cast<const unsigned*>(slot)) != 1u)
-        if ((++spins & 63u) == 0u && !wait_more(a, t0)) return false;
-    return true;
-}
-
-// ---------------------------------------------------------------------------
 // Exchange of the rows next to a band.  A row of the colour flipped in phase
 // p is published as tagged 64-bit words (32 bits of lattice, p + 1), double
 // buffered by the parity of p; its reader is the thread that owns the word

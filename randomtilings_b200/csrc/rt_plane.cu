@@ -44,7 +44,8 @@ namespace rtb {
 // Shared memory: planes [lattice][colour][plane][stored row][RS words];
 // stored row s is colour-array row a0 - H + s; word 0 and word WW + 1 of a
 // row are zero padding for the funnel shifts; then two masks per word.
-// A work item is the four words of a Philox call.
+// A work item is the four words of a Philox call.  Walks on several CTAs have more
+// phases than one block (launch_walk).
 template <int FAM, int LB>
 __global__ void __launch_bounds__(LB, 1) plane_kernel(const __grid_constant__ WalkArgs a) {
     using M = PlaneModel<FAM>;
@@ -106,11 +107,6 @@ __global__ void __launch_bounds__(LB, 1) plane_kernel(const __grid_constant__ Wa
     uint32_t key0 = 0, key1 = 0;
     int64_t dstep = 0;
     __syncthreads();
-    const bool no_exchange = nct > 1 && a.nphases <= H;
-    if (no_exchange && tid == 0 && !(cta == 0 && a.drop_phase == 0)) {
-        if (cta > 0) raise_loaded(slot(a, cta, 0, 0, 0, 0));
-        if (cta + 1 < nct) raise_loaded(slot(a, cta, 1, 0, 0, 0));
-    }
 
     int64_t blk = 0;
     for (int64_t b0 = 0; b0 < a.nphases; b0 += H, ++blk) {
@@ -359,12 +355,7 @@ __global__ void __launch_bounds__(LB, 1) plane_kernel(const __grid_constant__ Wa
         }
     }
 
-    bool ok = true;
-    if (no_exchange && tid == 0) {  // the neighbours may still be reading this band's rows
-        if (cta > 0) ok = wait_loaded(a, slot(a, cta - 1, 1, 0, 0, 0));
-        if (cta + 1 < nct) ok = ok && wait_loaded(a, slot(a, cta + 1, 0, 0, 0, 0));
-    }
-    if (__syncthreads_or(!ok)) return;
+    __syncthreads();
     // Store the band rows back as bytes.
     for (int l = 0; l < a.nlat; ++l)
         for (int c = 0; c < NC; ++c) {

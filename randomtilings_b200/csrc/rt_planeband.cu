@@ -7,7 +7,9 @@
 // one Philox call per step, so they make the calls of four steps at once, one
 // each, and exchange the words: a quarter of the calls.  Halo rows go from
 // the registers of their owner to the registers of the thread that keeps them
-// in the neighbouring CTA, with no index arithmetic.
+// in the neighbouring CTA, with no index arithmetic.  Every walk on several CTAs
+// makes an exchange (launch_walk): it orders a CTA's loads before its neighbours'
+// stores.
 //
 // What bounds it: the latency of a phase (barrier, neighbours, rule: 0.25 us)
 // and, on large lattices, instruction issue; the exchange every H phases adds
@@ -251,11 +253,6 @@ __global__ void __launch_bounds__(kBandBlock, 1) plane_band_kernel(const __grid_
     };
 
     __syncthreads();
-    const bool no_exchange = nct > 1 && a.nphases <= H;
-    if (no_exchange && tid == 0 && !(cta == 0 && a.drop_phase == 0)) {
-        if (has_top) raise_loaded(slot(a, cta, 0, 0, 0, 0));
-        if (has_bot) raise_loaded(slot(a, cta, 1, 0, 0, 0));
-    }
     uint32_t blk = 0;  // halo exchanges made (modulo 2^32, as the tags)
     int k = 0;         // phases since the last one
     const int s_top = has_top ? 1 : H, s_bot = H + nrows + (has_bot ? H - 1 : 0);
@@ -396,12 +393,6 @@ __global__ void __launch_bounds__(kBandBlock, 1) plane_band_kernel(const __grid_
             if (NC == 3) regular(std::integral_constant<int, 2 % NC>{});
             if (!ok) return;
         }
-    }
-    if (no_exchange) {  // the neighbours may still be reading this band's rows
-        bool ok = true;
-        if (tid == 0 && has_top) ok = wait_loaded(a, slot(a, cta - 1, 1, 0, 0, 0));
-        if (tid == 0 && has_bot) ok = ok && wait_loaded(a, slot(a, cta + 1, 0, 0, 0, 0));
-        if (__syncthreads_or(!ok)) return;
     }
 
     // Band rows back to bytes: a warp writes one word after the other.

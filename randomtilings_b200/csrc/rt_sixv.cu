@@ -85,7 +85,8 @@ __global__ void __launch_bounds__(256) sixv_step_kernel(const __grid_constant__ 
 // (32 bits of heights and the exchange's number), double-buffered by its
 // parity.  A CTA publishes exchange t + 1 only after it read exchange t, which
 // each neighbour published after reading exchange t - 1 from it, so a slot is
-// rewritten only after it was read.  Every wait is bounded: past timeout_ns the
+// rewritten only after it was read, and no CTA writes its band back before its
+// neighbours have read it.  Every wait is bounded: past timeout_ns the
 // CTA sets ERR_TIMEOUT in *err and returns, and the others see it.  The launch
 // is cooperative, so every CTA is resident.
 //
@@ -200,11 +201,6 @@ __global__ void __launch_bounds__(1024, 1) sixv_band_kernel(const __grid_constan
     using C1 = std::integral_constant<int, 1>;
 
     __syncthreads();
-    const bool no_exchange = nct > 1 && (a.steps + 1) / 2 <= H;
-    if (no_exchange && tid == 0 && !(cta == 0 && a.drop_blk == 0)) {
-        if (has_top) raise_loaded(sixv_slot(a, cta, 0, 0, 0));
-        if (has_bot) raise_loaded(sixv_slot(a, cta, 1, 0, 0));
-    }
     int k = 0;          // pairs of steps since the last exchange
     uint32_t blk = 0;   // exchanges made
     for (int64_t s = 0; s < a.steps; s += 2) {
@@ -280,12 +276,6 @@ __global__ void __launch_bounds__(1024, 1) sixv_band_kernel(const __grid_constan
         if (__syncthreads_or(!ok)) return;
         k = 0;
         ++blk;
-    }
-    if (no_exchange) {  // the neighbours may still be reading this band's rows
-        bool ok = true;
-        if (tid == 0 && has_top) ok = wait_loaded(a, sixv_slot(a, cta - 1, 1, 0, 0));
-        if (tid == 0 && has_bot) ok = ok && wait_loaded(a, sixv_slot(a, cta + 1, 0, 0, 0));
-        if (__syncthreads_or(!ok)) return;
     }
     for (int l = 0; l < NLAT; ++l)
         for (int e = tid; e < nrows * S; e += BLOCK) {
@@ -472,6 +462,9 @@ rt_status run_epoch(rt_sixv* h, int n, int nlat, int64_t sweeps, uint64_t key, u
             int H = ctas == 1 ? 1 : std::min(rows_max() <= 8 ? 4 : 2, S / ctas);
             auto bytes = [&]() { return (size_t)nlat * (rows_max() + 2 * H) * 8 * a.Q * sizeof(int16_t); };
             while (H > 1 && bytes() + sizeof(uint32_t[16]) > (size_t)optin) --H;
+            // Several CTAs make an exchange in every epoch, be it of one sweep (two
+            // pairs): it orders a CTA's loads of its halo before its neighbours' stores.
+            if (ctas > 1) H = (int)std::min<int64_t>(H, 2 * sweeps - 1);
             const size_t smem = bytes();
             const size_t xbytes = (size_t)ctas * 2 * 2 * nlat * (H * 4 * a.Q) * sizeof(unsigned long long);
             bool one = h->thr[0] > 0 && h->thr[0] < 1u << 23;

@@ -376,6 +376,11 @@ rt_status launch_walk(const WalkPlan& plan, WalkArgs& args, cudaStream_t stream,
     args.xwords = plan.xwords;
     args.xslots = plan.xslots;
     args.depth = plan.depth;
+    // A CTA of a band kernel reads its neighbours' rows when it starts and writes its
+    // own when it ends; what orders the two is an exchange, whose rows are sent after
+    // the loads.  So a walk on several CTAs makes at least one: blocks are shorter than
+    // the walk.  (Planned depths suit longer walks; a halo of fewer rows needs less.)
+    if (plan.ctas > 1 && args.nphases <= plan.depth) args.depth = (int)std::max<int64_t>(1, args.nphases - 1);
     args.pwords = plan.pwords;
     void* kargs[] = {&args};
     cudaError_t e;

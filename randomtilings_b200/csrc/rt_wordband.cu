@@ -6,7 +6,9 @@
 // with their generators, which go on in step with their owners' -- and after
 // phase k of a block of H phases the rows within H - k - 1 of the band are
 // current.  Then each CTA's first and last H rows go to its neighbours through
-// tagged words (rt_exchange.cuh), all words of a thread in one round trip.
+// tagged words (rt_exchange.cuh), all words of a thread in one round trip.  H is
+// less than the walk's phases (launch_walk), so that no CTA writes its band back
+// before its neighbours have read it.
 //
 // What bounds it: the latency of a phase -- the draws, the word's update, the
 // barrier, 0.2 us a step on one CTA -- and the exchange, 1.5 us or so every H
@@ -142,11 +144,6 @@ __global__ void __launch_bounds__(LB, 1) word_band_kernel(const __grid_constant_
         until = until_special(0);
     }
     __syncthreads();
-    const bool no_exchange = nct > 1 && a.nphases <= H;
-    if (no_exchange && tid == 0 && !(cta == 0 && drop_blk == 0)) {
-        if (has_top) raise_loaded(slot(a, cta, 0, 0, 0, 0));
-        if (has_bot) raise_loaded(slot(a, cta, 1, 0, 0, 0));
-    }
     WordPhase P = s_phase[word_phase_index(d)];
     while (more) {
         uint32_t d_next = 0u;
@@ -234,12 +231,6 @@ __global__ void __launch_bounds__(LB, 1) word_band_kernel(const __grid_constant_
         if (__syncthreads_or(!ok)) return;
         k = 0;
         ++blk;
-    }
-    if (no_exchange) {  // the neighbours may still be reading this band's rows
-        bool ok = true;
-        if (tid == 0 && has_top) ok = wait_loaded(a, slot(a, cta - 1, 1, 0, 0, 0));
-        if (tid == 0 && has_bot) ok = ok && wait_loaded(a, slot(a, cta + 1, 0, 0, 0, 0));
-        if (__syncthreads_or(!ok)) return;
     }
     for (int l = 0; l < NL; ++l)
         for (int c = 0; c < NC; ++c) {

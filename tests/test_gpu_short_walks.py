@@ -1,7 +1,7 @@
-"""Walks that end before the first halo exchange: a band's rows are written only
-after the neighbours have read them.  A withheld flag ends the walk with a timeout;
-walks of one step to just beyond a block of phases, on many CTAs and again and
-again, equal the oracle."""
+"""Walks of fewer phases than the planned halo has rows: a band's rows are written
+only after the neighbours have read them, so every walk on several CTAs makes an
+exchange.  A withheld one ends the walk with a timeout; walks of one step to just
+beyond a block of phases, on many CTAs and again and again, equal the oracle."""
 from __future__ import annotations
 
 import numpy as np
@@ -29,7 +29,7 @@ def _check(tiler, t, want, steps, seed):
 
 
 def _withheld(monkeypatch, make, t):
-    """The first CTA withholds its flag: its neighbour may not write."""
+    """The first CTA withholds its rows: its neighbour may not write."""
     import randomtilings_b200 as rt
 
     monkeypatch.setenv("RT_TEST_DROP_PUBLISH", "0")
@@ -122,8 +122,7 @@ def test_short_large_plane_band_walks(monkeypatch, model, steps):
 
 
 # Bands of four rows with halos of four, and of 7 to 11 rows with halos of four
-# and two: one sweep is two pairs of steps, and no exchange comes before the
-# third pair or the fifth.
+# and two; one sweep is two pairs of steps.
 @pytest.mark.parametrize("n", [90, 333, 1000, 1601])
 @pytest.mark.parametrize("sweeps", [1, 2, 3])
 def test_short_six_vertex_walks(n, sweeps):
@@ -137,7 +136,7 @@ def test_short_six_vertex_walks(n, sweeps):
 @pytest.mark.parametrize("n", [90, 1601])
 @pytest.mark.parametrize("sweeps", [1, 40])
 def test_six_vertex_bands_wait_for_their_neighbours(monkeypatch, n, sweeps):
-    """The first CTA withholds its flag, or its rows of the first exchange."""
+    """The first CTA withholds its rows of the first exchange."""
     import randomtilings_b200 as rt
 
     h = np.array(rt.SixVertexTiler.MaxHeights(n), dtype=np.int32)
