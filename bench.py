@@ -419,6 +419,8 @@ def run_b200(args) -> None:
             "warm_vs_cold": warm,
             "gpu_launches": int(launches) * args.steps,
             "phases_per_launch": int(phases),
+            "phases_note": "of the schedule: one per colour step and the final Update; the kernel takes a run of "
+                           "same-colour steps as one",
             "clocks": clocks,
             "wall_s_timed_region": wall,
         }
@@ -880,7 +882,7 @@ def main() -> None:
     # --set full of a 600-colour-step launch of this build: 1,160,960 B read, 0 written).  The
     # lattice stays on chip, so a launch of any number of colour steps moves the same bytes; a
     # timed run cannot read DRAM counters, so the figure comes from that capture.
-    ap.add_argument("--traffic", type=float, default=1160960.0,
+    ap.add_argument("--traffic", type=float, default=1074176.0,
                     help="dram bytes per walk launch from an ncu capture (reported in roofline.traffic)")
     ap.add_argument("--batch-chains", type=int, default=4096)
     ap.add_argument("--batch-sweeps", type=int, default=5000)

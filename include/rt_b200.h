@@ -179,7 +179,10 @@ void* rt_stream(rt_tiler* h);
  * address in *d_tiling; it stays valid until the next rt_upload / rt_walk
  * or rt_destroy, and is overwritten by the next rt_download / rt_device_tiling. */
 rt_status rt_device_tiling(rt_tiler* h, int32_t** d_tiling);
-/* Counters of the last run: phases executed and kernel launches issued. */
+/* Counters of the last run: the phases of its schedule (colour models: one per
+ * colour step and the final Update, although a kernel may take a run of steps of
+ * one colour as one; triangle dimers: the array updates of the launch) and the
+ * kernel launches issued. */
 rt_status rt_last_run_info(rt_tiler* h, int64_t* phases, int64_t* launches);
 
 /* No counterpart in the reference.  For callers that may not allocate GPU

@@ -216,8 +216,8 @@ struct rt_tiler {
     bool plan_td_fits = false;
     bool td_fits = false;   // triangle dimers: the uploaded arrays' values fit the bit planes
     int kernel_choice = 0;  // 0 auto, 1 generic walk kernel only, 2 word kernel only (RT_WALK_KERNEL)
-    int ctas_hint = 0;      // word kernel grid (RT_WALK_CTAS; 0 = one CTA per SM)
-    int depth_hint = 0;     // bit-plane kernel: phases per halo exchange (RT_PLANE_DEPTH; 0 = up to 8)
+    int ctas_hint = 0;      // CTAs of the walk (RT_WALK_CTAS; 0 = by size)
+    int depth_hint = 0;     // bit-plane kernels: phases per halo exchange (RT_PLANE_DEPTH; 0 = by size)
     int64_t drop_phase = -1;  // RT_TEST_DROP_PUBLISH: a phase whose rows CTA 0 withholds (bounded-wait tests)
     int64_t last_phases = 0, last_launches = 0;
     uint64_t timeout_ns = 5000000000ull;

@@ -979,12 +979,7 @@ extern "C" rt_status rt_mixed_chain_spec(int64_t seed, int32_t* model, int32_t* 
 
 namespace rtb {
 
-// The graph the height-function projection relaxes over (rt_project.cu):
-// vertex side *n, per vertex its kind (0 outside the domain, 1 interior,
-// 2 boundary -- as DomainToVertices marks them) and a bit per neighbour
-// direction whose edge touches the domain with both ends inside it.
-// Directions: dominoes (i+1, j), (i-1, j), (i, j+1), (i, j-1); lozenges
-// (i, j+1), (i-1, j+1), (i-1, j), (i, j-1), (i+1, j-1), (i+1, j).
+// Dominoes have M x M faces, lozenges M x 2M.
 int domain_side(int model, int64_t dlen) {
     if (model == RT_DOMINO) {
         const int m = isqrt_exact(dlen);
@@ -994,6 +989,12 @@ int domain_side(int model, int64_t dlen) {
     return m < 2 || (int64_t)2 * m * m != dlen ? -1 : m;
 }
 
+// The graph of the height plans (rt_height.cu): vertex side *n, per vertex its kind
+// (0 outside the domain, 1 interior, 2 boundary -- as DomainToVertices marks them)
+// and a bit per neighbour direction whose edge touches the domain with both ends
+// inside it.  Directions: dominoes (i+1, j), (i-1, j), (i, j+1), (i, j-1); lozenges
+// (i, j+1), (i-1, j+1), (i-1, j), (i, j-1), (i+1, j-1), (i+1, j).  The projection
+// finds the same on the device (rt_domain.cuh).
 bool lipschitz_graph(int model, const int32_t* d, int64_t dlen, int* n_out, std::vector<uint8_t>* kind,
                      std::vector<uint8_t>* edges) {
     if (!d) return false;

@@ -40,7 +40,7 @@ struct WalkPlan {
     int wpad = 0;    // shared-memory row stride (elements)
     int xwords = 0;  // exchange words per halo row
     int xslots = 1;  // arrays exchanged per phase
-    int depth = 1;   // bit-plane kernel: phases per halo exchange
+    int depth = 1;   // band kernels: phases per halo exchange
     int pwords = 0;  // bit-plane kernel: words per row
     bool cluster = false;     // the CTAs are one thread-block cluster (else a cooperative launch)
     bool merge_runs = false;  // the kernel takes a run of same-colour steps as one phase
@@ -57,14 +57,15 @@ rt_status allow_shared(const void* fn, int device, size_t smem, std::string* err
 // Launch configuration of a one-cluster plan; `attr` outlives *cfg.
 void walk_launch_config(const WalkPlan& plan, cudaLaunchConfig_t* cfg, cudaLaunchAttribute (&attr)[1]);
 rt_status launch_walk(const WalkPlan& plan, WalkArgs& args, cudaStream_t stream, std::string* err);
-// Word-parallel kernel of the int8 models (rt_word.cu): uniform TinyMT32J
-// parameters or fast mode.  ctas_hint <= 0: one CTA per SM.
+// Word-parallel kernels of the int8 models: uniform TinyMT32J parameters or fast
+// mode.  On bands with halo rows (plan_word_band) where they fit, else rt_word.cu.
+// ctas_hint 0: a grid by size; < 0: so too, and rt_word.cu only.
 bool word_family(int family);
 // weighted: the instantiation that reads per-site thresholds (WalkArgs::wper > 0).
 rt_status plan_word_walk(int family, int device, int nlat, int rows, int width, bool philox, int ctas_hint,
                          WalkPlan* plan, std::string* err, bool weighted = false);
-// The same, one word per thread, on bands with halo rows (rt_wordband.cu); an
-// error if the bands do not fit it.
+// One word per thread, on bands with halo rows (rt_wordband.cu); an error if the
+// bands do not fit it.
 rt_status plan_word_band(int family, int device, int nlat, int rows, int width, bool philox, int ctas_hint, bool weighted,
                          WalkPlan* plan, std::string* err);
 // Bit-plane kernel of a single triangle-dimer walk (rt_td.cu), for arrays whose
@@ -74,17 +75,18 @@ rt_status plan_td_walk(int device, int rows, int width, bool philox, int ctas_hi
 // 1,024 sites.  ctas_hint <= 0: by size.
 rt_status plan_recttri_walk(int device, int rows, int width, bool philox, int ctas_hint, WalkPlan* plan,
                             std::string* err);
-// Bit-plane kernel of the int8 models (rt_plane.cu, RT_RNG_PLANES).
-// ctas_hint / depth_hint <= 0: one CTA per SM / the largest depth up to 8.
+// Bit-plane kernels of the int8 models (RT_RNG_PLANES): rt_planeband.cu up to 2,048
+// words a CTA, else rt_plane.cu.  ctas_hint / depth_hint <= 0: by size, a depth of up
+// to 32 / one CTA per SM, up to 8.
 rt_status plan_plane_walk(int family, int device, int nlat, int rows, int width, int ctas_hint, int depth_hint,
                           WalkPlan* plan, std::string* err);
 // The kernel a walk runs on, as every walk entry point chooses it: the
-// bit-plane kernel in RT_RNG_PLANES mode; otherwise the word kernel for the
+// bit-plane kernels in RT_RNG_PLANES mode; otherwise the word kernels for the
 // int8 models with uniform generator parameters (unless kernel_choice = 1),
 // the triangle dimers' bit-plane kernel for arrays whose values fit it
-// (td_fits), and the rectangle-triangle kernel; falling back to the generic walk kernel for every other case and
-// for any band those kernels cannot hold (kernel_choice = 2 forbids the
-// fallback).
+// (td_fits), and the rectangle-triangle kernel; falling back to the generic walk
+// kernel for every other case and for any band those kernels cannot hold
+// (kernel_choice = 2 forbids the fallback).
 rt_status choose_plan(int family, int device, int nlat, int rows, int cols, int width, bool uniform, bool fast,
                       bool planes, bool weighted, bool td_fits, int kernel_choice, int ctas_hint, int depth_hint,
                       WalkPlan* plan, std::string* err);

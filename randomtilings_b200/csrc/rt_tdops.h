@@ -30,7 +30,7 @@ enum : uint32_t {
     TD_BFLY_SAME = 26,      // a = t, b = p1 | p2 << 2                  (UpdateButterflysFlipped?1)
     TD_BFLY_21 = 27,        // a = t, b = p1
     TD_BFLY_22 = 28,        // a = t, b = p1
-    TD_BFLY_23_LOZ = 29,    // a = t, b = p1: pass 23, then the lozenges from that butterfly array
+    TD_BFLY_23_LOZ = 29,    // a = t, b = p1: passes 30 and 31 at once (the full program the schedule is checked against)
     TD_BFLY_23 = 30,        // a = t, b = p1: pass 23 alone
     TD_LOZ_FROM_BFLY = 31   // a = t                                    (UpdateLozengeFromButterflys{H,L,R})
 };

@@ -7,10 +7,10 @@
 // these only on states that are no dimer covers, by at most one bit, which the
 // planes keep too: any start whose values fit the planes gives the integer
 // rule's values.  Every bit of every array is a plane of its own, 32 sites of
-// a row per 32-bit word, 56 planes in all, and each phase op is written as
-// boolean algebra on the words: one work item updates 32 sites of a row at
-// once.  A neighbour at column j +- 1 is a
-// funnel shift of two adjacent words.  Sums of weighted conditions (the
+// a row per 32-bit word, 56 planes in all (51 without the carries, for the
+// largest batched chains), and each phase op is written as boolean algebra on
+// the words: one work item updates 32 sites of a row at once.  A neighbour at
+// column j +- 1 is a funnel shift of two adjacent words.  Sums of weighted conditions (the
 // digits a + 2 b + 3 c of the reference's rules) use a bit-sliced ripple
 // adder, so every value is the one the integer rule computes.
 //

@@ -110,10 +110,10 @@ struct WordNbr {
 
 // One phase on one word of one lattice (planes at `lat`, a pending Update or
 // none), in two parts: `begin` reads the word and its own row (sel_tab: the
-// column shifts, null where no table is at hand), `finish` takes
-// the rows next to it.  m0 / m1: byte masks (0xff) of the phase's draws --
-// dominoes: m0 where the site toggles (heat bath: becomes 12, else 3);
-// lozenges: m0 where a cube is added, m1 where one is removed.
+// column shifts, null where no table is at hand), `finish` takes the rows next to
+// it.  m0 / m1: byte masks (0xff) of the phase's draws -- dominoes: m0 where the
+// site toggles (heat bath: becomes 12, else 3); lozenges: m0 where a cube is added,
+// m1 where one is removed.
 template <int FAM>
 struct WordOp {
     static constexpr bool DOM = FAM != FAM_LOZENGE8;
